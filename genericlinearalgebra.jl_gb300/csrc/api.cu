@@ -1674,7 +1674,8 @@ int gla_plan_bucket_config(gla_plan_t p, int b, int* nmax, int* matrices, int* n
   *nmax = bk.nmax;
   *matrices = bk.count;
   *nt_tri = bk.nt_tri;
-  *lanes_per_warp = bk.lpw > 0 ? bk.lpw : (p->prec == GLA_PREC_F64 ? 16 : 8);
+  const bool grp = p->prec == GLA_PREC_F64 && p->jobz == 'V';  // four lanes per matrix: at most 8
+  *lanes_per_warp = bk.lpw > 0 ? (grp ? std::min(bk.lpw, 8) : bk.lpw) : (grp ? 2 : p->prec == GLA_PREC_F64 ? 16 : 8);
   return 0;
 }
 
