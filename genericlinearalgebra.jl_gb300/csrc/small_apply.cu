@@ -10,19 +10,45 @@
 //
 // A sweep touches columns (i, i+1) for consecutive i, so each row keeps the
 // column shared by two neighbouring rotations in a register ("carry"): one
-// shared-memory load, one store and four FP arithmetic instructions per row
-// per rotation. Rotations are staged through shared memory in chunks.
+// shared-memory load, one store and four (FP64: three) FP arithmetic
+// instructions per row per rotation. Rotations are staged through shared
+// memory in chunks.
+//
+// FP64 is bound by its pipe (64 cycles a warp instruction), so there a
+// rotation is three shears instead of four products: for c >= 0 and
+// t = s / (1 + c), |t| <= 1, x += t y; y -= s x; x += t y gives c x + s y
+// and c y - s x with the rounding of a rotation of that angle; for c < 0 the
+// opposite rotation is applied and both results change sign (on the integer
+// pipe). t is formed once per rotation while a chunk is staged. Replay of
+// 512 matrices of order 128: 12.5 ms with four products, 10.9 with shears; of
+// order 112: 8.3 and 5.9 ms.
 #include "gla_launch.h"
 #include "gla_small.cuh"
 
 namespace gla {
 
-constexpr int kRotChunk = 512;
+template <class T>
+constexpr int kRotChunk = sizeof(T) == 8 ? 256 : 512;  // at least one sweep (< kSmallMaxN rotations)
 
 size_t apply_smem_bytes(int n, int elem) {
-  // S[n*(n+1)] | rotation chunk (2*kRotChunk) | keys (u64, n) | rank (int, n) | headers (3n+4)
-  return (size_t)elem * ((size_t)n * (n + 1) + 2 * kRotChunk) + 8 * (size_t)n + 4 * (size_t)n +
-         4 * (3 * (size_t)n + 4) + 16;
+  // S[n*(n+1)] | rotation chunk (2 per rotation) | keys (u64, n) | rank (int, n) | headers (3n+4)
+  // | FP64: sign masks of the chunk's rotations
+  const int chunk = elem == 8 ? kRotChunk<double> : kRotChunk<float>;
+  return (size_t)elem * ((size_t)n * (n + 1) + 2 * chunk) + 8 * (size_t)n + 4 * (size_t)n +
+         4 * (3 * (size_t)n + 4) + 16 + (elem == 8 ? 4 * (size_t)chunk : 0);
+}
+
+// t = s / (1 + c), 1 <= 1 + c <= 2: the reciprocal's seed and one cubic step.
+GLA_DEV double shear(double c, double s) {
+  const double q = 1.0 + c;
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(q));
+  const double e = fma(-q, x, 1.0);
+  x = fma(x, fma(e, e, e), x);
+  return s * x;
+}
+GLA_DEV double flip_sign(double x, unsigned m) {
+  return __hiloint2double((int)((unsigned)__double2hiint(x) ^ m), __double2loint(x));
 }
 
 // V: Q in (from k_tridiag or a previous pass) and the rotated, sorted
@@ -52,7 +78,7 @@ __global__ void __launch_bounds__(128) k_apply(const SmallDesc* __restrict__ des
   const int tid = threadIdx.x, NT = blockDim.x;
   T* S = reinterpret_cast<T*>(smem_raw);
   T* buf = S + (size_t)n * ld;
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(buf + 2 * kRotChunk);
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(buf + 2 * kRotChunk<T>);
   int* rank = reinterpret_cast<int*>(keys + n);
   T* Vg = V + (ROWS2 ? 2 * dsc.w_off : dsc.a_off);  // column-major, leading dimension nr
 
@@ -71,6 +97,7 @@ __global__ void __launch_bounds__(128) k_apply(const SmallDesc* __restrict__ des
   // ---- replay this pass's rotations: whole sweeps per staged chunk
   const T* myrot = rot + 2 * dsc.rot_off;
   unsigned* hs = reinterpret_cast<unsigned*>(rank + n);
+  unsigned* sgn = hs + 3 * n + 4;  // FP64 only
   const int nhdr = st.nhdr;
   for (int h = tid; h < nhdr; h += NT) hs[h] = hdr[dsc.hdr_off + h];
   const int r = tid;
@@ -81,10 +108,48 @@ __global__ void __launch_bounds__(128) k_apply(const SmallDesc* __restrict__ des
     // sweeps [h, h2) whose rotations fit in the chunk (a sweep has < n <= kRotChunk)
     __syncthreads();
     int h2 = h, tot = 0;
-    while (h2 < nhdr && tot + hdr_count(hs[h2]) <= kRotChunk) tot += hdr_count(hs[h2++]);
-    for (int q = tid; q < 2 * tot; q += NT) buf[q] = myrot[2 * q0 + q];
+    while (h2 < nhdr && tot + hdr_count(hs[h2]) <= kRotChunk<T>) tot += hdr_count(hs[h2++]);
+    if constexpr (sizeof(T) == 8) {
+      for (int q = tid; q < tot; q += NT) {
+        const double2 cs = reinterpret_cast<const double2*>(myrot)[q0 + q];
+        const unsigned m = (unsigned)__double2hiint(cs.x) & 0x80000000u;
+        const double s = flip_sign(cs.y, m);
+        buf[2 * q] = shear(flip_sign(cs.x, m), s);
+        buf[2 * q + 1] = s;
+        sgn[q] = m;
+      }
+    } else {
+      for (int q = tid; q < 2 * tot; q += NT) buf[q] = myrot[2 * q0 + q];
+    }
     __syncthreads();
-    if (row) {
+    if constexpr (sizeof(T) == 8) {
+      if (row) {
+        const double2* ts = reinterpret_cast<const double2*>(buf);
+        const unsigned* sg = sgn;
+        for (int hh = h; hh < h2; hh++) {
+          const unsigned hw = hs[hh];
+          const int start = hdr_start(hw), cnt = hdr_count(hw);
+          const int step = hdr_up(hw) ? ld : -ld;  // to the next column
+          T* col = Sr + (size_t)start * ld;
+          T carry = col[-step], v = col[0];
+          for (int k = 0; k < cnt; k++) {
+            const double2 r2 = ts[k];
+            const unsigned m = sg[k];
+            const T vnext = (k + 1 < cnt) ? col[step] : T(0);
+            T x = fma(r2.x, v, carry);
+            const T y = fma(-r2.y, x, v);
+            x = fma(r2.x, y, x);
+            col[-step] = flip_sign(x, m);
+            carry = flip_sign(y, m);
+            v = vnext;
+            col += step;
+          }
+          col[-step] = carry;
+          ts += cnt;
+          sg += cnt;
+        }
+      }
+    } else if (row) {
       const T* cs = buf;
       for (int hh = h; hh < h2; hh++) {
         const unsigned hw = hs[hh];
