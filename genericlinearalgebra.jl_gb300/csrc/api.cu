@@ -301,10 +301,10 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
       }
     }
     bk.nt = std::max(32, (bk.nmax + 31) / 32 * 32);
-    // FP32 reductions are latency bound: two threads per row halve the
-    // per-thread loops of the tridiagonalisation (FP64 keeps one: its cost
-    // is the FP64 pipe, not latency)
-    bk.nt_tri = precision == GLA_PREC_F64 ? bk.nt : std::min(256, 2 * bk.nt);
+    // two threads per row: FP32 reductions are latency bound, and an FP64 CTA
+    // of one warp per 32 rows leaves its sub-partitions' FP64 units idle at
+    // every reduction and barrier
+    bk.nt_tri = std::min(256, 2 * bk.nt);
     if (bk.count) p->buckets.push_back(bk);
   }
 
@@ -415,9 +415,17 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
   if (err == cudaSuccess) err = cudaMemset(p->d_scale, 0, sizeof(int) * std::max<int64_t>(batch, 1));
   if (err == cudaSuccess) err = cudaMallocHost((void**)&p->pin_pending, sizeof(int) * kMaxBuckets);
   if (err == cudaSuccess) err = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming);
+  // The largest orders have the longest pipeline, so their CTAs go first:
+  // falling stream priorities from the first bucket on (as many levels as the
+  // device has). Without them every bucket's reduction shares the SMs and
+  // the largest bucket's chase starts late.
+  int prio_low = 0, prio_high = 0;
+  if (err == cudaSuccess) err = cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
+  int prio = prio_high;
   for (Bucket& bk : p->buckets) {
-    if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&bk.stream, cudaStreamNonBlocking);
+    if (err == cudaSuccess) err = cudaStreamCreateWithPriority(&bk.stream, cudaStreamNonBlocking, prio);
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&bk.join, cudaEventDisableTiming);
+    prio = std::min(prio + 1, prio_low);
   }
   if (p->nchunks) {
     if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&p->s_in, cudaStreamNonBlocking);

@@ -26,10 +26,10 @@
 namespace gla {
 
 size_t tridiag_smem_bytes(int n, int nt, int elem, bool) {
-  // redm[32] u64 | red[32] (8-byte slots) | S[n*ld] | vv,uu,ww,taus [n] | part[8*nt]
+  // redm[32] u64 | red[32] (8-byte slots) | S[n*ld] | vv,uu,ww,taus [n] | part[8*nt], FP64 part[nt]
   // (the FP32 tridiagonal solver reuses S and part once Q is in global memory)
   const size_t ld = (size_t)((n + 1) | 1);
-  return 512 + (size_t)elem * ((size_t)n * ld + 4 * (size_t)n + 8 * (size_t)nt);
+  return 512 + (size_t)elem * ((size_t)n * ld + 4 * (size_t)n + (elem == 8 ? 1 : 8) * (size_t)nt);
 }
 
 template <class T, class Tin, bool WANTQ, bool STEIN>

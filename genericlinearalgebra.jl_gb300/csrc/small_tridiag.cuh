@@ -33,6 +33,21 @@ GLA_DEV void block_sum_max(T v, unsigned long long m, T* red, unsigned long long
     redm[wid] = m;
   }
   __syncthreads();
+  if constexpr (sizeof(T) == 8) {
+    // the warps' sums by three shuffles (nw <= 8): every warp would queue
+    // nw - 1 additions on the FP64 pipe
+    T s = (lane & 7) < nw ? red[lane & 7] : T(0);
+    unsigned long long x = (lane & 7) < nw ? redm[lane & 7] : 0ull;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+      unsigned long long w = __shfl_xor_sync(0xffffffffu, x, o);
+      x = w > x ? w : x;
+    }
+    sum = s;
+    mx = x;
+    return;
+  }
   T s = red[0];
   unsigned long long x = redm[0];
   for (int i = 1; i < nw; i++) {
@@ -42,6 +57,43 @@ GLA_DEV void block_sum_max(T v, unsigned long long m, T* red, unsigned long long
   sum = s;
   mx = x;
 }
+
+// The same for a sum alone.
+GLA_DEV double block_sum8(double v, double* red) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  v = warp_sum(v);
+  __syncthreads();
+  if (lane == 0) red[wid] = v;
+  __syncthreads();
+  double s = (lane & 7) < nw ? red[lane & 7] : 0.0;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+GLA_DEV float block_sum8(float v, float* red) { return block_sum(v, red); }
+
+// The reflector's scalars from x1 and the column's squared norm (FP64, both
+// well inside the normal range): nu = copysign(norm, x1), tau = (x1 + nu)/nu
+// and 1/(x1 + nu), each from one hardware seed and a cubic correction (12
+// FP64 instructions where the IEEE square root and divisions take about 45;
+// with block_sum8 and two threads per row, the reduction and Q of one matrix
+// of order 64 went from 0.62 to 0.42 ms, of 512 of order 128 from 7.7 to 5.8).
+GLA_DEV void reflector_scalars(double x0, double sumsq, double& nu, double& tau, double& scl) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(sumsq));
+  const double h = sumsq * y;
+  const double e = fma(-h, y, 1.0);
+  const double q = e * fma(e, 0.375, 0.5);
+  const double norm = fma(h, q, h), rnorm = fma(y, q, y);
+  nu = copysign(norm, x0);
+  const double xi1 = x0 + nu;
+  tau = fma(fabs(x0), rnorm, 1.0);
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(xi1));
+  const double d = fma(-xi1, x, 1.0);
+  scl = fma(x, fma(d, d, d), x);
+}
+GLA_DEV void reflector_scalars(float, float, float&, float&, float&) {}
 
 // Leading dimension of the staged matrix: odd, so that transposed accesses
 // (stride ld across the lanes of a warp) spread over all shared-memory banks.
@@ -192,22 +244,28 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
       // LinearAlgebra.reflector!: norm (scaled only when maxabs^2 would
       // overflow or underflow), nu = copysign(norm, x1), x1 += nu,
       // x[2:] /= x1, tau = x1/nu, x[1] = -nu.
-      const T maxabs = AbsBits<T>::from(mb);
-      const T mm = maxabs * maxabs;
-      T normu;
-      if (isfinite((T)m * mm) && mm != 0) {
-        normu = prec<T>::sqrt_ieee(sumsq);
+      T nu, scl;
+      const int mbe = (int)(mb >> 52);  // (FP64) biased exponent of the largest entry
+      if (sizeof(T) == 8 && mbe > 1023 - 400 && mbe < 1023 + 400) {
+        reflector_scalars(x0, sumsq, nu, tau, scl);
       } else {
-        const T r = (tid < m) ? xi / maxabs : T(0);
-        T s2;
-        unsigned long long dummy;
-        block_sum_max<T>(r * r, 0ull, red, redm, s2, dummy);
-        normu = maxabs * prec<T>::sqrt_ieee(s2);
+        const T maxabs = AbsBits<T>::from(mb);
+        const T mm = maxabs * maxabs;
+        T normu;
+        if (isfinite((T)m * mm) && mm != 0) {
+          normu = prec<T>::sqrt_ieee(sumsq);
+        } else {
+          const T r = (tid < m) ? xi / maxabs : T(0);
+          T s2;
+          unsigned long long dummy;
+          block_sum_max<T>(r * r, 0ull, red, redm, s2, dummy);
+          normu = maxabs * prec<T>::sqrt_ieee(s2);
+        }
+        nu = tcopysign(normu, x0);
+        const T xi1 = x0 + nu;
+        tau = prec<T>::div_ieee(xi1, nu);
+        scl = prec<T>::tame(xi1) ? prec<T>::rcp(xi1) : prec<T>::div_ieee(T(1), xi1);
       }
-      const T nu = tcopysign(normu, x0);
-      const T xi1 = x0 + nu;
-      tau = prec<T>::div_ieee(xi1, nu);
-      const T scl = prec<T>::tame(xi1) ? prec<T>::rcp(xi1) : prec<T>::div_ieee(T(1), xi1);
       if (tid < m) {
         const T v = (tid == 0) ? T(1) : xi * scl;
         vv[tid] = v;
@@ -225,6 +283,7 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
       int P = NT / R;
       P = P > 8 ? 8 : P;
       const int p = tid / R, i = tid - p * R;
+      const int ps = sizeof(T) == 8 ? R : NT;  // FP64: NT partial sums in all, more CTAs per SM
       if (p < P && i < m) {
         const int j0 = (p * m) / P, j1 = ((p + 1) * m) / P;
         T acc0 = 0, acc1 = 0;
@@ -236,19 +295,19 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
           acc1 = fma(At[a1], vv[j + 1], acc1);
         }
         if (j < j1) acc0 = fma(At[(j <= i) ? (j * ld + i) : (i * ld + j)], vv[j], acc0);
-        part[p * NT + i] = acc0 + acc1;
+        part[p * ps + i] = acc0 + acc1;
       }
       __syncthreads();
       T ui = 0;
       if (tid < m) {
         T s = part[tid];
-        for (int q = 1; q < P; q++) s += part[q * NT + tid];
+        for (int q = 1; q < P; q++) s += part[q * ps + tid];
         ui = tau * s;
         uu[tid] = ui;
       }
       // xi = tau * (v' u)
       const T vi = (tid < m) ? vv[tid] : T(0);
-      const T xsum = block_sum(vi * ui, red);
+      const T xsum = block_sum8(vi * ui, red);
       const T xiv = tau * xsum;
       if (tid < m) ww[tid] = xiv * vi - ui;
       __syncthreads();
@@ -301,7 +360,7 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
       if (tau == T(0)) continue;  // uniform: taus is shared
       T part = T(0);
       for (int i = k + 1 + tid; i < n; i += NT) part = fma(r[i], (i == k + 1) ? T(1) : S[(size_t)k * ld + i], part);
-      const T dot = block_sum(part, red);
+      const T dot = block_sum8(part, red);
       const T f = tau * dot;
       for (int i = k + 1 + tid; i < n; i += NT) r[i] = fma(-f, (i == k + 1) ? T(1) : S[(size_t)k * ld + i], r[i]);
       __syncthreads();
