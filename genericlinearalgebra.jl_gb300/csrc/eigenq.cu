@@ -254,6 +254,7 @@ int gla_dormtr(char side, char uplo, char trans, int64_t m, int64_t n, const dou
     F = q->frev;
     ldf = nq;
   }
+  if ((rc = large_clear_error(q->c, st))) return rc;
   if (side == 'L') {
     if (!upper) return large_ormtr(q->c, A, lda, tau, C, ldc, st, ni, trans == 'T');
     // op(Q_U) C = P op(Q_L) (P C)

@@ -68,6 +68,26 @@ cudaError_t oz_slice_rows(OzWork* w, const float* hi, const float* lo, long long
                           cudaStream_t st);
 bool oz_fits(const OzWork* w, int m, int n, int K);
 
+// ---- FP64-accurate tensor-core GEMM (ozaki64.cuh / ozaki64.cu) and the
+// stages of the FP64 path that run on it. One object per large context of
+// order n; err: the word its bounded waits set (the context's).
+struct Oz64;
+int oz64_create(Oz64** out, int n, int* err);
+void oz64_destroy(Oz64* w);
+size_t oz64_bytes(const Oz64* w);
+constexpr int kOz64MinMerge = 256;   // smallest merge whose level runs on it
+constexpr int kOz64MinUpdate = 128;  // smallest trailing order whose update does
+// A[t:, t:] -= V W' + W V' (lower triangle of the order-n matrix A): V the
+// first nbp <= 32 columns of VW (leading dimension n), W the next nbp.
+cudaError_t oz64_rank2k(Oz64* w, const double* VW, int nbp, int t, double* A, long long lda, cudaStream_t st);
+// Problems whose sizes are known on the device only: d[0 .. nprob), not
+// transposed, at most m1max x mmax with k <= mmax (a level of the tree).
+cudaError_t oz64_grouped(Oz64* w, const GemmDesc* d, int nprob, int m1max, int mmax, cudaStream_t st);
+// Z := Q Z (trans: Q' Z) from the reflectors Y (n x n columns with their unit
+// elements, zeros above and in the last column; overwritten) and tau.
+cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Z, long long ldz, int ncol, bool trans,
+                        cudaStream_t st);
+
 // ---- adjoint of one large eigen-decomposition (large_adjoint.cu):
 // Abar = V (diag(wbar) + sym(F o (V' Vbar))) V' for orders up to nmax of
 // the context (its tensor-core slice buffers and float-pair planes,
@@ -86,6 +106,7 @@ cudaError_t sytrd_plan_create(SytrdPlan** out, int n, bool f64, bool tc = false)
 void sytrd_plan_destroy(SytrdPlan* p);
 cudaError_t sytrd_enqueue(SytrdPlan* p, void* A, long long lda, void* d, void* e, void* tau, cudaStream_t st);
 int* sytrd_error_word(SytrdPlan* p);
+void sytrd_set_oz64(SytrdPlan* p, Oz64* oz);
 
 struct DcPlan;
 // bisect_leaves (FP32 only): the leaves go through the per-eigenvalue solver
@@ -95,6 +116,7 @@ int dc_plan_create(DcPlan** out, int n, bool f64, bool bisect_leaves = false);
 void dc_plan_destroy(DcPlan* p);
 // Z has leading dimension n; info gets one word per leaf.
 int dc_enqueue(DcPlan* p, void* d, const void* e, void* Z, int* leaf_info, cudaStream_t st);
+void dc_set_oz64(DcPlan* p, Oz64* oz);
 int* dc_fail_word(DcPlan* p);
 int dc_leaf_count(const DcPlan* p);
 size_t dc_plan_bytes(const DcPlan* p);
@@ -106,6 +128,7 @@ void backtr_plan_destroy(BacktrPlan* p);
 // Error word the back-transformation's tensor-core GEMMs set when a bounded
 // wait runs out (the large context passes its reduction's word).
 void backtr_set_error_word(BacktrPlan* p, int* err);
+void backtr_set_oz64(BacktrPlan* p, Oz64* oz);
 // Z := Q Z, or Q' Z when trans, for Z of ncol columns (-1: n).
 int backtr_enqueue(BacktrPlan* p, const void* A, long long lda, const void* tau, void* Z, long long ldz,
                    cudaStream_t st, int ncol = -1, bool trans = false);
@@ -137,6 +160,9 @@ int large_stedc(LargeCtx* c, void* d, const void* e, void* Z, long long ldz, int
 // Z := Q Z with Q = H_0 H_1 ... H_{n-2} from large_sytrd.
 int large_ormtr(LargeCtx* c, const void* A, long long lda, const void* tau, void* Z, long long ldz, cudaStream_t st,
                 int ncol = -1, bool trans = false);
+// Clears the word that bounded waits set (the reduction clears it itself):
+// before a back-transformation that does not follow a reduction.
+int large_clear_error(LargeCtx* c, cudaStream_t st);
 // Full eigen-decomposition of one matrix. tcode: kF64, kF32 or kF32FromF64
 // (double input solved in FP32; outputs float). Ain has leading dimension
 // lda and uplo 'L'/'U'; w gets the ascending eigenvalues, V (ldv) the

@@ -28,6 +28,7 @@ struct LargeCtx {
   SytrdPlan* sy = nullptr;
   DcPlan* dc = nullptr;
   BacktrPlan* bt = nullptr;
+  Oz64* oz = nullptr;   // FP64, orders above 128: the GEMMs on the tensor cores
   void* Aw = nullptr;   // working copy, n x n, leading dimension n
   void* Z = nullptr;    // eigenvectors, n x n
   void* d = nullptr;
@@ -134,6 +135,14 @@ int large_create(LargeCtx** out, int n, bool f64, bool refine_stage) {
   if (!rc) rc = dc_plan_create(&c->dc, n, f64, refine_stage);
   if (!rc) rc = backtr_plan_create(&c->bt, n, f64, !f64 && refine_stage);
   if (!rc) backtr_set_error_word(c->bt, sytrd_error_word(c->sy));
+  if (!rc && f64 && n > kSmallMaxN) {
+    rc = oz64_create(&c->oz, n, sytrd_error_word(c->sy));
+    if (!rc) {
+      sytrd_set_oz64(c->sy, c->oz);
+      dc_set_oz64(c->dc, c->oz);
+      backtr_set_oz64(c->bt, c->oz);
+    }
+  }
   auto alloc = [&](void** p, size_t bytes) {
     if (!rc) {
       cudaError_t e2 = cudaMalloc(p, std::max<size_t>(bytes, 16));
@@ -165,6 +174,7 @@ void large_destroy(LargeCtx* c) {
   sytrd_plan_destroy(c->sy);
   dc_plan_destroy(c->dc);
   backtr_plan_destroy(c->bt);
+  oz64_destroy(c->oz);
   cudaFree(c->Aw);
   cudaFree(c->Z);
   cudaFree(c->d);
@@ -186,11 +196,16 @@ void large_stage_ms(const LargeCtx* c, float* ms3) {
 
 size_t large_workspace_bytes(const LargeCtx* c) {
   const size_t el = c->f64 ? 8 : 4;
-  return el * (size_t)c->n * c->n * 4 + dc_plan_bytes(c->dc);
+  return el * (size_t)c->n * c->n * 4 + dc_plan_bytes(c->dc) + (c->oz ? oz64_bytes(c->oz) : 0);
 }
 
 int large_sytrd(LargeCtx* c, void* A, long long lda, void* d, void* e, void* tau, cudaStream_t st) {
   LG_CUDA(sytrd_enqueue(c->sy, A, lda, d, e, tau, st));
+  return 0;
+}
+
+int large_clear_error(LargeCtx* c, cudaStream_t st) {
+  LG_CUDA(cudaMemsetAsync(sytrd_error_word(c->sy), 0, sizeof(int), st));
   return 0;
 }
 
@@ -281,17 +296,21 @@ int large_stev(LargeCtx* c, const double* d, const double* e, double* w, double*
   LG_CUDA(cudaMemcpyAsync(c->d, d, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   LG_CUDA(cudaMemsetAsync(c->e, 0, sizeof(double) * n, st));
   if (n > 1) LG_CUDA(cudaMemcpyAsync(c->e, e, sizeof(double) * (n - 1), cudaMemcpyDeviceToDevice, st));
-  int rc = dc_enqueue(c->dc, c->d, c->e, c->Z, c->leaf_info, st);
+  int rc = large_clear_error(c, st);
+  if (rc) return rc;
+  rc = dc_enqueue(c->dc, c->d, c->e, c->Z, c->leaf_info, st);
   if (rc) return rc;
   LG_CUDA(cudaMemcpyAsync(w, c->d, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   if (Z)
     LG_CUDA(cudaMemcpy2DAsync(Z, sizeof(double) * ldz, c->Z, sizeof(double) * n, sizeof(double) * n, n,
                               cudaMemcpyDeviceToDevice, st));
+  LG_CUDA(cudaMemcpyAsync(c->h_stat, sytrd_error_word(c->sy), sizeof(int), cudaMemcpyDeviceToHost, st));
   LG_CUDA(cudaMemcpyAsync(c->h_stat + 1, dc_fail_word(c->dc), sizeof(int), cudaMemcpyDeviceToHost, st));
   const int nleaf = dc_leaf_count(c->dc);
   std::vector<int> li(nleaf);
   LG_CUDA(cudaMemcpyAsync(li.data(), c->leaf_info, sizeof(int) * nleaf, cudaMemcpyDeviceToHost, st));
   LG_CUDA(cudaStreamSynchronize(st));
+  if (c->h_stat[0]) return -1000 - (int)cudaErrorLaunchTimeout;
   int bad = c->h_stat[1] ? 1 : 0;
   bool nonfinite = false;
   for (int x : li) {

@@ -138,9 +138,11 @@ struct BacktrPlan {
   void* W2 = nullptr;   // T W, kBT x n (leading dimension kBT)
   float* Yt = nullptr;  // FP32 with tensor cores: Y transposed
   int* err = nullptr;   // error word of the tensor-core GEMMs (set by backtr_set_error_word)
+  Oz64* oz = nullptr;   // FP64: the whole application on the tensor cores (set by backtr_set_oz64)
 };
 
 void backtr_set_error_word(BacktrPlan* p, int* err) { p->err = err; }
+void backtr_set_oz64(BacktrPlan* p, Oz64* oz) { p->oz = oz; }
 
 int backtr_plan_create(BacktrPlan** out, int n, bool f64, bool tc) {
   *out = nullptr;
@@ -203,6 +205,10 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
   k_form_y<T><<<dim3((n + 255) / 256, n), 256, 0, st>>>(A, lda, Y, n, tc ? (T*)p.Yt : (T*)nullptr);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return -1000 - (int)err;
+  if (sizeof(T) == 8 && p.oz) {
+    err = oz64_backtr(p.oz, (double*)Y, (const double*)tau, (double*)Zall, ldz, ncol, trans, st);
+    return err == cudaSuccess ? 0 : -1000 - (int)err;
+  }
   k_larft<T><<<p.nblk, 256, larft_smem_bytes<T>(), st>>>(Y, tau, (T*)p.Tm, n);
   if ((err = cudaGetLastError()) != cudaSuccess) return -1000 - (int)err;
   const bool f64 = sizeof(T) == 8;

@@ -642,6 +642,7 @@ struct DcPlan {
   void* em = nullptr;
   int* d_fail = nullptr;
   long long u_stride = 0;
+  Oz64* oz = nullptr;       // FP64: eigenvector updates on the tensor cores (set by dc_set_oz64)
   DcArrays<double> a64{};
   DcArrays<float> a32{};
 };
@@ -768,7 +769,10 @@ int dc_run(DcPlan& p, T* d, const T* e, T* Z, int* info, cudaStream_t st) {
     const size_t psm = (size_t)mp2 * (sizeof(unsigned long long) + sizeof(int));
     k_dc_post<T><<<lv.count, 1024, psm, st>>>(al, mp2);
     DC_CUDA(cudaGetLastError());
-    DC_CUDA(gemm_launch_grouped(sizeof(T) == 8, al.gdesc, 2 * lv.count, lv.m1max + 1, lv.mmax, st));
+    if (sizeof(T) == 8 && p.oz && lv.mmax >= kOz64MinMerge)
+      DC_CUDA(oz64_grouped(p.oz, al.gdesc, 2 * lv.count, lv.m1max, lv.mmax, st));
+    else
+      DC_CUDA(gemm_launch_grouped(sizeof(T) == 8, al.gdesc, 2 * lv.count, lv.m1max + 1, lv.mmax, st));
     k_dc_copydefl<T><<<dim3(lv.mmax, lv.count), 256, 0, st>>>(al);
     DC_CUDA(cudaGetLastError());
     k_dc_fail<T><<<1, 256, 0, st>>>(al.info, lv.count, p.d_fail);
@@ -901,6 +905,7 @@ int dc_enqueue(DcPlan* p, void* d, const void* e, void* Z, int* info, cudaStream
   return dc_run<float>(*p, (float*)d, (const float*)e, (float*)Z, info, st);
 }
 
+void dc_set_oz64(DcPlan* p, Oz64* oz) { p->oz = oz; }
 int* dc_fail_word(DcPlan* p) { return p->d_fail; }
 int dc_leaf_count(const DcPlan* p) { return p->nleaf; }
 size_t dc_plan_bytes(const DcPlan* p) {

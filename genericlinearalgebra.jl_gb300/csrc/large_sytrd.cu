@@ -443,6 +443,7 @@ struct SytrdPlan {
   unsigned* bar = nullptr;
   int* err = nullptr;
   bool f64 = true;
+  Oz64* oz = nullptr;     // FP64: trailing updates on the tensor cores (set by sytrd_set_oz64)
 };
 
 // [V | W] of a panel with nbp reflectors (V at VW, W at VW + nbp n, rows
@@ -545,6 +546,11 @@ cudaError_t sytrd_run(SytrdPlan& sp, T* A, long long lda, T* d, T* e, T* tau, cu
     const int t = k0 + nbp;
     if (t < n - 1) {  // trailing update A[t:, t:] -= V W' + W V' (lower tiles)
       if (sizeof(T) == 4 && sytrd_update_tc(sp, (float*)A, lda, n, t, nbp, st, &err)) {
+        if (err != cudaSuccess) return err;
+        continue;
+      }
+      if (sizeof(T) == 8 && sp.oz && n - t >= kOz64MinUpdate) {
+        err = oz64_rank2k(sp.oz, (const double*)VW, nbp, t, (double*)A, lda, st);
         if (err != cudaSuccess) return err;
         continue;
       }
@@ -657,5 +663,6 @@ cudaError_t sytrd_enqueue(SytrdPlan* sp, void* A, long long lda, void* d, void* 
 }
 
 int* sytrd_error_word(SytrdPlan* sp) { return sp->err; }
+void sytrd_set_oz64(SytrdPlan* sp, Oz64* oz) { sp->oz = oz; }
 
 }  // namespace gla
