@@ -39,9 +39,21 @@
 
 namespace gla {
 
-constexpr int kTW = 32;        // SYMV unit width (columns)
-constexpr int kRC = 64;        // SYMV unit height (rows): 2 rows per lane
-constexpr int kMaxTC = 16384 / kTW;  // tile columns at the largest order
+// Shapes of a SYMV unit (one warp): CW columns, NQ rows per lane. A unit is
+// a serial chain of FP64 instructions of 64 cycles each (2 CW NQ products,
+// and CW or so additions to reduce its column sums), so small trailing
+// orders, where every warp has at most one unit, want small units, and large
+// ones, which fill the FP64 units anyway, those with the fewest additions
+// per product. FP64 panels take the first shape whose max_m holds their
+// trailing order (other limits by a factor of 0.7 or 1.4 cost 1 to 4%); FP32
+// panels, bound by latency, the last.
+struct UnitShape {
+  int cw, nq, max_m;
+};
+constexpr int kMaxOrder = 16384;
+constexpr UnitShape kShapes[] = {{8, 1, 560}, {16, 1, 1000}, {16, 2, 1500}, {32, 2, kMaxOrder}};
+constexpr int kNumShapes = 4;
+constexpr int kMaxTC = kMaxOrder / 32;  // tile columns a launch may cover (560/8 and 1500/16 are fewer)
 constexpr int kDotRows = 1024; // rows per dot-product unit
 constexpr int kPT = 256;       // threads per CTA
 constexpr long long kSpinLimit = 1ll << 26;
@@ -57,71 +69,75 @@ struct SytrdArgs {
   T* d;
   T* e;
   T* tau;
-  T* P;              // row partials   [nTC][n]
-  T* Qp;             // column partials [nCH][n]
+  T* P;              // row partials    [tile column - Jbase][n]
+  T* Qp;             // column partials [chunk of rows][n]
   T* normp;          // [G]
   T* qfp;            // [G]
   T* dots;           // [3][kSytrdNB][nDCH]
   int nDCH;
-  const int* ustart; // first SYMV unit of each tile column; ustart[nTC] = total
+  const int* ustart; // of this shape: first SYMV unit of each tile column; ustart[nTC] = total
   int nTC;
   unsigned* bar;     // arrival counter (monotonic over the launches of one tridiagonalisation)
   unsigned bar_base; // counter value when this launch starts
   int* err;
 };
 
+// Sum over the lanes of the warp that differ in the lane bits of [lo, 32).
+template <class T>
+GLA_DEV T lane_sum(T v, int lo) {
+  for (int o = 16; o >= lo; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// Four sums over the warp at once, six additions in all: lane 8 k ends with
+// the sum of v[k].
+template <class T>
+GLA_DEV T warp_sum4(const T (&v)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool u = lane & 16, w = lane & 8;
+  const T a = (u ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, u ? v[0] : v[2], 16);
+  const T b = (u ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, u ? v[1] : v[3], 16);
+  T x = (w ? b : a) + __shfl_xor_sync(0xffffffffu, w ? a : b, 8);
+  x += __shfl_xor_sync(0xffffffffu, x, 4);
+  x += __shfl_xor_sync(0xffffffffu, x, 2);
+  return x + __shfl_xor_sync(0xffffffffu, x, 1);
+}
+
 // Grid barrier on a monotonic arrival counter: barrier number k of a launch
 // completes when the counter reaches (k + 1) * gridDim.x. Thread 0 of each
 // CTA arrives with a release add and polls with acquire loads; the wait is
 // bounded (kSpinLimit polls) and a timeout sets the error word, which every
-// waiting CTA also watches. The verdict is broadcast through shared memory
-// so that all threads of a CTA return the same value.
-GLA_DEV bool grid_sync(unsigned* bar, int* err, unsigned& target) {
+// waiting CTA also watches now and then. The verdict is broadcast through shared memory
+// so that all threads of a CTA return the same value. Before it arrives, the
+// CTA's part of a sum goes out: the warps' parts in part[0 .. 8), added by
+// warp 0 into *out.
+template <class T>
+GLA_DEV bool grid_sync(unsigned* bar, int* err, unsigned& target, const T* part, T* out) {
   __shared__ int s_ok;
   target += gridDim.x;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-    volatile int* verr = err;
-    long long it = 0;
-    for (;;) {
-      unsigned v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-      if ((int)(v - target) >= 0) break;
-      if (*verr) break;
-      if (++it > kSpinLimit) {
-        atomicExch(err, 1);
-        break;
+  if (threadIdx.x < 32) {
+    T v = part[threadIdx.x & 7];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (threadIdx.x == 0) {
+      *out = v;
+      // (cumulative: it also releases what the CTA's other threads wrote
+      // before the __syncthreads above)
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+      volatile int* verr = err;
+      bool ok = false;
+      for (long long it = 1; it <= kSpinLimit; it++) {
+        unsigned c;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(bar) : "memory");
+        ok = (int)(c - target) >= 0;
+        if (ok || ((it & 255) == 0 && *verr)) break;
       }
+      if (!ok) atomicExch(err, 1);
+      s_ok = ok;
     }
-    s_ok = *verr == 0;
   }
   __syncthreads();
   return s_ok != 0;
-}
-
-// Deterministic block sum of up to 4 values (every CTA gets the same bits
-// for the same inputs). `buf` alternates between two shared slots so that
-// consecutive calls need a single __syncthreads each.
-template <class T, int K>
-GLA_DEV void block_sum(T (&v)[K], T (*sred)[kPT / 32][4], int& buf) {
-#pragma unroll
-  for (int k = 0; k < K; k++)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-  if ((threadIdx.x & 31) == 0)
-#pragma unroll
-    for (int k = 0; k < K; k++) sred[buf][threadIdx.x >> 5][k] = v[k];
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    T s = T(0);
-#pragma unroll
-    for (int i = 0; i < kPT / 32; i++) s += sred[buf][i][k];
-    v[k] = s;
-  }
-  buf ^= 1;
 }
 
 // a_i = A[i, j] below row s (the raw reflector column), 0 elsewhere. The
@@ -135,33 +151,35 @@ GLA_DEV T a_at(const T* __restrict__ A, long long ld, int j, int s, int i) {
 // One warp: SYMV unit (tile column J, chunk ch) of the trailing lower
 // triangle on the raw column a, row by row (lane l holds row r0 + l + 32 q);
 // all loads of the unit are issued before its FMAs. Adds the row sums to
-// P[J][r] and the column sums to Qp[ch][c]; returns the unit's part of a'A_t a.
-template <class T>
+// P[J - Jbase][r] and the column sums to Qp[ch][c]; returns the unit's part
+// of a'A_t a.
+template <class T, int CW, int NQ>
 __device__ T symv_unit(const SytrdArgs<T>& a, int j, int s, int J, int ch, T* svcol) {
-  constexpr int NQ = kRC / 32;
+  constexpr int RC = 32 * NQ;
   const int lane = threadIdx.x & 31, n = a.n;
   const long long ld = a.ld;
   const T* __restrict__ A = a.A;
-  const int c0 = J * kTW, r0 = c0 + ch * kRC;
-  const int cc = c0 + lane;
+  const int c0 = J * CW, r0 = c0 + ch * RC;
+  constexpr int kRep = 32 / CW;  // lanes that end with the same column sum
+  const int cc = c0 + lane / kRep;
   const T vc = cc < n ? a_at(A, ld, j, s, cc) : T(0);
   const T* __restrict__ base = A + (long long)c0 * ld + r0 + lane;
-  const int ncol = min(kTW, n - c0);
-  T x[NQ][kTW], vr[NQ];
+  const int ncol = min(CW, n - c0);
+  T x[NQ][CW], vr[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; q++) {
     const int r = r0 + lane + 32 * q;
     const bool rin = r < n;
     const T* rowp = base + 32 * q;
 #pragma unroll
-    for (int ci = 0; ci < kTW; ci++) x[q][ci] = (rin && ci < ncol) ? rowp[(long long)ci * ld] : T(0);
+    for (int ci = 0; ci < CW; ci++) x[q][ci] = (rin && ci < ncol) ? rowp[(long long)ci * ld] : T(0);
     vr[q] = rin ? a_at(A, ld, j, s, r) : T(0);
   }
-  svcol[lane] = vc;
+  if (lane % kRep == 0) svcol[lane / kRep] = vc;
   __syncwarp();
-  T colacc[kTW];
+  T colacc[CW];
 #pragma unroll
-  for (int ci = 0; ci < kTW; ci++) colacc[ci] = T(0);
+  for (int ci = 0; ci < CW; ci++) colacc[ci] = T(0);
   T qf = T(0);
 #pragma unroll
   for (int q = 0; q < NQ; q++) {
@@ -169,29 +187,34 @@ __device__ T symv_unit(const SytrdArgs<T>& a, int j, int s, int J, int ch, T* sv
     const bool diag = ch == 0 && q == 0;  // diagonal tile: lower part only (row >= column)
     T rowacc = T(0);
 #pragma unroll
-    for (int ci = 0; ci < kTW; ci++) {
+    for (int ci = 0; ci < CW; ci++) {
       const T xr = (diag && lane < ci) ? T(0) : x[q][ci];
       const T xc = (diag && lane <= ci) ? T(0) : x[q][ci];
       rowacc = fma(xr, svcol[ci], rowacc);
       colacc[ci] = fma(xc, vr[q], colacc[ci]);
     }
     const int r = r0 + lane + 32 * q;
-    if (r < n) a.P[(long long)J * n + r] = rowacc;
+    if (r < n) a.P[(long long)(J - a.k0 / CW) * n + r] = rowacc;
     qf = fma(rowacc, vr[q], qf);
   }
-  // reduce-scatter the 32 column sums across the warp: lane l keeps column l
+  // reduce-scatter the column sums across the warp: lane l keeps column l / kRep
 #pragma unroll
-  for (int half = 16; half >= 1; half >>= 1) {
-    const bool up = (lane & half) != 0;
+  for (int half = CW / 2; half >= 1; half >>= 1) {
+    const int bit = half * kRep;
+    const bool up = (lane & bit) != 0;
 #pragma unroll
     for (int i = 0; i < half; i++) {
       const T send = up ? colacc[i] : colacc[i + half];
       const T keep = up ? colacc[i + half] : colacc[i];
-      colacc[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+      colacc[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
     }
   }
-  if (cc < n) a.Qp[(long long)ch * n + cc] = colacc[0];
-  qf = fma(colacc[0], vc, qf);
+#pragma unroll
+  for (int o = kRep / 2; o >= 1; o >>= 1) colacc[0] += __shfl_xor_sync(0xffffffffu, colacc[0], o);
+  if (lane % kRep == 0) {
+    if (cc < n) a.Qp[(long long)ch * n + cc] = colacc[0];
+    qf = fma(colacc[0], vc, qf);
+  }
   __syncwarp();
   return qf;
 }
@@ -208,20 +231,81 @@ GLA_DEV void own_rows(int s, int n, int& lo, int& hi) {
 // rows k0 + 1 .. n - 1, fixed for the panel).
 GLA_DEV __host__ int panel_rows(int k0, int n, int G) { return (n - k0 - 1 + G - 1) / G; }
 
+// beta = -copysign(norm, alpha), tau = (beta - alpha) / beta and 1 / (alpha -
+// beta) from alpha and sigma, the squared norm below it; beta = alpha and
+// zeros when sigma is zero. FP64: one seed and one cubic step per square root
+// and reciprocal, 10 instructions in a row; the norm in even lanes and its
+// reciprocal in odd ones.
+GLA_DEV void panel_scalars(double alpha, double sigma, double& beta, double& tau, double& scale) {
+  if ((__double_as_longlong(sigma) << 1) == 0) {
+    beta = alpha;
+    tau = scale = 0.0;
+    return;
+  }
+  const bool odd = threadIdx.x & 1;
+  const double nrm2 = fma(alpha, alpha, sigma);
+  double y, x;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(nrm2));
+  const double h = nrm2 * y;
+  const double e = fma(-h, y, 1.0);
+  const double q = e * fma(e, 0.375, 0.5);
+  const double hy = odd ? y : h;
+  const double r = fma(hy, q, hy);
+  const double nrm = __shfl_sync(0xffffffffu, r, 0), rn = __shfl_sync(0xffffffffu, r, 1);
+  beta = copysign(nrm, -alpha);
+  // even: alpha - beta = sign(alpha) (|alpha| + norm); odd: tau = 1 + |alpha| / norm
+  const double d = fma(odd ? fabs(alpha) : 1.0, odd ? rn : nrm, odd ? 1.0 : fabs(alpha));
+  tau = __shfl_sync(0xffffffffu, d, 1);
+  const double dd = copysign(__shfl_sync(0xffffffffu, d, 0), alpha);
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(dd));
+  const double ed = fma(-dd, x, 1.0);
+  scale = fma(x, fma(ed, ed, ed), x);
+}
+GLA_DEV void panel_scalars(float alpha, float sigma, float& beta, float& tau, float& scale) {
+  if (sigma == 0.f) {
+    beta = alpha;
+    tau = scale = 0.f;
+    return;
+  }
+  const float nrm2 = fmaf(alpha, alpha, sigma);
+  const float nrm = nrm2 * prec<float>::rsqrt(nrm2);
+  beta = -copysignf(nrm, alpha);
+  tau = (beta - alpha) * prec<float>::rcp(beta);
+  scale = prec<float>::rcp(alpha - beta);
+}
+
 // Dot-product unit kinds, in work-list order after the SYMV units.
-constexpr int kDotA = 0;  // sum_r a_r A[r, s]        (cross term of v'A_t v)
+constexpr int kDotA = 0;  // 2 sum_r a_r A[r, s]      (cross term of v'A_t v)
 constexpr int kDotV = 1;  // sum_r a_r V[r, q], q < c
 constexpr int kDotW = 2;  // sum_r a_r W[r, q]
 
-template <class T>
+// Microseconds per column (reduction of order 777 / 4096 in FP64, of order
+// 2048 in FP32): 9.4 / 27.1 and 7.6, of which the two grid barriers are about
+// 3.5; before units by shape, this split and the short serial chains below
+// 19.4 / 32.9 and 7.9.
+//
+// Work split of phase B. FP64: warps 0 .. 3 read and add up the column's
+// scalars, warp 0 derives the reflector's from them (warp 1 the sums over the
+// panel's earlier columns), warps 4 .. 7 hold the CTA's rows: an FP64
+// addition costs 64 cycles per warp whatever its lanes hold, and the two
+// warps of a sub-partition queue for it, so sums go through as few additions
+// as there are (four sums in six), and by one warp. FP32, bound by the round
+// trips to L2: all warps do both, with as many loads in flight as there are
+// threads.
+template <class T, int CW, int NQ>
 __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
+  constexpr int RC = 32 * NQ;
+  constexpr bool kSplit = sizeof(T) == 8;
+  constexpr int kRowT = kSplit ? kPT / 2 : kPT, kRedT = kRowT, kRedW = kRedT / 32;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int n = a.n, G = gridDim.x, g = blockIdx.x;
   const long long ld = a.ld, ldv = a.ldv;
   T* __restrict__ A = a.A;
-  __shared__ T sred[2][kPT / 32][4];
+  __shared__ T spart[8];       // the warps' parts of the sum that the next barrier carries
+  __shared__ T sred[kRedW][4];  // the scalars' sums by warp
   __shared__ T svcol[kPT / 32][32];
   __shared__ T sdotV[kSytrdNB], sdotW[kSytrdNB], sVs[kSytrdNB], sWs[kSytrdNB];
+  __shared__ T spv[kSytrdNB], sqv[kSytrdNB], sS[4];
   __shared__ int sust[kMaxTC + 1];
   __shared__ T sscal[4];
   // this CTA's V and W rows of the panel (rows lo0 .. lo0 + R0 - 1, columns
@@ -232,47 +316,51 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
   T* sWr = sVr + (size_t)R0 * kSytrdNB;
   const int lo0 = min(n, a.k0 + 1 + g * R0), hi0 = min(n, lo0 + R0);
   for (int i = tid; i < 2 * R0 * kSytrdNB; i += kPT) sVr[i] = T(0);
-  int rb = 0;
   unsigned bar_target = a.bar_base;
-  for (int i = tid; i <= a.nTC; i += kPT) sust[i] = a.ustart[i];
+  const int Jb = a.k0 / CW, nJ = a.nTC - Jb;  // tile columns of the panel's trailing matrix
+  for (int i = tid; i <= nJ; i += kPT) sust[i] = a.ustart[Jb + i];
+  // rows: tpr threads per row
+  int tpr = 1;
+  while (tpr < 32 && tpr * 2 * R0 <= kRowT) tpr *= 2;
+  const int rpp = kRowT / tpr;  // rows per pass (more rows than threads take several)
 
   // panel start: norm partial of column k0 below the subdiagonal
   {
     const int j = a.k0, s = j + 1;
     int lo, hi;
     own_rows(s, n, lo, hi);
-    T part[1] = {T(0)};
+    T part = T(0);
     for (int i = lo + tid; i < hi; i += kPT)
       if (i > s) {
         const T x = A[i + (long long)j * ld];
-        part[0] = fma(x, x, part[0]);
+        part = fma(x, x, part);
       }
-    block_sum(part, sred, rb);
-    if (tid == 0) a.normp[g] = part[0];
+    part = lane_sum(part, 1);
+    if (lane == 0) spart[wid] = part;
   }
-  if (!grid_sync(a.bar, a.err, bar_target)) return;
+  if (!grid_sync(a.bar, a.err, bar_target, spart, a.normp + g)) return;
 
   for (int c = 0; c < a.nbp; c++) {
     const int j = a.k0 + c, s = j + 1, m = n - s;
-    const int J0 = s / kTW;
+    const int J0 = s / CW;
+    const int ndch = (m + kDotRows - 1) / kDotRows;
     // ---------------- phase A: SYMV and dot products on the raw column a
     {
-      const int usym0 = sust[J0], nsym = sust[a.nTC] - usym0;
-      const int ndch = (m + kDotRows - 1) / kDotRows;
+      const int usym0 = sust[J0 - Jb], nsym = sust[nJ] - usym0;
       const int ndot = (2 * c + 1) * ndch;
-      T qf[1] = {T(0)};
+      T qf = T(0);
       // unit u goes to CTA u % G, so every CTA gets an even share
       for (int k = wid;; k += kPT / 32) {
         const int u = g + G * k;
         if (u >= nsym + ndot) break;
         if (u < nsym) {
           const int ug = usym0 + u;
-          int lo = J0, hi = a.nTC - 1;  // tile column: last J with sust[J] <= ug
+          int lo = J0 - Jb, hi = nJ - 1;  // tile column: last J with sust[J] <= ug
           while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
             if (sust[mid] <= ug) lo = mid; else hi = mid - 1;
           }
-          qf[0] += symv_unit(a, j, s, lo, ug - sust[lo], svcol[wid]);
+          qf += symv_unit<T, CW, NQ>(a, j, s, Jb + lo, ug - sust[lo], svcol[wid]);
         } else {
           const int du = u - nsym;
           const int kind = du < ndch ? kDotA : (du - ndch) / (c * ndch) + 1;
@@ -282,147 +370,237 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
                                                   : (kind == kDotV ? a.V : a.W) + (long long)q * ldv;
           const int r0 = s + 1 + chn * kDotRows, r1 = min(n, r0 + kDotRows);
           T acc = T(0);
+#pragma unroll 4
           for (int r = r0 + lane; r < r1; r += 32) acc = fma(X[r], A[r + (long long)j * ld], acc);
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+          acc = lane_sum(acc, 1);
+          if (kind == kDotA) acc += acc;  // the quadratic form has it twice
           if (lane == 0) a.dots[((long long)kind * kSytrdNB + q) * a.nDCH + chn] = acc;
         }
       }
-      block_sum(qf, sred, rb);
-      if (tid == 0) a.qfp[g] = qf[0];
+      qf = lane_sum(qf, 1);
+      if (lane == 0) spart[wid] = qf;
     }
-    if (!grid_sync(a.bar, a.err, bar_target)) return;
+    if (!grid_sync(a.bar, a.err, bar_target, spart, a.qfp + g)) return;
 
     // ---------------- phase B: reflector scalars, y, w, reflector store, next column
-    const int ndch = (m + kDotRows - 1) / kDotRows;
-    const int Js = s / kTW;
-    const int nchs = (n - Js * kTW + kRC - 1) / kRC;
-    const int R = R0;
-    int tpr = 1;
-    while (tpr < 32 && tpr * 2 * R <= kPT) tpr *= 2;
-    const int sub = tid % tpr;
-    const int rl = tid / tpr;  // this thread's row of the CTA's panel rows
-    const int i = lo0 + rl;
-    const bool act = i < hi0 && i >= s;
-    const int ii = act ? i : s;  // idle threads read row s (always in range)
-    const int rc = rl < R ? rl : R - 1;  // (idle threads: any cached row)
-    // (1) every load of the phase, independent of the reductions
-    T red[4] = {T(0), T(0), T(0), T(0)};  // sigma, a'A_t a, sum a_r A[r,s], y_s raw
-    for (int t = tid; t < G; t += kPT) {
-      red[0] += a.normp[t];
-      red[1] += a.qfp[t];
-    }
-    for (int k = tid; k < ndch; k += kPT) red[2] += a.dots[((long long)kDotA * kSytrdNB) * a.nDCH + k];
-    if (tid < c) {
-      T sv = T(0), sw = T(0);
-      for (int k = 0; k < ndch; k++) {
-        sv += a.dots[((long long)kDotV * kSytrdNB + tid) * a.nDCH + k];
-        sw += a.dots[((long long)kDotW * kSytrdNB + tid) * a.nDCH + k];
+    const int Js = s / CW;
+    const bool rows = !kSplit || wid >= 4;
+    const int rt = kSplit ? tid & (kRowT - 1) : tid, sub = rt % tpr, rl0 = rt / tpr;
+    // (1) every load of the phase is issued before the first sum needs one
+    // (loops that load and add would each wait for L2 in turn); what does not
+    // fit the registers follows in batches. Rows: kU parts of a row's y in P
+    // and in Qp per thread; cP, cQ: those the CTA's rows have at most.
+    constexpr int kU = kSplit ? 4 : 16;
+    const int Jhi = (max(hi0, lo0 + 1) - 1) / CW, Jlo = max(lo0, s) / CW;
+    const int cP = (min(Jhi, a.nTC - 1) - J0 + tpr) / tpr;
+    const int cQ = ((n - min(Jlo, a.nTC - 1) * CW + RC - 1) / RC + tpr - 1) / tpr;
+    T tp[kU], tq[kU], ai = T(0), Ais = T(0);
+    auto load_parts = [&](int ii, int u0) {
+      const int Ji = ii / CW, nch = (n - Ji * CW + RC - 1) / RC;
+      const T* pp = a.P + (long long)(J0 - Jb) * n + ii;
+      const T* pq = a.Qp + ii;
+#pragma unroll
+      for (int u = 0; u < kU; u++) {
+        const int k = sub + (u0 + u) * tpr;
+        if (u0 + u < cP) tp[u] = k <= Ji - J0 ? pp[(long long)k * n] : T(0);
+        if (u0 + u < cQ) tq[u] = k < nch ? pq[(long long)k * n] : T(0);
       }
-      sdotV[tid] = sv;
-      sdotW[tid] = sw;
-      sVs[tid] = a.V[s + (long long)tid * ldv];
-      sWs[tid] = a.W[s + (long long)tid * ldv];
-    }
-    for (int k = tid - 64; k >= 0 && k < nchs; k += kPT - 64) red[3] += a.Qp[(long long)k * n + s];
-    if (tid == 63) red[3] += a.P[(long long)Js * n + s];
+    };
+    auto add_parts = [&](int u0, T& y) {
+#pragma unroll
+      for (int u = 0; u < kU; u++) {
+        if (u0 + u < cP) y += tp[u];
+        if (u0 + u < cQ) y += tq[u];
+      }
+    };
+    auto row_of = [&](int rl) {  // idle threads read row s (always in range)
+      const int i = lo0 + rl;
+      return (rl < R0 && i < hi0 && i >= s) ? i : s;
+    };
     const T alpha = A[s + (long long)j * ld];
     const T Ass = A[s + (long long)s * ld];
-    T yraw = T(0);
-    {
-      const int Ji = ii / kTW;
-      for (int Jx = J0 + sub; Jx <= Ji; Jx += tpr) yraw += a.P[(long long)Jx * n + ii];
-      const int nch = (n - Ji * kTW + kRC - 1) / kRC;
-      for (int k = sub; k < nch; k += tpr) yraw += a.Qp[(long long)k * n + ii];
+    if (rows) {
+      const int ii = row_of(rl0);
+      ai = a_at(A, ld, j, s, ii);
+      Ais = A[ii + (long long)s * ld];
+      load_parts(ii, 0);
     }
-    const T ai = a_at(A, ld, j, s, ii);
-    const T Ais = A[ii + (long long)s * ld];
-    block_sum(red, sred, rb);  // also publishes sdotV/sdotW/sVs/sWs
-    // (2) reflector scalars and the q-sums once, in warp 0 (lanes over q;
-    // FP64 work repeated by every warp would queue on the FP64 pipe)
-    if (wid == 0) {
-      const T sigma = red[0];
-      T beta, tau, scale;
-      if (sigma == T(0)) {
-        beta = alpha;
-        tau = T(0);
-        scale = T(0);
-      } else {
-        const T nrm2 = fma(alpha, alpha, sigma);
-        const T nrm = nrm2 * prec<T>::rsqrt(nrm2);
-        beta = -copysign(nrm, alpha);
-        tau = (beta - alpha) * prec<T>::rcp(beta);
-        scale = prec<T>::rcp(alpha - beta);
-      }
-      // p = V'v, q = W'v with v = scale a + e_s; y_s and v'A_t v by linearity
-      T pq = T(0), corr = T(0);
-      if (lane < c) {
-        const T pv = fma(scale, sdotV[lane], sVs[lane]), qv = fma(scale, sdotW[lane], sWs[lane]);
-        pq = pv * qv;
-        corr = sVs[lane] * qv + sWs[lane] * pv;
-      }
+    T yraw = T(0);
+    if (!kSplit || !rows) {
+      const int nchs = (n - Js * CW + RC - 1) / RC;
+      constexpr int kN = kSplit ? 2 : 1, kD = 4;
+      T pn[kN], pf[kN], pc[kN], da = T(0), px = T(0), vs = T(0), ws = T(0), dv[kD], dw[kD];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        pq += __shfl_xor_sync(0xffffffffu, pq, o);
-        corr += __shfl_xor_sync(0xffffffffu, corr, o);
+      for (int u = 0; u < kN; u++) {
+        const int t = tid + u * kRedT;
+        pn[u] = t < G ? a.normp[t] : T(0);
+        pf[u] = t < G ? a.qfp[t] : T(0);
+        pc[u] = t < nchs ? a.Qp[(long long)t * n + s] : T(0);
       }
-      if (lane == 0) {
-        const T vAv = scale * scale * red[1] + T(2) * scale * red[2] + Ass;
-        const T hw = T(0.5) * tau * tau * (vAv - T(2) * pq);  // w = tau y - hw v
-        const T y_s = scale * red[3] + Ass - corr;
-        sscal[0] = tau;
-        sscal[1] = scale;
-        sscal[2] = hw;
-        sscal[3] = tau * y_s - hw;  // w_s
-        if (g == 0) {
-          if (c == 0) a.d[j] = A[j + (long long)j * ld];  // later columns: written by the previous step
-          a.e[j] = beta;
-          a.tau[j] = tau;
+      if (tid < ndch) da = a.dots[((long long)kDotA * kSytrdNB) * a.nDCH + tid];
+      if (tid == 0) px = a.P[(long long)(Js - Jb) * n + s];
+      const T* pv = a.dots + ((long long)kDotV * kSytrdNB + lane) * a.nDCH;
+      const T* pw = a.dots + ((long long)kDotW * kSytrdNB + lane) * a.nDCH;
+      if (wid == 1) {
+        if (lane < c) {
+          vs = a.V[s + (long long)lane * ldv];
+          ws = a.W[s + (long long)lane * ldv];
+        }
+#pragma unroll
+        for (int u = 0; u < kD; u++) {
+          dv[u] = lane < c && u < ndch ? pv[u] : T(0);
+          dw[u] = lane < c && u < ndch ? pw[u] : T(0);
+        }
+      }
+      T red[4] = {pn[0], pf[0], da, pc[0]};  // sigma, a'A_t a, 2 sum a_r A[r,s], y_s raw
+      if (kN > 1 && G > kRedT) {
+        red[0] += pn[kN - 1];
+        red[1] += pf[kN - 1];
+      }
+      if (kN > 1 && nchs > kRedT) red[3] += pc[kN - 1];
+      if (wid == 0) red[3] += px;
+      for (int t = tid + kN * kRedT; t < G; t += kRedT) {
+        red[0] += a.normp[t];
+        red[1] += a.qfp[t];
+      }
+      for (int k = tid + kN * kRedT; k < nchs; k += kRedT) red[3] += a.Qp[(long long)k * n + s];
+      for (int k = tid + kRedT; k < ndch; k += kRedT) red[2] += a.dots[((long long)kDotA * kSytrdNB) * a.nDCH + k];
+      const T x = warp_sum4(red);
+      if ((lane & 7) == 0) sred[wid][lane >> 3] = x;
+      if (wid == 1) {
+        T dV = dv[0], dW = dw[0];
+#pragma unroll
+        for (int u = 1; u < kD; u++)
+          if (u < ndch) {
+            dV += dv[u];
+            dW += dw[u];
+          }
+        for (int k = kD; k < ndch; k++)
+          if (lane < c) {
+            dV += pv[k];
+            dW += pw[k];
+          }
+        sdotV[lane] = dV;
+        sdotW[lane] = dW;
+        sVs[lane] = vs;
+        sWs[lane] = ws;
+      }
+    }
+    if (rows) add_parts(0, yraw);
+    __syncthreads();
+    // (2) The reflector's scalars in warp 0; meanwhile the sums over the
+    // panel's earlier columns in warp 1, and with them the coefficients of
+    // what depends on scale. With v = scale a + e_s, p = V'v, q = W'v:
+    //   v'A_t v - 2 p'q = (k2 scale + k1) scale + k0,  y_s = k3 scale + k0,
+    //   k2 = a'A_t a - 2 sum dV dW, k1 = 2 a'A[:, s] - 2 sum (dV Ws + Vs dW),
+    //   k0 = A[s, s] - 2 sum Vs Ws, k3 = y_s raw - sum (dV Ws + Vs dW).
+    // Every step is one instruction of a serial chain (64 cycles in FP64), so
+    // lanes 0 and 1 do two different products at once where the chain forks.
+    if (wid < 2) {
+      T x = sred[(lane >> 2) & (kRedW - 1)][lane & 3];
+#pragma unroll
+      for (int o = 4; o < 4 * kRedW; o *= 2) x += __shfl_xor_sync(0xffffffffu, x, o);
+      if (wid == 1) {
+        const T dV = sdotV[lane], dW = sdotW[lane], vs = sVs[lane], ws = sWs[lane];
+        const T v[4] = {dV * dW, fma(dV, ws, vs * dW), vs * ws, T(0)};
+        const T S = warp_sum4(v);
+        // lane 0: k2, 1: k1, 2: k0, 3: k3
+        const T Sk = __shfl_sync(0xffffffffu, S, lane == 0 ? 0 : lane == 2 ? 16 : 8);
+        const T b = __shfl_sync(0xffffffffu, x, lane == 0 ? 1 : lane == 1 ? 2 : 3);
+        const T k = fma(lane == 3 ? T(-1) : T(-2), Sk, lane == 2 ? Ass : b);
+        if (lane < 4) sS[lane] = k;
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+      } else {
+        const T sigma = __shfl_sync(0xffffffffu, x, 0);
+        T beta, tau, scale;
+        panel_scalars(alpha, sigma, beta, tau, scale);
+        spv[lane] = fma(scale, sdotV[lane], sVs[lane]);
+        sqv[lane] = fma(scale, sdotW[lane], sWs[lane]);
+        const T h2 = T(0.5) * tau * tau;
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        const T k0 = sS[2];
+        // lane 0: k2 scale + k1, lane 1: y_s
+        const T u = fma(scale, lane == 0 ? sS[0] : sS[3], lane == 0 ? sS[1] : k0);
+        const T hw = h2 * fma(u, scale, k0);  // (lane 0) w = tau y - hw v
+        const T y_s = __shfl_sync(0xffffffffu, u, 1);
+        if (lane == 0) {
+          sscal[0] = tau;
+          sscal[1] = scale;
+          sscal[2] = hw;
+          sscal[3] = fma(tau, y_s, -hw);  // w_s
+          if (g == 0) {
+            if (c == 0) a.d[j] = A[j + (long long)j * ld];  // later columns: written by the previous step
+            a.e[j] = beta;
+            a.tau[j] = tau;
+          }
         }
       }
     }
     __syncthreads();
-    const T tau = sscal[0], scale = sscal[1], hw = sscal[2], w_s = sscal[3];
     const bool last_in_panel = c + 1 == a.nbp;
     const bool update_next = !last_in_panel || s == n - 1;
     // (3) own rows
-    T y = T(0), xn = T(0);
-    for (int q = sub; q < c; q += tpr) {
-      const T vq = sVr[(size_t)rc * kSytrdNB + q], wq = sWr[(size_t)rc * kSytrdNB + q];
-      const T pv = fma(scale, sdotV[q], sVs[q]), qv = fma(scale, sdotW[q], sWs[q]);
-      y -= vq * qv + wq * pv;
-      xn += vq * sWs[q] + wq * sVs[q];
-    }
-    if (sub == 0) y += scale * yraw + Ais;
-    else y += scale * yraw;
-    for (int o = tpr / 2; o > 0; o >>= 1) {
-      y += __shfl_xor_sync(0xffffffffu, y, o, tpr);
-      xn += __shfl_xor_sync(0xffffffffu, xn, o, tpr);
-    }
-    const T vi = ii == s ? T(1) : scale * ai;
-    const T wi = tau * y - hw * vi;
-    xn += vi * w_s + wi;  // the q = c term: v_s = 1, w_s
-    T npart[1] = {T(0)};
-    if (act && sub == 0) {
-      a.V[ii + (long long)c * ldv] = vi;
-      a.W[ii + (long long)c * ldv] = wi;
-      sVr[(size_t)rl * kSytrdNB + c] = vi;
-      sWr[(size_t)rl * kSytrdNB + c] = wi;
-      if (ii > s) A[ii + (long long)j * ld] = vi;
-      if (update_next) {
-        // A[s, s] is read by every CTA in this phase: its new value goes to d[s]
-        const T x = Ais - xn;
-        if (ii == s)
-          a.d[s] = x;
-        else
-          A[ii + (long long)s * ld] = x;
-        if (ii > s + 1) npart[0] = x * x;
+    T npart = T(0);
+    if (rows) {
+      const T tau = sscal[0], scale = sscal[1], hw = sscal[2], w_s = sscal[3];
+      for (int rl = rl0; rl < rpp * ((R0 + rpp - 1) / rpp); rl += rpp) {
+        const int i = lo0 + rl, ii = row_of(rl);
+        const bool act = rl < R0 && i < hi0 && i >= s;
+        if (rl != rl0) {
+          ai = a_at(A, ld, j, s, ii);
+          Ais = A[ii + (long long)s * ld];
+          yraw = T(0);
+          load_parts(ii, 0);
+          add_parts(0, yraw);
+        }
+        for (int u0 = kU; u0 < max(cP, cQ); u0 += kU) {
+          load_parts(ii, u0);
+          add_parts(u0, yraw);
+        }
+        const int rc = rl < R0 ? rl : R0 - 1;  // (idle threads: any cached row)
+        T y = T(0), xn = T(0);
+        for (int q = sub; q < c; q += tpr) {
+          const T vq = sVr[(size_t)rc * kSytrdNB + q], wq = sWr[(size_t)rc * kSytrdNB + q];
+          y = fma(vq, sqv[q], fma(wq, spv[q], y));
+          xn = fma(vq, sWs[q], fma(wq, sVs[q], xn));
+        }
+        y = fma(scale, yraw, -y);
+        // y and xn over the row's tpr lanes: the halves swap one of the two first
+        if (tpr > 1) {
+          const int h = tpr / 2;
+          const bool up = sub >= h;
+          T z = (up ? xn : y) + __shfl_xor_sync(0xffffffffu, up ? y : xn, h);
+          for (int o = h / 2; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+          const T other = __shfl_xor_sync(0xffffffffu, z, h);
+          y = up ? other : z;
+          xn = up ? z : other;
+        }
+        y += Ais;
+        const T vi = ii == s ? T(1) : scale * ai;
+        const T wi = fma(tau, y, -hw * vi);
+        xn += fma(vi, w_s, wi);  // the q = c term: v_s = 1, w_s
+        if (act && sub == 0) {
+          a.V[ii + (long long)c * ldv] = vi;
+          a.W[ii + (long long)c * ldv] = wi;
+          sVr[(size_t)rl * kSytrdNB + c] = vi;
+          sWr[(size_t)rl * kSytrdNB + c] = wi;
+          if (ii > s) A[ii + (long long)j * ld] = vi;
+          if (update_next) {
+            // A[s, s] is read by every CTA in this phase: its new value goes to d[s]
+            const T x = Ais - xn;
+            if (ii == s)
+              a.d[s] = x;
+            else
+              A[ii + (long long)s * ld] = x;
+            if (ii > s + 1) npart = fma(x, x, npart);
+          }
+        }
       }
+      npart = lane_sum(npart, tpr);  // (lanes with sub > 0 hold zero)
     }
-    block_sum(npart, sred, rb);
-    if (tid == 0) a.normp[g] = npart[0];
+    if (lane == 0) spart[wid] = npart;
     if (c + 1 < a.nbp)
-      if (!grid_sync(a.bar, a.err, bar_target)) return;
+      if (!grid_sync(a.bar, a.err, bar_target, spart, a.normp + g)) return;
   }
 }
 
@@ -430,8 +608,9 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
 
 struct SytrdPlan {
   int n = 0, G = 0;
-  int nTC = 0, nCH = 0, nDCH = 0;
-  int* ustart = nullptr;
+  int nDCH = 0;
+  int* ustart = nullptr;  // the shapes' tables, one after another
+  int uoff[kNumShapes] = {};
   void* P = nullptr;
   void* Qp = nullptr;
   void* normp = nullptr;
@@ -504,6 +683,22 @@ bool sytrd_update_tc(SytrdPlan& sp, float* A, long long lda, int n, int t, int n
   return true;
 }
 
+int panel_shape(int m, bool f64) {
+  int sh = 0;
+  while (sh + 1 < kNumShapes && (!f64 || m > kShapes[sh].max_m)) sh++;
+  return sh;
+}
+template <class T>
+const void* panel_kernel(int sh) {
+  static_assert(kNumShapes == 4, "one kernel per shape");
+  if constexpr (sizeof(T) == 8) {
+    if (sh == 0) return (const void*)k_sytrd_panel<T, kShapes[0].cw, kShapes[0].nq>;
+    if (sh == 1) return (const void*)k_sytrd_panel<T, kShapes[1].cw, kShapes[1].nq>;
+    if (sh == 2) return (const void*)k_sytrd_panel<T, kShapes[2].cw, kShapes[2].nq>;
+  }
+  return (const void*)k_sytrd_panel<T, kShapes[3].cw, kShapes[3].nq>;
+}
+
 template <class T>
 cudaError_t sytrd_run(SytrdPlan& sp, T* A, long long lda, T* d, T* e, T* tau, cudaStream_t st) {
   const int n = sp.n;
@@ -524,8 +719,6 @@ cudaError_t sytrd_run(SytrdPlan& sp, T* A, long long lda, T* d, T* e, T* tau, cu
   a.qfp = (T*)sp.qfp;
   a.dots = (T*)sp.dots;
   a.nDCH = sp.nDCH;
-  a.ustart = sp.ustart;
-  a.nTC = sp.nTC;
   a.bar = sp.bar;
   a.err = sp.err;
   T* VW = (T*)sp.VW;
@@ -539,8 +732,11 @@ cudaError_t sytrd_run(SytrdPlan& sp, T* A, long long lda, T* d, T* e, T* tau, cu
     a.W = VW + (long long)nbp * n;
     a.bar_base = bar_base;
     bar_base += 2u * (unsigned)nbp * (unsigned)sp.G;  // barriers per launch: 1 + nbp + (nbp - 1)
+    const int sh = panel_shape(n - k0 - 1, sizeof(T) == 8);
+    a.nTC = (n + kShapes[sh].cw - 1) / kShapes[sh].cw;
+    a.ustart = sp.ustart + sp.uoff[sh];
     void* args[] = {(void*)&a};
-    err = cudaLaunchCooperativeKernel((const void*)k_sytrd_panel<T>, dim3(sp.G), dim3(kPT), args,
+    err = cudaLaunchCooperativeKernel(panel_kernel<T>(sh), dim3(sp.G), dim3(kPT), args,
                                       2 * (size_t)panel_rows(k0, n, sp.G) * kSytrdNB * sizeof(T), st);
     if (err != cudaSuccess) return err;
     const int t = k0 + nbp;
@@ -590,26 +786,35 @@ cudaError_t sytrd_plan_create(SytrdPlan** out, int n, bool f64, bool tc) {
   // is a property of the kernel, shared by every plan: always the largest
   // order's, so that a plan made later never lowers it below an earlier
   // plan's launches.
-  const void* kfn = f64 ? (const void*)k_sytrd_panel<double> : (const void*)k_sytrd_panel<float>;
-  const int vwbytes = 2 * panel_rows(0, kMaxTC * kTW, std::max(nsm, 1)) * kSytrdNB * (f64 ? 8 : 4);
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, vwbytes);
-  if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, kPT, vwbytes);
-  if (err == cudaSuccess && per < 1) err = cudaErrorCooperativeLaunchTooLarge;
+  const int vwbytes = 2 * panel_rows(0, kMaxOrder, std::max(nsm, 1)) * kSytrdNB * (f64 ? 8 : 4);
+  for (int sh = f64 ? 0 : kNumShapes - 1; sh < kNumShapes; sh++) {
+    const void* kfn = f64 ? panel_kernel<double>(sh) : panel_kernel<float>(sh);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, vwbytes);
+    if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, kPT, vwbytes);
+    if (err == cudaSuccess && per < 1) err = cudaErrorCooperativeLaunchTooLarge;
+  }
   if (err != cudaSuccess) {
     delete sp;
     return err;
   }
   sp->G = nsm;  // one CTA per SM (co-residency of a cooperative launch)
-  sp->nTC = (n + kTW - 1) / kTW;
-  sp->nCH = (n + kRC - 1) / kRC;
   sp->nDCH = (n + kDotRows - 1) / kDotRows;
-  std::vector<int> ustart(sp->nTC + 1);
-  int total = 0;
-  for (int J = 0; J < sp->nTC; J++) {
-    ustart[J] = total;
-    total += (n - J * kTW + kRC - 1) / kRC;  // chunks of tile column J
+  // unit tables of the shapes, and the partial buffers that hold any of them
+  std::vector<int> ustart;
+  size_t np = 0, nq = 0;
+  for (int sh = 0; sh < kNumShapes; sh++) {
+    const UnitShape& u = kShapes[sh];
+    const int ntc = (n + u.cw - 1) / u.cw, rc = 32 * u.nq, m = std::min(n, f64 || sh == kNumShapes - 1 ? u.max_m + 1 : 0);
+    sp->uoff[sh] = (int)ustart.size();
+    int total = 0;
+    for (int J = 0; J < ntc; J++) {
+      ustart.push_back(total);
+      total += (n - J * u.cw + rc - 1) / rc;  // chunks of tile column J
+    }
+    ustart.push_back(total);
+    np = std::max(np, (size_t)(m + u.cw - 1) / u.cw + 1);
+    nq = std::max(nq, (size_t)(m + u.cw + rc - 1) / rc + 1);
   }
-  ustart[sp->nTC] = total;
   std::vector<int> bk(4 * kSytrdNB);
   const int last = (n - 1) % kSytrdNB == 0 ? kSytrdNB : (n - 1) % kSytrdNB;
   for (int kk = 0; kk < 2 * kSytrdNB; kk++) bk[kk] = kk < kSytrdNB ? kSytrdNB + kk : kk - kSytrdNB;
@@ -619,8 +824,8 @@ cudaError_t sytrd_plan_create(SytrdPlan** out, int n, bool f64, bool tc) {
     if (err == cudaSuccess) err = cudaMalloc(p, std::max<size_t>(bytes, 16));
   };
   alloc((void**)&sp->ustart, sizeof(int) * ustart.size());
-  alloc(&sp->P, el * (size_t)sp->nTC * n);
-  alloc(&sp->Qp, el * (size_t)sp->nCH * n);
+  alloc(&sp->P, el * np * n);
+  alloc(&sp->Qp, el * nq * n);
   alloc(&sp->normp, el * sp->G);
   alloc(&sp->qfp, el * sp->G);
   alloc(&sp->dots, el * 3 * kSytrdNB * sp->nDCH);
