@@ -6,8 +6,8 @@
 //
 // Cuppen's splitting: T = diag(T1, T2) + rho u u' with u = e_p + sign(beta)
 // e_{p+1} at every split (beta = e[p], rho = |beta|, T1's last and T2's
-// first diagonal entries reduced by rho). Leaves (orders <= kLeafMax) are
-// solved by the batched small-matrix QL path. A merge of two solved halves
+// first diagonal entries reduced by rho). Leaves are solved by the batched
+// small-matrix path. A merge of two solved halves
 // Q1' T1 Q1 = D1, Q2' T2 Q2 = D2 is the rank-one problem D + rho z z' with
 // z = [last row of Q1; sign(beta) first row of Q2] / sqrt(2), rho = 2|beta|:
 //   1. sort D (merge of two ascending lists) and deflate: entries with
@@ -42,7 +42,12 @@
 
 namespace gla {
 
-constexpr int kLeafMax = 64;
+// Largest leaf: FP64 leaves go through the QL chase, whose time grows with
+// the square of the order (1.3 ms for leaves of 47, 0.15 ms for 16, and the
+// replay of their rotations with its cube) where a level of merges costs
+// about 0.1 ms; FP32 leaves mostly through the per-eigenvalue solver, one
+// launch of 20 us at 64.
+constexpr int kLeafMaxF64 = 16, kLeafMaxF32 = 64;
 constexpr int kPrepThreads = 1024;
 constexpr int kPrepChunk = 1024;
 
@@ -56,6 +61,49 @@ template <>
 struct dc_eps<float> {
   static constexpr float u = 0x1p-24f;
 };
+
+// 1/x and 1/sqrt(x) to about one unit in the last place: FP64 from a hardware
+// seed and one cubic step (3 and 4 instructions of 64 cycles, where the IEEE
+// division takes 9), FP32 from the hardware's division and square root.
+GLA_DEV double dc_rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+GLA_DEV float dc_rcp(float x) { return 1.f / x; }
+GLA_DEV double dc_sqrt(double x) {  // x >= 0
+  if (prec<double>::biased_exp(x) < 64) return sqrt(x);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = x * y;
+  const double e = fma(-h, y, 1.0);
+  return fma(h * e, fma(e, 0.375, 0.5), h);
+}
+GLA_DEV float dc_sqrt(float x) { return sqrtf(x); }
+
+// Four sums over the warp in six additions; every lane gets all of them.
+template <class T>
+GLA_DEV void dc_sum4(T (&v)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool u = lane & 16, w = lane & 8;
+  const T a = (u ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, u ? v[0] : v[2], 16);
+  const T b = (u ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, u ? v[1] : v[3], 16);
+  T x = (w ? b : a) + __shfl_xor_sync(0xffffffffu, w ? a : b, 8);
+  x += __shfl_xor_sync(0xffffffffu, x, 4);
+  x += __shfl_xor_sync(0xffffffffu, x, 2);
+  x += __shfl_xor_sync(0xffffffffu, x, 1);
+#pragma unroll
+  for (int k = 0; k < 4; k++) v[k] = __shfl_sync(0xffffffffu, x, 8 * k);
+}
+GLA_DEV bool sign_bit(double x) { return __double2hiint(x) < 0; }
+GLA_DEV bool sign_bit(float x) { return __float_as_int(x) < 0; }
+GLA_DEV unsigned long long abs_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+GLA_DEV unsigned long long abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+GLA_DEV void from_bits(unsigned long long b, double& x) { x = __longlong_as_double((long long)b); }
+GLA_DEV void from_bits(unsigned long long b, float& x) { x = __uint_as_float((unsigned)b); }
 
 struct MergeInfo {
   int o, m1, m2;
@@ -138,9 +186,11 @@ __global__ void __launch_bounds__(kPrepThreads) k_dc_prep(DcArrays<T> a) {
   const T sgn = beta < T(0) ? T(-1) : T(1);
   const T rho = T(2) * fabs(beta);
   const T rs2 = T(0.70710678118654752440);
-  __shared__ T sred[kPrepThreads / 32];
+  __shared__ unsigned long long sred[kPrepThreads / 32];
+  __shared__ int scnt[kPrepThreads / 32], sfirst;
+  const int lane = tid & 31, wid = tid >> 5;
   // z, merged order, max |D|
-  T dmax = T(0);
+  unsigned long long dbits = 0;
   for (int i = tid; i < m; i += kPrepThreads) {
     const T di = a.dd[o + i];
     T zi;
@@ -166,88 +216,121 @@ __global__ void __launch_bounds__(kPrepThreads) k_dc_prep(DcArrays<T> a) {
     a.sZ[o + rank] = zi;
     a.ssrc[o + rank] = i;
     a.ctype[o + i] = i < m1 ? 0 : 1;
-    dmax = fmax(dmax, fabs(di));
+    const unsigned long long bi = abs_bits(di);
+    dbits = bi > dbits ? bi : dbits;
   }
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, s));
-  if ((tid & 31) == 0) sred[tid >> 5] = dmax;
+  dbits = warp_max_u64(dbits);
+  if (lane == 0) sred[wid] = dbits;
+  if (tid == 0) sfirst = 0x7fffffff;
   __syncthreads();
-  dmax = T(0);
-  for (int i = 0; i < kPrepThreads / 32; i++) dmax = fmax(dmax, sred[i]);
+  dbits = warp_max_u64(sred[lane]);
+  T dmax;
+  from_bits(dbits, dmax);
   const T tol = T(8) * dc_eps<T>::u * fmax(dmax, rho);
-  for (int t = tid; t < m; t += kPrepThreads) a.zdef[o + t] = rho * fabs(a.sZ[o + t]) <= tol;
+  // entries that the size of z keeps, in order, and the others: thread t takes
+  // `per` consecutive ones
+  const int per = (m + kPrepThreads - 1) / kPrepThreads;
+  const int b0 = min(m, tid * per), b1 = min(m, b0 + per);
+  int cnt = 0;
+  for (int t = b0; t < b1; t++) {
+    const int z = rho * fabs(a.sZ[o + t]) <= tol;
+    a.zdef[o + t] = z;
+    cnt += !z;
+  }
+  int inc = cnt;  // inclusive scan over the block
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, d);
+    if (lane >= d) inc += v;
+  }
+  if (lane == 31) scnt[wid] = inc;
   __syncthreads();
-
-  // sequential pair deflation by thread 0 over chunks staged in shared memory
-  __shared__ T cD[kPrepChunk], cZ[kPrepChunk];
-  __shared__ int cS[kPrepChunk], cF[kPrepChunk];
-  int k = 0, nf = 0, nr = 0;
-  T Dp = T(0), zp = T(0);
-  int sp = -1;
-  for (int c0 = 0; c0 < m; c0 += kPrepChunk) {
-    const int cn = min(kPrepChunk, m - c0);
-    __syncthreads();
-    for (int t = tid; t < cn; t += kPrepThreads) {
-      cD[t] = a.sD[o + c0 + t];
-      cZ[t] = a.sZ[o + c0 + t];
-      cS[t] = a.ssrc[o + c0 + t];
-      cF[t] = a.zdef[o + c0 + t];
+  int before = lane < wid ? scnt[lane] : 0, nk = scnt[lane];
+  before = __reduce_add_sync(0xffffffffu, before) + inc - cnt;
+  nk = __reduce_add_sync(0xffffffffu, nk);
+  for (int t = b0; t < b1; t++) {
+    const T Dt = a.sD[o + t];
+    const int st = a.ssrc[o + t];
+    if (a.zdef[o + t]) {
+      a.fd[o + t - before] = Dt;
+      a.fsrc[o + t - before] = st;
+    } else {
+      a.kd[o + before] = Dt;
+      a.kz[o + before] = a.sZ[o + t];
+      a.ksrc[o + before] = st;
+      before++;
     }
-    __syncthreads();
-    if (tid == 0) {
-      for (int t = 0; t < cn; t++) {
-        const T Dt = cD[t], zt = cZ[t];
-        const int st = cS[t];
-        if (cF[t]) {
-          a.fd[o + nf] = Dt;
-          a.fsrc[o + nf] = st;
-          nf++;
-          continue;
-        }
-        if (sp < 0) {
-          Dp = Dt;
-          zp = zt;
-          sp = st;
-          continue;
-        }
-        const T r2 = zp * zp + zt * zt;
-        if (fabs(Dt - Dp) * fabs(zp * zt) <= tol * r2) {
-          const T r = sqrt(r2);
-          const T cs = zt / r, sn = zp / r;
-          a.rc[o + nr] = cs;
-          a.rs[o + nr] = sn;
-          a.rp[o + nr] = sp;
-          a.rt[o + nr] = st;
-          nr++;
-          if (a.ctype[o + sp] != a.ctype[o + st]) {
-            a.ctype[o + sp] = 2;
-            a.ctype[o + st] = 2;
+  }
+  __syncthreads();
+  // the first kept pair that deflates, all pairs side by side: up to it the
+  // kept list is final
+  auto deflates = [&](T D1, T z1, T D2, T z2) { return fabs(D2 - D1) * fabs(z1 * z2) <= tol * (z1 * z1 + z2 * z2); };
+  for (int t = tid; t + 1 < nk; t += kPrepThreads)
+    if (deflates(a.kd[o + t], a.kz[o + t], a.kd[o + t + 1], a.kz[o + t + 1])) {
+      atomicMin(&sfirst, t);
+      break;
+    }
+  __syncthreads();
+  const int first = sfirst;
+  int k = nk, nf = m - nk, nr = 0;
+  if (first < nk) {
+    // from there on pair by pair in thread 0, over chunks staged in shared memory
+    __shared__ T cD[kPrepChunk], cZ[kPrepChunk];
+    __shared__ int cS[kPrepChunk];
+    T Dp = a.kd[o + first], zp = a.kz[o + first];
+    int sp = a.ksrc[o + first];
+    k = first;
+    for (int c0 = first + 1; c0 < nk; c0 += kPrepChunk) {
+      const int cn = min(kPrepChunk, nk - c0);
+      __syncthreads();
+      for (int t = tid; t < cn; t += kPrepThreads) {
+        cD[t] = a.kd[o + c0 + t];
+        cZ[t] = a.kz[o + c0 + t];
+        cS[t] = a.ksrc[o + c0 + t];
+      }
+      __syncthreads();
+      if (tid == 0) {
+        for (int t = 0; t < cn; t++) {
+          const T Dt = cD[t], zt = cZ[t];
+          const int st = cS[t];
+          if (deflates(Dp, zp, Dt, zt)) {
+            const T r = sqrt(zp * zp + zt * zt);
+            const T cs = zt / r, sn = zp / r;
+            a.rc[o + nr] = cs;
+            a.rs[o + nr] = sn;
+            a.rp[o + nr] = sp;
+            a.rt[o + nr] = st;
+            nr++;
+            if (a.ctype[o + sp] != a.ctype[o + st]) {
+              a.ctype[o + sp] = 2;
+              a.ctype[o + st] = 2;
+            }
+            a.fd[o + nf] = cs * cs * Dp + sn * sn * Dt;
+            a.fsrc[o + nf] = sp;
+            nf++;
+            Dp = sn * sn * Dp + cs * cs * Dt;
+            zp = r;
+            sp = st;
+          } else {
+            a.kd[o + k] = Dp;
+            a.kz[o + k] = zp;
+            a.ksrc[o + k] = sp;
+            k++;
+            Dp = Dt;
+            zp = zt;
+            sp = st;
           }
-          a.fd[o + nf] = cs * cs * Dp + sn * sn * Dt;
-          a.fsrc[o + nf] = sp;
-          nf++;
-          Dp = sn * sn * Dp + cs * cs * Dt;
-          zp = r;
-          sp = st;
-        } else {
-          a.kd[o + k] = Dp;
-          a.kz[o + k] = zp;
-          a.ksrc[o + k] = sp;
-          k++;
-          Dp = Dt;
-          zp = zt;
-          sp = st;
         }
       }
     }
-  }
-  if (tid == 0) {
-    if (sp >= 0) {
+    if (tid == 0) {
       a.kd[o + k] = Dp;
       a.kz[o + k] = zp;
       a.ksrc[o + k] = sp;
       k++;
     }
+  }
+  if (tid == 0) {
     mi->k = k;
     mi->nf = nf;
     mi->nrot = nr;
@@ -294,108 +377,97 @@ __global__ void __launch_bounds__(256) k_dc_secular(DcArrays<T> a) {
     return;
   }
   const bool last = j == k - 1;
-  int og;
-  T lo, hi;
-  if (!last) {
-    const T mid = T(0.5) * (D[j] + D[j + 1]);
-    T f = T(0);
-    for (int i = lane; i < k; i += 32) f += Z[i] * Z[i] / (D[i] - mid);
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) f += __shfl_xor_sync(0xffffffffu, f, s);
-    f += irho;
-    if (f >= T(0)) {
-      og = j;
-      lo = T(0);
-      hi = mid - D[j];
-    } else {
-      og = j + 1;
-      lo = mid - D[j + 1];
-      hi = T(0);
-    }
-  } else {
-    og = j;
+  int og = j;
+  T lo = T(0), hi, tau;
+  if (last) {
     T z2 = T(0);
-    for (int i = lane; i < k; i += 32) z2 += Z[i] * Z[i];
+    for (int i = lane; i < k; i += 32) z2 = fma(Z[i], Z[i], z2);
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) z2 += __shfl_xor_sync(0xffffffffu, z2, s);
-    lo = T(0);
     hi = rho * z2 * (T(1) + T(4) * eps);
+    tau = T(0.5) * hi;
+  } else {
+    hi = T(0.5) * (D[j + 1] - D[j]);
+    tau = hi;  // the middle of the interval, which also tells the nearer pole
   }
-  const T Dorg = D[og];
-  const T dL = D[j] - Dorg;
-  const T dR = last ? T(0) : D[j + 1] - Dorg;
-  T tau = T(0.5) * (lo + hi);
+  T Dorg = D[j];
+  T dL = T(0), dR = last ? T(0) : D[j + 1] - Dorg;
   bool conv = false;
   for (int it = 0; it < 100; it++) {
-    T psi = T(0), dpsi = T(0), phi = T(0), dphi = T(0);
+    T v[4] = {T(0), T(0), T(0), T(0)};  // psi, psi', phi, phi'
     for (int i = lane; i < k; i += 32) {
-      const T del = (D[i] - Dorg) - tau;
-      const T t = Z[i] / del;
-      const T term = Z[i] * t, der = t * t;
+      const T z = Z[i];
+      const T t = z * dc_rcp((D[i] - Dorg) - tau);
       if (i <= j) {
-        psi += term;
-        dpsi += der;
+        v[0] = fma(z, t, v[0]);
+        v[1] = fma(t, t, v[1]);
       } else {
-        phi += term;
-        dphi += der;
+        v[2] = fma(z, t, v[2]);
+        v[3] = fma(t, t, v[3]);
       }
     }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-      psi += __shfl_xor_sync(0xffffffffu, psi, s);
-      dpsi += __shfl_xor_sync(0xffffffffu, dpsi, s);
-      phi += __shfl_xor_sync(0xffffffffu, phi, s);
-      dphi += __shfl_xor_sync(0xffffffffu, dphi, s);
+    dc_sum4(v);
+    const T psi = v[0], dpsi = v[1], phi = v[2], dphi = v[3];
+    const T g = (irho + psi) + phi;
+    const bool neg = sign_bit(g);
+    if (it == 0 && !last) {
+      if (neg) {  // the root lies in the upper half: origin at the upper pole
+        og = j + 1;
+        Dorg = D[og];
+        tau -= dR;
+        dL = -dR;
+        dR = T(0);
+        lo = tau;
+        hi = T(0);
+      }
+    } else if (neg) {
+      lo = tau;
+    } else {
+      hi = tau;
     }
-    const T g = irho + psi + phi;
-    const T gtol = eps * (irho + (T(8) + T(k) / T(16)) * (fabs(psi) + fabs(phi)) + T(2) * fabs(tau) * (dpsi + dphi));
-    if (fabs(g) <= gtol) {
+    const T gtol = eps * fma(T(2) * fabs(tau), dpsi + dphi, fma(T(8) + T(k) / T(16), fabs(psi) + fabs(phi), irho));
+    if (abs_bits(g) <= abs_bits(gtol)) {
       conv = true;
       break;
     }
-    if (g < T(0)) lo = tau; else hi = tau;
-    if (hi - lo <= T(4) * eps * fmax(fabs(lo), fabs(hi))) {
+    const T span = T(4) * eps * (abs_bits(lo) > abs_bits(hi) ? lo : hi);
+    if (abs_bits(hi - lo) <= abs_bits(span)) {
       conv = true;
       break;
     }
     const T DL = dL - tau;
-    T eta;
+    T tn = T(0);
     bool ok = false;
+    const unsigned long long klo = sort_key(lo), khi = sort_key(hi);
+    auto inside = [&](T x) { return sort_key(x) > klo && sort_key(x) < khi; };
     if (!last) {
+      // c + model of psi at the left pole, of phi at the right one: the root of
+      // c x^2 - qa x + qb nearest the current point
       const T DR = dR - tau;
-      const T c = g - DL * dpsi - DR * dphi;
-      const T qa = c * (DL + DR) + DL * DL * dpsi + DR * DR * dphi;
+      const T p1 = DL * dpsi, p2 = DR * dphi;
+      const T c = (g - p1) - p2;
+      const T qa = fma(c, DL + DR, fma(DL, p1, DR * p2));
       const T qb = DL * DR * g;
-      if (fabs(c) <= eps * fabs(qa)) {
-        if (qa != T(0)) {
-          eta = qb / qa;
-          ok = true;
-        }
-      } else {
-        T disc = qa * qa - T(4) * qb * c;
-        disc = disc > T(0) ? sqrt(disc) : T(0);
-        const T tq = qa >= T(0) ? T(0.5) * (qa + disc) : T(0.5) * (qa - disc);
-        const T e1 = tq / c;
-        const T e2 = tq != T(0) ? qb / tq : e1;
-        const bool in1 = e1 > DL && e1 < DR, in2 = e2 > DL && e2 < DR;
-        if (in1 != in2) {
-          eta = in1 ? e1 : e2;
-          ok = true;
-        } else if (in1) {
-          eta = fabs(e1) < fabs(e2) ? e1 : e2;
-          ok = true;
-        }
+      T disc = fma(qa, qa, T(-4) * qb * c);
+      disc = sign_bit(disc) ? T(0) : dc_sqrt(disc);
+      if (sign_bit(qa) || qa == T(0))
+        tn = tau + (qa - disc) * dc_rcp(T(2) * c);
+      else
+        tn = tau + T(2) * qb * dc_rcp(qa + disc);
+      ok = inside(tn);
+      if (!ok) {  // the other root
+        tn = tau + (sign_bit(qa) ? T(2) * qb * dc_rcp(qa - disc) : (qa + disc) * dc_rcp(T(2) * c));
+        ok = inside(tn);
       }
     } else {
-      const T c = g - DL * dpsi;
+      const T p1 = DL * dpsi, c = g - p1;
       if (c > T(0)) {
-        eta = DL + DL * DL * dpsi / c;
-        ok = true;
+        tn = tau + fma(DL * p1, dc_rcp(c), DL);
+        ok = inside(tn);
       }
     }
-    T tn = ok ? tau + eta : T(0.5) * (lo + hi);
-    if (!(tn > lo && tn < hi)) tn = T(0.5) * (lo + hi);
-    const bool small_step = fabs(tn - tau) <= T(2) * eps * fabs(tau);
+    if (!ok) tn = T(0.5) * (lo + hi);
+    const bool small_step = abs_bits(tn - tau) <= abs_bits(T(2) * eps * tau);
     tau = tn;
     if (small_step) {
       conv = true;
@@ -429,7 +501,7 @@ __global__ void __launch_bounds__(256) k_dc_zhat(DcArrays<T> a) {
       den = rho;
     else
       den = j < i ? D[j] - Di : D[j + 1] - Di;
-    prod *= num / den;
+    prod *= num * dc_rcp(den);
   }
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) prod *= __shfl_xor_sync(0xffffffffu, prod, s);
@@ -453,7 +525,7 @@ __global__ void __launch_bounds__(256) k_dc_vec(DcArrays<T> a) {
   __shared__ T sred[8];
   T ss = T(0);
   for (int i = threadIdx.x; i < k; i += 256) {
-    const T u = a.zh[o + i] / ((D[i] - Dorg) - tau);
+    const T u = a.zh[o + i] * dc_rcp((D[i] - Dorg) - tau);
     U[i] = u;
     ss = fma(u, u, ss);
   }
@@ -793,7 +865,8 @@ int dc_plan_create(DcPlan** out, int n, bool f64, bool bisect_leaves) {
   std::vector<std::vector<MergeInfo>> by_depth;
   std::vector<int> leaf_o, leaf_m, splits;
   int depth = 0;
-  while ((n + (1 << depth) - 1) >> depth > kLeafMax) depth++;
+  const int leaf_max = f64 ? kLeafMaxF64 : kLeafMaxF32;
+  while ((n + (1 << depth) - 1) >> depth > leaf_max) depth++;
   build_tree(0, n, 0, depth, by_depth, leaf_o, leaf_m, splits);
   // levels bottom-up (deepest merges first)
   for (int dpt = (int)by_depth.size() - 1; dpt >= 0; dpt--) {
