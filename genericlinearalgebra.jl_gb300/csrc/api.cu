@@ -795,6 +795,16 @@ int plan_execute(gla_plan_t p, const void* A, void* w, void* V, int* info, cudaS
         GLA_CUDA(cudaMemcpyAsync(p->pin_pending + b, p->d_pending + b, sizeof(int), cudaMemcpyDeviceToHost, s));
     } else {
       p->mark(b, GLA_PHASE_CHASE, 0, s);
+      if (work_t == kF32 && p->tol == kTolF32) {
+        // the default tolerance: every eigenvalue by bisection, to the last
+        // bit; another tolerance is a deflation threshold and keeps the chase
+        GLA_CUDA(launch_bisect_values(bk.count, bk.nmax, s, p->d_desc, p->d_perm_bucket + bk.start, p->d_d, p->d_e, w,
+                                      info));
+        p->mark(b, GLA_PHASE_CHASE, 1, s);
+        GLA_CUDA(cudaEventRecord(bk.join, s));
+        GLA_CUDA(cudaStreamWaitEvent(st, bk.join, 0));
+        continue;
+      }
       GLA_CUDA(launch_chase(work_t, kAlgoPWK, bk.count, chase_smem_bytes(bk.nmax, el), s, p->d_desc,
                             p->d_perm_bucket + bk.start, p->d_d, p->d_e, p->d_cst, nullptr, nullptr, info, p->tol,
                             kMaxSweepsPerN, p->d_pending + b, p->d_stats, bk.lpw));

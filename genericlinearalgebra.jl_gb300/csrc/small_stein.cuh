@@ -97,6 +97,31 @@ GLA_DEV float eig_bisect(int n, const float* d, const float* e2, int k, float lo
   return 0.5f * (lo + hi);
 }
 
+// The same to the last bit: until no float lies between lo and hi, then hi,
+// the smallest x with more than k eigenvalues below or at it (an eigenvalue
+// that splits off exactly comes back exactly).
+GLA_DEV float eig_bisect_full(int n, const float* d, const float* e2, int k, float lo, float hi, float pivmin) {
+  for (int it = 0; it < 160; it++) {
+    const float x1 = 0.5f * (lo + hi);
+    if (!(x1 > lo && x1 < hi)) break;
+    const float x0 = 0.5f * (lo + x1), x2 = 0.5f * (x1 + hi);  // (may round to an end: then unused)
+    int c0, c1, c2;
+    sturm3(n, d, e2, x0, x1, x2, pivmin, c0, c1, c2);
+    if (c1 > k) {
+      hi = x1;
+      if (x0 > lo && x0 < hi) {
+        if (c0 > k) hi = x0; else lo = x0;
+      }
+    } else {
+      lo = x1;
+      if (x2 > lo && x2 < hi) {
+        if (c2 > k) hi = x2; else lo = x2;
+      }
+    }
+  }
+  return hi;
+}
+
 // Eigenvector of eigenvalue lam by the twisted factorisation, written to
 // column k of Y (Y[i * ldy + k], row i). Returns false when the vector is
 // not finite. e: off-diagonal, e2 = e^2.

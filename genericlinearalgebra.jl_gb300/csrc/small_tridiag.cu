@@ -100,6 +100,73 @@ cudaError_t launch_stein_tri(int nblocks, int nmax, cudaStream_t st, const Small
   return cudaGetLastError();
 }
 
+// Eigenvalues of FP32 matrices (jobz 'N'): one CTA per matrix, one thread per
+// eigenvalue, bisection on Sturm counts of (d, e) scaled by an exact power of
+// two, to the last bit, in place of the root-free chase and the sort. That
+// chase is one serial recurrence of about n^2 steps per matrix (550 cycles
+// each: 5.1 ms for 1000 matrices of orders 8 .. 128 with everything beside
+// it), bisection 15 to 20 passes of n steps for all eigenvalues at once.
+__global__ void __launch_bounds__(128) k_bisect_values(const SmallDesc* __restrict__ descs,
+                                                       const int* __restrict__ perm, const float* __restrict__ dg_all,
+                                                       const float* __restrict__ eg_all, float* __restrict__ wout,
+                                                       const int* __restrict__ info) {
+  __shared__ float dd[kSmallMaxN], e2[kSmallMaxN], red[3][4];
+  const int mid = perm[blockIdx.x];
+  const SmallDesc dsc = descs[mid];
+  const int n = dsc.n, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+  if (info[mid] == -1) {
+    if (tid < n) wout[dsc.w_off + tid] = NAN;
+    return;
+  }
+  const float d = tid < n ? dg_all[dsc.w_off + tid] : 0.f;
+  const float e = tid + 1 < n ? eg_all[dsc.w_off + tid] : 0.f;
+  float m = fmaxf(fabsf(d), fabsf(e));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) red[0][wid] = m;
+  __syncthreads();
+  for (int w = 0; w < nw; w++) m = fmaxf(m, red[0][w]);
+  const int ex = m > 0.f ? ilogbf(m) : 0;
+  const float ds = ldexpf(d, -ex), es = ldexpf(e, -ex);
+  if (tid < n) {
+    dd[tid] = ds;
+    e2[tid] = es * es;
+  }
+  // Gershgorin interval: |e| of the entry before through the warp and, at its edge, shared memory
+  __syncthreads();
+  const float ep = tid > 0 && tid < n ? sqrtf(e2[tid - 1]) : 0.f;
+  const float ai = (fabsf(es) + ep) * 1.0001f;
+  float lo = tid < n ? ds - ai : 3.0e38f, hi = tid < n ? ds + ai : -3.0e38f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (lane == 0) {
+    red[1][wid] = lo;
+    red[2][wid] = hi;
+  }
+  __syncthreads();
+  for (int w = 0; w < nw; w++) {
+    lo = fminf(lo, red[1][w]);
+    hi = fmaxf(hi, red[2][w]);
+  }
+  const float pivmin = 0x1p-120f;
+  const float widen = 2.f * (float)n * prec<float>::eps * fmaxf(fabsf(lo), fabsf(hi)) + 2.f * pivmin;
+  if (tid < n) {
+    const float x = eig_bisect_full(n, dd, e2, tid, lo - widen, hi + widen, pivmin);
+    wout[dsc.w_off + tid] = fabsf(x) <= 4.f * pivmin ? 0.f : ldexpf(x, ex);
+  }
+}
+
+cudaError_t launch_bisect_values(int nblocks, int nmax, cudaStream_t st, const SmallDesc* descs, const int* perm,
+                                 const void* d, const void* e, void* w, const int* info) {
+  if (nblocks <= 0) return cudaSuccess;
+  const int nt = std::max(32, (nmax + 31) / 32 * 32);
+  k_bisect_values<<<nblocks, nt, 0, st>>>(descs, perm, (const float*)d, (const float*)e, (float*)w, info);
+  return cudaGetLastError();
+}
+
 template <class T, class Tin, bool Q, bool ST = false> static void set_tri_attr() {
   cudaFuncSetAttribute(k_tridiag<T, Tin, Q, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)tridiag_smem_bytes(kSmallMaxN, 256, sizeof(T), ST));
