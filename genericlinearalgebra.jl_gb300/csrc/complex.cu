@@ -159,69 +159,66 @@ __global__ void __launch_bounds__(256) k_zgroup(const double* __restrict__ E, in
   }
 }
 
-// X = re V, Y = im V (V interleaved, leading dimension ldv; X, Y n x n, ld n)
-__global__ void k_zsplit(const double* __restrict__ V, long long ldv, int n, double* __restrict__ X,
-                         double* __restrict__ Y) {
+// S = [X Y; Y -X] (2n x 2n, leading dimension 2n), X = re V, Y = im V (V
+// interleaved, leading dimension ldv).
+__global__ void k_zstack(const double* __restrict__ V, long long ldv, int n, double* __restrict__ S) {
   const int j = blockIdx.y;
+  const long long n2 = 2LL * n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    X[i + (long long)j * n] = V[2 * (i + j * ldv)];
-    Y[i + (long long)j * n] = V[2 * (i + j * ldv) + 1];
+    const double x = V[2 * (i + j * ldv)], y = V[2 * (i + j * ldv) + 1];
+    S[i + j * n2] = x;
+    S[n + i + j * n2] = y;
+    S[i + (n + j) * n2] = y;
+    S[n + i + (n + j) * n2] = -x;
   }
 }
-__global__ void k_zmerge(const double* __restrict__ X, const double* __restrict__ Y, int n, double* __restrict__ V,
-                         long long ldv) {
+// XY = [X Y] (n x 2n)
+__global__ void k_zsplit(const double* __restrict__ V, long long ldv, int n, double* __restrict__ XY) {
   const int j = blockIdx.y;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    V[2 * (i + j * ldv)] = X[i + (long long)j * n];
-    V[2 * (i + j * ldv) + 1] = Y[i + (long long)j * n];
+    XY[i + (long long)j * n] = V[2 * (i + j * ldv)];
+    XY[i + (long long)(n + j) * n] = V[2 * (i + j * ldv) + 1];
   }
 }
-// R = I - V^H V from P = re(V^H V), Q = im(V^H V): Rr = I - P, Ri = -Q (in place)
-__global__ void k_zresid(int n, double* __restrict__ P, double* __restrict__ Q) {
+__global__ void k_zmerge(const double* __restrict__ XY, int n, double* __restrict__ V, long long ldv) {
   const int j = blockIdx.y;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const long long idx = i + (long long)j * n;
-    P[idx] = (i == j ? 1.0 : 0.0) - P[idx];
-    Q[idx] = -Q[idx];
+    V[2 * (i + j * ldv)] = XY[i + (long long)j * n];
+    V[2 * (i + j * ldv) + 1] = XY[i + (long long)(n + j) * n];
+  }
+}
+// From PQ = [re(V^H V), im(V^H V)] (n x 2n) the halves of R = I - V^H V as
+// the right operand of [X Y] (2n x 2n): [Rr Ri; -Ri Rr] / 2.
+__global__ void k_zresid(int n, const double* __restrict__ PQ, double* __restrict__ R) {
+  const int j = blockIdx.y;
+  const long long n2 = 2LL * n;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double rr = 0.5 * ((i == j ? 1.0 : 0.0) - PQ[i + (long long)j * n]);
+    const double ri = -0.5 * PQ[i + (long long)(n + j) * n];
+    R[i + j * n2] = rr;
+    R[n + i + j * n2] = -ri;
+    R[i + (n + j) * n2] = ri;
+    R[n + i + (n + j) * n2] = rr;
   }
 }
 
-// One Newton-Schulz step on V (n x n complex, interleaved), with six n x n
-// real work arrays in W.
-int z_orthonormalise(double* V, long long ldv, int n, double* W, cudaStream_t st) {
+// One Newton-Schulz step V (I + R/2) on V (n x n complex, interleaved), as
+// two real products with everything stacked (8 n^2 doubles of work in W):
+// V^H V = [X; Y]' [X Y; Y -X] and [X Y] [Rr Ri; -Ri Rr] / 2.
+int z_orthonormalise(double* V, long long ldv, int n, double* W, gla::Oz64Gemm** oz, cudaStream_t st) {
   const long long nn = (long long)n * n;
-  double *X = W, *Y = W + nn, *P = W + 2 * nn, *Q = W + 3 * nn, *X2 = W + 4 * nn, *Y2 = W + 5 * nn;
+  double *S = W, *PQ = W + 4 * nn, *XY = W + 6 * nn;
+  const int n2 = 2 * n;
   const dim3 g2((n + 255) / 256, n);
-  k_zsplit<<<g2, 256, 0, st>>>(V, ldv, n, X, Y);
+  k_zstack<<<g2, 256, 0, st>>>(V, ldv, n, S);
   Z_CUDA(cudaGetLastError());
-  auto gemm = [&](bool ta, const double* A, const double* B, double* C, double alpha, double beta) {
-    gla::GemmDesc g{};
-    g.m = g.n = g.k = n;
-    g.A = A;
-    g.lda = n;
-    g.B = B;
-    g.ldb = n;
-    g.C = C;
-    g.ldc = n;
-    g.alpha = alpha;
-    g.beta = beta;
-    return gla::gemm_launch(true, ta, false, false, g, 1, st);
-  };
-  // V^H V = (X'X + Y'Y) + i (X'Y - Y'X)
-  Z_CUDA(gemm(true, X, X, P, 1.0, 0.0));
-  Z_CUDA(gemm(true, Y, Y, P, 1.0, 1.0));
-  Z_CUDA(gemm(true, X, Y, Q, 1.0, 0.0));
-  Z_CUDA(gemm(true, Y, X, Q, -1.0, 1.0));
-  k_zresid<<<g2, 256, 0, st>>>(n, P, Q);
+  Z_CUDA(gla::oz64_gemm(oz, true, n, n2, n2, S, n2, S, n2, PQ, n, false, st));
+  k_zresid<<<g2, 256, 0, st>>>(n, PQ, S);
+  k_zsplit<<<g2, 256, 0, st>>>(V, ldv, n, XY);
   Z_CUDA(cudaGetLastError());
-  // V (I + R/2): X2 = X + (X Rr - Y Ri)/2, Y2 = Y + (X Ri + Y Rr)/2
-  Z_CUDA(cudaMemcpyAsync(X2, X, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
-  Z_CUDA(cudaMemcpyAsync(Y2, Y, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
-  Z_CUDA(gemm(false, X, P, X2, 0.5, 1.0));
-  Z_CUDA(gemm(false, Y, Q, X2, -0.5, 1.0));
-  Z_CUDA(gemm(false, X, Q, Y2, 0.5, 1.0));
-  Z_CUDA(gemm(false, Y, P, Y2, 0.5, 1.0));
-  k_zmerge<<<g2, 256, 0, st>>>(X2, Y2, n, V, ldv);
+  Z_CUDA(cudaMemcpyAsync(PQ, XY, sizeof(double) * 2 * nn, cudaMemcpyDeviceToDevice, st));
+  Z_CUDA(gla::oz64_gemm(oz, false, n, n2, n2, PQ, n, S, n2, XY, n, true, st));
+  k_zmerge<<<g2, 256, 0, st>>>(XY, n, V, ldv);
   Z_CUDA(cudaGetLastError());
   return 0;
 }
@@ -231,6 +228,7 @@ struct ZWork {
   double* w2 = nullptr;
   double* scratch = nullptr;
   int* idx = nullptr;
+  gla::Oz64Gemm* oz = nullptr;
   size_t cap_E = 0, cap_w2 = 0, cap_scratch = 0, cap_idx = 0;
 };
 std::mutex g_z_mu;
@@ -257,6 +255,7 @@ void release_complex_cache() {
   cudaFree(g_z.w2);
   cudaFree(g_z.scratch);
   cudaFree(g_z.idx);
+  oz64_gemm_release(&g_z.oz);
   g_z = ZWork();
 }
 }  // namespace gla
@@ -280,7 +279,7 @@ int gla_zheev(char jobz, char uplo, int64_t n, const double* A, int64_t lda, dou
   std::lock_guard<std::mutex> lk(g_z_mu);
   const int nn = (int)n, n2 = 2 * nn;
   Z_CUDA(cudaStreamSynchronize(st));  // the buffers may be reallocated
-  Z_CUDA(grow(&g_z.E, &g_z.cap_E, (size_t)6 * nn * nn));  // E (4 n^2), later the 6 n^2 work arrays
+  Z_CUDA(grow(&g_z.E, &g_z.cap_E, (size_t)8 * nn * nn));  // E (4 n^2), later the 8 n^2 work arrays
   Z_CUDA(grow(&g_z.w2, &g_z.cap_w2, (size_t)n2));
   k_zembed<<<dim3((nn + 255) / 256, nn), 256, 0, st>>>(A, lda, nn, uplo == 'L', g_z.E);
   Z_CUDA(cudaGetLastError());
@@ -343,10 +342,10 @@ int gla_zheev(char jobz, char uplo, int64_t n, const double* A, int64_t lda, dou
                                    ldv, g_z.scratch);
       Z_CUDA(cudaGetLastError());
     }
-    // E's real eigenvectors are consumed (stream order); its 6 n^2 doubles
+    // E's real eigenvectors are consumed (stream order); its 8 n^2 doubles
     // hold the work arrays of the orthonormalisation step
     if (nn > 1) {
-      int rc2 = z_orthonormalise(V, ldv, nn, g_z.E, st);
+      int rc2 = z_orthonormalise(V, ldv, nn, g_z.E, &g_z.oz, st);
       if (rc2) return rc2;
     }
   }

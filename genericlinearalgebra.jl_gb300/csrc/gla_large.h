@@ -88,6 +88,17 @@ cudaError_t oz64_grouped(Oz64* w, const GemmDesc* d, int nprob, int m1max, int m
 cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Z, long long ldz, int ncol, bool trans,
                         cudaStream_t st);
 
+// C = op(A) B (+ C when add), FP64, column-major, m x n x k: on the tensor
+// cores when every extent reaches kOz64MinGemm, by the SIMT GEMM below that
+// (there the slicing and launches cost more than the product). *w, made by
+// the first call, holds the operand buffers, which grow; calls that share it
+// run on one stream after another. Should a bounded wait run out, C is NaN.
+struct Oz64Gemm;
+constexpr int kOz64MinGemm = 128;
+cudaError_t oz64_gemm(Oz64Gemm** w, bool ta, int m, int n, int k, const double* A, long long lda, const double* B,
+                      long long ldb, double* C, long long ldc, bool add, cudaStream_t st);
+void oz64_gemm_release(Oz64Gemm** w);
+
 // ---- adjoint of one large eigen-decomposition (large_adjoint.cu):
 // Abar = V (diag(wbar) + sym(F o (V' Vbar))) V' for orders up to nmax of
 // the context (its tensor-core slice buffers and float-pair planes,

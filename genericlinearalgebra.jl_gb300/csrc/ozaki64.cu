@@ -315,4 +315,96 @@ cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Zall, lon
   return cudaSuccess;
 }
 
+
+// ---- a single product of any shape, with operand buffers that grow
+struct Oz64Gemm {
+  unsigned char* buf = nullptr;
+  int* words = nullptr;
+  size_t bytes = 0, nwords = 0;
+  int* err = nullptr;
+};
+
+namespace {
+template <class P>
+cudaError_t grow(P** p, size_t* cap, size_t need, size_t unit) {
+  if (*cap >= need) return cudaSuccess;
+  cudaFree(*p);
+  *p = nullptr;
+  *cap = 0;
+  cudaError_t e = cudaMalloc((void**)p, unit * need);
+  if (e == cudaSuccess) *cap = need;
+  return e;
+}
+}  // namespace
+
+void oz64_gemm_release(Oz64Gemm** w) {
+  if (!*w) return;
+  cudaFree((*w)->buf);
+  cudaFree((*w)->words);
+  cudaFree((*w)->err);
+  delete *w;
+  *w = nullptr;
+}
+
+cudaError_t oz64_gemm(Oz64Gemm** wp, bool ta, int m, int n, int k, const double* A, long long lda, const double* B,
+                      long long ldb, double* C, long long ldc, bool add, cudaStream_t st) {
+  if (m <= 0 || n <= 0) return cudaSuccess;
+  if (m < kOz64MinGemm || n < kOz64MinGemm || k < kOz64MinGemm) {
+    GemmDesc g{};
+    g.m = m;
+    g.n = n;
+    g.k = k;
+    g.A = A;
+    g.lda = lda;
+    g.B = B;
+    g.ldb = ldb;
+    g.C = C;
+    g.ldc = ldc;
+    g.alpha = 1.0;
+    g.beta = add ? 1.0 : 0.0;
+    return gemm_launch(true, ta, false, false, g, 1, st);
+  }
+  cudaError_t e;
+  if (!*wp) {
+    Oz64Gemm* w = new (std::nothrow) Oz64Gemm();
+    if (!w) return cudaErrorMemoryAllocation;
+    e = cudaMalloc((void**)&w->err, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(w->err, 0, sizeof(int));
+    if (e == cudaSuccess) e = set_attributes();
+    if (e != cudaSuccess) {
+      oz64_gemm_release(&w);
+      return e;
+    }
+    *wp = w;
+  }
+  Oz64Gemm* w = *wp;
+  const int ba = blocks(m), bb = blocks(n), ks = slabs(k);
+  if ((e = grow(&w->buf, &w->bytes, (size_t)(ba + bb) * ks * kSlab, 1)) != cudaSuccess) return e;
+  if ((e = grow(&w->words, &w->nwords, 2 * (size_t)(ba + bb) * kBM, sizeof(int))) != cudaSuccess) return e;
+  Operand a{w->buf, w->words, (unsigned*)(w->words + ba * kBM)};
+  Operand b{w->buf + (size_t)ba * ks * kSlab, w->words + 2 * ba * kBM, (unsigned*)(w->words + (2 * ba + bb) * kBM)};
+  Source sa{A, lda, m, k, nullptr}, sb{B, ldb, n, k, nullptr};
+  if (ta) {
+    k_max_cols<<<ba * kBM / 8, 256, 0, st>>>(sa, ba * kBM, a.mx);
+    k_tile<false><<<dim3(ba, ks), 256, kSlab, st>>>(sa, a);
+  } else {
+    if ((e = cudaMemsetAsync(a.mx, 0, sizeof(unsigned) * ba * kBM, st)) != cudaSuccess) return e;
+    k_max_rows<<<dim3((m + 255) / 256, (k + 63) / 64), 256, 0, st>>>(sa, a.mx);
+    k_tile<true><<<dim3(ba, ks), 256, kSlab, st>>>(sa, a);
+  }
+  k_max_cols<<<bb * kBM / 8, 256, 0, st>>>(sb, bb * kBM, b.mx);
+  k_tile<false><<<dim3(bb, ks), 256, kSlab, st>>>(sb, b);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  Args g{};
+  g.seg[0] = Seg{a.base, b.base, a.exps, b.exps, ks, ks, ks};
+  g.M = m;
+  g.N = n;
+  g.C = C;
+  g.ldc = ldc;
+  g.add = add ? 1 : 0;
+  g.err = w->err;
+  k_gemm<1><<<tiles(m, n), kThreads, kSmem, st>>>(g);
+  return cudaGetLastError();
+}
+
 }  // namespace gla

@@ -230,7 +230,7 @@ __global__ void k_qlmat(const double* __restrict__ Cc, int n, double* __restrict
       for (int c = 0; c < 4; c++) Lv[(r * n + i) + (long long)(c * n + j) * n4] = lsign(r, c) * a[r ^ c];
   }
 }
-// G = [M0; M1; M2; M3] -> R = I - M in place
+// G = [M0; M1; M2; M3] -> R / 2 = (I - M) / 2 in place
 __global__ void k_qresid(int n, double* __restrict__ G) {
   const int j = blockIdx.y;
   const long long n4 = 4LL * n;
@@ -238,12 +238,12 @@ __global__ void k_qresid(int n, double* __restrict__ G) {
 #pragma unroll
     for (int m = 0; m < 4; m++) {
       const long long idx = (m * n + i) + j * n4;
-      G[idx] = (m == 0 && i == j ? 1.0 : 0.0) - G[idx];
+      G[idx] = 0.5 * ((m == 0 && i == j ? 1.0 : 0.0) - G[idx]);
     }
 }
 
 // One Newton-Schulz step on V (n x n quaternions); W holds 28 n^2 doubles.
-int q_orthonormalise(double* V, long long ldv, int n, double* W, cudaStream_t st) {
+int q_orthonormalise(double* V, long long ldv, int n, double* W, gla::Oz64Gemm** oz, cudaStream_t st) {
   const long long nn = (long long)n * n, n4 = 4LL * n;
   double *Lv = W, *Cc = W + 16 * nn, *G = W + 20 * nn, *Out = W + 24 * nn;
   const dim3 g2((n + 255) / 256, n);
@@ -251,27 +251,12 @@ int q_orthonormalise(double* V, long long ldv, int n, double* W, cudaStream_t st
   Q_CUDA(cudaGetLastError());
   k_qlmat<<<g2, 256, 0, st>>>(Cc, n, Lv);
   Q_CUDA(cudaGetLastError());
-  gla::GemmDesc g{};
-  g.m = (int)n4;
-  g.n = n;
-  g.k = (int)n4;
-  g.A = Lv;
-  g.lda = n4;
-  g.B = Cc;
-  g.ldb = n4;
-  g.C = G;
-  g.ldc = n4;
-  g.alpha = 1.0;
-  g.beta = 0.0;
-  Q_CUDA(gla::gemm_launch(true, true, false, false, g, 1, st));  // G = L(V)' Cc
+  const int m4 = (int)n4;
+  Q_CUDA(gla::oz64_gemm(oz, true, m4, n, m4, Lv, n4, Cc, n4, G, n4, false, st));  // G = L(V)' Cc
   k_qresid<<<g2, 256, 0, st>>>(n, G);
   Q_CUDA(cudaGetLastError());
   Q_CUDA(cudaMemcpyAsync(Out, Cc, sizeof(double) * 4 * nn, cudaMemcpyDeviceToDevice, st));
-  g.B = G;
-  g.C = Out;
-  g.alpha = 0.5;
-  g.beta = 1.0;
-  Q_CUDA(gla::gemm_launch(true, false, false, false, g, 1, st));  // Out = Cc + L(V) R / 2
+  Q_CUDA(gla::oz64_gemm(oz, false, m4, n, m4, Lv, n4, G, n4, Out, n4, true, st));  // Out = Cc + L(V) R / 2
   k_qmerge<<<g2, 256, 0, st>>>(Out, n, V, ldv);
   Q_CUDA(cudaGetLastError());
   return 0;
@@ -282,6 +267,7 @@ struct QWork {
   double* w4 = nullptr;
   double* scratch = nullptr;
   int* idx = nullptr;
+  gla::Oz64Gemm* oz = nullptr;
   size_t cap_E = 0, cap_w4 = 0, cap_scratch = 0, cap_idx = 0;
 };
 std::mutex g_qh_mu;
@@ -322,6 +308,7 @@ void release_quaternion_cache() {
   cudaFree(g_qh.w4);
   cudaFree(g_qh.scratch);
   cudaFree(g_qh.idx);
+  oz64_gemm_release(&g_qh.oz);
   g_qh = QWork();
 }
 }  // namespace gla
@@ -409,7 +396,7 @@ int gla_qheev(char jobz, char uplo, int64_t n, const double* A, int64_t lda, dou
     // L(A)'s real eigenvectors are consumed (stream order); its buffer holds
     // the work arrays of the orthonormalisation step
     if (nn > 1) {
-      const int rc2 = q_orthonormalise(V, ldv, nn, g_qh.E, st);
+      const int rc2 = q_orthonormalise(V, ldv, nn, g_qh.E, &g_qh.oz, st);
       if (rc2) return rc2;
     }
   }

@@ -64,3 +64,24 @@ def test_eigenq_products(G, n, cols):
     kept = [j for j in range(cols) if j not in lost]
     assert not np.isfinite(Y[1:, lost]).any()
     assert np.array_equal(Y[:, kept], X[:, kept])
+
+
+@pytest.mark.parametrize("n", [127, 128, 129, 200])
+def test_complex_and_quaternion_orthonormalisation(G, n):
+    # the Newton-Schulz step's products change from the FP64 pipe to the
+    # tensor cores at order 128
+    from helpers import qherm_random, qmul, qH, qeye, qnorm
+    rng = np.random.default_rng(n)
+    B = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    A = (B + B.conj().T) / 2
+    r = G.eigen(A)
+    nA = np.linalg.norm(A, 2)
+    assert np.abs(r.values - np.linalg.eigvalsh(A)).max() <= 16 * n * EPS64 * nA
+    assert np.linalg.norm(A @ r.vectors - r.vectors * r.values, 2) <= 1e-13 * nA
+    assert np.linalg.norm(r.vectors.conj().T @ r.vectors - np.eye(n), 2) <= 1e-13
+    m = n // 2 if n < 200 else n
+    A = qherm_random(m, rng)
+    r = G.eigen(G.QuaternionMatrix(A))
+    V, nA = r.vectors, qnorm(A)
+    assert qnorm(qmul(A, V) - V * r.values[None, :, None]) <= 1e-13 * nA
+    assert qnorm(qmul(qH(V), V) - qeye(m)) <= 1e-13
