@@ -16,12 +16,15 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstdio>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <new>
 #include <numeric>
+#include <thread>
 #include <tuple>
 #include <vector>
 
@@ -50,6 +53,7 @@ constexpr int kAsyncPasses = 2;     // chase passes enqueued without a host chec
 constexpr int kGraphPasses = 4;     // chase passes of a capture-safe (GLA_FLAG_GRAPH) execute
 constexpr int kMaxBuckets = 8;      // size buckets of width 16 over (0, 128]
 constexpr int kMaxChunks = 4;       // host-execute pipeline: chunks of the batch
+constexpr int kMaxSide = 8;         // large matrices solved side by side
 
 #define GLA_CUDA(x)                                  \
   do {                                               \
@@ -138,8 +142,22 @@ struct gla_plan_s {
   LargeAdjoint* adj_large = nullptr;  // adjoint context of the orders above GLA_MAX_SMALL_N
   // orders above GLA_MAX_SMALL_N: solved one at a time by the large path
   std::vector<int> large_idx;           // batch indices, in batch order
-  std::map<int, LargeCtx*> large_ctx;   // one context per distinct order
-  std::map<int, RefineLarge*> large_ref;  // F32_REFINED: refinement per distinct order
+  std::vector<int> large_chain;         // the chain each of them belongs to
+  // A chain is a context (and, for F32_REFINED, the refinement) of one order
+  // and the matrices it solves one after another. Chains of orders up to
+  // kSideBySideMaxN, when there are several, run side by side, each on a
+  // stream and a host thread of its own: one such matrix keeps a tenth of the
+  // GPU busy. An order has as many chains then as it has matrices, at most
+  // kMaxSide; otherwise one.
+  struct LargeChain {
+    int n = 0;
+    bool side = false;
+    LargeCtx* ctx = nullptr;
+    RefineLarge* ref = nullptr;
+    std::vector<int> items;  // positions in large_idx
+  };
+  std::vector<LargeChain> chains;       // the ones that run side by side first, largest orders first
+  std::vector<cudaStream_t> side_streams;
   int large_iters = 0;                  // refinement iterations of the last execute (max)
   double large_refine_n3 = 0;           // sum over large matrices of iterations * n^3
   float large_refine_ms = 0.f;          // host-timed refinement of the last execute
@@ -186,6 +204,7 @@ struct gla_plan_s {
 
 namespace {
 int autotune_plan(gla_plan_t p, int base_flags);
+int make_chains(gla_plan_t p, const int64_t* n);
 }
 
 extern "C" {
@@ -440,25 +459,11 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
   }
   if (err == cudaSuccess && !p->large_idx.empty())
     err = cudaMallocHost((void**)&p->h_large_info, sizeof(int) * p->large_idx.size());
-  for (int b : p->large_idx) {
-    if (err != cudaSuccess) break;
-    const int nb = (int)n[b];
-    if (p->large_ctx.count(nb)) continue;
-    LargeCtx* c = nullptr;
-    int rc = large_create(&c, nb, precision == GLA_PREC_F64, precision == GLA_PREC_F32_REFINED);
+  if (err == cudaSuccess && !p->large_idx.empty()) {
+    const int rc = make_chains(p, n);
     if (rc) {
       gla_plan_destroy(p);
       return rc;
-    }
-    p->large_ctx[nb] = c;
-    if (precision == GLA_PREC_F32_REFINED) {
-      RefineLarge* r = nullptr;
-      rc = refine_large_create(&r, nb);
-      if (rc) {
-        gla_plan_destroy(p);
-        return rc;
-      }
-      p->large_ref[nb] = r;
     }
   }
   if (p->timing)
@@ -509,8 +514,11 @@ int gla_plan_destroy(gla_plan_t p) {
   cudaFree(p->d_adj);
   cudaFree(p->h_adj);
   large_adjoint_destroy(p->adj_large);
-  for (auto& kv : p->large_ctx) large_destroy(kv.second);
-  for (auto& kv : p->large_ref) refine_large_destroy(kv.second);
+  for (auto& ch : p->chains) {
+    large_destroy(ch.ctx);
+    refine_large_destroy(ch.ref);
+  }
+  for (cudaStream_t s : p->side_streams) cudaStreamDestroy(s);
   cudaFreeHost(p->h_large_info);
   delete p;
   return 0;
@@ -616,54 +624,171 @@ int enqueue_refine(gla_plan_t p, int b, const void* A, int lower, void* Vout, vo
   return 0;
 }
 
-// Matrices above the small-matrix limit, one at a time on the caller's
-// stream (each large solve uses the whole GPU).
-int execute_large(gla_plan_t p, const void* A, void* w, void* V, int* info, cudaStream_t st) {
+// The plan's chains of large matrices, their contexts and, where several of
+// them run side by side, the streams.
+int make_chains(gla_plan_t p, const int64_t* n) {
+  const bool f64 = p->prec == GLA_PREC_F64, refined = p->prec == GLA_PREC_F32_REFINED;
+  std::map<int, std::vector<int>, std::greater<int>> by_order;  // positions in large_idx
+  int nside = 0;
+  for (size_t k = 0; k < p->large_idx.size(); k++) {
+    const int nb = (int)n[p->large_idx[k]];
+    by_order[nb].push_back((int)k);
+    nside += nb <= kSideBySideMaxN;
+  }
+  // (phase times are sums over matrices that have the GPU to themselves)
+  bool side = nside >= 2 && !p->timing;
+  p->large_chain.resize(p->large_idx.size());
+  for (;;) {
+    int rc = 0;
+    for (int want = side ? 1 : 0; want >= 0 && !rc; want--)
+      for (auto& kv : by_order) {
+        const bool sd = side && kv.first <= kSideBySideMaxN;
+        if (sd != (want == 1)) continue;
+        const int nch = sd ? std::min<int>(kMaxSide, (int)kv.second.size()) : 1;
+        for (int c = 0; c < nch && !rc; c++) {
+          p->chains.emplace_back();
+          gla_plan_s::LargeChain& ch = p->chains.back();
+          ch.n = kv.first;
+          ch.side = sd;
+          rc = large_create(&ch.ctx, ch.n, f64, refined, sd);
+          if (!rc && refined) rc = refine_large_create(&ch.ref, ch.n, sd);
+          for (size_t q = c; q < kv.second.size(); q += nch) {
+            ch.items.push_back(kv.second[q]);
+            p->large_chain[kv.second[q]] = (int)p->chains.size() - 1;
+          }
+        }
+        if (rc) break;
+      }
+    if (rc == -1000 - (int)cudaErrorNotSupported && side) {  // no cluster: one after another
+      for (auto& ch : p->chains) {
+        large_destroy(ch.ctx);
+        refine_large_destroy(ch.ref);
+      }
+      p->chains.clear();
+      side = false;
+      continue;
+    }
+    if (rc) return rc;
+    break;
+  }
+  if (side) {
+    int nch = 0;
+    for (auto& ch : p->chains) nch += ch.side;
+    p->side_streams.resize(std::min(kMaxSide, nch), nullptr);
+    for (cudaStream_t& s : p->side_streams) GLA_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  }
+  return 0;
+}
+
+// Statistics of the large matrices of one execute.
+struct LargeStats {
+  int iters = 0;
+  double n3 = 0;
+  float ms = 0.f;
+};
+
+// Matrix k (position in large_idx) on its chain's context and stream st.
+int solve_large(gla_plan_t p, int k, const void* A, void* w, void* V, int* info, cudaStream_t st, LargeStats* stats) {
   const size_t ioe = p->io_elem();
+  const int b = p->large_idx[k];
+  const int nb = (int)p->n[b];
+  const gla_plan_s::LargeChain& ch = p->chains[p->large_chain[k]];
+  // offsets of matrix b in the packed arenas
+  int64_t aoff = 0, woff = 0;
+  for (int q = 0; q < b; q++) {
+    aoff += p->n[q] * p->n[q];
+    woff += p->n[q];
+  }
+  const void* Ab = (const char*)A + ioe * aoff;
+  void* wb = (char*)w + ioe * woff;
+  void* Vb = (p->jobz == 'V' && V) ? (char*)V + ioe * aoff : nullptr;
+  int inf = 0;
+  int rc;
+  if (p->prec == GLA_PREC_F32_REFINED) {
+    // FP32 solve of the rounded matrix straight into the refinement's
+    // buffers, then refinement against the FP64 input
+    RefineLarge* r = ch.ref;
+    rc = large_syev(ch.ctx, kF32FromF64, true, p->uplo == 'L', Ab, nb, refine_large_wbuf(r), refine_large_xbuf(r), nb,
+                    &inf, st);
+    if (rc) return rc;
+    if (inf == 0) {
+      const auto t0 = std::chrono::steady_clock::now();
+      rc = refine_large_run(r, (const double*)Ab, nb, p->uplo == 'L', refine_large_xbuf(r), nb, refine_large_wbuf(r),
+                            (double*)wb, (double*)Vb, nb, st);
+      stats->ms += std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
+      stats->n3 += (double)refine_large_iters(r) * nb * (double)nb * nb;
+      if (rc == -1)
+        inf = -1;
+      else if (rc)
+        return rc;
+      stats->iters = std::max(stats->iters, refine_large_iters(r));
+    } else if (inf == -1) {  // non-finite input: NaN outputs (all bits set), as on the other paths
+      GLA_CUDA(cudaMemsetAsync(wb, 0xff, ioe * nb, st));
+      if (Vb) GLA_CUDA(cudaMemsetAsync(Vb, 0xff, ioe * nb * nb, st));
+    }
+  } else {
+    const int tc = p->prec == GLA_PREC_F64 ? kF64 : kF32;
+    rc = large_syev(ch.ctx, tc, p->jobz == 'V', p->uplo == 'L', Ab, nb, wb, Vb, nb, &inf, st);
+    if (rc) return rc;
+  }
+  p->h_large_info[k] = inf;
+  GLA_CUDA(cudaMemcpyAsync(info + b, p->h_large_info + k, sizeof(int), cudaMemcpyHostToDevice, st));
+  return 0;
+}
+
+// Matrices above the small-matrix limit: those that need the whole GPU one
+// after another on the caller's stream, then the chains that run side by
+// side, largest orders first, each by one of up to kMaxSide host threads with
+// a stream of its own. Every chain's work is waited for before this returns
+// (each solve reads its status back anyway). A thread that cannot be started
+// leaves its chains to the others, at least this one.
+int execute_large(gla_plan_t p, const void* A, void* w, void* V, int* info, cudaStream_t st) {
   p->large_iters = 0;
   p->large_refine_n3 = 0;
   p->large_refine_ms = 0.f;
-  for (size_t k = 0; k < p->large_idx.size(); k++) {
-    const int b = p->large_idx[k];
-    const int nb = (int)p->n[b];
-    // offsets of matrix b in the packed arenas
-    int64_t aoff = 0, woff = 0;
-    for (int q = 0; q < b; q++) {
-      aoff += p->n[q] * p->n[q];
-      woff += p->n[q];
-    }
-    const void* Ab = (const char*)A + ioe * aoff;
-    void* wb = (char*)w + ioe * woff;
-    void* Vb = (p->jobz == 'V' && V) ? (char*)V + ioe * aoff : nullptr;
-    int inf = 0;
-    int rc;
-    if (p->prec == GLA_PREC_F32_REFINED) {
-      // FP32 solve of the rounded matrix straight into the refinement's
-      // buffers, then refinement against the FP64 input
-      RefineLarge* r = p->large_ref[nb];
-      rc = large_syev(p->large_ctx[nb], kF32FromF64, true, p->uplo == 'L', Ab, nb, refine_large_wbuf(r),
-                      refine_large_xbuf(r), nb, &inf, st);
+  if (p->large_idx.empty()) return 0;
+  int nside = 0;
+  for (const auto& ch : p->chains) nside += ch.side;
+  std::vector<LargeStats> stats(p->side_streams.size() + 1);
+  for (size_t c = nside; c < p->chains.size(); c++)
+    for (int k : p->chains[c].items) {
+      const int rc = solve_large(p, k, A, w, V, info, st, &stats[0]);
       if (rc) return rc;
-      if (inf == 0) {
-        const auto t0 = std::chrono::steady_clock::now();
-        rc = refine_large_run(r, (const double*)Ab, nb, p->uplo == 'L', refine_large_xbuf(r), nb,
-                              refine_large_wbuf(r), (double*)wb, (double*)Vb, nb, st);
-        p->large_refine_ms +=
-            std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
-        p->large_refine_n3 += (double)refine_large_iters(r) * nb * (double)nb * nb;
-        if (rc == -1)
-          inf = -1;
-        else if (rc)
-          return rc;
-        p->large_iters = std::max(p->large_iters, refine_large_iters(r));
+    }
+  if (nside) {
+    int dev = 0;
+    GLA_CUDA(cudaGetDevice(&dev));
+    GLA_CUDA(cudaEventRecord(p->fork, st));
+    std::atomic<int> next{0}, status{0};
+    auto worker = [&](int t) {
+      cudaStream_t s = p->side_streams[t];
+      cudaError_t e = cudaSetDevice(dev);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(s, p->fork, 0);
+      int rc = e == cudaSuccess ? 0 : -1000 - (int)e;
+      for (int c; !rc && !status.load() && (c = next.fetch_add(1)) < nside;)
+        for (int k : p->chains[c].items)
+          if ((rc = solve_large(p, k, A, w, V, info, s, &stats[t + 1]))) break;
+      e = cudaStreamSynchronize(s);
+      if (!rc && e != cudaSuccess) rc = -1000 - (int)e;
+      int none = 0;
+      if (rc) status.compare_exchange_strong(none, rc);
+    };
+    std::vector<std::thread> threads;
+    for (size_t t = 1; t < p->side_streams.size(); t++) {
+      try {
+        threads.emplace_back(worker, (int)t);
+      } catch (...) {
+        break;
       }
-    } else {
-      const int tc = p->prec == GLA_PREC_F64 ? kF64 : kF32;
-      rc = large_syev(p->large_ctx[nb], tc, p->jobz == 'V', p->uplo == 'L', Ab, nb, wb, Vb, nb, &inf, st);
-      if (rc) return rc;
     }
-    p->h_large_info[k] = inf;
-    GLA_CUDA(cudaMemcpyAsync(info + b, p->h_large_info + k, sizeof(int), cudaMemcpyHostToDevice, st));
+    worker(0);
+    for (std::thread& t : threads) t.join();
+    if (status.load()) return status.load();
+  }
+  for (const LargeStats& s : stats) {
+    p->large_iters = std::max(p->large_iters, s.iters);
+    p->large_refine_n3 += s.n3;
+    p->large_refine_ms += s.ms;
   }
   return 0;
 }
@@ -1176,9 +1301,9 @@ int gla_plan_phase_times(gla_plan_t p, float* ms) {
     }
   // large matrices: tridiagonalisation, divide and conquer (reported as the
   // chase phase), back-transformation (reported as apply)
-  for (int b : p->large_idx) {
+  for (size_t k = 0; k < p->large_idx.size(); k++) {
     float st[3];
-    large_stage_ms(p->large_ctx[(int)p->n[b]], st);
+    large_stage_ms(p->chains[p->large_chain[k]].ctx, st);
     ms[GLA_PHASE_TRIDIAG] += st[0];
     ms[GLA_PHASE_CHASE] += st[1];
     ms[GLA_PHASE_APPLY] += st[2];

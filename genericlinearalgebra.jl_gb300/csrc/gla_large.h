@@ -118,6 +118,11 @@ void sytrd_plan_destroy(SytrdPlan* p);
 cudaError_t sytrd_enqueue(SytrdPlan* p, void* A, long long lda, void* d, void* e, void* tau, cudaStream_t st);
 int* sytrd_error_word(SytrdPlan* p);
 void sytrd_set_oz64(SytrdPlan* p, Oz64* oz);
+// Every panel on one thread-block cluster, so that several reductions run on
+// SMs of their own; false (and unchanged) above kSideBySideMaxN or where the
+// device cannot hold the cluster.
+constexpr int kSideBySideMaxN = 1024;
+bool sytrd_set_cluster_only(SytrdPlan* p);
 
 struct DcPlan;
 // bisect_leaves (FP32 only): the leaves go through the per-eigenvalue solver
@@ -151,7 +156,10 @@ struct LargeCtx;
 // divide-and-conquer leaves go through the per-eigenvalue solver and its
 // trailing updates and back-transformation through the 3xTF32 tensor-core
 // GEMM. Plain FP32 solves keep the QL leaves and the FP32 SIMT GEMMs.
-int large_create(LargeCtx** out, int n, bool f64, bool refine_stage = false);
+// side: the context runs beside others of the same plan, on streams of their
+// own: no launch of it may need the whole GPU at once (its panels run on one
+// cluster; cudaErrorNotSupported where they cannot).
+int large_create(LargeCtx** out, int n, bool f64, bool refine_stage = false, bool side = false);
 void large_destroy(LargeCtx* c);
 size_t large_workspace_bytes(const LargeCtx* c);
 // Stage times of the last large_syev (ms): tridiagonalisation (with the
@@ -190,7 +198,7 @@ int large_stev(LargeCtx* c, const double* d, const double* e, double* w, double*
 
 // ---- refinement of FP32 eigenpairs of one large matrix (large_refine.cu)
 struct RefineLarge;
-int refine_large_create(RefineLarge** out, int n);
+int refine_large_create(RefineLarge** out, int n, bool side = false);
 void refine_large_destroy(RefineLarge* r);
 // Buffers the FP32 solve can write straight into: eigenvectors (n x n,
 // leading dimension n) and eigenvalues (n).

@@ -123,7 +123,7 @@ __global__ void k_large_store(const T* __restrict__ d, const T* __restrict__ Z, 
 
 }  // namespace
 
-int large_create(LargeCtx** out, int n, bool f64, bool refine_stage) {
+int large_create(LargeCtx** out, int n, bool f64, bool refine_stage, bool side) {
   *out = nullptr;
   LargeCtx* c = new (std::nothrow) LargeCtx();
   if (!c) return -1000 - (int)cudaErrorMemoryAllocation;
@@ -132,6 +132,7 @@ int large_create(LargeCtx** out, int n, bool f64, bool refine_stage) {
   const size_t el = f64 ? 8 : 4;
   cudaError_t err = sytrd_plan_create(&c->sy, n, f64, !f64 && refine_stage);
   int rc = err == cudaSuccess ? 0 : -1000 - (int)err;
+  if (!rc && side && !sytrd_set_cluster_only(c->sy)) rc = -1000 - (int)cudaErrorNotSupported;
   if (!rc) rc = dc_plan_create(&c->dc, n, f64, refine_stage);
   if (!rc) rc = backtr_plan_create(&c->bt, n, f64, !f64 && refine_stage);
   if (!rc) backtr_set_error_word(c->bt, sytrd_error_word(c->sy));

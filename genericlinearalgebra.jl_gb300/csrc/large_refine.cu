@@ -62,6 +62,7 @@ constexpr double kResTheta = 0.1;
 
 struct RefineLarge {
   int n = 0;
+  bool side = false;  // runs beside others (large_create)
   float *Ahi = nullptr, *Alo = nullptr, *Xhi = nullptr, *Xlo = nullptr, *Phi = nullptr, *Plo = nullptr;
   float *Rres = nullptr, *T = nullptr, *E = nullptr, *XE = nullptr, *Ghi = nullptr, *Glo = nullptr;
   float* Cbuf = nullptr;   // cluster matrices, packed
@@ -365,11 +366,12 @@ __global__ void k_ref_store(const float* __restrict__ Xhi, const float* __restri
 
 }  // namespace
 
-int refine_large_create(RefineLarge** out, int n) {
+int refine_large_create(RefineLarge** out, int n, bool side) {
   *out = nullptr;
   RefineLarge* r = new (std::nothrow) RefineLarge();
   if (!r) return -1000 - (int)cudaErrorMemoryAllocation;
   r->n = n;
+  r->side = side;
   const size_t nn = (size_t)n * n;
   cudaError_t err = cudaSuccess;
   auto alloc = [&](void** p, size_t bytes) {
@@ -491,7 +493,7 @@ static int solve_clusters(RefineLarge* r, const std::vector<int>& cs, const std:
     if (it != r->big.end()) {
       lc = it->second;
     } else {
-      int rc = large_create(&lc, cc[k], false, true);
+      int rc = large_create(&lc, cc[k], false, true, r->side);
       if (rc) return rc;
       r->big[cc[k]] = lc;
     }

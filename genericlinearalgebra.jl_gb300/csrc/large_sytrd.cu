@@ -54,6 +54,13 @@ constexpr int kMaxOrder = 16384;
 constexpr UnitShape kShapes[] = {{8, 1, 560}, {16, 1, 1000}, {16, 2, 1500}, {32, 2, kMaxOrder}};
 constexpr int kNumShapes = 4;
 constexpr int kMaxTC = kMaxOrder / 32;  // tile columns a launch may cover (560/8 and 1500/16 are fewer)
+// Trailing orders up to these run a panel on one cluster of 16 CTAs: the
+// cluster's barrier saves what the other SMs would have shortened the column
+// by (FP32 order 500: 6.1 us a column on the cluster, 6.3 on 152 SMs; order
+// 1000: 7.6 and 7.1. FP64 order 200: 7.3 and 8.5; order 400: 10.2 and 9.3).
+// A plan that solves several matrices side by side runs all of their panels
+// so (SytrdPlan::cluster_only), each on SMs of its own.
+constexpr int kClusterG = 16, kClusterMaxF64 = 200, kClusterMaxF32 = 700;
 constexpr int kDotRows = 1024; // rows per dot-product unit
 constexpr int kPT = 256;       // threads per CTA
 constexpr long long kSpinLimit = 1ll << 26;
@@ -110,11 +117,28 @@ GLA_DEV T warp_sum4(const T (&v)[4]) {
 // so that all threads of a CTA return the same value. Before it arrives, the
 // CTA's part of a sum goes out: the warps' parts in part[0 .. 8), added by
 // warp 0 into *out.
-template <class T>
+//
+// CL: the grid is one thread-block cluster, and the barrier is the cluster's
+// (0.4 us instead of 1.7; release and acquire at cluster scope cover the
+// CTAs' global writes). The hardware schedules a cluster as a whole, so there
+// is nothing to spin on.
+template <class T, bool CL>
 GLA_DEV bool grid_sync(unsigned* bar, int* err, unsigned& target, const T* part, T* out) {
   __shared__ int s_ok;
   target += gridDim.x;
   __syncthreads();
+  if (CL) {
+    if (threadIdx.x < 32) {
+      T v = part[threadIdx.x & 7];
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (threadIdx.x == 0) *out = v;
+      __syncwarp();
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return true;
+  }
   if (threadIdx.x < 32) {
     T v = part[threadIdx.x & 7];
 #pragma unroll
@@ -292,7 +316,7 @@ constexpr int kDotW = 2;  // sum_r a_r W[r, q]
 // as there are (four sums in six), and by one warp. FP32, bound by the round
 // trips to L2: all warps do both, with as many loads in flight as there are
 // threads.
-template <class T, int CW, int NQ>
+template <class T, int CW, int NQ, bool CL>
 __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
   constexpr int RC = 32 * NQ;
   constexpr bool kSplit = sizeof(T) == 8;
@@ -338,7 +362,7 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
     part = lane_sum(part, 1);
     if (lane == 0) spart[wid] = part;
   }
-  if (!grid_sync(a.bar, a.err, bar_target, spart, a.normp + g)) return;
+  if (!grid_sync<T, CL>(a.bar, a.err, bar_target, spart, a.normp + g)) return;
 
   for (int c = 0; c < a.nbp; c++) {
     const int j = a.k0 + c, s = j + 1, m = n - s;
@@ -380,7 +404,7 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
       qf = lane_sum(qf, 1);
       if (lane == 0) spart[wid] = qf;
     }
-    if (!grid_sync(a.bar, a.err, bar_target, spart, a.qfp + g)) return;
+    if (!grid_sync<T, CL>(a.bar, a.err, bar_target, spart, a.qfp + g)) return;
 
     // ---------------- phase B: reflector scalars, y, w, reflector store, next column
     const int Js = s / CW;
@@ -600,7 +624,7 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
     }
     if (lane == 0) spart[wid] = npart;
     if (c + 1 < a.nbp)
-      if (!grid_sync(a.bar, a.err, bar_target, spart, a.normp + g)) return;
+      if (!grid_sync<T, CL>(a.bar, a.err, bar_target, spart, a.normp + g)) return;
   }
 }
 
@@ -622,6 +646,8 @@ struct SytrdPlan {
   unsigned* bar = nullptr;
   int* err = nullptr;
   bool f64 = true;
+  bool cluster = false;   // the device can hold a cluster: small trailing orders run on it
+  bool cluster_only = false;  // and all others too
   Oz64* oz = nullptr;     // FP64: trailing updates on the tensor cores (set by sytrd_set_oz64)
 };
 
@@ -689,14 +715,41 @@ int panel_shape(int m, bool f64) {
   return sh;
 }
 template <class T>
-const void* panel_kernel(int sh) {
+const void* panel_kernel(int sh, bool cluster) {
   static_assert(kNumShapes == 4, "one kernel per shape");
   if constexpr (sizeof(T) == 8) {
-    if (sh == 0) return (const void*)k_sytrd_panel<T, kShapes[0].cw, kShapes[0].nq>;
-    if (sh == 1) return (const void*)k_sytrd_panel<T, kShapes[1].cw, kShapes[1].nq>;
-    if (sh == 2) return (const void*)k_sytrd_panel<T, kShapes[2].cw, kShapes[2].nq>;
+    if (cluster && sh == 0) return (const void*)k_sytrd_panel<T, kShapes[0].cw, kShapes[0].nq, true>;
+    if (cluster && sh == 1) return (const void*)k_sytrd_panel<T, kShapes[1].cw, kShapes[1].nq, true>;
+    if (cluster && sh == 2) return (const void*)k_sytrd_panel<T, kShapes[2].cw, kShapes[2].nq, true>;
+    if (sh == 0) return (const void*)k_sytrd_panel<T, kShapes[0].cw, kShapes[0].nq, false>;
+    if (sh == 1) return (const void*)k_sytrd_panel<T, kShapes[1].cw, kShapes[1].nq, false>;
+    if (sh == 2) return (const void*)k_sytrd_panel<T, kShapes[2].cw, kShapes[2].nq, false>;
   }
-  return (const void*)k_sytrd_panel<T, kShapes[3].cw, kShapes[3].nq>;
+  if (cluster) return (const void*)k_sytrd_panel<T, kShapes[3].cw, kShapes[3].nq, true>;
+  return (const void*)k_sytrd_panel<T, kShapes[3].cw, kShapes[3].nq, false>;
+}
+// One panel: over the whole GPU as a cooperative launch, or as one cluster.
+template <class T>
+cudaError_t launch_panel(const SytrdPlan& sp, const SytrdArgs<T>& a, int sh, bool cluster, cudaStream_t st) {
+  const int G = cluster ? kClusterG : sp.G;
+  cudaLaunchAttribute at[1];
+  if (cluster) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kClusterG;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  } else {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(G);
+  cfg.blockDim = dim3(kPT);
+  cfg.dynamicSmemBytes = 2 * (size_t)panel_rows(a.k0, a.n, G) * kSytrdNB * sizeof(T);
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  void* args[] = {(void*)&a};
+  return cudaLaunchKernelExC(&cfg, panel_kernel<T>(sh, cluster), args);
 }
 
 template <class T>
@@ -730,15 +783,16 @@ cudaError_t sytrd_run(SytrdPlan& sp, T* A, long long lda, T* d, T* e, T* tau, cu
     a.nbp = nbp;
     a.V = VW;
     a.W = VW + (long long)nbp * n;
+    const int m = n - k0 - 1;
+    const bool cluster = sp.cluster && (sp.cluster_only || m <= (sizeof(T) == 8 ? kClusterMaxF64 : kClusterMaxF32));
     a.bar_base = bar_base;
-    bar_base += 2u * (unsigned)nbp * (unsigned)sp.G;  // barriers per launch: 1 + nbp + (nbp - 1)
-    const int sh = panel_shape(n - k0 - 1, sizeof(T) == 8);
+    if (!cluster) bar_base += 2u * (unsigned)nbp * (unsigned)sp.G;  // barriers per launch: 1 + nbp + (nbp - 1)
+    // (a cluster has a tenth of the warps: the shape of a trailing order
+    // with that many units per warp)
+    const int sh = panel_shape(cluster ? std::min(3 * m, kMaxOrder) : m, sizeof(T) == 8);
     a.nTC = (n + kShapes[sh].cw - 1) / kShapes[sh].cw;
     a.ustart = sp.ustart + sp.uoff[sh];
-    void* args[] = {(void*)&a};
-    err = cudaLaunchCooperativeKernel(panel_kernel<T>(sh), dim3(sp.G), dim3(kPT), args,
-                                      2 * (size_t)panel_rows(k0, n, sp.G) * kSytrdNB * sizeof(T), st);
-    if (err != cudaSuccess) return err;
+    if ((err = launch_panel(sp, a, sh, cluster, st)) != cudaSuccess) return err;
     const int t = k0 + nbp;
     if (t < n - 1) {  // trailing update A[t:, t:] -= V W' + W V' (lower tiles)
       if (sizeof(T) == 4 && sytrd_update_tc(sp, (float*)A, lda, n, t, nbp, st, &err)) {
@@ -788,10 +842,34 @@ cudaError_t sytrd_plan_create(SytrdPlan** out, int n, bool f64, bool tc) {
   // plan's launches.
   const int vwbytes = 2 * panel_rows(0, kMaxOrder, std::max(nsm, 1)) * kSytrdNB * (f64 ? 8 : 4);
   for (int sh = f64 ? 0 : kNumShapes - 1; sh < kNumShapes; sh++) {
-    const void* kfn = f64 ? panel_kernel<double>(sh) : panel_kernel<float>(sh);
+    const void* kfn = f64 ? panel_kernel<double>(sh, false) : panel_kernel<float>(sh, false);
     if (err == cudaSuccess) err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, vwbytes);
     if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, kPT, vwbytes);
     if (err == cudaSuccess && per < 1) err = cudaErrorCooperativeLaunchTooLarge;
+  }
+  if (err == cudaSuccess) {  // a cluster of kClusterG CTAs, where the device can hold one
+    const int csmem = 2 * ((kSideBySideMaxN + kClusterG) / kClusterG) * kSytrdNB * (f64 ? 8 : 4);
+    const void* kfn = nullptr;
+    for (int sh = f64 ? 0 : kNumShapes - 1; sh < kNumShapes; sh++) {
+      kfn = f64 ? panel_kernel<double>(sh, true) : panel_kernel<float>(sh, true);
+      if (err == cudaSuccess) err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem);
+      if (err == cudaSuccess) err = cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
+    if (err == cudaSuccess) {
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = kClusterG;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(kClusterG);
+      cfg.blockDim = dim3(kPT);
+      cfg.dynamicSmemBytes = csmem;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int nc = 0;
+      sp->cluster = cudaOccupancyMaxActiveClusters(&nc, kfn, &cfg) == cudaSuccess && nc >= 1;
+      if (!sp->cluster) cudaGetLastError();
+    }
   }
   if (err != cudaSuccess) {
     delete sp;
@@ -869,5 +947,9 @@ cudaError_t sytrd_enqueue(SytrdPlan* sp, void* A, long long lda, void* d, void* 
 
 int* sytrd_error_word(SytrdPlan* sp) { return sp->err; }
 void sytrd_set_oz64(SytrdPlan* sp, Oz64* oz) { sp->oz = oz; }
+bool sytrd_set_cluster_only(SytrdPlan* sp) {
+  sp->cluster_only = sp->cluster && sp->n <= kSideBySideMaxN;
+  return sp->cluster_only;
+}
 
 }  // namespace gla
