@@ -199,21 +199,29 @@ __global__ void k_ref_rres(const float* __restrict__ Xhi, const float* __restric
 // of the Davis-Kahan kind would then not be small), some pair (i, j) across
 // p with |i - j| <= kWin has |t_ij| > kTheta |lam_j - lam_i|, or the gap is
 // at rounding level.
-__global__ void k_ref_couple(const float* __restrict__ T, const double* __restrict__ lam,
-                             const float* __restrict__ rn, int n, int* __restrict__ couple) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per p, lanes over the pairs (one thread per p took 125 us at order
+// 2048 and 150 at 1000: up to 528 pairs in a row, an FP64 difference each).
+__global__ void __launch_bounds__(256) k_ref_couple(const float* __restrict__ T, const double* __restrict__ lam,
+                                                    const float* __restrict__ rn, int n, int* __restrict__ couple) {
+  const int p = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p >= n - 1) return;
   const double lmax = fmax(fabs(lam[0]), fabs(lam[n - 1]));
   const double gp = fabs(lam[p + 1] - lam[p]);
-  int c = gp <= 64.0 * 0x1p-52 * lmax || gp * kResTheta <= (double)fmaxf(rn[p], rn[p + 1]);
-  for (int i = max(0, p - kWin + 1); i <= p && !c; i++)
-    for (int j = p + 1; j <= min(n - 1, i + kWin) && !c; j++) {
+  bool c = gp <= 64.0 * 0x1p-52 * lmax || gp * kResTheta <= (double)fmaxf(rn[p], rn[p + 1]);
+  // i = p - a, j = i + b with a < b <= kWin: lane b - 1, one a at a time
+  for (int a = 0; a < kWin && a <= p && !c; a++) {
+    const int i = p - a, j = i + lane + 1;
+    bool over = false;
+    if (j > p && j < n) {
       const float gap = (float)fabs(lam[j] - lam[i]);
       const float t = fmaxf(fabsf(T[i + (long long)j * n]), fabsf(T[j + (long long)i * n]));
-      c = t > kTheta * gap;
+      over = t > kTheta * gap;
     }
-  couple[p] = c;
+    c = __any_sync(0xffffffffu, over);
+  }
+  if (lane == 0) couple[p] = c;
 }
+static_assert(kWin == 32, "one lane per distance");
 
 // dst[:, j] = src[:, perm[j]] (n x n, leading dimension n).
 __global__ void k_ref_gather(const float* __restrict__ src, float* __restrict__ dst, const int* __restrict__ perm,
@@ -225,6 +233,16 @@ __global__ void k_ref_gather(const float* __restrict__ src, float* __restrict__ 
 
 __device__ __forceinline__ void atomic_max_pos(float* a, float v) {
   atomicMax(reinterpret_cast<int*>(a), __float_as_int(v));  // v >= 0
+}
+
+// 1/x to about one unit in the last place (a hardware seed and one cubic
+// step: 3 FP64 instructions, where the IEEE division takes 9); x far from the
+// ends of the range.
+__device__ __forceinline__ double ref_rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 
 // The correction E (FP32); max |E_ij| over separated pairs into scal[0].
@@ -260,10 +278,10 @@ __global__ void k_ref_e(const float* __restrict__ T, const float* __restrict__ G
         // tfloor; rotations below 1e-8 cost nothing in orthogonality and are
         // kept (they carry the residual's last bits)
         const double t = 0.5 * ((double)T[idx] + (double)T[j + (long long)i * n]);
-        const double rot = t / gap;
+        const double rot = t * ref_rcp(gap);
         sep = (fabs(t) <= tfloor && fabs(rot) > 1e-8) ? 0.f : (float)rot;
       } else {
-        sep = (float)((double)T[idx] / gap);
+        sep = (float)((double)T[idx] * ref_rcp(gap));
       }
       em = fmaxf(em, fabsf(sep));
       e = polish ? sep - 0.5f * (Ghi[g] + Glo[g]) : sep;
@@ -547,7 +565,7 @@ int refine_large_run(RefineLarge* r, const double* A, long long lda, bool lower,
       RF_CUDA(oz_slice(r->oz32, true, r->Xhi, nullptr, n, n, n, 4, st));
       RF_CUDA(oz_slice(r->oz32, false, r->Rres, nullptr, n, n, n, 4, st));
       RF_CUDA(oz_gemm(r->oz32, n, n, n, r->T, nullptr, n, false, st));
-      k_ref_couple<<<(n + 255) / 256, 256, 0, st>>>(r->T, r->lam, r->rn, n, r->couple);
+      k_ref_couple<<<(n + 7) / 8, 256, 0, st>>>(r->T, r->lam, r->rn, n, r->couple);
       RF_CUDA(cudaGetLastError());
       RF_CUDA(cudaMemcpyAsync(r->h_lam.data(), r->lam, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
       RF_CUDA(cudaMemcpyAsync(r->h_couple.data(), r->couple, sizeof(int) * (n - 1), cudaMemcpyDeviceToHost, st));
