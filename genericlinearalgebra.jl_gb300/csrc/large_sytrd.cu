@@ -56,12 +56,18 @@ constexpr int kNumShapes = 4;
 constexpr int kMaxTC = kMaxOrder / 32;  // tile columns a launch may cover (560/8 and 1500/16 are fewer)
 // Trailing orders up to these run a panel on one cluster of 16 CTAs: the
 // cluster's barrier saves what the other SMs would have shortened the column
-// by (FP32 order 500: 6.1 us a column on the cluster, 6.3 on 152 SMs; order
-// 1000: 7.6 and 7.1. FP64 order 200: 7.3 and 8.5; order 400: 10.2 and 9.3).
+// by (FP32 order 500: 4.7 us a column on the cluster, 5.7 on 152 SMs; order
+// 1000 with its last 700 columns, its last 400 or none on the cluster: 5.6,
+// 5.5 and 5.9. FP64 order 200: 7.3 and 8.5; order 400: 10.2 and 9.3).
 // A plan that solves several matrices side by side runs all of their panels
 // so (SytrdPlan::cluster_only), each on SMs of its own.
 constexpr int kClusterG = 16, kClusterMaxF64 = 200, kClusterMaxF32 = 700;
-constexpr int kDotRows = 1024; // rows per dot-product unit
+// Rows per dot-product unit. An FP32 unit waits for L2 (eight rows a lane, in
+// two batches of loads, 6.6 us a column at order 2048; 32 rows 7.6); in FP64
+// the warps are occupied as it is, and shorter units add their reductions
+// (order 1500: 10.9 us with 1024 rows, 11.4 with 256).
+template <class T>
+constexpr int kDotRows = sizeof(T) == 8 ? 1024 : 256;
 constexpr int kPT = 256;       // threads per CTA
 constexpr long long kSpinLimit = 1ll << 26;
 
@@ -304,7 +310,7 @@ constexpr int kDotV = 1;  // sum_r a_r V[r, q], q < c
 constexpr int kDotW = 2;  // sum_r a_r W[r, q]
 
 // Microseconds per column (reduction of order 777 / 4096 in FP64, of order
-// 2048 in FP32): 9.4 / 27.1 and 7.6, of which the two grid barriers are about
+// 2048 in FP32): 9.1 / 26.9 and 6.0, of which the two grid barriers are about
 // 3.5; before units by shape, this split and the short serial chains below
 // 19.4 / 32.9 and 7.9.
 //
@@ -367,7 +373,7 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
   for (int c = 0; c < a.nbp; c++) {
     const int j = a.k0 + c, s = j + 1, m = n - s;
     const int J0 = s / CW;
-    const int ndch = (m + kDotRows - 1) / kDotRows;
+    const int ndch = (m + kDotRows<T> - 1) / kDotRows<T>;
     // ---------------- phase A: SYMV and dot products on the raw column a
     {
       const int usym0 = sust[J0 - Jb], nsym = sust[nJ] - usym0;
@@ -392,7 +398,7 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
           const int q = rem / ndch, chn = rem % ndch;
           const T* __restrict__ X = kind == kDotA ? A + (long long)s * ld
                                                   : (kind == kDotV ? a.V : a.W) + (long long)q * ldv;
-          const int r0 = s + 1 + chn * kDotRows, r1 = min(n, r0 + kDotRows);
+          const int r0 = s + 1 + chn * kDotRows<T>, r1 = min(n, r0 + kDotRows<T>);
           T acc = T(0);
 #pragma unroll 4
           for (int r = r0 + lane; r < r1; r += 32) acc = fma(X[r], A[r + (long long)j * ld], acc);
@@ -412,29 +418,31 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
     const int rt = kSplit ? tid & (kRowT - 1) : tid, sub = rt % tpr, rl0 = rt / tpr;
     // (1) every load of the phase is issued before the first sum needs one
     // (loops that load and add would each wait for L2 in turn); what does not
-    // fit the registers follows in batches. Rows: kU parts of a row's y in P
-    // and in Qp per thread; cP, cQ: those the CTA's rows have at most.
-    constexpr int kU = kSplit ? 4 : 16;
+    // fit the registers follows in a loop. Rows: kU parts of a row's y in P
+    // and in Qp per thread; cP, cQ: those the CTA's rows have at most. More
+    // than four parts cost FP32 more in predicated instructions than the
+    // loop does (16 parts: 6.6 us a column at order 2048, 8: 6.1, 4: 5.9).
+    constexpr int kU = 4;
     const int Jhi = (max(hi0, lo0 + 1) - 1) / CW, Jlo = max(lo0, s) / CW;
     const int cP = (min(Jhi, a.nTC - 1) - J0 + tpr) / tpr;
     const int cQ = ((n - min(Jlo, a.nTC - 1) * CW + RC - 1) / RC + tpr - 1) / tpr;
     T tp[kU], tq[kU], ai = T(0), Ais = T(0);
-    auto load_parts = [&](int ii, int u0) {
+    auto load_parts = [&](int ii) {
       const int Ji = ii / CW, nch = (n - Ji * CW + RC - 1) / RC;
       const T* pp = a.P + (long long)(J0 - Jb) * n + ii;
       const T* pq = a.Qp + ii;
 #pragma unroll
       for (int u = 0; u < kU; u++) {
-        const int k = sub + (u0 + u) * tpr;
-        if (u0 + u < cP) tp[u] = k <= Ji - J0 ? pp[(long long)k * n] : T(0);
-        if (u0 + u < cQ) tq[u] = k < nch ? pq[(long long)k * n] : T(0);
+        const int k = sub + u * tpr;
+        if (u < cP) tp[u] = k <= Ji - J0 ? pp[(long long)k * n] : T(0);
+        if (u < cQ) tq[u] = k < nch ? pq[(long long)k * n] : T(0);
       }
     };
-    auto add_parts = [&](int u0, T& y) {
+    auto add_parts = [&](T& y) {
 #pragma unroll
       for (int u = 0; u < kU; u++) {
-        if (u0 + u < cP) y += tp[u];
-        if (u0 + u < cQ) y += tq[u];
+        if (u < cP) y += tp[u];
+        if (u < cQ) y += tq[u];
       }
     };
     auto row_of = [&](int rl) {  // idle threads read row s (always in range)
@@ -447,12 +455,12 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
       const int ii = row_of(rl0);
       ai = a_at(A, ld, j, s, ii);
       Ais = A[ii + (long long)s * ld];
-      load_parts(ii, 0);
+      load_parts(ii);
     }
     T yraw = T(0);
     if (!kSplit || !rows) {
       const int nchs = (n - Js * CW + RC - 1) / RC;
-      constexpr int kN = kSplit ? 2 : 1, kD = 4;
+      constexpr int kN = kSplit ? 2 : 1, kD = kSplit ? 4 : 8;
       T pn[kN], pf[kN], pc[kN], da = T(0), px = T(0), vs = T(0), ws = T(0), dv[kD], dw[kD];
 #pragma unroll
       for (int u = 0; u < kN; u++) {
@@ -510,7 +518,7 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
         sWs[lane] = ws;
       }
     }
-    if (rows) add_parts(0, yraw);
+    if (rows) add_parts(yraw);
     __syncthreads();
     // (2) The reflector's scalars in warp 0; meanwhile the sums over the
     // panel's earlier columns in warp 1, and with them the coefficients of
@@ -570,16 +578,21 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
       for (int rl = rl0; rl < rpp * ((R0 + rpp - 1) / rpp); rl += rpp) {
         const int i = lo0 + rl, ii = row_of(rl);
         const bool act = rl < R0 && i < hi0 && i >= s;
+        int k0p = sub + kU * tpr;  // the parts beyond the first batch
         if (rl != rl0) {
           ai = a_at(A, ld, j, s, ii);
           Ais = A[ii + (long long)s * ld];
           yraw = T(0);
-          load_parts(ii, 0);
-          add_parts(0, yraw);
+          k0p = sub;
         }
-        for (int u0 = kU; u0 < max(cP, cQ); u0 += kU) {
-          load_parts(ii, u0);
-          add_parts(u0, yraw);
+        if (rl != rl0 || max(cP, cQ) > kU) {
+          const int Ji = ii / CW, nch = (n - Ji * CW + RC - 1) / RC;
+          const T* pp = a.P + (long long)(J0 - Jb) * n + ii;
+          const T* pq = a.Qp + ii;
+#pragma unroll 4
+          for (int k = k0p; k <= Ji - J0; k += tpr) yraw += pp[(long long)k * n];
+#pragma unroll 4
+          for (int k = k0p; k < nch; k += tpr) yraw += pq[(long long)k * n];
         }
         const int rc = rl < R0 ? rl : R0 - 1;  // (idle threads: any cached row)
         T y = T(0), xn = T(0);
@@ -876,7 +889,8 @@ cudaError_t sytrd_plan_create(SytrdPlan** out, int n, bool f64, bool tc) {
     return err;
   }
   sp->G = nsm;  // one CTA per SM (co-residency of a cooperative launch)
-  sp->nDCH = (n + kDotRows - 1) / kDotRows;
+  const int dot_rows = f64 ? kDotRows<double> : kDotRows<float>;
+  sp->nDCH = (n + dot_rows - 1) / dot_rows;
   // unit tables of the shapes, and the partial buffers that hold any of them
   std::vector<int> ustart;
   size_t np = 0, nq = 0;
