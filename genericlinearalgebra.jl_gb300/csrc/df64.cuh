@@ -77,10 +77,32 @@ GLA_DEV df64 df_mac(df64 acc, df64 a, float b) {
 
 GLA_DEV df64 df_mul(df64 a, df64 b) { return df_mac(df_make(0.f, 0.f), a, b); }
 
+// a - b rounded to a float once (the high parts' difference is exact in two
+// floats).
+GLA_DEV float df_diff(df64 a, df64 b) {
+  float s, e;
+  two_sum(a.hi, -b.hi, s, e);
+  return s + (e + (a.lo - b.lo));
+}
+
 // Conversions (FP64 instructions: use outside inner loops only).
 GLA_DEV df64 df_from(double x) {
   const float h = (float)x;
   return df_make(h, (float)(x - (double)h));
+}
+// df_from(a 2^-se) on the integer pipe: df_from and ldexp take five FP64-pipe
+// instructions, 64 cycles each for a warp.
+GLA_DEV df64 df_scaled(double a, int se) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a), m = b & 0xfffffffffffffull;
+  const int e = (int)(b >> 52) & 0x7ff, ef = e - 1023 - se + 127;  // biased exponents of a, and of hi as a float
+  if (e == 0 || e == 0x7ff || ef < 64 || ef > 250) return a == 0.0 ? df_make(0.f, 0.f) : df_from(ldexp(a, -se));
+  const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
+  // hi: to nearest, ties to even, at bit 29 (a carry runs into the exponent)
+  const unsigned ht = (unsigned)(m >> 29), hm = (unsigned)((m + 0xfffffffull + (ht & 1u)) >> 29);
+  const int lo = (int)((unsigned)m & 0x1fffffffu) - (int)((hm - ht) << 29);
+  const float l = (float)lo * __int_as_float((ef - 52) << 23);
+  return df_make(__uint_as_float(sign | (((unsigned)ef << 23) + hm)),
+                 __uint_as_float(__float_as_uint(l) ^ sign));
 }
 GLA_DEV double df_to(df64 a) { return (double)a.hi + (double)a.lo; }
 

@@ -55,4 +55,20 @@ GLA_DEV unsigned long long sort_key(float x) {
 
 enum Algo { kAlgoQL = 0, kAlgoQR = 1, kAlgoPWK = 2 };
 
+// use(idx, load(idx)) for idx < total over the CTA's threads, the loads of U
+// indices in flight before the first is used: a plain loop over an array in
+// L2 or HBM waits for each of its loads in turn.
+template <int U, class L, class F>
+GLA_DEV void batched(int total, const L& load, const F& use) {
+  const int NT = blockDim.x;
+  for (int b = threadIdx.x; b < total; b += U * NT) {
+    decltype(load(0)) v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) v[u] = load(min(b + u * NT, total - 1));
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (b + u * NT < total) use(b + u * NT, v[u]);
+  }
+}
+
 }  // namespace gla

@@ -186,14 +186,18 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
   const float* X0 = X32 + ao;
   float* Asf = reinterpret_cast<float*>(As);
   float an2 = 0.f;
-  for (int idx = tid; idx < n * n; idx += kRT) {
-    int i, k;
-    split_idx(idx, n, inv_n, i, k);
-    const double a = (lower ? (i >= k) : (i <= k)) ? Ag[idx] : Ag[(size_t)i * n + k];
-    const df64 ad = df_from(ldexp(a, -se));
-    A2[idx] = ad;
-    an2 = fmaf(ad.hi, ad.hi, an2);
-  }
+  batched<8>(
+      n * n,
+      [&](int idx) {
+        int i, k;
+        split_idx(idx, n, inv_n, i, k);
+        return (lower ? (i >= k) : (i <= k)) ? Ag[idx] : Ag[(size_t)i * n + k];
+      },
+      [&](int idx, double a) {
+        const df64 ad = df_scaled(a, se);
+        A2[idx] = ad;
+        an2 = fmaf(ad.hi, ad.hi, an2);
+      });
   const float anorm = sqrtf(block_sum_f(an2, red));
   if (TC) tcs::col_exps(n, A2, expA);  // A is symmetric: its row exponents
   const df64 zero = df_make(0.f, 0.f);
@@ -303,13 +307,17 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
     }
     __syncthreads();
     float sd2 = 0.f, r2 = 0.f;
-    for (int idx = tid; idx < n * n; idx += kRT) {
+    struct SR {
+      df64 s, r;
+    };
+    auto load_sr = [&](int idx) { return SR{cS[idx], cR[idx]}; };
+    batched<8>(n * n, load_sr, [&](int idx, const SR& x) {
       int i, j;
       split_idx(idx, n, inv_n, i, j);
-      const float sv = (i == j) ? (float)(df_to(cS[idx]) - lam[i]) : cS[idx].hi;
+      const float sv = (i == j) ? (float)(df_to(x.s) - lam[i]) : x.s.hi;
       sd2 = fmaf(sv, sv, sd2);
-      r2 = fmaf(cR[idx].hi, cR[idx].hi, r2);
-    }
+      r2 = fmaf(x.r.hi, x.r.hi, r2);
+    });
     const float sdn = sqrtf(block_sum_f(sd2, red));
     const float rn = sqrtf(block_sum_f(r2, red));
     const float delta = 2.f * (sdn + anorm * rn);
@@ -377,22 +385,22 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
     // floor; rotations below 1e-8 cost nothing and are kept
     const float tfloor = (float)(1e-14 * lmax_s);
     float emax = 0.f, rmax = 0.f;
-    for (int idx = tid; idx < n * n; idx += kRT) {
+    batched<8>(n * n, load_sr, [&](int idx, const SR& x) {
       int i, j;
       split_idx(idx, n, inv_n, i, j);
-      const float rhalf = 0.5f * (cR[idx].hi + cR[idx].lo);
+      const float rhalf = 0.5f * (x.r.hi + x.r.lo);
       rmax = fmaxf(rmax, fabsf(rhalf));
       float e = rhalf;
       if (cid[i] != cid[j]) {
-        const float gap = (float)(lam[j] - lam[i]);
-        const df64 num = df_mac(cS[idx], lamdf[j], cR[idx]);
+        const float gap = df_diff(lamdf[j], lamdf[i]);
+        const df64 num = df_mac(x.s, lamdf[j], x.r);
         const float rot = (num.hi + num.lo) / gap;
-        const float sij = cS[idx].hi + cS[idx].lo;
+        const float sij = x.s.hi + x.s.lo;
         if (!(fabsf(sij) <= tfloor && fabsf(sij / gap) > 1e-8f)) e = rot;
       }
       E[idx] = e;
       emax = fmaxf(emax, fabsf(e));
-    }
+    });
     emax = block_max_f(emax, red);
     rmax = 2.f * block_max_f(rmax, red);
     // ---- X <- X + X E (FP32 product, see above), then Rayleigh-Ritz inside clusters
@@ -400,10 +408,13 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
         n, [&](int i, int k) { return it == 0 ? X0[(size_t)k * n + i] : X[(size_t)k * n + i].hi; },
         [&](int k, int j) { return E[(size_t)j * n + k]; }, [&](int i, int j, float v) { T1[(size_t)j * n + i] = v; },
         Asf, Bsf, false);
-    for (int idx = tid; idx < n * n; idx += kRT) {
-      const df64 x = it == 0 ? df_make(X0[idx], 0.f) : X[idx];
-      Y[idx] = df_add(x, df_make(T1[idx], 0.f));
-    }
+    struct XT {
+      df64 x;
+      float t;
+    };
+    batched<8>(
+        n * n, [&](int idx) { return XT{it == 0 ? df_make(X0[idx], 0.f) : X[idx], T1[idx]}; },
+        [&](int idx, const XT& v) { Y[idx] = df_add(v.x, df_make(v.t, 0.f)); });
     __syncthreads();
     if (big_s) {
       const int ncl = ncl_s;
@@ -528,10 +539,13 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
   }
   __syncthreads();
   if (V)
-    for (int j = 0; j < n; j++) {
-      const int dst = rank[j];
-      for (int i = tid; i < n; i += kRT) V[(size_t)dst * n + i] = df_to(X[(size_t)j * n + i]);
-    }
+    batched<8>(
+        n * n, [&](int idx) { return X[idx]; },
+        [&](int idx, df64 x) {
+          int i, j;
+          split_idx(idx, n, inv_n, i, j);
+          V[(size_t)rank[j] * n + i] = df_to(x);
+        });
 }
 
 // Dynamic shared memory of the refinement kernels: the tensor-core slabs,

@@ -2,6 +2,7 @@
 // matrix, n <= 128), shared by its kernel (small_tridiag.cu) and by the
 // persistent FP32 + refinement kernel (refine.cu). See small_tridiag.cu.
 #pragma once
+#include "df64.cuh"
 #include "gla_small.cuh"
 #include "small_stein.cuh"
 
@@ -167,22 +168,26 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
 
   const Tin* Ag = A + dsc.a_off;
   // ---- load the referenced triangle (mirroring 'U' into 'L'), check finiteness
-  // (flat over the n^2 entries, so that every thread has several
-  // independent loads in flight; column j = idx / n by a float reciprocal,
-  // exact for idx < 2^14: the quotient's fraction stays >= 1/(2n) from 1)
+  // (flat over the n^2 entries; column j = idx / n by a float reciprocal,
+  // exact for idx < 2^14: the quotient's fraction stays >= 1/(2n) from 1;
+  // entries outside the triangle are not read and count as zero)
   int bad = 0;
   unsigned long long amax = 0;
   const float inv_n = 1.f / (float)n;
-#pragma unroll 4
-  for (int idx = tid; idx < n * n; idx += NT) {
-    const int j = (int)(((float)idx + 0.5f) * inv_n), i = idx - j * n;
-    if (lower ? (i >= j) : (i <= j)) {
-      Tin v = Ag[idx];
-      bad |= !isfinite(v);
-      unsigned long long b = AbsBits<Tin>::get(v);
-      amax = b > amax ? b : amax;
-    }
-  }
+  auto in_triangle = [&](int idx, int& i, int& j) {
+    j = (int)(((float)idx + 0.5f) * inv_n);
+    i = idx - j * n;
+    return lower ? (i >= j) : (i <= j);
+  };
+  auto entry = [&](int idx) {
+    int i, j;
+    return in_triangle(idx, i, j) ? Ag[idx] : Tin(0);
+  };
+  batched<sizeof(T) == 8 ? 4 : 8>(n * n, entry, [&](int, Tin v) {
+    bad |= !isfinite(v);
+    const unsigned long long b = AbsBits<Tin>::get(v);
+    amax = b > amax ? b : amax;
+  });
   bad = __syncthreads_or(bad);
   if (tid == 0) {
     ChaseState st;
@@ -218,16 +223,13 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
     }
     if (tid == 0) scale_exp[mid] = sexp;
   }
-#pragma unroll 4
-  for (int idx = tid; idx < n * n; idx += NT) {
-    const int j = (int)(((float)idx + 0.5f) * inv_n), i = idx - j * n;
-    if (lower ? (i >= j) : (i <= j)) {
-      Tin v = Ag[idx];
-      T t = (sizeof(Tin) != sizeof(T)) ? (T)ldexp((double)v, -sexp) : (T)v;
-      if (lower) S[j * ld + i] = t;
-      else S[i * ld + j] = t;
-    }
-  }
+  batched<sizeof(T) == 8 ? 4 : 8>(n * n, entry, [&](int idx, Tin v) {
+    int i, j;
+    if (!in_triangle(idx, i, j)) return;
+    const T t = (sizeof(Tin) != sizeof(T)) ? (T)df_scaled((double)v, sexp).hi : (T)v;
+    if (lower) S[j * ld + i] = t;
+    else S[i * ld + j] = t;
+  });
   __syncthreads();
 
   // ---- symtriLower!: k = 0 .. n-3
