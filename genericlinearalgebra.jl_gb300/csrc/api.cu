@@ -74,7 +74,7 @@ cudaError_t cache_alloc(P** slot, size_t bytes) {
 struct Bucket {
   int nmax;   // largest order in the bucket
   int nt;     // threads per CTA (apply)
-  int nt_tri; // threads per CTA (tridiagonalisation)
+  int nt_tri; // threads per CTA (tridiagonalisation; FP64, the FP32 stage takes 256)
   int lpw = 0;  // chase: matrices per warp (0: the launcher's default)
   int start;  // first index into perm_bucket (orders descending inside the bucket)
   int count;
@@ -320,9 +320,8 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
       }
     }
     bk.nt = std::max(32, (bk.nmax + 31) / 32 * 32);
-    // two threads per row: FP32 reductions are latency bound, and an FP64 CTA
-    // of one warp per 32 rows leaves its sub-partitions' FP64 units idle at
-    // every reduction and barrier
+    // two threads per row: an FP64 CTA of one warp per 32 rows leaves its
+    // sub-partitions' FP64 units idle at every reduction and barrier
     bk.nt_tri = std::min(256, 2 * bk.nt);
     if (bk.count) p->buckets.push_back(bk);
   }
@@ -1700,7 +1699,8 @@ int tune_measure(const TuneKey& k, int count, int base_flags, TuneVal* out) {
   const int nt = std::max(32, (n + 31) / 32 * 32);
   TuneVal best{1, k.fam == 0 ? 16 : 8, 1e30f, 1e30f};
   for (int mult = 1; mult <= 4 && rc == 0; mult *= 2) {
-    if (mult > 1 && nt * mult / 2 >= 256) break;  // the shape would repeat the previous one
+    // the shape would repeat the previous one (the FP32 stage has one shape)
+    if (mult > 1 && (k.fam != 0 || nt * mult / 2 >= 256)) break;
     float t = 0, c = 0;
     rc = tune_probe(prec, k.jobz, n, count, base_flags, mult, best.lpw, A, w, V, info, &t, &c);
     if (rc == 0 && t < best.tri_ms) {

@@ -9,7 +9,8 @@
 // triangles run the 'L' reduction (the 'U' variant :507-564 reduces the
 // mirrored matrix in reverse order and yields the same eigenpairs).
 //
-// Work split (FP64 on GB300 costs ~68 cycles per warp instruction no matter
+// FP32: the matrix in registers, see small_tridiag_f32.cuh.
+// FP64 work split (FP64 on GB300 costs ~68 cycles per warp instruction no matter
 // how many lanes are active, so every FP64 loop is spread over all lanes):
 //   norm / dot products: one element per thread + block reduction,
 //   SYMV: rows x (1, 2 or 4 column parts),
@@ -26,10 +27,9 @@
 namespace gla {
 
 size_t tridiag_smem_bytes(int n, int nt, int elem, bool) {
-  // redm[32] u64 | red[32] (8-byte slots) | S[n*ld] | vv,uu,ww,taus [n] | part[8*nt], FP64 part[nt]
-  // (the FP32 tridiagonal solver reuses S and part once Q is in global memory)
-  const size_t ld = (size_t)((n + 1) | 1);
-  return 512 + (size_t)elem * ((size_t)n * ld + 4 * (size_t)n + (elem == 8 ? 1 : 8) * (size_t)nt);
+  // redm[32] u64 | red[32] (8-byte slots) | S[n*ld] | vv,uu,ww,taus [n] | part: FP64 [nt], FP32 [8*256]
+  // (the FP32 tridiagonal solver reuses S and part once the reflectors are in global memory)
+  return 512 + (size_t)elem * (stage_words(n, elem) + 4 * (size_t)n + (elem == 8 ? (size_t)nt : 8 * (size_t)kRegNT));
 }
 
 template <class T, class Tin, bool WANTQ, bool STEIN>
@@ -191,6 +191,7 @@ cudaError_t launch_tridiag(int tcode, bool wantq, int nblocks, int nt, size_t sm
                            void* Q, int* info, ChaseState* cst, int* scale_exp, bool stein, void* w,
                            void* qtmp, void* rows2) {
   if (nblocks <= 0) return cudaSuccess;
+  if (tcode != kF64) nt = kRegNT;  // (small_tridiag_f32.cuh)
 #define GLA_TRI(T, Tin, WQ, ST)                                                                                 \
   k_tridiag<T, Tin, WQ, ST><<<nblocks, nt, smem, st>>>(descs, perm, (const Tin*)A, lower, (T*)d, (T*)e, (T*)Q, \
                                                        info, cst, scale_exp, (T*)w, (T*)qtmp, (T*)rows2)

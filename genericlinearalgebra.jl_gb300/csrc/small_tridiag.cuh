@@ -2,9 +2,12 @@
 // matrix, n <= 128), shared by its kernel (small_tridiag.cu) and by the
 // persistent FP32 + refinement kernel (refine.cu). See small_tridiag.cu.
 #pragma once
+#include <type_traits>
+
 #include "df64.cuh"
 #include "gla_small.cuh"
 #include "small_stein.cuh"
+#include "small_tridiag_f32.cuh"
 
 namespace gla {
 
@@ -19,8 +22,8 @@ template <> struct AbsBits<float> {
 };
 
 // Sum and max (of non-negative bit patterns) over the block.
-template <class T>
-GLA_DEV void block_sum_max(T v, unsigned long long m, T* red, unsigned long long* redm, T& sum, unsigned long long& mx) {
+GLA_DEV void block_sum_max(double v, unsigned long long m, double* red, unsigned long long* redm, double& sum,
+                           unsigned long long& mx) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -34,26 +37,15 @@ GLA_DEV void block_sum_max(T v, unsigned long long m, T* red, unsigned long long
     redm[wid] = m;
   }
   __syncthreads();
-  if constexpr (sizeof(T) == 8) {
-    // the warps' sums by three shuffles (nw <= 8): every warp would queue
-    // nw - 1 additions on the FP64 pipe
-    T s = (lane & 7) < nw ? red[lane & 7] : T(0);
-    unsigned long long x = (lane & 7) < nw ? redm[lane & 7] : 0ull;
+  // the warps' sums by three shuffles (nw <= 8): every warp would queue
+  // nw - 1 additions on the FP64 pipe
+  double s = (lane & 7) < nw ? red[lane & 7] : 0.0;
+  unsigned long long x = (lane & 7) < nw ? redm[lane & 7] : 0ull;
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-      s += __shfl_xor_sync(0xffffffffu, s, o);
-      unsigned long long w = __shfl_xor_sync(0xffffffffu, x, o);
-      x = w > x ? w : x;
-    }
-    sum = s;
-    mx = x;
-    return;
-  }
-  T s = red[0];
-  unsigned long long x = redm[0];
-  for (int i = 1; i < nw; i++) {
-    s += red[i];
-    x = redm[i] > x ? redm[i] : x;
+  for (int o = 4; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    unsigned long long w = __shfl_xor_sync(0xffffffffu, x, o);
+    x = w > x ? w : x;
   }
   sum = s;
   mx = x;
@@ -71,7 +63,6 @@ GLA_DEV double block_sum8(double v, double* red) {
   for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
 }
-GLA_DEV float block_sum8(float v, float* red) { return block_sum(v, red); }
 
 // The reflector's scalars from x1 and the column's squared norm (FP64, both
 // well inside the normal range): nu = copysign(norm, x1), tau = (x1 + nu)/nu
@@ -94,144 +85,131 @@ GLA_DEV void reflector_scalars(double x0, double sumsq, double& nu, double& tau,
   const double d = fma(-xi1, x, 1.0);
   scl = fma(x, fma(d, d, d), x);
 }
-GLA_DEV void reflector_scalars(float, float, float&, float&, float&) {}
 
 // Leading dimension of the staged matrix: odd, so that transposed accesses
 // (stride ld across the lanes of a warp) spread over all shared-memory banks.
-GLA_DEV int stage_ld(int n) { return (n + 1) | 1; }
+__host__ __device__ inline int stage_ld(int n) { return (n + 1) | 1; }
+// Words of the staged matrix (FP32: of the staged reflectors if these take
+// more, and a multiple of 16 bytes).
+__host__ __device__ inline size_t stage_words(int n, int elem) {
+  const size_t s = (size_t)n * stage_ld(n);
+  if (elem == 8) return s;
+  const size_t v = reg_v_words(n);
+  return ((s > v ? s : v) + 3) & ~(size_t)3;
+}
 
-// X = Q Y (n x n, Q column-major with leading dimension ld, Y row-major in
-// Ys with leading dimension ldy), stored column-major to Xg. Thread tiles of
-// 8 x 8 outputs with rows and columns strided by ceil(n/8), so that the
-// threads of a warp read consecutive (or identical) words.
-GLA_DEV void small_gemm_qy(int n, const float* __restrict__ S, int ld, const float* __restrict__ Ys, int ldy,
-                           float* __restrict__ Xg) {
-  const int nt8 = (n + 7) >> 3;
-  for (int t = threadIdx.x; t < nt8 * nt8; t += blockDim.x) {
-    const int ti = t % nt8, tk = t / nt8;
-    float acc[8][8];
+// The part of tridiag_body after the staging, float with the matrix in
+// registers (small_tridiag_f32.cuh). vv: the words after the staged matrix.
+template <int NB, bool WANTQ, bool STEIN>
+GLA_DEV void tridiag_body_regs(int mid, const SmallDesc& dsc, float* S, int ld, float* vv, float* __restrict__ dout,
+                               float* __restrict__ eout, float* __restrict__ Qout, ChaseState* __restrict__ cst,
+                               float* __restrict__ wout, float* __restrict__ qtmp, int sexp,
+                               float* __restrict__ rows2) {
+  constexpr int RU = 2 * NB;
+  const int n = dsc.n, tid = threadIdx.x;
+  float *dd = vv + n, *ee = vv + 2 * n, *taus = vv + 3 * n, *part = vv + 4 * n;
+  float* Qt = STEIN ? qtmp + dsc.a_off : nullptr;
+  // STEIN: S holds the vectors of the tridiagonal while the reflectors wait in
+  // Qt; else they stay in S
+  tridiag_regs<NB>(n, S, ld, dd, ee, taus, part, [&](int k, int i, float v) {
+    if (!WANTQ && !rows2) return;
+    if (!STEIN)
+      S[(size_t)k * (8 * RU) + v_place<RU>(i)] = v;
+    else if (i < n)
+      Qt[(size_t)k * n + i] = v;
+  });
+  for (int i = tid; i < n; i += kRegNT) {
+    dout[dsc.w_off + i] = dd[i];
+    eout[dsc.w_off + i] = ee[i];
+  }
+  if constexpr (!WANTQ) {
+    if (!rows2) return;
+    // eigen2!'s rows 1 and n of Q (see tridiag_body_shared), row n in the
+    // registers of warp 0
+    __syncthreads();
+    const int lane = tid & 31;
+    float* R2 = rows2 + 2 * dsc.w_off;
+    if (tid >= 32) return;
+    float r[4];
 #pragma unroll
-    for (int u = 0; u < 8; u++)
+    for (int q = 0; q < 4; q++) r[q] = lane + 32 * q == n - 1 ? 1.f : 0.f;
+    for (int k = 0; k + 2 < n; k++) {
+      float v[4], dot = 0.f;
 #pragma unroll
-      for (int v = 0; v < 8; v++) acc[u][v] = 0.f;
-    int iu[8], kv[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      iu[u] = min(ti + nt8 * u, n - 1);  // clamped: rows/columns past n are computed and not stored
-      kv[u] = min(tk + nt8 * u, n - 1);
-    }
-    for (int j = 0; j < n; j++) {
-      float q[8], y[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++) q[u] = S[(size_t)j * ld + iu[u]];
-#pragma unroll
-      for (int v = 0; v < 8; v++) y[v] = Ys[(size_t)j * ldy + kv[v]];
-#pragma unroll
-      for (int u = 0; u < 8; u++)
-#pragma unroll
-        for (int v = 0; v < 8; v++) acc[u][v] = fmaf(q[u], y[v], acc[u][v]);
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++)
-#pragma unroll
-      for (int v = 0; v < 8; v++) {
-        const int i = ti + nt8 * u, k = tk + nt8 * v;
-        if (i < n && k < n) Xg[(size_t)k * n + i] = acc[u][v];
+      for (int q = 0; q < 4; q++) {
+        v[q] = lane + 32 * q < n ? S[(size_t)k * (8 * RU) + v_place<RU>(lane + 32 * q)] : 0.f;
+        dot = fmaf(r[q], v[q], dot);
       }
+      const float f = taus[k] * warp_sum(dot);
+#pragma unroll
+      for (int q = 0; q < 4; q++) r[q] = fmaf(-f, v[q], r[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int i = lane + 32 * q;
+      if (i < n) {
+        R2[2 * i] = i == 0 ? 1.f : 0.f;
+        R2[2 * i + 1] = r[q];
+      }
+    }
+  } else {
+    float* Qg = Qout + dsc.a_off;
+    auto identity = [&](int i, int c) { return i == c ? 1.f : 0.f; };
+    auto store = [&](int i, int c, float v) { Qg[(size_t)c * n + i] = v; };
+    if constexpr (STEIN) {
+      auto fetch = [&]() {
+        __syncthreads();
+        batched<8>(
+            max(n - 2, 0) * (8 * RU),
+            [&](int idx) {
+              const int k = idx / (8 * RU), i = idx % (8 * RU);
+              return i < n ? Qt[(size_t)k * n + i] : 0.f;
+            },
+            [&](int idx, float v) {
+              const int k = idx / (8 * RU), i = idx % (8 * RU);
+              S[(size_t)k * (8 * RU) + v_place<RU>(i)] = v;
+            });
+        __syncthreads();
+      };
+      // Y in S (leading dimension ld), e^2, eigenvalues and flags in part
+      // (8 x 256 >= 3 n + 8 words)
+      float* e2s = part;
+      float* lams = e2s + n;
+      int* misc = reinterpret_cast<int*>(lams + n);  // [0] give up, [1] clusters, [2 + 2c], [3 + 2c] bounds
+      const bool solved = stein_solve(n, dd, ee, e2s, lams, S, ld, misc, reinterpret_cast<float*>(misc + n + 8));
+      if (solved) {
+        for (int k = tid; k < n; k += kRegNT) wout[dsc.w_off + k] = sexp ? ldexpf(lams[k], sexp) : lams[k];
+        if (tid == 0) {
+          ChaseState st;
+          st.bs = n;
+          st.nsweeps = 0;
+          st.nrot = 0;
+          st.nhdr = 0;
+          st.status = kChaseDone;
+          st.applied = 1;
+          cst[mid] = st;
+        }
+      }
+      // X = Q Y, or Q for the QL chase (whose state stays "running")
+      apply_q_regs<NB>(
+          n, S, taus, [&](int i, int c) { return solved ? S[(size_t)i * ld + c] : identity(i, c); }, fetch, store);
+    } else {
+      apply_q_regs<NB>(n, S, taus, identity, []() {}, store);
+    }
   }
 }
 
-// STEIN (float only): after forming Q, solve the tridiagonal in the same CTA
-// (small_stein.cuh) and write X = Q Y and the ascending eigenvalues (times
-// 2^scale) to wout, marking the matrix done for the chase; a matrix the
-// solver leaves to the QL chase gets Q as usual. Q goes to qtmp (an n x n
-// float scratch per matrix, arena layout) first, so that the solver's
-// arrays reuse the shared memory of the reduction.
-template <class T, class Tin, bool WANTQ, bool STEIN>
-GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __restrict__ descs,
-                          const Tin* __restrict__ A, int lower, T* __restrict__ dout, T* __restrict__ eout,
-                          T* __restrict__ Qout, int* __restrict__ info, ChaseState* __restrict__ cst,
-                          int* __restrict__ scale_exp, T* __restrict__ wout, T* __restrict__ qtmp,
-                          T* __restrict__ rows2 = nullptr) {
-  const SmallDesc dsc = descs[mid];
-  const int n = dsc.n;
-  const int ld = stage_ld(n);
-  const int tid = threadIdx.x, NT = blockDim.x;
-  unsigned long long* redm = reinterpret_cast<unsigned long long*>(smem_raw);
-  T* red = reinterpret_cast<T*>(smem_raw + 256);
-  T* S = reinterpret_cast<T*>(smem_raw + 512);
-  T* vv = S + (size_t)n * ld;
+// The part of tridiag_body after the staging, FP64: the matrix in shared memory.
+template <bool WANTQ>
+GLA_DEV void tridiag_body_shared(const SmallDesc& dsc, double* S, int ld, double* vv, double* red,
+                                 unsigned long long* redm, double* __restrict__ dout, double* __restrict__ eout,
+                                 double* __restrict__ Qout, double* __restrict__ rows2) {
+  using T = double;
+  const int n = dsc.n, tid = threadIdx.x, NT = blockDim.x;
   T* uu = vv + n;
   T* ww = uu + n;
   T* taus = ww + n;
   T* part = taus + n;
-
-  const Tin* Ag = A + dsc.a_off;
-  // ---- load the referenced triangle (mirroring 'U' into 'L'), check finiteness
-  // (flat over the n^2 entries; column j = idx / n by a float reciprocal,
-  // exact for idx < 2^14: the quotient's fraction stays >= 1/(2n) from 1;
-  // entries outside the triangle are not read and count as zero)
-  int bad = 0;
-  unsigned long long amax = 0;
-  const float inv_n = 1.f / (float)n;
-  auto in_triangle = [&](int idx, int& i, int& j) {
-    j = (int)(((float)idx + 0.5f) * inv_n);
-    i = idx - j * n;
-    return lower ? (i >= j) : (i <= j);
-  };
-  auto entry = [&](int idx) {
-    int i, j;
-    return in_triangle(idx, i, j) ? Ag[idx] : Tin(0);
-  };
-  batched<sizeof(T) == 8 ? 4 : 8>(n * n, entry, [&](int, Tin v) {
-    bad |= !isfinite(v);
-    const unsigned long long b = AbsBits<Tin>::get(v);
-    amax = b > amax ? b : amax;
-  });
-  bad = __syncthreads_or(bad);
-  if (tid == 0) {
-    ChaseState st;
-    st.bs = 0;
-    st.nsweeps = 0;
-    st.nrot = 0;
-    st.nhdr = 0;
-    st.status = bad ? kChaseDone : kChaseRunning;
-    st.applied = 0;
-    cst[mid] = st;
-    info[mid] = bad ? -1 : 0;
-  }
-  if (bad) return;
-  // Reduced-precision runs scale the matrix by an exact power of two so that
-  // its largest entry is near 1 (no overflow/underflow in the narrow type).
-  int sexp = 0;
-  if (sizeof(Tin) != sizeof(T)) {
-    unsigned long long mx = amax;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      unsigned long long w = __shfl_xor_sync(0xffffffffu, mx, o);
-      mx = w > mx ? w : mx;
-    }
-    if ((tid & 31) == 0) redm[tid >> 5] = mx;
-    __syncthreads();
-    mx = redm[0];
-    for (int w = 1; w < (NT >> 5); w++) mx = redm[w] > mx ? redm[w] : mx;
-    __syncthreads();
-    if (mx != 0) {
-      int e2;
-      frexp(AbsBits<Tin>::from(mx), &e2);
-      sexp = e2;  // max |A| * 2^-sexp in [0.5, 1)
-    }
-    if (tid == 0) scale_exp[mid] = sexp;
-  }
-  batched<sizeof(T) == 8 ? 4 : 8>(n * n, entry, [&](int idx, Tin v) {
-    int i, j;
-    if (!in_triangle(idx, i, j)) return;
-    const T t = (sizeof(Tin) != sizeof(T)) ? (T)df_scaled((double)v, sexp).hi : (T)v;
-    if (lower) S[j * ld + i] = t;
-    else S[i * ld + j] = t;
-  });
-  __syncthreads();
-
   // ---- symtriLower!: k = 0 .. n-3
   for (int k = 0; k + 2 < n; k++) {
     const int m = n - k - 1;
@@ -240,7 +218,7 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
     const T x0 = xc[0];  // read before the reduction's barriers; thread 0 rewrites xc[0] below
     T sumsq;
     unsigned long long mb;
-    block_sum_max<T>(xi * xi, (tid < m) ? AbsBits<T>::get(xi) : 0ull, red, redm, sumsq, mb);
+    block_sum_max(xi * xi, (tid < m) ? AbsBits<T>::get(xi) : 0ull, red, redm, sumsq, mb);
     T tau = 0;
     if (mb != 0) {
       // LinearAlgebra.reflector!: norm (scaled only when maxabs^2 would
@@ -248,7 +226,7 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
       // x[2:] /= x1, tau = x1/nu, x[1] = -nu.
       T nu, scl;
       const int mbe = (int)(mb >> 52);  // (FP64) biased exponent of the largest entry
-      if (sizeof(T) == 8 && mbe > 1023 - 400 && mbe < 1023 + 400) {
+      if (mbe > 1023 - 400 && mbe < 1023 + 400) {
         reflector_scalars(x0, sumsq, nu, tau, scl);
       } else {
         const T maxabs = AbsBits<T>::from(mb);
@@ -260,7 +238,7 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
           const T r = (tid < m) ? xi / maxabs : T(0);
           T s2;
           unsigned long long dummy;
-          block_sum_max<T>(r * r, 0ull, red, redm, s2, dummy);
+          block_sum_max(r * r, 0ull, red, redm, s2, dummy);
           normu = maxabs * prec<T>::sqrt_ieee(s2);
         }
         nu = tcopysign(normu, x0);
@@ -285,7 +263,6 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
       int P = NT / R;
       P = P > 8 ? 8 : P;
       const int p = tid / R, i = tid - p * R;
-      const int ps = sizeof(T) == 8 ? R : NT;  // FP64: NT partial sums in all, more CTAs per SM
       if (p < P && i < m) {
         const int j0 = (p * m) / P, j1 = ((p + 1) * m) / P;
         T acc0 = 0, acc1 = 0;
@@ -297,13 +274,13 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
           acc1 = fma(At[a1], vv[j + 1], acc1);
         }
         if (j < j1) acc0 = fma(At[(j <= i) ? (j * ld + i) : (i * ld + j)], vv[j], acc0);
-        part[p * ps + i] = acc0 + acc1;
+        part[p * R + i] = acc0 + acc1;
       }
       __syncthreads();
       T ui = 0;
       if (tid < m) {
         T s = part[tid];
-        for (int q = 1; q < P; q++) s += part[q * ps + tid];
+        for (int q = 1; q < P; q++) s += part[q * R + tid];
         ui = tau * s;
         uu[tid] = ui;
       }
@@ -342,10 +319,6 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
     const T di = S[(size_t)i * ld + i], ei = (i + 1 < n) ? S[(size_t)i * ld + i + 1] : T(0);
     dg[i] = di;
     eg[i] = ei;
-    if (STEIN) {  // uu, ww are free after the reduction: d and e for the tridiagonal solver
-      uu[i] = di;
-      ww[i] = ei;
-    }
   }
   if (!WANTQ && rows2) {
     // eigen2! (src/eigenSelfAdjoint.jl:633-644): only rows 1 and n of Q,
@@ -424,41 +397,110 @@ GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __r
   for (int r = tid; r < n; r += NT) S[r] = (r == 0) ? T(1) : T(0);
   __syncthreads();
   T* Qg = Qout + dsc.a_off;
-  if constexpr (STEIN) {
-    float* Qt = qtmp + dsc.a_off;
-    for (int j = 0; j < n; j++)
-      for (int i = tid; i < n; i += NT) Qt[(size_t)j * n + i] = S[(size_t)j * ld + i];
-    __syncthreads();
-    // Y over S (leading dimension ld), e^2, eigenvalues and flags over part
-    // (8 NT >= 3 n + 8 words), d and e stay in uu and ww
-    float* Ys = S;
-    float* e2s = part;
-    float* lams = e2s + n;
-    int* misc = reinterpret_cast<int*>(lams + n);  // [0] give up, [1] clusters, [2 + 2c], [3 + 2c] bounds
-    // red and redm (64 8-byte slots) are free here: the solver's reduction scratch
-    const bool solved = stein_solve(n, uu, ww, e2s, lams, Ys, ld, misc, reinterpret_cast<float*>(redm));
-    if (solved) {
-      small_gemm_qy(n, Qt, n, Ys, ld, Qg);
-      for (int k = tid; k < n; k += NT) wout[dsc.w_off + k] = sexp ? ldexpf(lams[k], sexp) : lams[k];
-      if (tid == 0) {
-        ChaseState st;
-        st.bs = n;
-        st.nsweeps = 0;
-        st.nrot = 0;
-        st.nhdr = 0;
-        st.status = kChaseDone;
-        st.applied = 1;
-        cst[mid] = st;
-      }
-      return;
-    }
-    // left to the QL chase: Q, the chase state stays "running"
-    for (int j = 0; j < n; j++)
-      for (int i = tid; i < n; i += NT) Qg[(size_t)j * n + i] = Qt[(size_t)j * n + i];
-    return;
-  }
   for (int j = 0; j < n; j++)
     for (int i = tid; i < n; i += NT) Qg[(size_t)j * n + i] = S[(size_t)j * ld + i];
+}
+
+// Float runs with the matrix in registers (256 threads). STEIN (float only): after the reduction, solve the
+// tridiagonal in the same CTA (small_stein.cuh) and write X = Q Y and the
+// ascending eigenvalues (times 2^scale) to wout, marking the matrix done for
+// the chase; a matrix the solver leaves to the QL chase gets Q as usual. The
+// reflectors wait in qtmp (an n x n float scratch per matrix, arena layout)
+// meanwhile, so that the solver's arrays reuse the shared memory of the
+// reduction.
+template <class T, class Tin, bool WANTQ, bool STEIN>
+GLA_DEV void tridiag_body(int mid, unsigned char* smem_raw, const SmallDesc* __restrict__ descs,
+                          const Tin* __restrict__ A, int lower, T* __restrict__ dout, T* __restrict__ eout,
+                          T* __restrict__ Qout, int* __restrict__ info, ChaseState* __restrict__ cst,
+                          int* __restrict__ scale_exp, T* __restrict__ wout, T* __restrict__ qtmp,
+                          T* __restrict__ rows2 = nullptr) {
+  const SmallDesc dsc = descs[mid];
+  const int n = dsc.n;
+  const int ld = stage_ld(n);
+  const int tid = threadIdx.x, NT = blockDim.x;
+  unsigned long long* redm = reinterpret_cast<unsigned long long*>(smem_raw);
+  T* red = reinterpret_cast<T*>(smem_raw + 256);
+  T* S = reinterpret_cast<T*>(smem_raw + 512);
+  T* vv = S + stage_words(n, (int)sizeof(T));
+
+  const Tin* Ag = A + dsc.a_off;
+  // ---- load the referenced triangle (mirroring 'U' into 'L'), check finiteness
+  // (flat over the n^2 entries; column j = idx / n by a float reciprocal,
+  // exact for idx < 2^14: the quotient's fraction stays >= 1/(2n) from 1;
+  // entries outside the triangle are not read and count as zero)
+  int bad = 0;
+  unsigned long long amax = 0;
+  const float inv_n = 1.f / (float)n;
+  auto in_triangle = [&](int idx, int& i, int& j) {
+    j = (int)(((float)idx + 0.5f) * inv_n);
+    i = idx - j * n;
+    return lower ? (i >= j) : (i <= j);
+  };
+  auto entry = [&](int idx) {
+    int i, j;
+    return in_triangle(idx, i, j) ? Ag[idx] : Tin(0);
+  };
+  batched<sizeof(T) == 8 ? 4 : 8>(n * n, entry, [&](int, Tin v) {
+    bad |= !isfinite(v);
+    const unsigned long long b = AbsBits<Tin>::get(v);
+    amax = b > amax ? b : amax;
+  });
+  bad = __syncthreads_or(bad);
+  if (tid == 0) {
+    ChaseState st;
+    st.bs = 0;
+    st.nsweeps = 0;
+    st.nrot = 0;
+    st.nhdr = 0;
+    st.status = bad ? kChaseDone : kChaseRunning;
+    st.applied = 0;
+    cst[mid] = st;
+    info[mid] = bad ? -1 : 0;
+  }
+  if (bad) return;
+  // Reduced-precision runs scale the matrix by an exact power of two so that
+  // its largest entry is near 1 (no overflow/underflow in the narrow type).
+  int sexp = 0;
+  if (sizeof(Tin) != sizeof(T)) {
+    unsigned long long mx = amax;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      unsigned long long w = __shfl_xor_sync(0xffffffffu, mx, o);
+      mx = w > mx ? w : mx;
+    }
+    if ((tid & 31) == 0) redm[tid >> 5] = mx;
+    __syncthreads();
+    mx = redm[0];
+    for (int w = 1; w < (NT >> 5); w++) mx = redm[w] > mx ? redm[w] : mx;
+    __syncthreads();
+    if (mx != 0) {
+      int e2;
+      frexp(AbsBits<Tin>::from(mx), &e2);
+      sexp = e2;  // max |A| * 2^-sexp in [0.5, 1)
+    }
+    if (tid == 0) scale_exp[mid] = sexp;
+  }
+  batched<sizeof(T) == 8 ? 4 : 8>(n * n, entry, [&](int idx, Tin v) {
+    int i, j;
+    if (!in_triangle(idx, i, j)) return;
+    const T t = (sizeof(Tin) != sizeof(T)) ? (T)df_scaled((double)v, sexp).hi : (T)v;
+    if (lower) S[j * ld + i] = t;
+    else S[i * ld + j] = t;
+  });
+  __syncthreads();
+
+  if constexpr (sizeof(T) == 8) {
+    tridiag_body_shared<WANTQ>(dsc, S, ld, vv, red, redm, dout, eout, Qout, rows2);
+  } else {
+    auto body = [&](auto nb) {
+      tridiag_body_regs<decltype(nb)::value, WANTQ, STEIN>(mid, dsc, S, ld, vv, dout, eout, Qout, cst, wout, qtmp, sexp,
+                                                           rows2);
+    };
+    if (n <= 32) body(std::integral_constant<int, 2>());
+    else if (n <= 64) body(std::integral_constant<int, 4>());
+    else if (n <= 96) body(std::integral_constant<int, 6>());
+    else body(std::integral_constant<int, 8>());
+  }
 }
 
 }  // namespace gla

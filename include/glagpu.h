@@ -410,7 +410,8 @@ int gla_autotune_clear(void);
 int gla_autotune_save(const char* path);
 int gla_autotune_load(const char* path);
 /* The plan's size buckets (orders <= GLA_MAX_SMALL_N) and the launch shapes
- * each one runs with. */
+ * each one runs with (nt_tri: threads per CTA of the FP64 reduction; the FP32
+ * one has a single shape of 256 threads). */
 int gla_plan_buckets(gla_plan_t plan, int* count);
 int gla_plan_bucket_config(gla_plan_t plan, int bucket, int* nmax, int* matrices, int* nt_tri, int* lanes_per_warp);
 
