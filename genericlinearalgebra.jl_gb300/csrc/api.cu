@@ -397,9 +397,9 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
   // the tensor-core products' slice scratch, one per persistent CTA (orders
   // above 32 only); a second set for the pipeline's odd chunks, whose CTAs
   // run beside the even chunks' with the same block indices
-  const bool pcache = p->persistent && p->refine_tc && p->nmax > 32;
-  const size_t pcache_set = pcache ? (size_t)p->persist_grid * refine_pcache_bytes() : 0;
-  const size_t o_pcache = carve((p->nchunks ? 2 : 1) * pcache_set);
+  const bool ops = p->persistent && p->refine_tc;
+  const size_t ops_set = ops ? (size_t)p->persist_grid * refine_ops_bytes() : 0;
+  const size_t o_ops = carve((p->nchunks ? 2 : 1) * ops_set);
   p->ws_bytes = off;
   err = cudaMalloc((void**)&p->ws, p->ws_bytes);
   if (err != cudaSuccess) {
@@ -424,7 +424,7 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
   p->d_next = (int*)(w + o_next);
   p->d_chunk_order = (int*)(w + o_corder);
   if (refined) refine_carve(&p->rw, w + o_ref, aoff, woff, batch);
-  if (refined) p->rw.pcache = pcache ? (unsigned char*)(w + o_pcache) : nullptr;
+  if (refined) p->rw.ops = ops ? (unsigned char*)(w + o_ops) : nullptr;
   if (batch) err = cudaMemcpy(p->d_desc, desc.data(), sizeof(SmallDesc) * batch, cudaMemcpyHostToDevice);
   if (err == cudaSuccess && !perm_bucket.empty())
     err = cudaMemcpy(p->d_perm_bucket, perm_bucket.data(), sizeof(int) * perm_bucket.size(), cudaMemcpyHostToDevice);
@@ -1040,7 +1040,7 @@ int pipelined_body(gla_plan_t p, const void* A_host, void* w_host, void* V_host,
   GLA_CUDA(cudaStreamWaitEvent(p->s_in, p->fork, 0));
   GLA_CUDA(cudaStreamWaitEvent(p->s_out, p->fork, 0));
   RefineWork rw_odd = p->rw;
-  if (rw_odd.pcache) rw_odd.pcache += (size_t)p->persist_grid * refine_pcache_bytes();
+  if (rw_odd.ops) rw_odd.ops += (size_t)p->persist_grid * refine_ops_bytes();
   for (int c = 0; c < p->nchunks; c++) {
     const size_t a0 = ioe * p->chunk_a[c], ab = ioe * (p->chunk_a[c + 1] - p->chunk_a[c]);
     if (ab) GLA_CUDA(cudaMemcpyAsync(dA + a0, hA + a0, ab, cudaMemcpyHostToDevice, p->s_in));

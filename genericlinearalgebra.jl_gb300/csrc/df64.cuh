@@ -90,19 +90,32 @@ GLA_DEV df64 df_from(double x) {
   const float h = (float)x;
   return df_make(h, (float)(x - (double)h));
 }
-// df_from(a 2^-se) on the integer pipe: df_from and ldexp take five FP64-pipe
-// instructions, 64 cycles each for a warp.
+// df_from(a 2^-se) for |a| 2^-se <= 1 on the integer pipe (df_from and ldexp
+// take five FP64-pipe instructions, 64 cycles each for a warp, and ldexp's
+// code is long where it is unrolled).
 GLA_DEV df64 df_scaled(double a, int se) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(a), m = b & 0xfffffffffffffull;
-  const int e = (int)(b >> 52) & 0x7ff, ef = e - 1023 - se + 127;  // biased exponents of a, and of hi as a float
-  if (e == 0 || e == 0x7ff || ef < 64 || ef > 250) return a == 0.0 ? df_make(0.f, 0.f) : df_from(ldexp(a, -se));
+  unsigned long long b = (unsigned long long)__double_as_longlong(a);
+  int e = (int)(b >> 52) & 0x7ff;
+  if (e == 0) {  // zero or subnormal
+    if (a == 0.0) return df_make(0.f, 0.f);
+    b = (unsigned long long)__double_as_longlong(a * 0x1p54);
+    e = ((int)(b >> 52) & 0x7ff) - 54;
+  }
+  const unsigned long long m = b & 0xfffffffffffffull;
+  // biased exponent of hi as a float; small ones are built 2^128 larger
+  const int ef = e - 1023 - se + 127, eb = min(ef < 64 ? ef + 128 : ef, 250);
+  if (eb < 64) return df_make(0.f, 0.f);  // below 2^-190
   const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
   // hi: to nearest, ties to even, at bit 29 (a carry runs into the exponent)
   const unsigned ht = (unsigned)(m >> 29), hm = (unsigned)((m + 0xfffffffull + (ht & 1u)) >> 29);
-  const int lo = (int)((unsigned)m & 0x1fffffffu) - (int)((hm - ht) << 29);
-  const float l = (float)lo * __int_as_float((ef - 52) << 23);
-  return df_make(__uint_as_float(sign | (((unsigned)ef << 23) + hm)),
-                 __uint_as_float(__float_as_uint(l) ^ sign));
+  const int li = (int)((unsigned)m & 0x1fffffffu) - (int)((hm - ht) << 29);
+  float hi = __uint_as_float(sign | (((unsigned)eb << 23) + hm));
+  float lo = __uint_as_float(__float_as_uint((float)li * __int_as_float((eb - 52) << 23)) ^ sign);
+  if (ef < 64) {
+    hi = hi * 0x1p-64f * 0x1p-64f;
+    lo = lo * 0x1p-64f * 0x1p-64f;
+  }
+  return df_make(hi, lo);
 }
 GLA_DEV double df_to(df64 a) { return (double)a.hi + (double)a.lo; }
 

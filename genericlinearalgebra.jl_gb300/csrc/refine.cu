@@ -45,7 +45,7 @@ size_t refine_workspace_bytes(int64_t a_elems, int64_t, int64_t) {
   return (7 * sizeof(df64) + 4 * sizeof(float)) * (size_t)a_elems + 4096;
 }
 
-size_t refine_pcache_bytes() { return (size_t)tcs::kPCacheBytes; }
+__host__ __device__ size_t refine_ops_bytes() { return (size_t)tcs::kScratchOps * tcs::kOpBytes; }
 
 void refine_carve(RefineWork* rw, char* base, int64_t a_elems, int64_t, int64_t) {
   df64* p = reinterpret_cast<df64*>(base);
@@ -138,16 +138,29 @@ GLA_DEV void split_idx(int idx, int n, float inv_n, int& i, int& j) {
   i = idx - j * n;
 }
 
+// Entry idx of the upper triangle, column by column: (i, j), i <= j, for
+// idx < 2^13 + 2^6 (the square root of 8 idx + 1 < 2^17 is off by less than
+// the distance to the next column's).
+GLA_DEV void upper_idx(int idx, int& i, int& j) {
+  j = (int)(0.5f * (sqrtf((float)(8 * idx + 1)) - 1.f));
+  j += (j + 1) * (j + 2) / 2 <= idx;
+  j -= j * (j + 1) / 2 > idx;
+  i = idx - j * (j + 1) / 2;
+}
+
 // The refinement of matrix mid by the whole CTA (kRT threads). TC: the three
 // double-float products on the tensor cores through tcx (set up by the
-// kernel), else on the FP32 pipe.
-template <bool TC>
+// kernel), else on the FP32 pipe. OPS (with TC): tcx has the scratch of
+// tcs::gemm_sliced.
+template <bool TC, bool OPS>
 GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const double* __restrict__ A, int lower,
                          const float* __restrict__ X32, double* __restrict__ Vout, double* __restrict__ wout,
                          int* __restrict__ info, const int* __restrict__ scale_exp, const RefineWork& rw,
                          unsigned long long* __restrict__ stats, tcs::Ctx* tcx) {
-  __shared__ df64 As[16 * kTP];
-  __shared__ df64 Bs2[16 * kTP];
+  // two 16 x kTP pair tiles, or two 16 x kTPF float tiles
+  __shared__ __align__(16) df64 AsBs[16 * kTPF];
+  df64 *As = AsBs, *Bs2 = AsBs + 16 * kTP;
+  static_assert(kTPF >= 2 * kTP, "both pair tiles");
   __shared__ double lam[kSmallMaxN];
   __shared__ df64 lamdf[kSmallMaxN];
   __shared__ float red[kRT / 32];
@@ -186,12 +199,15 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
   const float* X0 = X32 + ao;
   float* Asf = reinterpret_cast<float*>(As);
   float an2 = 0.f;
+  auto a_entry = [&](int i, int k) {
+    return (lower ? (i >= k) : (i <= k)) ? Ag[(size_t)k * n + i] : Ag[(size_t)i * n + k];
+  };
   batched<8>(
       n * n,
       [&](int idx) {
         int i, k;
         split_idx(idx, n, inv_n, i, k);
-        return (lower ? (i >= k) : (i <= k)) ? Ag[idx] : Ag[(size_t)i * n + k];
+        return a_entry(i, k);
       },
       [&](int idx, double a) {
         const df64 ad = df_scaled(a, se);
@@ -199,7 +215,12 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
         an2 = fmaf(ad.hi, ad.hi, an2);
       });
   const float anorm = sqrtf(block_sum_f(an2, red));
-  if (TC) tcs::col_exps(n, A2, expA);  // A is symmetric: its row exponents
+  if (TC) {
+    batched<8>(
+        n * n, [&](int idx) { return X0[idx]; }, [&](int idx, float x) { X[idx] = df_make(x, 0.f); });
+    tcs::col_exps(n, A2, expA);  // A is symmetric: its row exponents (ends with a barrier)
+    if (OPS) tcs::slice_operand(tcx->ops, 0, -1, n, A2, expA);
+  }  // A is symmetric: its row exponents
   const df64 zero = df_make(0.f, 0.f);
   auto zinit = [&](int, int) { return zero; };
   df64* cS = S0;
@@ -208,59 +229,49 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
   float emax_prev = 1e30f;
   for (int it = 0; it < kMaxRefineIters; it++) {
     if (TC) {
-      // Y = A X; S = X'Y and R = I - X'X (upper triangles, mirrored); on the
-      // first iteration X is X0, the FP32 eigenvectors (exact floats)
-      df64* Sd = it == 0 ? S0 : S;
-      df64* Rd = it == 0 ? R0 : R;
-      const df64* Xc = X;
-      auto xk = [&](int k, int j) { return it == 0 ? df_make(X0[(size_t)j * n + k], 0.f) : Xc[(size_t)j * n + k]; };
-      auto xt = [&](int i, int k) { return it == 0 ? df_make(X0[(size_t)i * n + k], 0.f) : Xc[(size_t)i * n + k]; };
+      // Y = A X; S = X'Y and R = I - X'X (upper triangles)
       int* expX = expQ + n;
-      if (it == 0)
-        tcs::col_exps(n, X0, expX);
-      else
-        tcs::col_exps(n, Xc, expX);
-      tcs::gemm(
-          *tcx, n, expA, expX, [&](int i, int k) { return A2[(size_t)k * n + i]; }, xk,
-          [&](int i, int j, df64 v) { Y[(size_t)j * n + i] = v; }, false);
-      tcs::col_exps(n, Y, expQ);
-      // [S | X'X] = X' [Y | X] as one product (X' sliced once): columns j < n
-      // give S, columns n + j give X'X; upper triangles, mirrored
-      tcs::gemm(
-          *tcx, n, 2 * n, expX, expQ, xt,
-          [&](int k, int j) { return j < n ? Y[(size_t)j * n + k] : xk(k, j - n); },
-          [&](int i, int j, df64 v) {
-            if (j < n) {
-              if (i <= j) {
-                Sd[(size_t)j * n + i] = v;
-                Sd[(size_t)i * n + j] = v;
+      tcs::col_exps(n, X, expX);
+      if constexpr (OPS) {
+        tcs::slice_operand(tcx->ops, 1, 0, n, X, expX);
+        tcs::gemm_sliced(*tcx, n, 1, 0, expA, expX, expQ, nullptr, Y);
+        tcs::col_exps(n, Y, expQ);
+        tcs::slice_operand(tcx->ops, -1, (n + 7) >> 3, n, Y, expQ);
+        tcs::gemm_sliced(*tcx, n, 2, 1, expX, expX, expQ, R, S);
+      } else {
+        const df64* Xc = X;
+        tcs::gemm(
+            *tcx, n, expA, expX, [&](int i, int k) { return A2[(size_t)k * n + i]; },
+            [&](int k, int j) { return Xc[(size_t)j * n + k]; },
+            [&](int i, int j, df64 v) { Y[(size_t)j * n + i] = v; }, false);
+        tcs::col_exps(n, Y, expQ);
+        // [S | X'X] = X' [Y | X] as one product (X' sliced once): columns j < n
+        // give S, columns n + j give X'X; upper triangles
+        tcs::gemm(
+            *tcx, n, 2 * n, expX, expQ, [&](int i, int k) { return Xc[(size_t)i * n + k]; },
+            [&](int k, int j) { return j < n ? Y[(size_t)j * n + k] : Xc[(size_t)(j - n) * n + k]; },
+            [&](int i, int j, df64 v) {
+              if (j < n) {
+                if (i <= j) S[(size_t)j * n + i] = v;
+              } else if (i <= j - n) {
+                R[(size_t)(j - n) * n + i] = df_add(df_make(i == j - n ? 1.f : 0.f, 0.f), df_neg(v));
               }
-            } else {
-              const int jj = j - n;
-              if (i <= jj) {
-                const df64 r = df_add(df_make(i == jj ? 1.f : 0.f, 0.f), df_neg(v));
-                Rd[(size_t)jj * n + i] = r;
-                Rd[(size_t)i * n + jj] = r;
-              }
-            }
-          },
-          false);
+            },
+            false);
+      }
       if (!tcs::ok(*tcx)) break;  // a tensor-core wait ran out: reported as not converged
-      cS = Sd;
-      cR = Rd;
+      cS = S;
+      cR = R;
     } else if (it == 0) {
       // ---- first iteration on the FP32 eigenvectors X0 (exact floats)
       tile_gemm_df<float>(
           n, [&](int i, int k) { return A2[(size_t)k * n + i]; }, [&](int k, int j) { return X0[(size_t)j * n + k]; },
           zinit, [&](int i, int j, df64 v) { Y[(size_t)j * n + i] = v; }, As, Bsf, false);
-      // S0 = X0'Y computed as (Y'X0) (symmetric): upper triangle, mirrored
+      // S0 = X0'Y computed as (Y'X0) (symmetric): upper triangle
       tile_gemm_df<float>(
           n, [&](int i, int k) { return Y[(size_t)i * n + k]; }, [&](int k, int j) { return X0[(size_t)j * n + k]; },
           zinit,
-          [&](int i, int j, df64 v) {
-            S0[(size_t)j * n + i] = v;
-            S0[(size_t)i * n + j] = v;
-          },
+          [&](int i, int j, df64 v) { S0[(size_t)j * n + i] = v; },
           As, Bsf, true);
       tile_gemm_df<float>(
           n, [&](int i, int k) { return df_make(X0[(size_t)i * n + k], 0.f); },
@@ -268,23 +279,19 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
           [&](int i, int j, df64 v) {
             const df64 r = df_add(df_make(i == j ? 1.f : 0.f, 0.f), df_neg(v));
             R0[(size_t)j * n + i] = r;
-            R0[(size_t)i * n + j] = r;
           },
           As, Bsf, true);
       cS = S0;
       cR = R0;
     } else {
-      // ---- explicit: Y = A X ; S = X'Y ; R = I - X'X (upper triangles, mirrored)
+      // ---- explicit: Y = A X ; S = X'Y ; R = I - X'X (upper triangles)
       tile_gemm_df<df64>(
           n, [&](int i, int k) { return A2[(size_t)k * n + i]; }, [&](int k, int j) { return X[(size_t)j * n + k]; },
           zinit, [&](int i, int j, df64 v) { Y[(size_t)j * n + i] = v; }, As, Bs2, false);
       tile_gemm_df<df64>(
           n, [&](int i, int k) { return X[(size_t)i * n + k]; }, [&](int k, int j) { return Y[(size_t)j * n + k]; },
           zinit,
-          [&](int i, int j, df64 v) {
-            S[(size_t)j * n + i] = v;
-            S[(size_t)i * n + j] = v;
-          },
+          [&](int i, int j, df64 v) { S[(size_t)j * n + i] = v; },
           As, Bs2, true);
       tile_gemm_df<df64>(
           n, [&](int i, int k) { return X[(size_t)i * n + k]; }, [&](int k, int j) { return X[(size_t)j * n + k]; },
@@ -292,7 +299,6 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
           [&](int i, int j, df64 v) {
             const df64 r = df_add(df_make(i == j ? 1.f : 0.f, 0.f), df_neg(v));
             R[(size_t)j * n + i] = r;
-            R[(size_t)i * n + j] = r;
           },
           As, Bs2, true);
       cS = S;
@@ -310,13 +316,19 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
     struct SR {
       df64 s, r;
     };
-    auto load_sr = [&](int idx) { return SR{cS[idx], cR[idx]}; };
-    batched<8>(n * n, load_sr, [&](int idx, const SR& x) {
+    auto load_sr = [&](int idx) {
       int i, j;
-      split_idx(idx, n, inv_n, i, j);
+      upper_idx(idx, i, j);
+      return SR{cS[(size_t)j * n + i], cR[(size_t)j * n + i]};
+    };
+    const int nup = n * (n + 1) / 2;
+    batched<8>(nup, load_sr, [&](int idx, const SR& x) {
+      int i, j;
+      upper_idx(idx, i, j);
       const float sv = (i == j) ? (float)(df_to(x.s) - lam[i]) : x.s.hi;
-      sd2 = fmaf(sv, sv, sd2);
-      r2 = fmaf(x.r.hi, x.r.hi, r2);
+      const float m = (i == j) ? 1.f : 2.f;
+      sd2 = fmaf(m * sv, sv, sd2);
+      r2 = fmaf(m * x.r.hi, x.r.hi, r2);
     });
     const float sdn = sqrtf(block_sum_f(sd2, red));
     const float rn = sqrtf(block_sum_f(r2, red));
@@ -385,35 +397,38 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
     // floor; rotations below 1e-8 cost nothing and are kept
     const float tfloor = (float)(1e-14 * lmax_s);
     float emax = 0.f, rmax = 0.f;
-    batched<8>(n * n, load_sr, [&](int idx, const SR& x) {
+    batched<6>(nup, load_sr, [&](int idx, const SR& x) {
       int i, j;
-      split_idx(idx, n, inv_n, i, j);
+      upper_idx(idx, i, j);
       const float rhalf = 0.5f * (x.r.hi + x.r.lo);
       rmax = fmaxf(rmax, fabsf(rhalf));
-      float e = rhalf;
+      float eij = rhalf, eji = rhalf;
       if (cid[i] != cid[j]) {
         const float gap = df_diff(lamdf[j], lamdf[i]);
-        const df64 num = df_mac(x.s, lamdf[j], x.r);
-        const float rot = (num.hi + num.lo) / gap;
         const float sij = x.s.hi + x.s.lo;
-        if (!(fabsf(sij) <= tfloor && fabsf(sij / gap) > 1e-8f)) e = rot;
+        if (!(fabsf(sij) <= tfloor && fabsf(sij) > 1e-8f * fabsf(gap))) {
+          const df64 nij = df_mac(x.s, lamdf[j], x.r), nji = df_mac(x.s, lamdf[i], x.r);
+          eij = (nij.hi + nij.lo) / gap;
+          eji = (nji.hi + nji.lo) / -gap;
+        }
       }
-      E[idx] = e;
-      emax = fmaxf(emax, fabsf(e));
+      E[(size_t)j * n + i] = eij;
+      E[(size_t)i * n + j] = eji;
+      emax = fmaxf(emax, fmaxf(fabsf(eij), fabsf(eji)));
     });
     emax = block_max_f(emax, red);
     rmax = 2.f * block_max_f(rmax, red);
     // ---- X <- X + X E (FP32 product, see above), then Rayleigh-Ritz inside clusters
     tile_gemm_f32(
-        n, [&](int i, int k) { return it == 0 ? X0[(size_t)k * n + i] : X[(size_t)k * n + i].hi; },
+        n, [&](int i, int k) { return !TC && it == 0 ? X0[(size_t)k * n + i] : X[(size_t)k * n + i].hi; },
         [&](int k, int j) { return E[(size_t)j * n + k]; }, [&](int i, int j, float v) { T1[(size_t)j * n + i] = v; },
-        Asf, Bsf, false);
+        Asf, Asf + 16 * kTPF);
     struct XT {
       df64 x;
       float t;
     };
     batched<8>(
-        n * n, [&](int idx) { return XT{it == 0 ? df_make(X0[idx], 0.f) : X[idx], T1[idx]}; },
+        n * n, [&](int idx) { return XT{!TC && it == 0 ? df_make(X0[idx], 0.f) : X[idx], T1[idx]}; },
         [&](int idx, const XT& v) { Y[idx] = df_add(v.x, df_make(v.t, 0.f)); });
     __syncthreads();
     if (big_s) {
@@ -425,23 +440,24 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
         float* Z = jac + k * k;
         // C = (I + R/2) S (I + R/2) - mu I restricted to the cluster, shifted by
         // the mean mu of its lam (first order in R, FP32 after the shift)
+        auto sym = [&](const df64* M, int i, int j) { return M[(size_t)max(i, j) * n + min(i, j)]; };
         double mu = 0;
         for (int a = 0; a < k; a++) mu += lam[ord[r0 + a]];
         mu /= k;
         for (int idx = tid; idx < k * k; idx += kRT) {
           const int a = idx % k, b = idx / k;
           const int ia = ord[r0 + a], ib = ord[r0 + b];
-          df64 sv = cS[(size_t)ib * n + ia];
+          df64 sv = sym(cS, ia, ib);
           if (a == b) sv = df_add(sv, df_from(-mu));
           float corr = 0.f;
           for (int q = 0; q < k; q++) {
             const int iq = ord[r0 + q];
-            const float sq_b = cS[(size_t)ib * n + iq].hi - (q == b ? (float)mu : 0.f);
-            const float sa_q = cS[(size_t)iq * n + ia].hi - (a == q ? (float)mu : 0.f);
-            corr = fmaf(cR[(size_t)iq * n + ia].hi, sq_b, corr);
-            corr = fmaf(sa_q, cR[(size_t)ib * n + iq].hi, corr);
+            const float sq_b = sym(cS, iq, ib).hi - (q == b ? (float)mu : 0.f);
+            const float sa_q = sym(cS, ia, iq).hi - (a == q ? (float)mu : 0.f);
+            corr = fmaf(sym(cR, ia, iq).hi, sq_b, corr);
+            corr = fmaf(sa_q, sym(cR, iq, ib).hi, corr);
           }
-          C[b * k + a] = (sv.hi + sv.lo) + 0.5f * corr + (float)mu * cR[(size_t)ib * n + ia].hi;
+          C[b * k + a] = (sv.hi + sv.lo) + 0.5f * corr + (float)mu * sym(cR, ia, ib).hi;
         }
         __syncthreads();
         float offc = 0.f;
@@ -568,7 +584,7 @@ __global__ void __launch_bounds__(kRT) k_refine(const SmallDesc* __restrict__ de
   if (cst && cst[mid].applied == kRefinedInKernel) return;  // (uniform) before any TMEM is taken
   tcs::Ctx tcx;
   if (TC) tcs::setup(tcx, &tsh, rsm, rw.err);
-  refine_body<TC>(mid, descs, A, lower, X32, Vout, wout, info, scale_exp, rw, stats, &tcx);
+  refine_body<TC, false>(mid, descs, A, lower, X32, Vout, wout, info, scale_exp, rw, stats, &tcx);
   if (TC) tcs::teardown(tcx);
 }
 
@@ -594,7 +610,7 @@ __global__ void __launch_bounds__(kRT, 2)
   tcs::Ctx tcx;
   if (TC)
     tcs::setup(tcx, &tsh, smem_raw, rw.err,
-               rw.pcache ? rw.pcache + (size_t)blockIdx.x * tcs::kPCacheBytes : nullptr);
+               rw.ops + (size_t)blockIdx.x * refine_ops_bytes());
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_idx = atomicAdd(next, 1);
@@ -606,7 +622,7 @@ __global__ void __launch_bounds__(kRT, 2)
                                             qtmp);
     __syncthreads();
     if (cst[mid].applied == 1) {  // solved in FP32 (small_stein.cuh)
-      refine_body<TC>(mid, descs, A, lower, X32, Vout, wout, info, scale_exp, rw, stats, &tcx);
+      refine_body<TC, TC>(mid, descs, A, lower, X32, Vout, wout, info, scale_exp, rw, stats, &tcx);
       __syncthreads();
       if (threadIdx.x == 0) cst[mid].applied = kRefinedInKernel;
     }

@@ -9,8 +9,9 @@
 // 16 x 16 grid keeps the entries (ty + 16 u, tx + 16 v) of the full symmetric
 // matrix, so that a step is at most NB^2 independent FMAs per thread, and the
 // cyclic distribution lets whole register rows and columns drop out as the
-// trailing matrix shrinks (the loops over u and v start at the block kb of
-// the current column, which is unrolled). Two barriers a column: 1900 to 2100
+// trailing matrix shrinks (the loops over u and v start at the block KB of
+// the current column, for which the code is unrolled; one loop with a switch
+// around the FMAs took 196 us where this takes 128). Two barriers a column: 1900 to 2100
 // cycles with two CTAs on the SM (order 128: 385 -> 128 us a matrix).
 //
 // The reflectors are applied to X = Q Y by warps that own whole columns of X
@@ -145,16 +146,15 @@ GLA_DEV void tridiag_regs_block(float (&a)[NB][NB], int n, float* dd, float* ee,
           float norm;
           if (isfinite((float)(n - k - 1) * mm) && mm != 0.f) {
             norm = prec<float>::sqrt_ieee(s2);
-          } else {
+          } else {  // squares out of range: by an exact power of two
+            const int ex = min(max((int)(mb >> 23) - 127, -126), 126);
+            const float dn = __int_as_float((127 - ex) << 23), up = __int_as_float((127 + ex) << 23);
             float q2 = 0.f;
 #pragma unroll
-            for (int v = KB; v < NB; v++) {
-              const float q = x[v] / maxabs;
-              q2 = fmaf(q, q, q2);
-            }
+            for (int v = KB; v < NB; v++) q2 = fmaf(x[v] * dn, x[v] * dn, q2);
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) q2 += __shfl_xor_sync(half, q2, o);
-            norm = maxabs * prec<float>::sqrt_ieee(q2);
+            norm = up * prec<float>::sqrt_ieee(q2);
           }
           nu = copysignf(norm, x0);
           const float xi1 = x0 + nu;
@@ -216,13 +216,13 @@ GLA_DEV void tridiag_regs_block(float (&a)[NB][NB], int n, float* dd, float* ee,
   if constexpr (KB + 1 < NB) tridiag_regs_block<NB, KB + 1>(a, n, dd, ee, taus, xs, storev);
 }
 
-// The reflectors 16 KB + 15 .. 0 of apply_q_regs, in that order.
-template <int NB, int KB>
+// The reflectors 32 QB + 31 .. 0 of apply_q_regs, in that order.
+template <int NB, int QB>
 GLA_DEV void apply_q_block(float (&x)[2 * NB][NB / 2], int n, const float* Vs, const float* taus) {
-  constexpr int RU = 2 * NB, CV = NB / 2, U0 = (2 * KB) & ~3;  // rows below 8 U0 are zero in v
+  constexpr int RU = 2 * NB, CV = NB / 2, U0 = 4 * QB;  // rows below 8 U0 are zero in v
   const int lr = threadIdx.x & 7;
 #pragma unroll 1
-  for (int k = min(16 * KB + 15, n - 3); k >= 16 * KB; k--) {
+  for (int k = min(32 * QB + 31, n - 3); k >= 32 * QB; k--) {
     const float* vk = Vs + (size_t)k * (8 * RU);
     float v[RU], d[CV];
 #pragma unroll
@@ -255,7 +255,7 @@ GLA_DEV void apply_q_block(float (&x)[2 * NB][NB / 2], int n, const float* Vs, c
       for (int u = U0; u < RU; u++) x[u][c] = fmaf(v[u], t, x[u][c]);
     }
   }
-  if constexpr (KB > 0) apply_q_block<NB, KB - 1>(x, n, Vs, taus);
+  if constexpr (QB > 0) apply_q_block<NB, QB - 1>(x, n, Vs, taus);
 }
 
 // X = H_0 H_1 ... H_{n-3} Y for Y read through y(i, c), X stored through
@@ -279,7 +279,7 @@ GLA_DEV void apply_q_regs(int n, const float* Vs, const float* taus, const Y& y,
       x[u][c] = (i < n && cc < n) ? y(i, cc) : 0.f;
     }
   ready();
-  if (wid * 2 * NB < n) apply_q_block<NB, NB - 1>(x, n, Vs, taus);
+  if (wid * 2 * NB < n) apply_q_block<NB, NB / 2 - 1>(x, n, Vs, taus);
 #pragma unroll
   for (int u = 0; u < RU; u++)
 #pragma unroll

@@ -80,62 +80,73 @@ GLA_DEV void tile_gemm_df(int n, const LA& la, const LB& lb, const IN& init, con
   __syncthreads();
 }
 
-// FP32 variant of tile_gemm_df (the X E update).
-template <class LA, class LB, class ST>
-GLA_DEV void tile_gemm_f32(int n, const LA& la, const LB& lb, const ST& store, float* As, float* Bs, bool upper) {
+// C(i, j) = sum_k la(i, k) lb(k, j) in FP32 for n <= 128 (the X E update):
+// one tile of 16 TM x 16 TM outputs, TM x TM per thread in quads of rows and
+// columns 64 apart, so that the operands come as float4 (TM = 8: 64 FMAs per
+// four shared-memory loads; with 4 x 4 outputs read word by word the product
+// of order 128 took 49 us with two CTAs on the SM). As, Bs: 16 x kTPF each.
+constexpr int kTPF = 132;
+template <int TM, class LA, class LB, class ST>
+GLA_DEV void tile_gemm_f32_tm(int n, const LA& la, const LB& lb, const ST& store, float* As, float* Bs) {
+  constexpr int NG = TM / 4;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int kk_ld = tid & 15, ii_ld = tid >> 4;
-  for (int i0 = 0; i0 < n; i0 += 64) {
-    for (int j0 = 0; j0 < n; j0 += 64) {
-      if (upper && j0 + 63 < i0) continue;
-      float acc[4][4];
+  const int kk_ld = tid & 15, ii_ld = tid >> 4;  // this thread loads (kk_ld, ii_ld + 16 q), q < TM
+  float acc[TM][TM];
 #pragma unroll
-      for (int u = 0; u < 4; u++)
+  for (int u = 0; u < TM; u++)
 #pragma unroll
-        for (int v = 0; v < 4; v++) acc[u][v] = 0.f;
-      float ra[4], rb[4];
-      auto fetch = [&](int k0) {
-        const int k = k0 + kk_ld;
+    for (int v = 0; v < TM; v++) acc[u][v] = 0.f;
+  float ra[TM], rb[TM];
+  auto fetch = [&](int k0) {
+    const int k = k0 + kk_ld;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const int i = i0 + ii_ld + 16 * q, j = j0 + ii_ld + 16 * q;
-          ra[q] = (i < n && k < n) ? la(i, k) : 0.f;
-          rb[q] = (j < n && k < n) ? lb(k, j) : 0.f;
-        }
-      };
-      fetch(0);
-      for (int k0 = 0; k0 < n; k0 += 16) {
-        __syncthreads();
+    for (int q = 0; q < TM; q++) {
+      const int i = ii_ld + 16 * q;
+      const bool in = i < n && k < n;
+      ra[q] = in ? la(i, k) : 0.f;
+      rb[q] = in ? lb(k, i) : 0.f;
+    }
+  };
+  fetch(0);
+#pragma unroll 1
+  for (int k0 = 0; k0 < n; k0 += 16) {
+    __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-          As[kk_ld * kTP + ii_ld + 16 * q] = ra[q];
-          Bs[kk_ld * kTP + ii_ld + 16 * q] = rb[q];
-        }
-        __syncthreads();
-        if (k0 + 16 < n) fetch(k0 + 16);
-#pragma unroll 4
-        for (int kk = 0; kk < 16; kk++) {
-          float a[4], b[4];
+    for (int q = 0; q < TM; q++) {
+      As[kk_ld * kTPF + ii_ld + 16 * q] = ra[q];
+      Bs[kk_ld * kTPF + ii_ld + 16 * q] = rb[q];
+    }
+    __syncthreads();
+    if (k0 + 16 < n) fetch(k0 + 16);
+#pragma unroll 2
+    for (int kk = 0; kk < 16; kk++) {
+      float a[TM], b[TM];
 #pragma unroll
-          for (int u = 0; u < 4; u++) a[u] = As[kk * kTP + tx + 16 * u];
-#pragma unroll
-          for (int v = 0; v < 4; v++) b[v] = Bs[kk * kTP + ty + 16 * v];
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-#pragma unroll
-            for (int v = 0; v < 4; v++) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
-        }
+      for (int g = 0; g < NG; g++) {
+        const float4 x = *reinterpret_cast<const float4*>(As + kk * kTPF + 64 * g + 4 * tx);
+        const float4 y = *reinterpret_cast<const float4*>(Bs + kk * kTPF + 64 * g + 4 * ty);
+        a[4 * g] = x.x, a[4 * g + 1] = x.y, a[4 * g + 2] = x.z, a[4 * g + 3] = x.w;
+        b[4 * g] = y.x, b[4 * g + 1] = y.y, b[4 * g + 2] = y.z, b[4 * g + 3] = y.w;
       }
 #pragma unroll
-      for (int u = 0; u < 4; u++)
+      for (int u = 0; u < TM; u++)
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
-          const int i = i0 + tx + 16 * u, j = j0 + ty + 16 * v;
-          if (i < n && j < n && (!upper || i <= j)) store(i, j, acc[u][v]);
-        }
+        for (int v = 0; v < TM; v++) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
     }
   }
+#pragma unroll
+  for (int u = 0; u < TM; u++)
+#pragma unroll
+    for (int v = 0; v < TM; v++) {
+      const int i = 64 * (u >> 2) + 4 * tx + (u & 3), j = 64 * (v >> 2) + 4 * ty + (v & 3);
+      if (i < n && j < n) store(i, j, acc[u][v]);
+    }
   __syncthreads();
+}
+template <class LA, class LB, class ST>
+GLA_DEV void tile_gemm_f32(int n, const LA& la, const LB& lb, const ST& store, float* As, float* Bs) {
+  if (n <= 64) tile_gemm_f32_tm<4>(n, la, lb, store, As, Bs);
+  else tile_gemm_f32_tm<8>(n, la, lb, store, As, Bs);
 }
 
 }  // namespace gla
