@@ -394,8 +394,8 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
     }
   }
   const size_t o_corder = carve(sizeof(int) * chunk_order.size());
-  // the tensor-core products' slice scratch, one per persistent CTA (orders
-  // above 32 only); a second set for the pipeline's odd chunks, whose CTAs
+  // the slices of the tensor-core products' operands, one set per persistent CTA;
+  // a second one for the pipeline's odd chunks, whose CTAs
   // run beside the even chunks' with the same block indices
   const bool ops = p->persistent && p->refine_tc;
   const size_t ops_set = ops ? (size_t)p->persist_grid * refine_ops_bytes() : 0;

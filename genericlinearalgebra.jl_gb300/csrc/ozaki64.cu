@@ -52,7 +52,6 @@ cudaError_t set_attributes() {
     set((const void*)k_slice_vw, kSlab);
     set((const void*)k_slice_blockcol, kSlab);
     set((const void*)k_slice_w, kSlab);
-    set((const void*)k_larft128, kLarftSmem);
   });
   return attr;
 }
@@ -239,7 +238,9 @@ cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Zall, lon
   sg.nks = -4;
   sg.ncols = 1 << 30;
   k_gemm_steps<<<dim3(2, nblk), kThreads, kSmem, st>>>(g, sg);
-  k_larft128<<<nblk, 256, kLarftSmem, st>>>(w->G, tau, w->T, nref);
+  k_larft_leaf<<<dim3(kBM / kLeafT, nblk), 256, 0, st>>>(w->G, tau, w->T, nref);
+  k_larft_merge<32><<<dim3(4, 2, nblk), 256, 0, st>>>(w->G, w->T);
+  k_larft_merge<64><<<dim3(16, 1, nblk), 256, 0, st>>>(w->G, w->T);
   // V_b = Y_b T_b (or Y_b T_b') over Y, then V by block columns
   k_slice_blockcol<<<dim3(nb, nblk), 256, kSlab, st>>>(Y, n, n, (int)nbp, vr, vexp);
   const int trows = nblk * kBM;  // the T factors' columns, one after another

@@ -699,79 +699,63 @@ __global__ void __launch_bounds__(kThreads, 1) k_group_gemm(const Group g) {
   gemm_body<1>(a, blockIdx.x, 0);
 }
 
-// ---- compact-WY factor of a block of 128 reflectors: T (upper triangular,
-// leading dimension 128) from the Gram matrix G = Y'Y and tau, T(i, i) =
-// tau_i, T(0:i, i) = -tau_i T(0:i, 0:i) G(0:i, i). The two halves of 64
-// columns run side by side (two lanes per dot product), then the corner is
-// T12 = -T11 G12 T22. One CTA per block; dynamic shared memory: G and T.
-constexpr int kHB = kBM / 2, kHld = kHB + 1, kHSize = kHB * kHld;  // a 64 x 64 quarter
-constexpr size_t kLarftSmem = sizeof(double) * (5 * (size_t)kHSize + kBM);
-__global__ void __launch_bounds__(256) k_larft128(const double* __restrict__ Gall, const double* __restrict__ tau,
-                                                  double* __restrict__ Tall, int nref) {
-  extern __shared__ __align__(16) unsigned char tsm[];
-  double* G = reinterpret_cast<double*>(tsm);  // quarters G11, G22, G12, column-major
-  double* T = G + 3 * kHSize;                  // quarters T11, T22
-  double* tv = T + 2 * kHSize;
-  const int b = blockIdx.x, tid = threadIdx.x;
-  const double* Gb = Gall + (size_t)b * kBM * kBM;
-  for (int i = tid; i < kHB * kHB; i += 256) {
-    const int r = i % kHB, c = i / kHB, o = r + c * kHld;
-    G[o] = Gb[r + c * kBM];
-    G[kHSize + o] = Gb[kHB + r + (kHB + c) * kBM];
-    G[2 * kHSize + o] = Gb[r + (kHB + c) * kBM];
-    T[o] = 0.0;
-    T[kHSize + o] = 0.0;
+// ---- compact-WY factors of the blocks of 128 reflectors: T (upper triangular,
+// leading dimension 128) from the Gram matrices G = Y'Y and tau, T(i, i) =
+// tau_i, T(0:i, i) = -tau_i T(0:i, 0:i) G(0:i, i). The recurrence runs inside
+// diagonal blocks of 32, one CTA each, eight lanes per dot product; two blocks
+// a, b of equal order join by T_ab = -T_aa G_ab T_bb, a few columns per CTA.
+// An SM does one FP64 warp instruction in 16 cycles, so it is the number of
+// SMs that counts: one CTA per block of 128 took 200 us.
+constexpr int kLeafT = 32;
+// grid: (diagonal block, block of 128)
+__global__ void __launch_bounds__(256) k_larft_leaf(const double* __restrict__ Gall, const double* __restrict__ tau,
+                                                    double* __restrict__ Tall, int nref) {
+  __shared__ double G[kLeafT][kLeafT + 1], T[kLeafT][kLeafT + 1], tv[kLeafT];  // [column][row]
+  const int o = blockIdx.x * kLeafT, b = blockIdx.y, tid = threadIdx.x;
+  const size_t off = (size_t)b * kBM * kBM + o + (size_t)o * kBM;
+  for (int i = tid; i < kLeafT * kLeafT; i += 256) {
+    const int r = i % kLeafT, c = i / kLeafT;
+    G[c][r] = Gall[off + r + c * kBM];
+    T[c][r] = 0.0;
   }
-  for (int i = tid; i < kBM; i += 256) tv[i] = b * kBM + i < nref ? tau[b * kBM + i] : 0.0;
+  if (tid < kLeafT) tv[tid] = b * kBM + o + tid < nref ? tau[b * kBM + o + tid] : 0.0;
   __syncthreads();
-  {
-    const int half = tid >> 7, r = (tid >> 1) & (kHB - 1), part = tid & 1;
-    const double* Gh = G + half * kHSize;
-    double* Th = T + half * kHSize;
-    for (int i = 0; i < kHB; i++) {
-      double s = 0.0;
-      if (r < i)
-        for (int q = r + part; q < i; q += 2) s = fma(Th[r + q * kHld], Gh[q + i * kHld], s);
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      if (part == 0) {
-        const double t = tv[half * kHB + i];
-        if (r < i) Th[r + i * kHld] = -t * s;
-        if (r == i) Th[r + i * kHld] = t;
-      }
-      __syncthreads();
+  const int r = tid >> 3, part = tid & 7;
+  for (int i = 0; i < kLeafT; i++) {
+    double s = 0.0;
+    for (int q = r + part; q < i; q += 8) s = fma(T[q][r], G[i][q], s);
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    if (part == 0) {
+      if (r < i) T[i][r] = -tv[i] * s;
+      if (r == i) T[i][r] = tv[i];
     }
+    __syncthreads();
   }
-  const int r = tid & (kHB - 1), c0 = tid >> 6;  // entries (r, c0 + 4 v) of the corner
-  double* G12 = G + 2 * kHSize;
-  const double* T22 = T + kHSize;
-  double m[16];
-#pragma unroll
-  for (int v = 0; v < 16; v++) m[v] = 0.0;
-  for (int q = 0; q < kHB; q++) {
-    const double x = G12[r + q * kHld];
-#pragma unroll
-    for (int v = 0; v < 16; v++) m[v] = fma(x, T22[q + (c0 + 4 * v) * kHld], m[v]);
+  for (int i = tid; i < kLeafT * kLeafT; i += 256) {
+    const int rr = i % kLeafT, c = i / kLeafT;
+    Tall[off + rr + c * kBM] = T[c][rr];
   }
+}
+
+// grid: (slice of the columns, pair, block of 128); H: order of the blocks joined
+template <int H>
+__global__ void __launch_bounds__(256) k_larft_merge(const double* __restrict__ Gall, double* __restrict__ Tall) {
+  constexpr int kC = 256 / H;  // columns per CTA, one entry per thread
+  __shared__ double M[kC][H + 1];
+  const int tid = threadIdx.x, r = tid % H, cc = tid / H, c = blockIdx.x * kC + cc;
+  const size_t aa = (size_t)blockIdx.z * kBM * kBM + (size_t)blockIdx.y * 2 * H * (kBM + 1);
+  const size_t ab = aa + (size_t)H * kBM, bb = ab + H;
+  double s = 0.0;
+#pragma unroll 16
+  for (int q = 0; q < H; q++) s = fma(Gall[ab + r + q * kBM], Tall[bb + q + c * kBM], s);  // G_ab T_bb
+  M[cc][r] = s;
   __syncthreads();
-#pragma unroll
-  for (int v = 0; v < 16; v++) G12[r + (c0 + 4 * v) * kHld] = m[v];  // G12 T22
-  __syncthreads();
-#pragma unroll
-  for (int v = 0; v < 16; v++) m[v] = 0.0;
-  for (int q = 0; q < kHB; q++) {
-    const double x = T[r + q * kHld];
-#pragma unroll
-    for (int v = 0; v < 16; v++) m[v] = fma(x, G12[q + (c0 + 4 * v) * kHld], m[v]);
-  }
-  double* Tb = Tall + (size_t)b * kBM * kBM;
-#pragma unroll
-  for (int v = 0; v < 16; v++) Tb[r + (kHB + c0 + 4 * v) * kBM] = -m[v];
-  for (int i = tid; i < kHB * kHB; i += 256) {
-    const int rr = i % kHB, c = i / kHB, o = rr + c * kHld;
-    Tb[rr + c * kBM] = T[o];
-    Tb[kHB + rr + (kHB + c) * kBM] = T22[o];
-    Tb[kHB + rr + c * kBM] = 0.0;
-  }
+  s = 0.0;
+#pragma unroll 16
+  for (int q = 0; q < H; q++) s = fma(Tall[aa + r + q * kBM], M[cc][q], s);
+  Tall[ab + r + c * kBM] = -s;
+  Tall[aa + H + r + c * kBM] = 0.0;
 }
 
 }  // namespace oz64
