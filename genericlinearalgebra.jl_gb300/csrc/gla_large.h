@@ -76,7 +76,6 @@ int oz64_create(Oz64** out, int n, int* err);
 void oz64_destroy(Oz64* w);
 size_t oz64_bytes(const Oz64* w);
 constexpr int kOz64MinMerge = 256;   // smallest merge whose level runs on it
-constexpr int kOz64MinUpdate = 128;  // smallest trailing order whose update does
 // A[t:, t:] -= V W' + W V' (lower triangle of the order-n matrix A): V the
 // first nbp <= 32 columns of VW (leading dimension n), W the next nbp.
 cudaError_t oz64_rank2k(Oz64* w, const double* VW, int nbp, int t, double* A, long long lda, cudaStream_t st);
