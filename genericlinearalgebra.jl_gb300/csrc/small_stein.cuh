@@ -73,6 +73,33 @@ GLA_DEV void sturm3(int n, const float* __restrict__ d, const float* __restrict_
   c2 = a2;
 }
 
+// [lo, hi], which holds all n eigenvalues, cut down for the k-th smallest, k =
+// threadIdx.x < n: one Sturm sequence per point of a grid of 3 NT, three per
+// thread, and a search in the counts, in place of log4(3 NT) quadsection
+// steps in which every thread makes its way there by itself (order 128, 256
+// threads: 12 steps become 8). cnt: 3 NT ints of shared scratch. All threads.
+GLA_DEV void grid_bracket(int n, const float* d, const float* e2, float& lo, float& hi, float pivmin, int* cnt) {
+  const int tid = threadIdx.x, P = 3 * blockDim.x;
+  const float l0 = lo, h0 = hi, step = (h0 - l0) / (float)(P + 1);
+  auto point = [&](int p) { return fmaf((float)(p + 1), step, l0); };
+  int c0, c1, c2;
+  sturm3(n, d, e2, point(3 * tid), point(3 * tid + 1), point(3 * tid + 2), pivmin, c0, c1, c2);
+  cnt[3 * tid] = c0;
+  cnt[3 * tid + 1] = c1;
+  cnt[3 * tid + 2] = c2;
+  __syncthreads();
+  if (tid < n) {
+    int a = -1, b = P;  // at most k below point(a), more below point(b)
+    while (b - a > 1) {
+      const int m = (a + b) >> 1;
+      if (cnt[m] > tid) b = m;
+      else a = m;
+    }
+    if (a >= 0) lo = point(a);
+    if (b < P) hi = point(b);
+  }
+}
+
 // The k-th smallest eigenvalue (0-based) in [lo, hi] by quadsection.
 GLA_DEV float eig_bisect(int n, const float* d, const float* e2, int k, float lo, float hi, float atol,
                          float pivmin) {
@@ -210,13 +237,14 @@ GLA_DEV bool mgs_cluster(int n, float* Y, int ldy, int c0, int c1) {
 
 // The whole solver for one matrix, run by every thread of the CTA (blockDim
 // >= n): dd, ee the diagonal and off-diagonal, e2s, lams (n floats each),
-// Ys (n x ldy), misc (n + 8 ints) and fscr (96 floats) shared scratch.
+// Ys (n x ldy), misc (n + 8 ints), fscr (96 floats) and cnt (3 blockDim ints)
+// shared scratch.
 // Returns (uniformly) true with the ascending eigenvalues in lams and the
 // orthonormal eigenvectors in the columns of Ys, or false when the matrix is
 // left to the QL chase.
 GLA_DEV bool stein_solve(int n, const float* __restrict__ dd, const float* __restrict__ ee, float* __restrict__ e2s,
                          float* __restrict__ lams, float* __restrict__ Ys, int ldy, int* __restrict__ misc,
-                         float* __restrict__ fscr) {
+                         float* __restrict__ fscr, int* __restrict__ cnt) {
   const int tid = threadIdx.x, NT = blockDim.x;
   // Gershgorin interval, ||T|| bound, pivmin (LAPACK dstebz's safeguards)
   float glo = 3.0e38f, ghi = -3.0e38f, e2max = 0.f;
@@ -252,6 +280,7 @@ GLA_DEV bool stein_solve(int n, const float* __restrict__ dd, const float* __res
   glo -= widen;
   ghi += widen;
   const float atol = 2.f * prec<float>::eps * tnorm + 4.f * pivmin;
+  grid_bracket(n, dd, e2s, glo, ghi, pivmin, cnt);
   if (tid < n) lams[tid] = eig_bisect(n, dd, e2s, tid, glo, ghi, atol, pivmin);
   __syncthreads();
   // strict: a zero gap is tight even when ||T|| = 0

@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(256) k_tridiag(const SmallDesc* __restrict__ d
                                      scale_exp, wout, qtmp, rows2);
 }
 
-size_t stein_tri_smem_bytes(int n) { return 512 + 4 * (2 * (size_t)n + stein_extra_words(n)); }
+size_t stein_tri_smem_bytes(int n) { return 512 + 4 * (2 * (size_t)n + stein_extra_words(n) + 3 * 128); }
 
 // Tridiagonal input on the FP32 stage (the leaves of the divide and conquer
 // of the FP32 + refinement path): the per-eigenvalue solver of
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(128) k_stein_tri(const SmallDesc* __restrict__
     ee[i] = (i + 1 < n) ? eg_all[dsc.w_off + i] : 0.f;
   }
   __syncthreads();
-  if (!stein_solve(n, dd, ee, e2s, lams, Ys, ldy, misc, fscr)) return;
+  if (!stein_solve(n, dd, ee, e2s, lams, Ys, ldy, misc, fscr, misc + n + 8)) return;
   float* Qg = Qout + dsc.a_off;
   for (int j = 0; j < n; j++)
     for (int i = tid; i < n; i += blockDim.x) Qg[(size_t)j * n + i] = Ys[(size_t)i * ldy + j];
@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(128) k_bisect_values(const SmallDesc* __restri
                                                        const float* __restrict__ eg_all, float* __restrict__ wout,
                                                        const int* __restrict__ info) {
   __shared__ float dd[kSmallMaxN], e2[kSmallMaxN], red[3][4];
+  __shared__ int cnt[3 * kSmallMaxN];
   const int mid = perm[blockIdx.x];
   const SmallDesc dsc = descs[mid];
   const int n = dsc.n, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
@@ -153,8 +154,11 @@ __global__ void __launch_bounds__(128) k_bisect_values(const SmallDesc* __restri
   }
   const float pivmin = 0x1p-120f;
   const float widen = 2.f * (float)n * prec<float>::eps * fmaxf(fabsf(lo), fabsf(hi)) + 2.f * pivmin;
+  lo -= widen;
+  hi += widen;
+  grid_bracket(n, dd, e2, lo, hi, pivmin, cnt);
   if (tid < n) {
-    const float x = eig_bisect_full(n, dd, e2, tid, lo - widen, hi + widen, pivmin);
+    const float x = eig_bisect_full(n, dd, e2, tid, lo, hi, pivmin);
     wout[dsc.w_off + tid] = fabsf(x) <= 4.f * pivmin ? 0.f : ldexpf(x, ex);
   }
 }

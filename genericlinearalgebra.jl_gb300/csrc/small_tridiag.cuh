@@ -172,11 +172,12 @@ GLA_DEV void tridiag_body_regs(int mid, const SmallDesc& dsc, float* S, int ld, 
         __syncthreads();
       };
       // Y in S (leading dimension ld), e^2, eigenvalues and flags in part
-      // (8 x 256 >= 3 n + 8 words)
+      // (8 x 256 >= 3 n + 104 + 3 x 256 words)
       float* e2s = part;
       float* lams = e2s + n;
       int* misc = reinterpret_cast<int*>(lams + n);  // [0] give up, [1] clusters, [2 + 2c], [3 + 2c] bounds
-      const bool solved = stein_solve(n, dd, ee, e2s, lams, S, ld, misc, reinterpret_cast<float*>(misc + n + 8));
+      const bool solved = stein_solve(n, dd, ee, e2s, lams, S, ld, misc, reinterpret_cast<float*>(misc + n + 8),
+                                      misc + n + 104);
       if (solved) {
         for (int k = tid; k < n; k += kRegNT) wout[dsc.w_off + k] = sexp ? ldexpf(lams[k], sexp) : lams[k];
         if (tid == 0) {
