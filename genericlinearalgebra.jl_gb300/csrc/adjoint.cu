@@ -55,10 +55,15 @@ __global__ void __launch_bounds__(kRT) k_adjoint(const SmallDesc* __restrict__ d
     lbar[i] = wbar[dsc.w_off + i];
     amax = fmax(amax, fabs(lam[i]));
   }
-  for (int idx = tid; idx < n * n; idx += kRT) {
-    V2[idx] = df_from(V[ao + idx]);
-    B2[idx] = df_from(Vbar[ao + idx]);
-  }
+  struct VB {
+    double v, b;
+  };
+  batched<4>(
+      n * n, [&](int idx) { return VB{V[ao + idx], Vbar[ao + idx]}; },
+      [&](int idx, const VB& x) {
+        V2[idx] = df_from_fast(x.v);
+        B2[idx] = df_from_fast(x.b);
+      });
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   if ((tid & 31) == 0) red[tid >> 5] = amax;
@@ -83,24 +88,32 @@ __global__ void __launch_bounds__(kRT) k_adjoint(const SmallDesc* __restrict__ d
         zinit, [&](int i, int j, df64 v) { M[(size_t)j * n + i] = v; }, As, Bs, false);
   }
   // M = diag(wbar) + sym(F o G), pairs (i, j) and (j, i) by one thread
-  for (int idx = tid; idx < n * n; idx += kRT) {
-    const int i = idx % n, j = idx / n;
-    if (i > j) continue;
-    if (i == j) {
-      M[idx] = df_from(lbar[i]);
-      continue;
-    }
-    const double gap = lam[j] - lam[i];
-    const df64 gij = M[(size_t)j * n + i], gji = M[(size_t)i * n + j];
-    df64 m = zero;
-    if (fabs(gap) > gap_min) {
-      // 0.5 F_ij (G_ij - G_ji), F_ij = 1/(lam_j - lam_i)
-      const df64 diff = df_add(gij, df_neg(gji));
-      m = df_mul(diff, df_from(0.5 / gap));
-    }
-    M[(size_t)j * n + i] = m;
-    M[(size_t)i * n + j] = m;
-  }
+  struct GG {
+    df64 ij, ji;
+  };
+  batched<4>(
+      n * (n + 1) / 2,
+      [&](int idx) {
+        int i, j;
+        upper_idx(idx, i, j);
+        return GG{M[(size_t)j * n + i], M[(size_t)i * n + j]};
+      },
+      [&](int idx, const GG& g) {
+        int i, j;
+        upper_idx(idx, i, j);
+        df64 m = zero;
+        const double gap = lam[j] - lam[i];
+        if (i == j) {
+          m = df_from(lbar[i]);
+        } else if (fabs(gap) > gap_min) {
+          // 0.5 F_ij (G_ij - G_ji), F_ij = 1/(lam_j - lam_i)
+          const int e = (__double2hiint(gap) >> 20) & 0x7ff;
+          const double f = e > 100 && e < 1946 ? 0.5 * rcp64(gap) : 0.5 / gap;
+          m = df_mul(df_add(g.ij, df_neg(g.ji)), df_from_fast(f));
+        }
+        M[(size_t)j * n + i] = m;
+        M[(size_t)i * n + j] = m;
+      });
   __syncthreads();
   // T = V M
   double* Ab = Abar + ao;

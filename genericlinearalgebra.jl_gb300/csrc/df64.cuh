@@ -117,6 +117,11 @@ GLA_DEV df64 df_scaled(double a, int se) {
   }
   return df_make(hi, lo);
 }
+// df_from without the FP64 pipe for 2^-60 < |x| < 2^120.
+GLA_DEV df64 df_from_fast(double x) {
+  const int e = (int)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff;
+  return e > 1023 - 60 && e < 1023 + 120 ? df_scaled(x, 0) : df_from(x);
+}
 GLA_DEV double df_to(df64 a) { return (double)a.hi + (double)a.lo; }
 
 }  // namespace gla

@@ -60,6 +60,15 @@ template <> struct prec<double> {
   }
 };
 
+// 1/x for normal x well inside the range: one hardware seed and a cubic
+// correction, four FP64 instructions where the IEEE division takes about 45.
+GLA_DEV double rcp64(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
 template <> struct prec<float> {
   static constexpr float eps = 0x1p-23f;           // Julia eps(Float32)
   static constexpr int mant = 23;

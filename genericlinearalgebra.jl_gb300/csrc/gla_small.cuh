@@ -71,4 +71,14 @@ GLA_DEV void batched(int total, const L& load, const F& use) {
   }
 }
 
+// Entry idx of the upper triangle, column by column: (i, j), i <= j, for
+// idx < 2^13 + 2^6 (the square root of 8 idx + 1 < 2^17 is off by less than
+// the distance to the next column's).
+GLA_DEV void upper_idx(int idx, int& i, int& j) {
+  j = (int)(0.5f * (sqrtf((float)(8 * idx + 1)) - 1.f));
+  j += (j + 1) * (j + 2) / 2 <= idx;
+  j -= j * (j + 1) / 2 > idx;
+  i = idx - j * (j + 1) / 2;
+}
+
 }  // namespace gla

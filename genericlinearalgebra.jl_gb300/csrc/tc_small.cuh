@@ -226,16 +226,24 @@ GLA_DEV void col_exps(int n, const T* __restrict__ M, int* out) {
 }
 
 // Scale exponents of the rows of an n x n column-major array: out[i] =
-// exp_of(max_j |hi(M(i, j))|), one thread per row (consecutive threads read
-// consecutive rows of a column); all threads of the CTA, ends with a barrier.
+// exp_of(max_j |hi(M(i, j))|), two threads per row, eight loads in flight
+// (consecutive threads read consecutive rows of a column); all 256 threads of
+// the CTA, ends with a barrier.
 template <class T>
 GLA_DEV void row_exps(int n, const T* __restrict__ M, int* out) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    float m = 0.f;
-#pragma unroll 4
-    for (int j = 0; j < n; j++) m = fmaxf(m, fabsf(hi_of(M[(size_t)j * n + i])));
-    out[i] = exp_of(m);
+  __shared__ float other[kM];
+  const int i = threadIdx.x & (kM - 1), ic = min(i, n - 1), h = threadIdx.x >> 7;
+  float m = 0.f;
+  for (int j0 = h * 8; j0 < n; j0 += 16) {
+    float x[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) x[u] = hi_of(M[(size_t)min(j0 + u, n - 1) * n + ic]);
+#pragma unroll
+    for (int u = 0; u < 8; u++) m = fmaxf(m, fabsf(x[u]));
   }
+  if (h == 1) other[i] = m;
+  __syncthreads();
+  if (h == 0 && i < n) out[i] = exp_of(fmaxf(m, other[i]));
   __syncthreads();
 }
 
