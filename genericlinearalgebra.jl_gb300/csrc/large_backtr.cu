@@ -24,7 +24,8 @@ constexpr int kBT = kBacktrNB;
 // Y (and, when Yt is given, its transpose: the K-major operand of the
 // tensor-core Z -= Y W2) from the reflectors stored below the subdiagonal.
 template <class T>
-__global__ void k_form_y(const T* __restrict__ A, long long lda, T* __restrict__ Y, int n, T* __restrict__ Yt) {
+__global__ void k_form_y(const T* __restrict__ A, long long lda, T* __restrict__ Y, int n, long long ldy,
+                         T* __restrict__ Yt) {
   const int j = blockIdx.y;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     T v;
@@ -34,8 +35,8 @@ __global__ void k_form_y(const T* __restrict__ A, long long lda, T* __restrict__
       v = T(1);
     else
       v = A[i + (long long)j * lda];
-    Y[i + (long long)j * n] = v;
-    if (Yt) Yt[j + (long long)i * n] = v;
+    Y[i + j * ldy] = v;
+    if (Yt) Yt[j + i * ldy] = v;
   }
 }
 
@@ -49,8 +50,8 @@ size_t larft_smem_bytes() {
 }
 
 template <class T>
-__global__ void __launch_bounds__(256) k_larft(const T* __restrict__ Y, const T* __restrict__ tau, T* __restrict__ Tm,
-                                               int n) {
+__global__ void __launch_bounds__(256) k_larft(const T* __restrict__ Y, long long ldy, const T* __restrict__ tau,
+                                               T* __restrict__ Tm, int n) {
   const int b = blockIdx.x, j0 = b * kBT, kb = min(kBT, n - 1 - j0);
   extern __shared__ __align__(16) unsigned char larft_sm[];
   T(*G)[kBT + 1] = reinterpret_cast<T(*)[kBT + 1]>(larft_sm);
@@ -67,7 +68,7 @@ __global__ void __launch_bounds__(256) k_larft(const T* __restrict__ Y, const T*
     for (int idx = tid; idx < 32 * kBT; idx += 256) {
       const int ii = idx % 32, c = idx / 32;
       const int i = i0 + ii;
-      Ys[ii][c] = (i < n && c < kb) ? Y[i + (long long)(j0 + c) * n] : T(0);
+      Ys[ii][c] = (i < n && c < kb) ? Y[i + (j0 + c) * ldy] : T(0);
     }
     __syncthreads();
 #pragma unroll 4
@@ -136,7 +137,12 @@ struct BacktrPlan {
   void* Tm = nullptr;
   void* Wp = nullptr;
   void* W2 = nullptr;   // T W, kBT x n (leading dimension kBT)
-  float* Yt = nullptr;  // FP32 with tensor cores: Y transposed
+  // FP32 with tensor cores: Y transposed; leading dimension of Y and Yt, a
+  // multiple of 16 bytes as their tensor maps want (otherwise n); and the same
+  // for Z where the caller's columns are not on 16-byte boundaries
+  float* Yt = nullptr;
+  long long ldy = 0;
+  float* Zp = nullptr;
   int* err = nullptr;   // error word of the tensor-core GEMMs (set by backtr_set_error_word)
   Oz64* oz = nullptr;   // FP64: the whole application on the tensor cores (set by backtr_set_oz64)
 };
@@ -158,11 +164,16 @@ int backtr_plan_create(BacktrPlan** out, int n, bool f64, bool tc) {
   auto alloc = [&](void** q, size_t bytes) {
     if (err == cudaSuccess) err = cudaMalloc(q, std::max<size_t>(bytes, 16));
   };
-  alloc(&p->Y, el * (size_t)n * n);
+  const bool use_tc = !f64 && tc && tc::tc_available();
+  p->ldy = use_tc ? (n + 3) & ~3 : n;
+  alloc(&p->Y, el * (size_t)p->ldy * n);
   alloc(&p->Tm, el * (size_t)p->nblk * kBT * kBT);
   alloc(&p->Wp, el * (size_t)p->splits * kBT * n);
   alloc(&p->W2, el * (size_t)kBT * n);
-  if (!f64 && tc && n % 4 == 0 && tc::tc_available()) alloc((void**)&p->Yt, sizeof(float) * (size_t)n * n);
+  if (use_tc) {
+    alloc((void**)&p->Yt, sizeof(float) * (size_t)p->ldy * n);
+    if (p->ldy != n) alloc((void**)&p->Zp, sizeof(float) * (size_t)p->ldy * n);
+  }
   if (err == cudaSuccess)
     err = f64 ? cudaFuncSetAttribute((const void*)k_larft<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)larft_smem_bytes<double>())
@@ -183,6 +194,7 @@ void backtr_plan_destroy(BacktrPlan* p) {
   cudaFree(p->Wp);
   cudaFree(p->W2);
   cudaFree(p->Yt);
+  cudaFree(p->Zp);
   delete p;
 }
 
@@ -191,31 +203,41 @@ void backtr_plan_destroy(BacktrPlan* p) {
 // B_b = I - Y_b T_b Y_b': Q Z applies the last block first, Q' Z applies
 // B_0' = I - Y_0 T_0' Y_0' first.
 template <class T>
-int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, long long ldz, int ncol, bool trans,
+int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, long long ldzu, int ncol, bool trans,
                cudaStream_t st) {
   const int n = p.n;
   if (n < 2 || ncol <= 0) return 0;
   T* Y = (T*)p.Y;
   // FP32 with tensor cores: both GEMMs of a block on tcgen05 (3xTF32) when
-  // the tensor maps of Y, Y' and Z can be built (16-byte-aligned columns)
+  // the tensor maps of Y, Y' and Z can be built (16-byte-aligned columns; a Z
+  // whose columns are not is copied into Zp and back: 2 n^2 words against
+  // n^3 products that take six times as long on the FP32 pipe)
   CUtensorMap mY, mYt;
-  const bool tc = sizeof(T) == 4 && p.Yt && p.err && (ldz % 4) == 0 && ((uintptr_t)Zall & 15) == 0 &&
-                  tc::tc_make_map(&mY, (const float*)Y, n, n, n, tc::kBM) &&
-                  tc::tc_make_map(&mYt, p.Yt, n, n, n, tc::kBM);
-  k_form_y<T><<<dim3((n + 255) / 256, n), 256, 0, st>>>(A, lda, Y, n, tc ? (T*)p.Yt : (T*)nullptr);
+  const bool aligned = (ldzu % 4) == 0 && ((uintptr_t)Zall & 15) == 0;
+  const long long ldy = p.ldy;
+  const bool tc = sizeof(T) == 4 && p.Yt && p.err && (aligned || p.Zp) &&
+                  tc::tc_make_map(&mY, (const float*)Y, n, n, ldy, tc::kBM) &&
+                  tc::tc_make_map(&mYt, p.Yt, n, n, ldy, tc::kBM);
+  k_form_y<T><<<dim3((n + 255) / 256, n), 256, 0, st>>>(A, lda, Y, n, ldy, tc ? (T*)p.Yt : (T*)nullptr);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return -1000 - (int)err;
   if (sizeof(T) == 8 && p.oz) {
-    err = oz64_backtr(p.oz, (double*)Y, (const double*)tau, (double*)Zall, ldz, ncol, trans, st);
+    err = oz64_backtr(p.oz, (double*)Y, (const double*)tau, (double*)Zall, ldzu, ncol, trans, st);
     return err == cudaSuccess ? 0 : -1000 - (int)err;
   }
-  k_larft<T><<<p.nblk, 256, larft_smem_bytes<T>(), st>>>(Y, tau, (T*)p.Tm, n);
+  k_larft<T><<<p.nblk, 256, larft_smem_bytes<T>(), st>>>(Y, ldy, tau, (T*)p.Tm, n);
   if ((err = cudaGetLastError()) != cudaSuccess) return -1000 - (int)err;
   const bool f64 = sizeof(T) == 8;
   const int bk = f64 ? GemmCfg<double>::BK : GemmCfg<float>::BK;
   for (int c0 = 0; c0 < ncol; c0 += n) {
   const int nc = std::min(n, ncol - c0);
-  T* Z = Zall + (long long)c0 * ldz;
+  T* const Zuser = Zall + (long long)c0 * ldzu;
+  const bool copied = tc && !aligned;
+  T* const Z = copied ? (T*)p.Zp : Zuser;
+  const long long ldz = copied ? ldy : ldzu;
+  if (copied && (err = cudaMemcpy2DAsync(Z, sizeof(T) * ldz, Zuser, sizeof(T) * ldzu, sizeof(T) * n, nc,
+                                         cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
+    return -1000 - (int)err;
   CUtensorMap mZ;
   const bool tcz = tc && tc::tc_make_map(&mZ, (const float*)Z, n, nc, ldz, tc::kBN);
   for (int bi = 0; bi < p.nblk; bi++) {
@@ -279,8 +301,8 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
     g.m = kb;
     g.n = nc;
     g.k = mrows;
-    g.A = Y + r0 + (long long)j0 * n;
-    g.lda = n;
+    g.A = Y + r0 + j0 * ldy;
+    g.lda = ldy;
     g.B = Z + r0;
     g.ldb = ldz;
     g.C = p.Wp;
@@ -301,8 +323,8 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
     h.m = mrows;
     h.n = nc;
     h.k = kb;
-    h.A = Y + r0 + (long long)j0 * n;
-    h.lda = n;
+    h.A = Y + r0 + j0 * ldy;
+    h.lda = ldy;
     h.B = p.W2;
     h.ldb = kBT;
     h.C = Z + r0;
@@ -311,6 +333,9 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
     h.beta = 1.0;
     if ((err = gemm_launch(f64, false, false, false, h, 1, st)) != cudaSuccess) return -1000 - (int)err;
   }
+  if (copied && (err = cudaMemcpy2DAsync(Zuser, sizeof(T) * ldzu, Z, sizeof(T) * ldz, sizeof(T) * n, nc,
+                                         cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
+    return -1000 - (int)err;
   }
   return 0;
 }
