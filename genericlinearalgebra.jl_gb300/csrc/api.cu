@@ -139,7 +139,15 @@ struct gla_plan_s {
   int* pin_pending = nullptr;
   df64* d_adj = nullptr;  // adjoint workspace (allocated by the first gla_plan_adjoint)
   double* h_adj = nullptr;  // device staging of gla_plan_adjoint_host
-  LargeAdjoint* adj_large = nullptr;  // adjoint context of the orders above GLA_MAX_SMALL_N
+  // adjoint of the orders above GLA_MAX_SMALL_N: a context and, where several
+  // matrices run side by side, a stream with its join event each
+  struct AdjointSide {
+    LargeAdjoint* ctx = nullptr;
+    cudaStream_t stream = nullptr;
+    cudaEvent_t join = nullptr;
+  };
+  std::vector<AdjointSide> adj_large;
+  cudaEvent_t adj_fork = nullptr;
   // orders above GLA_MAX_SMALL_N: solved one at a time by the large path
   std::vector<int> large_idx;           // batch indices, in batch order
   std::vector<int> large_chain;         // the chain each of them belongs to
@@ -512,7 +520,12 @@ int gla_plan_destroy(gla_plan_t p) {
   cudaFreeHost(p->pin_pending);
   cudaFree(p->d_adj);
   cudaFree(p->h_adj);
-  large_adjoint_destroy(p->adj_large);
+  if (p->adj_fork) cudaEventDestroy(p->adj_fork);
+  for (auto& a : p->adj_large) {
+    large_adjoint_destroy(a.ctx);
+    if (a.stream) cudaStreamDestroy(a.stream);
+    if (a.join) cudaEventDestroy(a.join);
+  }
   for (auto& ch : p->chains) {
     large_destroy(ch.ctx);
     refine_large_destroy(ch.ref);
@@ -1229,29 +1242,64 @@ int gla_plan_adjoint(gla_plan_t p, const double* w, const double* V, const doubl
   if (!(gap_rel == gap_rel)) return -7;
   const double gr = gap_rel > 0 ? gap_rel : 1e-10;
   cudaStream_t st = (cudaStream_t)stream;
+  if (!p->large_idx.empty()) {
+    if (!p->adj_fork) GLA_CUDA(cudaEventCreateWithFlags(&p->adj_fork, cudaEventDisableTiming));
+    GLA_CUDA(cudaEventRecord(p->adj_fork, st));
+  }
   if (p->nwork > 0) {  // orders <= GLA_MAX_SMALL_N: one CTA per matrix
     if (!p->d_adj) GLA_CUDA(cache_alloc(&p->d_adj, adjoint_workspace_bytes(p->a_elems)));
     GLA_CUDA(launch_adjoint(p->nwork, st, p->d_desc, p->d_perm_bucket, w, V, wbar, Vbar, Abar, p->d_adj, p->a_elems,
                             gr));
   }
-  if (!p->large_idx.empty()) {  // larger orders: three FP64 GEMMs each, one shared workspace
-    int nl = 0;
-    for (int b : p->large_idx) nl = std::max(nl, (int)p->n[b]);
-    if (!p->adj_large) {
-      int rc = large_adjoint_create(&p->adj_large, nl);
-      if (rc) return rc;
+  if (p->large_idx.empty()) return 0;
+  // larger orders: three FP64-accurate GEMMs each, about 17 launches. Those of
+  // an order up to kSideBySideMaxN leave most of the GPU idle, so several
+  // such matrices go over up to kMaxSide streams with a workspace each,
+  // beside the small orders (23 matrices of orders 129 .. 500 one after
+  // another: 4 ms); larger ones fill the GPU one at a time.
+  int nl = 0;
+  for (int b : p->large_idx) nl = std::max(nl, (int)p->n[b]);
+  const size_t sides = nl <= kSideBySideMaxN ? std::min<size_t>(kMaxSide, p->large_idx.size()) : 1;
+  while (p->adj_large.size() < sides) {
+    gla_plan_s::AdjointSide a;
+    int rc = large_adjoint_create(&a.ctx, nl);
+    if (!rc && sides > 1) {
+      cudaError_t e = cudaStreamCreateWithFlags(&a.stream, cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a.join, cudaEventDisableTiming);
+      if (e != cudaSuccess) rc = -1000 - (int)e;
     }
-    for (int b : p->large_idx) {
-      const int nb = (int)p->n[b];
-      int64_t aoff = 0, woff = 0;
-      for (int q = 0; q < b; q++) {
-        aoff += p->n[q] * p->n[q];
-        woff += p->n[q];
-      }
-      GLA_CUDA(large_adjoint(p->adj_large, nb, w + woff, V + aoff, nb, wbar + woff, Vbar + aoff, nb, Abar + aoff, nb,
-                             gr, st));
+    if (rc) {
+      large_adjoint_destroy(a.ctx);
+      if (a.stream) cudaStreamDestroy(a.stream);
+      if (a.join) cudaEventDestroy(a.join);
+      return rc;
     }
+    p->adj_large.push_back(a);
   }
+  std::vector<int64_t> aoff(p->n.size() + 1, 0), woff(p->n.size() + 1, 0);
+  for (size_t q = 0; q < p->n.size(); q++) {
+    aoff[q + 1] = aoff[q] + p->n[q] * p->n[q];
+    woff[q + 1] = woff[q] + p->n[q];
+  }
+  std::vector<int> order(p->large_idx.begin(), p->large_idx.end());
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return p->n[x] > p->n[y]; });
+  cudaError_t e = cudaSuccess;
+  if (sides > 1)
+    for (size_t t = 0; t < sides && e == cudaSuccess; t++) 
+      e = cudaStreamWaitEvent(p->adj_large[t].stream, p->adj_fork, 0);
+  for (size_t k = 0; k < order.size() && e == cudaSuccess; k++) {
+    const int b = order[k], nb = (int)p->n[b];
+    auto& a = p->adj_large[k % sides];
+    e = large_adjoint(a.ctx, nb, w + woff[b], V + aoff[b], nb, wbar + woff[b], Vbar + aoff[b], nb, Abar + aoff[b], nb,
+                      gr, sides > 1 ? a.stream : st);
+  }
+  if (sides > 1)
+    for (size_t t = 0; t < sides; t++) {  // joined even after an error: the caller may free the buffers
+      cudaError_t j = cudaEventRecord(p->adj_large[t].join, p->adj_large[t].stream);
+      if (j == cudaSuccess) j = cudaStreamWaitEvent(st, p->adj_large[t].join, 0);
+      if (e == cudaSuccess) e = j;
+    }
+  GLA_CUDA(e);
   return 0;
 }
 
