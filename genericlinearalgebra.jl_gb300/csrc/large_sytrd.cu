@@ -88,6 +88,9 @@ struct SytrdArgs {
   T* qfp;            // [G]
   T* dots;           // [3][kSytrdNB][nDCH]
   int nDCH;
+  const int2* F;     // fixed-point panels: the trailing matrix (leading dimension n), see fix_of
+  const int* fe;     // its exponents, [tile column][fch]
+  int fch;
   const int* ustart; // of this shape: first SYMV unit of each tile column; ustart[nTC] = total
   int nTC;
   unsigned* bar;     // arrival counter (monotonic over the launches of one tridiagonalisation)
@@ -249,6 +252,167 @@ __device__ T symv_unit(const SytrdArgs<T>& a, int j, int s, int J, int ch, T* sv
   return qf;
 }
 
+// ---- The FP64 SYMV in fixed point, for trailing orders above kFixedMin.
+//
+// Every entry of the trailing matrix meets the vector twice (row and column
+// sums), and an FP64 product costs a sub-partition 64 cycles: at order 4096
+// the SYMV took 16 of the 27 us of a column, at 70% of the FP64 rate. The
+// trailing matrix is the same for the 32 columns of a panel, so it is turned
+// once per panel into integers of 57 bits, scaled by the largest entry of
+// their 64 x 32 unit, as two digits of 28 bits; the vector is split alike
+// unit by unit. A product is then three 32 x 32 -> 64-bit multiply-adds of 4
+// cycles (the product of the low digits, 2^-58 of the unit's largest, is left
+// out), the sums are exact in 64 bits, and the reductions over lanes are
+// integer additions. What is rounded is the entries, at 2^-57 of their unit's
+// largest, and the unit's sums, at 2^-56: below the 2^-53 of each FP64 sum
+// (residual and orthogonality of orders 1100 .. 4096, also of graded
+// matrices, as with FP64 products to 3%).
+//
+// Reduction of order 4096: 26.9 -> 18.5 us a column, 1500: 10.9 -> 10.3. Below
+// about 1000 a warp has less than a unit of this size, and smaller FP64 units
+// are faster (a limit of 600: order 777 9.8 us a column instead of 9.1).
+constexpr int kFixedMin = 1000;
+constexpr int kFixW = 32, kFixR = 64;  // columns and rows of a unit (the last of kShapes)
+
+// e with |x| < 2^e for the top word of the largest |x| (at least 2^-400: the
+// working matrix has its largest entry in [1, 2)).
+GLA_DEV int fix_exp(unsigned top) { return max((int)(top >> 20) - 1022, -400); }
+GLA_DEV unsigned fix_top(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
+// x 2^(56 - e), |x| < 2^e, rounded: digits (hi, lo) with hi 2^28 + lo, |lo| <= 2^27.
+GLA_DEV int2 fix_of(double x, int e) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int ex = (int)(b >> 52) & 0x7ff, s = ex - 1019 - e;  // the mantissa's shift, at most 3
+  const unsigned long long m = (b & 0xfffffffffffffull) | (ex ? 1ull << 52 : 0ull);
+  const unsigned long long f = s >= 0 ? m << s : s > -64 ? ((m >> (-s - 1)) + 1) >> 1 : 0ull;
+  const long long v = (long long)b < 0 ? -(long long)f : (long long)f;
+  const int hi = (int)((v + (1ll << 27)) >> 28);
+  return make_int2(hi, (int)(v - ((long long)hi << 28)));
+}
+// The sum s1 2^56 + s2 2^28 of products of digits, in units of 2^56.
+GLA_DEV long long fix_sum(long long s1, long long s2) { return s1 + ((s2 + (1ll << 27)) >> 28); }
+// v 2^(e - 56), e >= -800.
+GLA_DEV double fix_value(long long v, int e) { return (double)v * __hiloint2double((1023 - 56 + e) << 20, 0); }
+
+// The units of the tile columns J0 .. of the lower triangle (grid: chunk of
+// rows, tile column).
+__global__ void __launch_bounds__(256) k_sytrd_fix(const double* __restrict__ A, long long ld, int n, int J0,
+                                                   int2* __restrict__ F, int* __restrict__ fe, int fch) {
+  __shared__ unsigned red[8];
+  const int J = J0 + blockIdx.y, c0 = J * kFixW, r0 = c0 + (int)blockIdx.x * kFixR, tid = threadIdx.x;
+  if (r0 >= n) return;
+  const int r = r0 + (tid & (kFixR - 1)), cb = c0 + (tid >> 6);
+  double x[8];
+  unsigned m = 0;
+#pragma unroll
+  for (int u = 0; u < 8; u++) {
+    const int c = cb + 4 * u;
+    x[u] = (r < n && c <= r) ? A[r + c * ld] : 0.0;
+    m = max(m, fix_top(x[u]));
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((tid & 31) == 0) red[tid >> 5] = m;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; w++) m = max(m, red[w]);
+  const int e = fix_exp(m);
+  if (tid == 0) fe[J * fch + blockIdx.x] = e;
+#pragma unroll
+  for (int u = 0; u < 8; u++) {
+    const int c = cb + 4 * u;
+    if (r < n && c < n) F[r + (long long)c * n] = fix_of(x[u], e);
+  }
+}
+
+// symv_unit<double, 32, 2> on F, eight columns at a time.
+GLA_DEV double symv_unit_fixed(const SytrdArgs<double>& a, int j, int s, int J, int ch, int2* sv) {
+  const int lane = threadIdx.x & 31, n = a.n;
+  const int c0 = J * kFixW, r0 = c0 + ch * kFixR, cc = c0 + lane;
+  int2 nx[2][8];  // the next eight columns, on their way while these are multiplied
+  auto fetch = [&](int h) {
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int r = r0 + lane + 32 * q;
+      const int2* base = a.F + r + (long long)(c0 + h) * n;
+#pragma unroll
+      for (int i = 0; i < 8; i++) nx[q][i] = (r < n && c0 + h + i < n) ? base[(long long)i * n] : make_int2(0, 0);
+    }
+  };
+  fetch(0);
+  const double vc = cc < n ? a_at(a.A, a.ld, j, s, cc) : 0.0;
+  double vr[2];
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int r = r0 + lane + 32 * q;
+    vr[q] = r < n ? a_at(a.A, a.ld, j, s, r) : 0.0;
+  }
+  const int ea = a.fe[J * a.fch + ch];
+  const int ec = fix_exp(__reduce_max_sync(0xffffffffu, fix_top(vc)));
+  const int er = fix_exp(__reduce_max_sync(0xffffffffu, max(fix_top(vr[0]), fix_top(vr[1]))));
+  sv[lane] = fix_of(vc, ec);
+  const int2 w[2] = {fix_of(vr[0], er), fix_of(vr[1], er)};
+  __syncwarp();
+  long long r1[2] = {0, 0}, r2[2] = {0, 0};
+  double qf = 0.0;
+#pragma unroll 1
+  for (int h = 0; h < kFixW; h += 8) {
+    int2 x[2][8];
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+      for (int i = 0; i < 8; i++) x[q][i] = nx[q][i];
+    if (h + 8 < kFixW) fetch(h + 8);
+    long long v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int2 xc = sv[h + i];
+      const bool diag = ch == 0 && lane == h + i;  // F is zero above the diagonal; on it only the row sum counts
+      long long c1 = 0, c2 = 0;
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int2 f = x[q][i];
+        r1[q] += (long long)f.x * xc.x;
+        r2[q] += (long long)f.x * xc.y;
+        r2[q] += (long long)f.y * xc.x;
+        const int wx = q == 0 && diag ? 0 : w[q].x, wy = q == 0 && diag ? 0 : w[q].y;
+        c1 += (long long)f.x * wx;
+        c2 += (long long)f.x * wy;
+        c2 += (long long)f.y * wx;
+      }
+      v[i] = fix_sum(c1, c2);
+    }
+    // column sums across the warp: lane l keeps column h + l / 4
+#pragma unroll
+    for (int half = 4; half >= 1; half >>= 1) {
+      const bool up = (lane & (4 * half)) != 0;
+#pragma unroll
+      for (int i = 0; i < half; i++) {
+        const long long send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * half);
+      }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    const int ci = h + (lane >> 2);
+    const double xv = __shfl_sync(0xffffffffu, vc, ci);
+    if ((lane & 3) == 0 && c0 + ci < n) {
+      const double y = fix_value(v[0], ea + er);
+      a.Qp[(long long)ch * n + c0 + ci] = y;
+      qf = fma(y, xv, qf);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int r = r0 + lane + 32 * q;
+    if (r < n) {
+      const double y = fix_value(fix_sum(r1[q], r2[q]), ea + ec);
+      a.P[(long long)(J - a.k0 / kFixW) * n + r] = y;
+      qf = fma(y, vr[q], qf);
+    }
+  }
+  __syncwarp();
+  return qf;
+}
+
 // Rows of the trailing range [s, n) owned by CTA g.
 GLA_DEV void own_rows(int s, int n, int& lo, int& hi) {
   const int m = n - s, G = gridDim.x;
@@ -310,7 +474,7 @@ constexpr int kDotV = 1;  // sum_r a_r V[r, q], q < c
 constexpr int kDotW = 2;  // sum_r a_r W[r, q]
 
 // Microseconds per column (reduction of order 777 / 4096 in FP64, of order
-// 2048 in FP32): 9.1 / 26.9 and 6.0, of which the two grid barriers are about
+// 2048 in FP32): 9.1 / 18.5 and 6.0, of which the two grid barriers are about
 // 3.5; before units by shape, this split and the short serial chains below
 // 19.4 / 32.9 and 7.9.
 //
@@ -322,7 +486,7 @@ constexpr int kDotW = 2;  // sum_r a_r W[r, q]
 // as there are (four sums in six), and by one warp. FP32, bound by the round
 // trips to L2: all warps do both, with as many loads in flight as there are
 // threads.
-template <class T, int CW, int NQ, bool CL>
+template <class T, int CW, int NQ, bool CL, bool FX = false>
 __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
   constexpr int RC = 32 * NQ;
   constexpr bool kSplit = sizeof(T) == 8;
@@ -390,7 +554,10 @@ __global__ void __launch_bounds__(kPT, 1) k_sytrd_panel(const SytrdArgs<T> a) {
             const int mid = (lo + hi + 1) >> 1;
             if (sust[mid] <= ug) lo = mid; else hi = mid - 1;
           }
-          qf += symv_unit<T, CW, NQ>(a, j, s, Jb + lo, ug - sust[lo], svcol[wid]);
+          if constexpr (FX)
+            qf += symv_unit_fixed(a, j, s, Jb + lo, ug - sust[lo], reinterpret_cast<int2*>(svcol[wid]));
+          else
+            qf += symv_unit<T, CW, NQ>(a, j, s, Jb + lo, ug - sust[lo], svcol[wid]);
         } else {
           const int du = u - nsym;
           const int kind = du < ndch ? kDotA : (du - ndch) / (c * ndch) + 1;
@@ -661,6 +828,9 @@ struct SytrdPlan {
   bool f64 = true;
   bool cluster = false;   // the device can hold a cluster: small trailing orders run on it
   bool cluster_only = false;  // and all others too
+  int2* F = nullptr;      // FP64, orders above kFixedMin: the trailing matrix in fixed point, n x n
+  int* fe = nullptr;      // exponents of its units, [tile column][fch]
+  int fch = 0;
   Oz64* oz = nullptr;     // FP64: trailing updates on the tensor cores (set by sytrd_set_oz64)
 };
 
@@ -728,9 +898,10 @@ int panel_shape(int m, bool f64) {
   return sh;
 }
 template <class T>
-const void* panel_kernel(int sh, bool cluster) {
+const void* panel_kernel(int sh, bool cluster, bool fixed = false) {
   static_assert(kNumShapes == 4, "one kernel per shape");
   if constexpr (sizeof(T) == 8) {
+    if (fixed) return (const void*)k_sytrd_panel<T, kFixW, kFixR / 32, false, true>;
     if (cluster && sh == 0) return (const void*)k_sytrd_panel<T, kShapes[0].cw, kShapes[0].nq, true>;
     if (cluster && sh == 1) return (const void*)k_sytrd_panel<T, kShapes[1].cw, kShapes[1].nq, true>;
     if (cluster && sh == 2) return (const void*)k_sytrd_panel<T, kShapes[2].cw, kShapes[2].nq, true>;
@@ -743,7 +914,8 @@ const void* panel_kernel(int sh, bool cluster) {
 }
 // One panel: over the whole GPU as a cooperative launch, or as one cluster.
 template <class T>
-cudaError_t launch_panel(const SytrdPlan& sp, const SytrdArgs<T>& a, int sh, bool cluster, cudaStream_t st) {
+cudaError_t launch_panel(const SytrdPlan& sp, const SytrdArgs<T>& a, int sh, bool cluster, bool fixed,
+                         cudaStream_t st) {
   const int G = cluster ? kClusterG : sp.G;
   cudaLaunchAttribute at[1];
   if (cluster) {
@@ -762,7 +934,7 @@ cudaError_t launch_panel(const SytrdPlan& sp, const SytrdArgs<T>& a, int sh, boo
   cfg.attrs = at;
   cfg.numAttrs = 1;
   void* args[] = {(void*)&a};
-  return cudaLaunchKernelExC(&cfg, panel_kernel<T>(sh, cluster), args);
+  return cudaLaunchKernelExC(&cfg, panel_kernel<T>(sh, cluster, fixed), args);
 }
 
 template <class T>
@@ -785,6 +957,9 @@ cudaError_t sytrd_run(SytrdPlan& sp, T* A, long long lda, T* d, T* e, T* tau, cu
   a.qfp = (T*)sp.qfp;
   a.dots = (T*)sp.dots;
   a.nDCH = sp.nDCH;
+  a.F = sp.F;
+  a.fe = sp.fe;
+  a.fch = sp.fch;
   a.bar = sp.bar;
   a.err = sp.err;
   T* VW = (T*)sp.VW;
@@ -802,10 +977,19 @@ cudaError_t sytrd_run(SytrdPlan& sp, T* A, long long lda, T* d, T* e, T* tau, cu
     if (!cluster) bar_base += 2u * (unsigned)nbp * (unsigned)sp.G;  // barriers per launch: 1 + nbp + (nbp - 1)
     // (a cluster has a tenth of the warps: the shape of a trailing order
     // with that many units per warp)
-    const int sh = panel_shape(cluster ? std::min(3 * m, kMaxOrder) : m, sizeof(T) == 8);
+    const bool fixed = sp.F && m > kFixedMin && !cluster;
+    const int sh = fixed ? kNumShapes - 1 : panel_shape(cluster ? std::min(3 * m, kMaxOrder) : m, sizeof(T) == 8);
+    if constexpr (sizeof(T) == 8) {
+      if (fixed) {
+        const int J0 = k0 / kFixW;
+        k_sytrd_fix<<<dim3((n - k0 + kFixR - 1) / kFixR, (n + kFixW - 1) / kFixW - J0), 256, 0, st>>>(
+            A, lda, n, J0, sp.F, sp.fe, sp.fch);
+        if ((err = cudaGetLastError()) != cudaSuccess) return err;
+      }
+    }
     a.nTC = (n + kShapes[sh].cw - 1) / kShapes[sh].cw;
     a.ustart = sp.ustart + sp.uoff[sh];
-    if ((err = launch_panel(sp, a, sh, cluster, st)) != cudaSuccess) return err;
+    if ((err = launch_panel(sp, a, sh, cluster, fixed, st)) != cudaSuccess) return err;
     const int t = k0 + nbp;
     if (t < n - 1) {  // trailing update A[t:, t:] -= V W' + W V' (lower tiles)
       if (sizeof(T) == 4 && sytrd_update_tc(sp, (float*)A, lda, n, t, nbp, st, &err)) {
@@ -856,8 +1040,9 @@ cudaError_t sytrd_plan_create(SytrdPlan** out, int n, bool f64, bool tc) {
   // order's, so that a plan made later never lowers it below an earlier
   // plan's launches.
   const int vwbytes = 2 * panel_rows(0, kMaxOrder, std::max(nsm, 1)) * kSytrdNB * (f64 ? 8 : 4);
-  for (int sh = f64 ? 0 : kNumShapes - 1; sh < kNumShapes; sh++) {
-    const void* kfn = f64 ? panel_kernel<double>(sh, false) : panel_kernel<float>(sh, false);
+  const bool fx = f64 && n > kFixedMin;
+  for (int sh = f64 ? 0 : kNumShapes - 1; sh < kNumShapes + fx; sh++) {  // (with fx the fixed-point kernel, last)
+    const void* kfn = f64 ? panel_kernel<double>(sh, false, sh == kNumShapes) : panel_kernel<float>(sh, false);
     if (err == cudaSuccess) err = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, vwbytes);
     if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, kPT, vwbytes);
     if (err == cudaSuccess && per < 1) err = cudaErrorCooperativeLaunchTooLarge;
@@ -925,6 +1110,11 @@ cudaError_t sytrd_plan_create(SytrdPlan** out, int n, bool f64, bool tc) {
   alloc(&sp->dots, el * 3 * kSytrdNB * sp->nDCH);
   alloc(&sp->VW, el * (size_t)n * 2 * kSytrdNB);
   alloc((void**)&sp->bkidx, sizeof(int) * bk.size());
+  if (fx) {
+    sp->fch = (n + kFixR - 1) / kFixR;
+    alloc((void**)&sp->F, sizeof(int2) * (size_t)n * n);
+    alloc((void**)&sp->fe, sizeof(int) * (size_t)((n + kFixW - 1) / kFixW) * sp->fch);
+  }
   alloc((void**)&sp->bar, 2 * sizeof(unsigned));
   alloc((void**)&sp->err, sizeof(int));
   if (err == cudaSuccess)
@@ -951,6 +1141,8 @@ void sytrd_plan_destroy(SytrdPlan* sp) {
   cudaFree(sp->VW);
   cudaFree(sp->VWt);
   cudaFree(sp->bkidx);
+  cudaFree(sp->F);
+  cudaFree(sp->fe);
   cudaFree(sp->bar);
   cudaFree(sp->err);
   delete sp;
