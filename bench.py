@@ -96,13 +96,13 @@ def refine_roofline(achieved, peak, batch, fp32):
     "tridiag" phase); peak = MEASURED_PEAKS.json bf16 (burst). The kernel is
     latency-bound (per-column barriers of the FP32 reduction, the slicing),
     so the fraction is small by construction; fp32 gives its FP32-pipe work
-    (reduction, Q, X = QY, X E) against the SGEMM FMA rate of this run.
+    (reduction, X = QY, X E) against the SGEMM FMA rate of this run.
     traffic: DRAM bytes of one launch over the first 1024 workload matrices
     (same order distribution), from an ncu capture, scaled by the matrix
     count; the algorithmic bytes are ~20 sum(n^2) = 0.48 GB per step, the
     rest is the per-matrix double-float scratch of the refinement (56 n^2
-    bytes) and the products' slice scratch (224 KB per CTA, rewritten for
-    every product), which do not stay in L2."""
+    bytes) and the products' slice scratch (0.9 MB per CTA, rewritten by
+    every iteration), which do not stay in L2."""
     return {"kernel": "k_solve_refine", "bound": "tensor", "achieved": achieved, "peak": peak,
             "unit": "TFLOP/s", "frac": (achieved / peak) if peak else None,
             "traffic": REFINE_DRAM_BYTES_PER_1024 * batch / 1024 if REFINE_DRAM_BYTES_PER_1024 else None,
@@ -412,14 +412,14 @@ def run_ours(args):
         # Roofline of the refined step's dominant kernel, the persistent
         # k_solve_refine (its time is the plan's "tridiag" phase): bf16
         # tensor flops of the refinement's sliced products (refine_roofline),
-        # and beside them its FP32-pipe flops: the reduction, Q and X = QY
-        # ((4/3 + 4/3 + 2) n^3) and X E (2 n^3 per iteration) against the
+        # and beside them its FP32-pipe flops: the reduction and X = QY
+        # ((4/3 + 2) n^3) and X E (2 n^3 per iteration) against the
         # SGEMM rate measured in this run.
         sg = measured_sgemm_tflops(torch)
         fused_ms = ph.get("tridiag", 0.0)
         sec = fused_ms * 1e-3
         tflops = 168.0 * c["refine_n3"] / sec / 1e12 if sec > 0 else 0.0
-        f32_flops = (4.0 / 3.0 + 4.0 / 3.0 + 2.0) * ns3 + 2.0 * c["refine_n3"]
+        f32_flops = (4.0 / 3.0 + 2.0) * ns3 + 2.0 * c["refine_n3"]
         f32_ach = f32_flops / sec / 1e12 if sec > 0 else 0.0
         mp = measured_peaks_file()
         bf16_peak = (mp or {}).get("bf16_tflops")

@@ -148,7 +148,7 @@ struct gla_plan_s {
   };
   std::vector<AdjointSide> adj_large;
   cudaEvent_t adj_fork = nullptr;
-  // orders above GLA_MAX_SMALL_N: solved one at a time by the large path
+  // orders above GLA_MAX_SMALL_N: solved by the large path
   std::vector<int> large_idx;           // batch indices, in batch order
   std::vector<int> large_chain;         // the chain each of them belongs to
   // A chain is a context (and, for F32_REFINED, the refinement) of one order

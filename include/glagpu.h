@@ -115,11 +115,13 @@ const char* gla_status_string(int status);
  * n[0..batch) (host array, 0 <= n[b] <= GLA_MAX_N).
  *
  * Orders up to GLA_MAX_SMALL_N are solved together (one CTA per matrix,
- * size-bucketed). Larger orders are solved one at a time with the whole GPU:
- * blocked Householder tridiagonalisation, divide and conquer on the
- * tridiagonal, compact-WY back-transformation; such plans synchronise the
- * stream inside execute and do not support GLA_FLAG_GRAPH or
- * GLA_PREC_F32_REFINED (those return -8 / -2).
+ * size-bucketed). Larger orders take the whole GPU one after another, or,
+ * where several of them are of order 1024 or less, run side by side (up to
+ * eight host threads with a stream each during the call): blocked Householder
+ * tridiagonalisation, divide and conquer on the tridiagonal, compact-WY
+ * back-transformation, with GLA_PREC_F32_REFINED in FP32 and refined; such
+ * plans synchronise the stream inside execute and do not support
+ * GLA_FLAG_GRAPH (-8).
  *
  * Packed arena layout used by the execute calls: matrix b is n[b] x n[b],
  * column-major with leading dimension n[b], at element offset
