@@ -66,8 +66,8 @@ GLA_DEV constexpr uint32_t idesc_n(int n) {
 }
 static_assert(kS * kNT <= kTmemCols, "level accumulators exceed the CTA's TMEM columns");
 // Slices of the operands in the scratch, K-major rows in slabs of K = 16. As
-// P: [slab][slice][8-row group][2 core matrices], so that a slab is one bulk
-// copy; A at slot 0 and X' at slot 1. As Q: the columns of [X | Y], the 8-column
+// P: [slab][8-row group][slice][2 core matrices], so that a slab's first rows,
+// those that the upper triangle's pass needs, are one bulk copy; A at slot 0 and X' at slot 1. As Q: the columns of [X | Y], the 8-column
 // groups of Y after those of X, [slab][4 groups][slice][group][2 core
 // matrices], so that a pass's part of a slab is one bulk copy; slots 2 and 3.
 constexpr int kRG = 256;                                     // one 8-row group of one slice of a slab
@@ -450,14 +450,14 @@ static __device__ __noinline__ void slice_operand(unsigned char* ops, int opP, i
     for (int t = 0; t < 4; t++) {
       const int kc = kc0 + t, ks = kc >> 1, in = (kc & 1) * 128 + lane * 4;
       if (kc >= nkc) break;
-      unsigned char* dp = ops + (size_t)opP * kOpBytes + ((size_t)ks * kS * nrg + rg) * kRG + in;
+      unsigned char* dp = ops + (size_t)opP * kOpBytes + (size_t)(ks * nrg + rg) * (kS * kRG) + in;
       unsigned char* dq =
           ops + (size_t)2 * kOpBytes + (size_t)(ks * nblk + (v >> 2)) * kStageQ + (v & 3) * kRG + in;
       uint32_t w[kS];
       slices7(x[t][0], x[t][1], e, w);
       if (opP >= 0)
 #pragma unroll
-        for (int s = 0; s < kS; s++) *reinterpret_cast<uint32_t*>(dp + s * nrg * kRG) = w[s];
+        for (int s = 0; s < kS; s++) *reinterpret_cast<uint32_t*>(dp + s * kRG) = w[s];
       if (vq >= 0)
 #pragma unroll
         for (int s = 0; s < kS; s++) *reinterpret_cast<uint32_t*>(dq + s * (kNT / 8) * kRG) = w[s];
@@ -465,9 +465,9 @@ static __device__ __noinline__ void slice_operand(unsigned char* ops, int opP, i
   }
 }
 
-// Descriptor of a K = 16 slab: row groups kRG bytes apart.
-GLA_DEV uint64_t desc_k16(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFF) | (uint64_t)(128u >> 4) << 16 | (uint64_t)((uint32_t)kRG >> 4) << 32 |
+// Descriptor of a K = 16 slab: row groups sbo bytes apart.
+GLA_DEV uint64_t desc_k16(uint32_t saddr, int sbo) {
+  return (uint64_t)((saddr >> 4) & 0x3FFF) | (uint64_t)(128u >> 4) << 16 | (uint64_t)((uint32_t)sbo >> 4) << 32 |
          (uint64_t)1 << 46;
 }
 
@@ -494,9 +494,12 @@ static __device__ __noinline__ bool gemm_sliced(Ctx& c, int n, int nq, int opP, 
     if (4 * av >= nv) return true;
     const uint32_t g = c.asked;
     if (g >= 2 && !oz::mbar_wait(&c.sh->empty[g & 1], ((g >> 1) - 1) & 1, c.err)) return false;
+    // the row groups that the pass's columns need (upper: up to the last column)
+    const int v1 = min(4 * av + 4, nv);
+    const int rows = nq == 1 || (4 * av < nrg && v1 > nrg) ? nrg : v1 <= nrg ? v1 : v1 - nrg;
     unsigned char* st = c.slabs + (g & 1) * kStage;
-    oz::mbar_expect_tx(&c.sh->full[g & 1], (uint32_t)(kS * nrg * kRG + kStageQ));
-    oz::bulk_g2s(st, srcP + (size_t)ak * (kS * nrg * kRG), (uint32_t)(kS * nrg * kRG), &c.sh->full[g & 1]);
+    oz::mbar_expect_tx(&c.sh->full[g & 1], (uint32_t)(rows * kS * kRG + kStageQ));
+    oz::bulk_g2s(st, srcP + (size_t)ak * (kS * nrg * kRG), (uint32_t)(rows * kS * kRG), &c.sh->full[g & 1]);
     oz::bulk_g2s(st + kStageP, srcQ + (size_t)(ak * nblk + av) * kStageQ, (uint32_t)kStageQ, &c.sh->full[g & 1]);
     c.asked = g + 1;
     if (++ak == nks) {
@@ -518,10 +521,10 @@ static __device__ __noinline__ bool gemm_sliced(Ctx& c, int n, int nq, int opP, 
         c.landed = g + 1;
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t st = oz::smem_u32(c.slabs + (g & 1) * kStage);
-        const uint64_t a0 = desc_k16(st), b0 = desc_k16(st + kStageP);
+        const uint64_t a0 = desc_k16(st, kS * kRG), b0 = desc_k16(st + kStageP, kRG);
 #pragma unroll
         for (int s = 1; s <= kS; s++)  // (see gemm)
-          oz::mma_f16(c.sh->tmem + (uint32_t)((s - 1) * kNT), a0 + (uint64_t)(((s - 1) * nrg * kRG) >> 4), b0,
+          oz::mma_f16(c.sh->tmem + (uint32_t)((s - 1) * kNT), a0 + (uint64_t)(((s - 1) * kRG) >> 4), b0,
                       idesc_n(kNT * (kS + 1 - s)), (ks == 0 && s == 1) ? 0u : 1u);
         oz::mma_commit(&c.sh->empty[g & 1]);
         if (ks + 1 == nks) oz::mma_commit(&c.sh->bar);
