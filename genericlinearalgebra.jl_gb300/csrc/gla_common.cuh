@@ -156,18 +156,4 @@ GLA_DEV unsigned long long warp_max_u64(unsigned long long v) {
   }
   return v;
 }
-
-// Block-wide sum over all threads of the block; red must hold blockDim/32
-// entries. Every thread gets the result.
-template <class T> GLA_DEV T block_sum(T v, T* red) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  v = warp_sum(v);
-  __syncthreads();
-  if (lane == 0) red[wid] = v;
-  __syncthreads();
-  T s = 0;
-  for (int i = 0; i < nw; i++) s += red[i];
-  return s;
-}
-
 }  // namespace gla

@@ -198,14 +198,7 @@ GLA_DEV int exp_of(float m) { return m > 0.f ? ilogbf(m) + 1 : 0; }
 // their loads in flight per warp (all threads of the CTA; ends with a barrier). A row of P whose
 // exponent is given this way (P = X', or P = A symmetric) needs no pass of
 // its own.
-template <class T>
-GLA_DEV float hi_of(const T& v);
-template <>
-GLA_DEV float hi_of<float>(const float& v) { return v; }
-template <>
-GLA_DEV float hi_of<df64>(const df64& v) { return v.hi; }
-template <class T>
-GLA_DEV void col_exps(int n, const T* __restrict__ M, int* out) {
+GLA_DEV void col_exps(int n, const df64* __restrict__ M, int* out) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int j0 = wid * 4; j0 < n; j0 += nw * 4) {
     float x[4][4], m[4];  // (n <= 128: a column is four loads; those past an end repeat the last entry)
@@ -213,7 +206,7 @@ GLA_DEV void col_exps(int n, const T* __restrict__ M, int* out) {
     for (int u = 0; u < 4; u++)
 #pragma unroll
       for (int q = 0; q < 4; q++)
-        x[u][q] = hi_of(M[(size_t)min(j0 + u, n - 1) * n + min(lane + 32 * q, n - 1)]);
+        x[u][q] = M[(size_t)min(j0 + u, n - 1) * n + min(lane + 32 * q, n - 1)].hi;
 #pragma unroll
     for (int u = 0; u < 4; u++) {
       m[u] = fmaxf(fmaxf(fabsf(x[u][0]), fabsf(x[u][1])), fmaxf(fabsf(x[u][2]), fabsf(x[u][3])));
@@ -229,15 +222,14 @@ GLA_DEV void col_exps(int n, const T* __restrict__ M, int* out) {
 // exp_of(max_j |hi(M(i, j))|), two threads per row, eight loads in flight
 // (consecutive threads read consecutive rows of a column); all 256 threads of
 // the CTA, ends with a barrier.
-template <class T>
-GLA_DEV void row_exps(int n, const T* __restrict__ M, int* out) {
+GLA_DEV void row_exps(int n, const df64* __restrict__ M, int* out) {
   __shared__ float other[kM];
   const int i = threadIdx.x & (kM - 1), ic = min(i, n - 1), h = threadIdx.x >> 7;
   float m = 0.f;
   for (int j0 = h * 8; j0 < n; j0 += 16) {
     float x[8];
 #pragma unroll
-    for (int u = 0; u < 8; u++) x[u] = hi_of(M[(size_t)min(j0 + u, n - 1) * n + ic]);
+    for (int u = 0; u < 8; u++) x[u] = M[(size_t)min(j0 + u, n - 1) * n + ic].hi;
 #pragma unroll
     for (int u = 0; u < 8; u++) m = fmaxf(m, fabsf(x[u]));
   }
