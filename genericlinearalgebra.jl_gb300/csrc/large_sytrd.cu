@@ -274,14 +274,16 @@ __device__ T symv_unit(const SytrdArgs<T>& a, int j, int s, int J, int ch, T* sv
 constexpr int kFixedMin = 1000;
 constexpr int kFixW = 32, kFixR = 64;  // columns and rows of a unit (the last of kShapes)
 
-// e with |x| < 2^e for the top word of the largest |x| (at least 2^-400: the
-// working matrix has its largest entry in [1, 2)).
-GLA_DEV int fix_exp(unsigned top) { return max((int)(top >> 20) - 1022, -400); }
+// e with |x| < 2^e for the top word of the largest |x|; subnormal numbers share
+// the least exponent. A reflector's column may be as small as it likes beside
+// the rest of the matrix (one coupled by 1e-140 to a block of size 1): it is
+// scaled up to size 1 after the product, so its digits keep their own exponent.
+GLA_DEV int fix_exp(unsigned top) { return max((int)(top >> 20), 1) - 1022; }
 GLA_DEV unsigned fix_top(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
 // x 2^(56 - e), |x| < 2^e, rounded: digits (hi, lo) with hi 2^28 + lo, |lo| <= 2^27.
 GLA_DEV int2 fix_of(double x, int e) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int ex = (int)(b >> 52) & 0x7ff, s = ex - 1019 - e;  // the mantissa's shift, at most 3
+  const int ex = (int)(b >> 52) & 0x7ff, s = max(ex, 1) - 1019 - e;  // the mantissa's shift, at most 3
   const unsigned long long m = (b & 0xfffffffffffffull) | (ex ? 1ull << 52 : 0ull);
   const unsigned long long f = s >= 0 ? m << s : s > -64 ? ((m >> (-s - 1)) + 1) >> 1 : 0ull;
   const long long v = (long long)b < 0 ? -(long long)f : (long long)f;
@@ -290,8 +292,12 @@ GLA_DEV int2 fix_of(double x, int e) {
 }
 // The sum s1 2^56 + s2 2^28 of products of digits, in units of 2^56.
 GLA_DEV long long fix_sum(long long s1, long long s2) { return s1 + ((s2 + (1ll << 27)) >> 28); }
-// v 2^(e - 56), e >= -800.
-GLA_DEV double fix_value(long long v, int e) { return (double)v * __hiloint2double((1023 - 56 + e) << 20, 0); }
+// v 2^(e - 56), zero where that is below 2^-960 (a unit of the matrix and a
+// column that are both tiny: times the column's scale, at most 2^511, that is
+// below 2^-440 of the matrix). e <= 1078, as the eigensolvers scale their matrix.
+GLA_DEV double fix_value(long long v, int e) {
+  return (double)v * __hiloint2double(max(1023 - 56 + e, 0) << 20, 0);
+}
 
 // The units of the tile columns J0 .. of the lower triangle (grid: chunk of
 // rows, tile column).
