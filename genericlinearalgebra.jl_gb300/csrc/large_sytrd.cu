@@ -433,17 +433,19 @@ GLA_DEV __host__ int panel_rows(int k0, int n, int G) { return (n - k0 - 1 + G -
 
 // beta = -copysign(norm, alpha), tau = (beta - alpha) / beta and 1 / (alpha -
 // beta) from alpha and sigma, the squared norm below it; beta = alpha and
-// zeros when sigma is zero. FP64: one seed and one cubic step per square root
-// and reciprocal, 10 instructions in a row; the norm in even lanes and its
-// reciprocal in odd ones.
+// zeros when sigma is zero, or when the whole column is so small (2^-500 beside
+// a matrix of size 1; FP32 2^-60) that its square leaves the normal range and
+// the seeds below: leaving it out moves the matrix by no more than its norm.
+// FP64: one seed and one cubic step per square root and reciprocal, 10
+// instructions in a row; the norm in even lanes and its reciprocal in odd ones.
 GLA_DEV void panel_scalars(double alpha, double sigma, double& beta, double& tau, double& scale) {
-  if ((__double_as_longlong(sigma) << 1) == 0) {
+  const double nrm2 = fma(alpha, alpha, sigma);
+  if ((__double_as_longlong(sigma) << 1) == 0 || prec<double>::biased_exp(nrm2) < 1023 - 1000) {
     beta = alpha;
     tau = scale = 0.0;
     return;
   }
   const bool odd = threadIdx.x & 1;
-  const double nrm2 = fma(alpha, alpha, sigma);
   double y, x;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(nrm2));
   const double h = nrm2 * y;
@@ -462,12 +464,12 @@ GLA_DEV void panel_scalars(double alpha, double sigma, double& beta, double& tau
   scale = fma(x, fma(ed, ed, ed), x);
 }
 GLA_DEV void panel_scalars(float alpha, float sigma, float& beta, float& tau, float& scale) {
-  if (sigma == 0.f) {
+  const float nrm2 = fmaf(alpha, alpha, sigma);
+  if (sigma == 0.f || nrm2 < 0x1p-120f) {
     beta = alpha;
     tau = scale = 0.f;
     return;
   }
-  const float nrm2 = fmaf(alpha, alpha, sigma);
   const float nrm = nrm2 * prec<float>::rsqrt(nrm2);
   beta = -copysignf(nrm, alpha);
   tau = (beta - alpha) * prec<float>::rcp(beta);

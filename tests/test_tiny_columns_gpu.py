@@ -41,3 +41,21 @@ def test_tiny_first_column(G, n):
     V = r.vectors.cpu().numpy()
     assert np.linalg.norm(A @ V - V * r.values.cpu().numpy(), 2) <= 1e-13 * np.abs(want).max()
     assert np.linalg.norm(V.T @ V - np.eye(n), 2) <= 1e-13
+
+
+@pytest.mark.parametrize("precision,c", [("f64", 1e-154), ("f64", 1e-157), ("f64", 1e-165), ("f32", 1e-19),
+                                         ("f32", 1e-20), ("f32", 1e-22), ("f32_refined", 1e-20)])
+@pytest.mark.parametrize("n", [150, 300, 1056])
+def test_first_column_whose_square_underflows(G, n, precision, c):
+    # the squared norm of the column is subnormal or zero in the working precision
+    import torch
+    A, want = coupled(n, c)
+    dt = torch.float32 if precision == "f32" else torch.float64
+    eps = 2.0 ** -23 if precision == "f32" else EPS64
+    r = G.eigen(torch.tensor(A, device="cuda", dtype=dt), precision=precision)
+    w, V = r.values.cpu().numpy().astype(np.float64), r.vectors.cpu().numpy().astype(np.float64)
+    nA = np.abs(want).max()
+    assert np.abs(w - want).max() <= 8 * n * eps * nA
+    if precision != "f32":
+        assert np.linalg.norm(A @ V - V * w, 2) <= 1e-13 * nA
+        assert np.linalg.norm(V.T @ V - np.eye(n), 2) <= 1e-13
