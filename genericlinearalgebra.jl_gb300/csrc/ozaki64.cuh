@@ -586,7 +586,8 @@ GLA_DEV void gemm_body(const Args& g, int tile, int split) {
         double x;
         bool bad;
         if (NSEG == 1) {
-          bad = max(a0, b0) == kBadExp;
+          // (a product without terms has no slices either: its exponents' words are an earlier one's)
+          bad = total > 0 && max(a0, b0) == kBadExp;
           x = to_double(H[c], L[c], a0 + b0);
           x = g.neg ? -x : x;
         } else {
