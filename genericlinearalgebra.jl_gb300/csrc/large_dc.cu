@@ -189,7 +189,11 @@ __global__ void __launch_bounds__(kPrepThreads) k_dc_prep(DcArrays<T> a) {
   __shared__ unsigned long long sred[kPrepThreads / 32];
   __shared__ int scnt[kPrepThreads / 32], sfirst;
   const int lane = tid & 31, wid = tid >> 5;
-  // z, merged order, max |D|
+  // z, merged order, max |D|. (The ranks are a permutation of finite values; with
+  // a NaN among them, which only a wait that ran out can bring, two may fall on
+  // one place: the places left out then hold an index in range as well.)
+  for (int i = tid; i < m; i += kPrepThreads) a.ssrc[o + i] = i;
+  __syncthreads();
   unsigned long long dbits = 0;
   for (int i = tid; i < m; i += kPrepThreads) {
     const T di = a.dd[o + i];
