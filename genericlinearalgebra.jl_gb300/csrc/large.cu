@@ -86,7 +86,7 @@ __global__ void k_large_load(const Tin* __restrict__ A, long long lda, int n, bo
                              const unsigned long long* __restrict__ amax, const int* __restrict__ nonfinite,
                              int* __restrict__ scale_exp) {
   const double am = __longlong_as_double((long long)*amax);
-  const int ex = (am > 0.0 && !*nonfinite) ? ilogb(am) : 0;
+  const int ex = (am > 0.0 && !*nonfinite) ? max(ilogb(am), -1022) : 0;  // (2^-ex stays finite)
   const double sc = ldexp(1.0, -ex);
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *scale_exp = ex;
   const bool bad = *nonfinite != 0;
@@ -98,6 +98,36 @@ __global__ void k_large_load(const Tin* __restrict__ A, long long lda, int n, bo
       v = (T)((double)x * sc);
     }
     Aw[i + (long long)j * n] = v;
+  }
+}
+
+// The same for a tridiagonal, in one CTA: d and e (n - 1 entries) times 2^-ex
+// with the largest in [1, 2) into dw and ew (n entries each, ew's last zero);
+// zeros for non-finite input. Divide and conquer orders its values by
+// comparisons and squares them, so it must meet neither NaN nor overflow.
+__global__ void __launch_bounds__(1024) k_tri_load(const double* __restrict__ d, const double* __restrict__ e, int n,
+                                                   double* __restrict__ dw, double* __restrict__ ew,
+                                                   int* __restrict__ nonfinite, int* __restrict__ scale_exp) {
+  __shared__ unsigned long long smax[32];
+  const int tid = threadIdx.x;
+  unsigned long long m = 0;  // (the bits of NaN and infinity are above those of every finite value)
+  for (int i = tid; i < n; i += 1024) {
+    m = max(m, abs_bits<double>(d[i]));
+    if (i + 1 < n) m = max(m, abs_bits<double>(e[i]));
+  }
+  m = warp_max_u64(m);
+  if ((tid & 31) == 0) smax[tid >> 5] = m;
+  __syncthreads();
+  m = warp_max_u64(smax[tid & 31]);
+  const bool bad = m >= 0x7ff0000000000000ull;
+  const int ex = bad || m == 0 ? 0 : ilogb(__longlong_as_double((long long)m));
+  if (tid == 0) {
+    *nonfinite = bad;
+    *scale_exp = ex;
+  }
+  for (int i = tid; i < n; i += 1024) {
+    dw[i] = bad ? 0.0 : ldexp(d[i], -ex);
+    ew[i] = bad || i + 1 >= n ? 0.0 : ldexp(e[i], -ex);
   }
 }
 
@@ -287,38 +317,35 @@ int large_syev(LargeCtx* c, int tcode, bool wantv, bool lower, const void* Ain, 
 }
 
 // SymTridiagonal input (the reference's eigen!(::SymTridiagonal),
-// src/eigenSelfAdjoint.jl:602-612): divide and conquer on (d, e) as given
-// (FP64 context), eigenvalues ascending into w, eigenvectors into Z (ldz)
-// when wanted. Synchronises st.
+// src/eigenSelfAdjoint.jl:602-612): divide and conquer on (d, e) scaled by a
+// power of two (FP64 context), eigenvalues ascending into w, eigenvectors into
+// Z (ldz) when wanted; NaN and info -1 for non-finite input. Synchronises st.
 int large_stev(LargeCtx* c, const double* d, const double* e, double* w, double* Z, long long ldz, int* info_host,
                cudaStream_t st) {
   const int n = c->n;
   if (!c->f64) return -1000 - (int)cudaErrorInvalidValue;
-  LG_CUDA(cudaMemcpyAsync(c->d, d, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-  LG_CUDA(cudaMemsetAsync(c->e, 0, sizeof(double) * n, st));
-  if (n > 1) LG_CUDA(cudaMemcpyAsync(c->e, e, sizeof(double) * (n - 1), cudaMemcpyDeviceToDevice, st));
+  int* nonfinite = c->flags + 2;
+  int* sexp = c->flags + 3;
+  k_tri_load<<<1, 1024, 0, st>>>(d, e, n, (double*)c->d, (double*)c->e, nonfinite, sexp);
+  LG_CUDA(cudaGetLastError());
   int rc = large_clear_error(c, st);
   if (rc) return rc;
   rc = dc_enqueue(c->dc, c->d, c->e, c->Z, c->leaf_info, st);
   if (rc) return rc;
-  LG_CUDA(cudaMemcpyAsync(w, c->d, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-  if (Z)
-    LG_CUDA(cudaMemcpy2DAsync(Z, sizeof(double) * ldz, c->Z, sizeof(double) * n, sizeof(double) * n, n,
-                              cudaMemcpyDeviceToDevice, st));
+  k_large_store<double, double><<<dim3(Z ? (n + 255) / 256 : 1, n), 256, 0, st>>>(
+      (const double*)c->d, (const double*)c->Z, n, w, Z, ldz, nonfinite, sexp);
+  LG_CUDA(cudaGetLastError());
   LG_CUDA(cudaMemcpyAsync(c->h_stat, sytrd_error_word(c->sy), sizeof(int), cudaMemcpyDeviceToHost, st));
   LG_CUDA(cudaMemcpyAsync(c->h_stat + 1, dc_fail_word(c->dc), sizeof(int), cudaMemcpyDeviceToHost, st));
+  LG_CUDA(cudaMemcpyAsync(c->h_stat + 2, nonfinite, sizeof(int), cudaMemcpyDeviceToHost, st));
   const int nleaf = dc_leaf_count(c->dc);
   std::vector<int> li(nleaf);
   LG_CUDA(cudaMemcpyAsync(li.data(), c->leaf_info, sizeof(int) * nleaf, cudaMemcpyDeviceToHost, st));
   LG_CUDA(cudaStreamSynchronize(st));
   if (c->h_stat[0]) return -1000 - (int)cudaErrorLaunchTimeout;
   int bad = c->h_stat[1] ? 1 : 0;
-  bool nonfinite = false;
-  for (int x : li) {
-    if (x < 0) nonfinite = true;
-    if (x > 0) bad += x;
-  }
-  *info_host = nonfinite ? -1 : bad;
+  for (int x : li) bad += x > 0 ? x : 0;
+  *info_host = c->h_stat[2] ? -1 : bad;
   return 0;
 }
 
