@@ -57,9 +57,10 @@ cudaError_t launch_stein_tri(int nblocks, int nmax, cudaStream_t st, const Small
                              const void* d, const void* e, void* Q, void* w, ChaseState* cst, const int* info);
 
 // FP32, values only: the ascending eigenvalues of (d, e) into w, NaN for
-// matrices whose info is -1 (blockDim >= n).
+// matrices whose info is -1 and, with info > 0, for those with an infinity or
+// NaN in d or e (blockDim >= n).
 cudaError_t launch_bisect_values(int nblocks, int nmax, cudaStream_t st, const SmallDesc* descs, const int* perm,
-                                 const void* d, const void* e, void* w, const int* info);
+                                 const void* d, const void* e, void* w, int* info);
 
 // Capture-safe executes: info = -2 for matrices whose chase is still running.
 cudaError_t launch_mark_unfinished(int nblocks, cudaStream_t st, const SmallDesc* descs, const int* perm,

@@ -109,7 +109,7 @@ cudaError_t launch_stein_tri(int nblocks, int nmax, cudaStream_t st, const Small
 __global__ void __launch_bounds__(128) k_bisect_values(const SmallDesc* __restrict__ descs,
                                                        const int* __restrict__ perm, const float* __restrict__ dg_all,
                                                        const float* __restrict__ eg_all, float* __restrict__ wout,
-                                                       const int* __restrict__ info) {
+                                                       int* __restrict__ info) {
   __shared__ float dd[kSmallMaxN], e2[kSmallMaxN], red[3][4];
   __shared__ int cnt[3 * kSmallMaxN];
   const int mid = perm[blockIdx.x];
@@ -121,6 +121,13 @@ __global__ void __launch_bounds__(128) k_bisect_values(const SmallDesc* __restri
   }
   const float d = tid < n ? dg_all[dsc.w_off + tid] : 0.f;
   const float e = tid + 1 < n ? eg_all[dsc.w_off + tid] : 0.f;
+  // a reduction that left the range (entries near the largest float): no
+  // eigenvalue is found, as the chase would report it
+  if (__syncthreads_or(!isfinite(d) || !isfinite(e))) {
+    if (tid < n) wout[dsc.w_off + tid] = NAN;
+    if (tid == 0) info[mid] = max(n - 1, 1);
+    return;
+  }
   float m = fmaxf(fabsf(d), fabsf(e));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -164,7 +171,7 @@ __global__ void __launch_bounds__(128) k_bisect_values(const SmallDesc* __restri
 }
 
 cudaError_t launch_bisect_values(int nblocks, int nmax, cudaStream_t st, const SmallDesc* descs, const int* perm,
-                                 const void* d, const void* e, void* w, const int* info) {
+                                 const void* d, const void* e, void* w, int* info) {
   if (nblocks <= 0) return cudaSuccess;
   const int nt = std::max(32, (nmax + 31) / 32 * 32);
   k_bisect_values<<<nblocks, nt, 0, st>>>(descs, perm, (const float*)d, (const float*)e, (float*)w, info);
