@@ -49,21 +49,27 @@ GLA_DEV float rcp_seed(float x) {
 }
 
 // Guarded pivot (LAPACK dlaebz / dstebz): a pivot smaller than pivmin in
-// magnitude is replaced by -pivmin.
-GLA_DEV float guard_piv(float q, float pivmin) { return fabsf(q) < pivmin ? -pivmin : q; }
+// magnitude is replaced by -pivmin. SIGNED: a positive one by pivmin, so that
+// the count is that of the pivot as it is and an entry that stands alone is met
+// exactly however small it is.
+template <bool SIGNED = false>
+GLA_DEV float guard_piv(float q, float pivmin) {
+  return fabsf(q) < pivmin ? (SIGNED && q > 0.f ? pivmin : -pivmin) : q;
+}
 
 // Numbers of eigenvalues of T below x0, x1, x2 (three interleaved Sturm
 // sequences). d: diagonal, e2: squared off-diagonal (shared memory, read
 // by every thread at the same index: broadcast).
+template <bool SIGNED = false>
 GLA_DEV void sturm3(int n, const float* __restrict__ d, const float* __restrict__ e2, float x0, float x1, float x2,
                     float pivmin, int& c0, int& c1, int& c2) {
-  float q0 = guard_piv(d[0] - x0, pivmin), q1 = guard_piv(d[0] - x1, pivmin), q2 = guard_piv(d[0] - x2, pivmin);
+  float q0 = guard_piv<SIGNED>(d[0] - x0, pivmin), q1 = guard_piv<SIGNED>(d[0] - x1, pivmin), q2 = guard_piv<SIGNED>(d[0] - x2, pivmin);
   int a0 = q0 < 0.f, a1 = q1 < 0.f, a2 = q2 < 0.f;
   for (int i = 1; i < n; i++) {
     const float di = d[i], ei = e2[i - 1];
-    q0 = guard_piv(fmaf(-ei, rcp_seed(q0), di - x0), pivmin);
-    q1 = guard_piv(fmaf(-ei, rcp_seed(q1), di - x1), pivmin);
-    q2 = guard_piv(fmaf(-ei, rcp_seed(q2), di - x2), pivmin);
+    q0 = guard_piv<SIGNED>(fmaf(-ei, rcp_seed(q0), di - x0), pivmin);
+    q1 = guard_piv<SIGNED>(fmaf(-ei, rcp_seed(q1), di - x1), pivmin);
+    q2 = guard_piv<SIGNED>(fmaf(-ei, rcp_seed(q2), di - x2), pivmin);
     a0 += q0 < 0.f;
     a1 += q1 < 0.f;
     a2 += q2 < 0.f;
@@ -78,12 +84,13 @@ GLA_DEV void sturm3(int n, const float* __restrict__ d, const float* __restrict_
 // thread, and a search in the counts, in place of log4(3 NT) quadsection
 // steps in which every thread makes its way there by itself (order 128, 256
 // threads: 12 steps become 8). cnt: 3 NT ints of shared scratch. All threads.
+template <bool SIGNED = false>
 GLA_DEV void grid_bracket(int n, const float* d, const float* e2, float& lo, float& hi, float pivmin, int* cnt) {
   const int tid = threadIdx.x, P = 3 * blockDim.x;
   const float l0 = lo, h0 = hi, step = (h0 - l0) / (float)(P + 1);
   auto point = [&](int p) { return fmaf((float)(p + 1), step, l0); };
   int c0, c1, c2;
-  sturm3(n, d, e2, point(3 * tid), point(3 * tid + 1), point(3 * tid + 2), pivmin, c0, c1, c2);
+  sturm3<SIGNED>(n, d, e2, point(3 * tid), point(3 * tid + 1), point(3 * tid + 2), pivmin, c0, c1, c2);
   cnt[3 * tid] = c0;
   cnt[3 * tid + 1] = c1;
   cnt[3 * tid + 2] = c2;
@@ -126,14 +133,17 @@ GLA_DEV float eig_bisect(int n, const float* d, const float* e2, int k, float lo
 
 // The same to the last bit: until no float lies between lo and hi, then hi,
 // the smallest x with more than k eigenvalues below or at it (an eigenvalue
-// that splits off exactly comes back exactly).
-GLA_DEV float eig_bisect_full(int n, const float* d, const float* e2, int k, float lo, float hi, float pivmin) {
+// that splits off exactly comes back exactly), or until both are within `zero`
+// of zero.
+GLA_DEV float eig_bisect_full(int n, const float* d, const float* e2, int k, float lo, float hi, float pivmin,
+                              float zero) {
   for (int it = 0; it < 160; it++) {
+    if (lo >= -zero && hi <= zero) break;
     const float x1 = 0.5f * (lo + hi);
     if (!(x1 > lo && x1 < hi)) break;
     const float x0 = 0.5f * (lo + x1), x2 = 0.5f * (x1 + hi);  // (may round to an end: then unused)
     int c0, c1, c2;
-    sturm3(n, d, e2, x0, x1, x2, pivmin, c0, c1, c2);
+    sturm3<true>(n, d, e2, x0, x1, x2, pivmin, c0, c1, c2);
     if (c1 > k) {
       hi = x1;
       if (x0 > lo && x0 < hi) {

@@ -102,7 +102,8 @@ cudaError_t launch_stein_tri(int nblocks, int nmax, cudaStream_t st, const Small
 
 // Eigenvalues of FP32 matrices (jobz 'N'): one CTA per matrix, one thread per
 // eigenvalue, bisection on Sturm counts of (d, e) scaled by an exact power of
-// two, to the last bit, in place of the root-free chase and the sort. That
+// two (the largest to about 2^62: its square is in range and the squares of
+// entries 2^-136 as large are too), to the last bit, in place of the root-free chase and the sort. That
 // chase is one serial recurrence of about n^2 steps per matrix (550 cycles
 // each: 5.1 ms for 1000 matrices of orders 8 .. 128 with everything beside
 // it), bisection 15 to 20 passes of n steps for all eigenvalues at once.
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(128) k_bisect_values(const SmallDesc* __restri
                                                        const int* __restrict__ perm, const float* __restrict__ dg_all,
                                                        const float* __restrict__ eg_all, float* __restrict__ wout,
                                                        int* __restrict__ info) {
-  __shared__ float dd[kSmallMaxN], e2[kSmallMaxN], red[3][4];
+  __shared__ float dd[kSmallMaxN], e2[kSmallMaxN], xs[kSmallMaxN], red[3][4];
   __shared__ int cnt[3 * kSmallMaxN];
   const int mid = perm[blockIdx.x];
   const SmallDesc dsc = descs[mid];
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(128) k_bisect_values(const SmallDesc* __restri
   if (lane == 0) red[0][wid] = m;
   __syncthreads();
   for (int w = 0; w < nw; w++) m = fmaxf(m, red[0][w]);
-  const int ex = m > 0.f ? ilogbf(m) : 0;
+  const int ex = m > 0.f ? ilogbf(m) - 62 : 0;
   const float ds = ldexpf(d, -ex), es = ldexpf(e, -ex);
   if (tid < n) {
     dd[tid] = ds;
@@ -163,11 +164,43 @@ __global__ void __launch_bounds__(128) k_bisect_values(const SmallDesc* __restri
   const float widen = 2.f * (float)n * prec<float>::eps * fmaxf(fabsf(lo), fabsf(hi)) + 2.f * pivmin;
   lo -= widen;
   hi += widen;
-  grid_bracket(n, dd, e2, lo, hi, pivmin, cnt);
-  if (tid < n) {
-    const float x = eig_bisect_full(n, dd, e2, tid, lo, hi, pivmin);
-    wout[dsc.w_off + tid] = fabsf(x) <= 4.f * pivmin ? 0.f : ldexpf(x, ex);
+  grid_bracket<true>(n, dd, e2, lo, hi, pivmin, cnt);
+  const float zero = 4.f * pivmin;
+  const float x = tid < n ? eig_bisect_full(n, dd, e2, tid, lo, hi, pivmin, zero) : 0.f;
+  if (tid < n) xs[tid] = x;
+  __syncthreads();
+  if (tid >= n) return;
+  float out = ldexpf(x, ex);
+  if (fabsf(x) <= zero) {
+    // Zero to within the guarded pivots (2^-180 of the matrix): zero, but for
+    // the entries that stand alone, which are eigenvalues as they are. Those
+    // below zero come first here, those above it last.
+    const float* dg = dg_all + dsc.w_off;
+    auto alone = [&](int i) {
+      return (i == 0 || e2[i - 1] == 0.f) && e2[i] == 0.f && fabsf(dd[i]) <= zero;  // (e2[n - 1] is zero)
+    };
+    int before = 0, here = 0, neg = 0, pos = 0;
+    for (int i = 0; i < n; i++) {
+      before += xs[i] < -zero;
+      here += fabsf(xs[i]) <= zero;
+      neg += alone(i) && dg[i] < 0.f;
+      pos += alone(i) && dg[i] > 0.f;
+    }
+    const int r = tid - before;
+    out = 0.f;
+    if (r < neg || r >= here - pos) {
+      const int want = r < neg ? r : r - (here - pos);
+      const bool up = r >= neg;
+      for (int i = 0; i < n; i++) {
+        if (!alone(i) || (up ? dg[i] <= 0.f : dg[i] >= 0.f)) continue;
+        int rank = 0;
+        for (int j = 0; j < n; j++)
+          rank += alone(j) && (up ? dg[j] > 0.f : dg[j] < 0.f) && (dg[j] < dg[i] || (dg[j] == dg[i] && j < i));
+        if (rank == want) out = dg[i];
+      }
+    }
   }
+  wout[dsc.w_off + tid] = out;
 }
 
 cudaError_t launch_bisect_values(int nblocks, int nmax, cudaStream_t st, const SmallDesc* descs, const int* perm,
