@@ -258,6 +258,7 @@ void release_complex_cache() {
   oz64_gemm_release(&g_z.oz);
   g_z = ZWork();
 }
+Oz64Gemm* complex_gemm() { return g_z.oz; }
 }  // namespace gla
 
 extern "C" {
@@ -349,8 +350,7 @@ int gla_zheev(char jobz, char uplo, int64_t n, const double* A, int64_t lda, dou
       if (rc2) return rc2;
     }
   }
-  Z_CUDA(cudaStreamSynchronize(st));  // the index tables live in host memory until here
-  return 0;
+  return gla::oz64_gemm_status(g_z.oz, st);  // (the index tables live in host memory until it has waited)
 }
 
 // Host-buffer form (stages through the device).

@@ -91,12 +91,21 @@ cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Z, long l
 // cores when every extent reaches kOz64MinGemm, by the SIMT GEMM below that
 // (there the slicing and launches cost more than the product). *w, made by
 // the first call, holds the operand buffers, which grow; calls that share it
-// run on one stream after another. Should a bounded wait run out, C is NaN.
+// run on one stream after another. Should a bounded wait run out, C is NaN and
+// oz64_gemm_status tells.
 struct Oz64Gemm;
 constexpr int kOz64MinGemm = 128;
 cudaError_t oz64_gemm(Oz64Gemm** w, bool ta, int m, int n, int k, const double* A, long long lda, const double* B,
                       long long ldb, double* C, long long ldc, bool add, cudaStream_t st);
 void oz64_gemm_release(Oz64Gemm** w);
+// Waits for st; 0, or cudaErrorLaunchTimeout's status when a wait of a product
+// since the last call ran out, whose mark it clears (w may be null: no product yet).
+int oz64_gemm_status(Oz64Gemm* w, cudaStream_t st);
+// For tests: leaves the mark such a wait would leave.
+cudaError_t oz64_gemm_mark(Oz64Gemm* w);
+// The products of gla_zheev and gla_qheev (null before their first call).
+Oz64Gemm* complex_gemm();
+Oz64Gemm* quaternion_gemm();
 
 // ---- adjoint of one large eigen-decomposition (large_adjoint.cu):
 // Abar = V (diag(wbar) + sym(F o (V' Vbar))) V' for orders up to nmax of

@@ -347,6 +347,23 @@ void oz64_gemm_release(Oz64Gemm** w) {
   *w = nullptr;
 }
 
+int oz64_gemm_status(Oz64Gemm* w, cudaStream_t st) {
+  int word = 0;
+  cudaError_t e = cudaSuccess;
+  if (w) e = cudaMemcpyAsync(&word, w->err, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && word) {
+    e = cudaMemsetAsync(w->err, 0, sizeof(int), st);
+    if (e == cudaSuccess) e = cudaErrorLaunchTimeout;
+  }
+  return e == cudaSuccess ? 0 : -1000 - (int)e;
+}
+
+cudaError_t oz64_gemm_mark(Oz64Gemm* w) {
+  const int word = 1;
+  return cudaMemcpy(w->err, &word, sizeof(int), cudaMemcpyHostToDevice);
+}
+
 cudaError_t oz64_gemm(Oz64Gemm** wp, bool ta, int m, int n, int k, const double* A, long long lda, const double* B,
                       long long ldb, double* C, long long ldc, bool add, cudaStream_t st) {
   if (m <= 0 || n <= 0) return cudaSuccess;

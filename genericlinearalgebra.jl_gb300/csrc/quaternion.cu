@@ -311,6 +311,7 @@ void release_quaternion_cache() {
   oz64_gemm_release(&g_qh.oz);
   g_qh = QWork();
 }
+Oz64Gemm* quaternion_gemm() { return g_qh.oz; }
 }  // namespace gla
 
 extern "C" {
@@ -400,8 +401,7 @@ int gla_qheev(char jobz, char uplo, int64_t n, const double* A, int64_t lda, dou
       if (rc2) return rc2;
     }
   }
-  Q_CUDA(cudaStreamSynchronize(st));  // the index tables live in host memory until here
-  return 0;
+  return gla::oz64_gemm_status(g_qh.oz, st);  // (the index tables live in host memory until it has waited)
 }
 
 // Host-buffer form (stages through the device).
