@@ -539,7 +539,17 @@ int gla_plan_destroy(gla_plan_t p) {
 int gla_plan_workspace_size(gla_plan_t p, size_t* bytes) {
   if (!p) return -1;
   if (!bytes) return -2;
-  *bytes = p->ws_bytes;
+  size_t b = p->ws_bytes;
+  for (const auto& ch : p->chains) {
+    b += large_workspace_bytes(ch.ctx);
+    if (ch.ref) b += refine_large_bytes(ch.ref);
+  }
+  for (const auto& a : p->adj_large) b += large_adjoint_bytes(a.ctx);
+  if (p->d_adj) b += adjoint_workspace_bytes(p->a_elems);
+  if (p->h_adj) b += sizeof(double) * (size_t)(3 * p->a_elems + 2 * p->w_elems);
+  if (p->h_A)  // staging of the host-buffer calls
+    b += p->io_elem() * (size_t)((p->jobz == 'V' ? 2 : 1) * p->a_elems + p->w_elems) + sizeof(int) * p->batch;
+  *bytes = b;
   return 0;
 }
 

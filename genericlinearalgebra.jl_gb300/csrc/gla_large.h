@@ -67,6 +67,15 @@ int* oz_error_word(OzWork* w);
 cudaError_t oz_slice_rows(OzWork* w, const float* hi, const float* lo, long long ld, int rows, int len, int S,
                           cudaStream_t st);
 bool oz_fits(const OzWork* w, int m, int n, int K);
+size_t oz_bytes(const OzWork* w);
+
+// cudaMalloc that adds what it got to *total (each object counts its own).
+inline cudaError_t counted_malloc(void** p, size_t bytes, size_t* total) {
+  const size_t b = bytes < 16 ? 16 : bytes;
+  const cudaError_t e = cudaMalloc(p, b);
+  if (e == cudaSuccess) *total += b;
+  return e;
+}
 
 // ---- FP64-accurate tensor-core GEMM (ozaki64.cuh / ozaki64.cu) and the
 // stages of the FP64 path that run on it. One object per large context of
@@ -114,6 +123,7 @@ Oz64Gemm* quaternion_gemm();
 struct LargeAdjoint;
 int large_adjoint_create(LargeAdjoint** out, int nmax);
 void large_adjoint_destroy(LargeAdjoint* a);
+size_t large_adjoint_bytes(const LargeAdjoint* a);
 cudaError_t large_adjoint(LargeAdjoint* a, int n, const double* w, const double* V, long long ldv,
                           const double* wbar, const double* Vbar, long long ldvb, double* Abar, long long lda,
                           double gap_rel, cudaStream_t st);
@@ -131,6 +141,7 @@ void sytrd_set_oz64(SytrdPlan* p, Oz64* oz);
 // device cannot hold the cluster.
 constexpr int kSideBySideMaxN = 1024;
 bool sytrd_set_cluster_only(SytrdPlan* p);
+size_t sytrd_plan_bytes(const SytrdPlan* p);
 
 struct DcPlan;
 // bisect_leaves (FP32 only): the leaves go through the per-eigenvalue solver
@@ -149,6 +160,7 @@ struct BacktrPlan;
 // tc (FP32 only): both GEMMs of every block on the tensor cores (3xTF32).
 int backtr_plan_create(BacktrPlan** out, int n, bool f64, bool tc = false);
 void backtr_plan_destroy(BacktrPlan* p);
+size_t backtr_plan_bytes(const BacktrPlan* p);
 // Error word the back-transformation's tensor-core GEMMs set when a bounded
 // wait runs out (the large context passes its reduction's word).
 void backtr_set_error_word(BacktrPlan* p, int* err);
@@ -169,7 +181,7 @@ struct LargeCtx;
 // cluster; cudaErrorNotSupported where they cannot).
 int large_create(LargeCtx** out, int n, bool f64, bool refine_stage = false, bool side = false);
 void large_destroy(LargeCtx* c);
-size_t large_workspace_bytes(const LargeCtx* c);
+size_t large_workspace_bytes(const LargeCtx* c);  // device memory of the context, in bytes
 // Stage times of the last large_syev (ms): tridiagonalisation (with the
 // load), divide and conquer, back-transformation (with the store).
 void large_stage_ms(const LargeCtx* c, float* ms3);
@@ -208,6 +220,7 @@ int large_stev(LargeCtx* c, const double* d, const double* e, double* w, double*
 struct RefineLarge;
 int refine_large_create(RefineLarge** out, int n, bool side = false);
 void refine_large_destroy(RefineLarge* r);
+size_t refine_large_bytes(const RefineLarge* r);  // (with the clusters' contexts it has made so far)
 // Buffers the FP32 solve can write straight into: eigenvectors (n x n,
 // leading dimension n) and eigenvalues (n).
 float* refine_large_xbuf(RefineLarge* r);

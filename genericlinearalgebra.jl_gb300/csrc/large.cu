@@ -36,6 +36,7 @@ struct LargeCtx {
   void* tau = nullptr;
   int* flags = nullptr; // [0] max |a| bits (low word), [1] high word, [2] non-finite, [3] scale exponent
   int* leaf_info = nullptr;
+  size_t bytes = 0;       // device memory held by the context itself
   int* h_stat = nullptr;  // pinned status words
   cudaEvent_t ev[4] = {};  // stage boundaries: load+sytrd | stedc | ormtr+store
   float ms[3] = {0, 0, 0}; // last solve: tridiagonalisation, divide and conquer, back-transformation
@@ -176,7 +177,7 @@ int large_create(LargeCtx** out, int n, bool f64, bool refine_stage, bool side) 
   }
   auto alloc = [&](void** p, size_t bytes) {
     if (!rc) {
-      cudaError_t e2 = cudaMalloc(p, std::max<size_t>(bytes, 16));
+      cudaError_t e2 = counted_malloc(p, bytes, &c->bytes);
       if (e2 != cudaSuccess) rc = -1000 - (int)e2;
     }
   };
@@ -226,8 +227,8 @@ void large_stage_ms(const LargeCtx* c, float* ms3) {
 }
 
 size_t large_workspace_bytes(const LargeCtx* c) {
-  const size_t el = c->f64 ? 8 : 4;
-  return el * (size_t)c->n * c->n * 4 + dc_plan_bytes(c->dc) + (c->oz ? oz64_bytes(c->oz) : 0);
+  return c->bytes + sytrd_plan_bytes(c->sy) + dc_plan_bytes(c->dc) + backtr_plan_bytes(c->bt) +
+         (c->oz ? oz64_bytes(c->oz) : 0);
 }
 
 int large_sytrd(LargeCtx* c, void* A, long long lda, void* d, void* e, void* tau, cudaStream_t st) {

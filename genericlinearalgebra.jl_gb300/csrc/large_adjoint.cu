@@ -135,6 +135,11 @@ int large_adjoint_create(LargeAdjoint** out, int nmax) {
   return 0;
 }
 
+size_t large_adjoint_bytes(const LargeAdjoint* a) {
+  const size_t nn = (size_t)a->nmax * a->nmax;
+  return oz_bytes(a->oz) + 8 * nn * sizeof(float) + (nn + 1) * sizeof(double);
+}
+
 void large_adjoint_destroy(LargeAdjoint* a) {
   if (!a) return;
   oz_destroy(a->oz);

@@ -144,9 +144,11 @@ struct BacktrPlan {
   long long ldy = 0;
   float* Zp = nullptr;
   int* err = nullptr;   // error word of the tensor-core GEMMs (set by backtr_set_error_word)
+  size_t bytes = 0;     // device memory held
   Oz64* oz = nullptr;   // FP64: the whole application on the tensor cores (set by backtr_set_oz64)
 };
 
+size_t backtr_plan_bytes(const BacktrPlan* p) { return p->bytes; }
 void backtr_set_error_word(BacktrPlan* p, int* err) { p->err = err; }
 void backtr_set_oz64(BacktrPlan* p, Oz64* oz) { p->oz = oz; }
 
@@ -162,7 +164,7 @@ int backtr_plan_create(BacktrPlan** out, int n, bool f64, bool tc) {
   const size_t el = f64 ? 8 : 4;
   cudaError_t err = cudaSuccess;
   auto alloc = [&](void** q, size_t bytes) {
-    if (err == cudaSuccess) err = cudaMalloc(q, std::max<size_t>(bytes, 16));
+    if (err == cudaSuccess) err = counted_malloc(q, bytes, &p->bytes);
   };
   const bool use_tc = !f64 && tc && tc::tc_available();
   p->ldy = use_tc ? (n + 3) & ~3 : n;

@@ -718,6 +718,7 @@ struct DcPlan {
   void* em = nullptr;
   int* d_fail = nullptr;
   long long u_stride = 0;
+  size_t bytes = 0;         // device memory held, the leaves' plan apart
   Oz64* oz = nullptr;       // FP64: eigenvector updates on the tensor cores (set by dc_set_oz64)
   DcArrays<double> a64{};
   DcArrays<float> a32{};
@@ -908,7 +909,7 @@ int dc_plan_create(DcPlan** out, int n, bool f64, bool bisect_leaves) {
   }
   cudaError_t err = cudaSuccess;
   auto alloc = [&](void** q, size_t bytes) {
-    if (err == cudaSuccess) err = cudaMalloc(q, std::max<size_t>(bytes, 16));
+    if (err == cudaSuccess) err = counted_malloc(q, bytes, &p->bytes);
   };
   alloc((void**)&p->d_info, sizeof(MergeInfo) * std::max(1, p->nmerge));
   alloc((void**)&p->d_gdesc, sizeof(GemmDesc) * 2 * std::max(1, p->nmerge));
@@ -986,8 +987,9 @@ void dc_set_oz64(DcPlan* p, Oz64* oz) { p->oz = oz; }
 int* dc_fail_word(DcPlan* p) { return p->d_fail; }
 int dc_leaf_count(const DcPlan* p) { return p->nleaf; }
 size_t dc_plan_bytes(const DcPlan* p) {
-  const size_t el = p->f64 ? 8 : 4;
-  return arrays_bytes(p->n, 8) + el * (size_t)p->n * (p->u_stride + p->n);
+  size_t leaves = 0;
+  gla_plan_workspace_size(p->leafplan, &leaves);
+  return p->bytes + leaves;
 }
 
 }  // namespace gla

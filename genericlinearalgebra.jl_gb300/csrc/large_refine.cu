@@ -63,6 +63,7 @@ constexpr double kResTheta = 0.1;
 struct RefineLarge {
   int n = 0;
   bool side = false;  // runs beside others (large_create)
+  size_t bytes = 0;   // device memory held by the object itself
   float *Ahi = nullptr, *Alo = nullptr, *Xhi = nullptr, *Xlo = nullptr, *Phi = nullptr, *Plo = nullptr;
   float *Rres = nullptr, *T = nullptr, *E = nullptr, *XE = nullptr, *Ghi = nullptr, *Glo = nullptr;
   float* Cbuf = nullptr;   // cluster matrices, packed
@@ -393,7 +394,7 @@ int refine_large_create(RefineLarge** out, int n, bool side) {
   const size_t nn = (size_t)n * n;
   cudaError_t err = cudaSuccess;
   auto alloc = [&](void** p, size_t bytes) {
-    if (err == cudaSuccess) err = cudaMalloc(p, std::max<size_t>(bytes, 16));
+    if (err == cudaSuccess) err = counted_malloc(p, bytes, &r->bytes);
   };
   float** bufs[] = {&r->Ahi, &r->Alo, &r->Xhi, &r->Xlo, &r->Phi, &r->Plo, &r->Rres, &r->T, &r->E, &r->XE, &r->Ghi,
                     &r->Glo, &r->Cbuf, &r->Wbuf};
@@ -449,6 +450,11 @@ void refine_large_destroy(RefineLarge* r) {
   delete r;
 }
 
+size_t refine_large_bytes(const RefineLarge* r) {
+  size_t b = r->bytes + oz_bytes(r->oz) + oz_bytes(r->ozx) + oz_bytes(r->oz32);
+  for (const auto& kv : r->big) b += large_workspace_bytes(kv.second);
+  return b;
+}
 int refine_large_iters(const RefineLarge* r) { return r->iters; }
 int refine_large_rotations(const RefineLarge* r) { return r->rotated; }
 float* refine_large_xbuf(RefineLarge* r) { return r->Xhi; }

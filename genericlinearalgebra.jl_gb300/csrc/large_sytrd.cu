@@ -834,6 +834,7 @@ struct SytrdPlan {
   unsigned* bar = nullptr;
   int* err = nullptr;
   bool f64 = true;
+  size_t bytes = 0;       // device memory held
   bool cluster = false;   // the device can hold a cluster: small trailing orders run on it
   bool cluster_only = false;  // and all others too
   int2* F = nullptr;      // FP64, orders above kFixedMin: the trailing matrix in fixed point, n x n
@@ -1108,7 +1109,7 @@ cudaError_t sytrd_plan_create(SytrdPlan** out, int n, bool f64, bool tc) {
   for (int kk = 0; kk < 2 * last; kk++) bk[2 * kSytrdNB + kk] = kk < last ? last + kk : kk - last;
   const size_t el = f64 ? 8 : 4;
   auto alloc = [&](void** p, size_t bytes) {
-    if (err == cudaSuccess) err = cudaMalloc(p, std::max<size_t>(bytes, 16));
+    if (err == cudaSuccess) err = counted_malloc(p, bytes, &sp->bytes);
   };
   alloc((void**)&sp->ustart, sizeof(int) * ustart.size());
   alloc(&sp->P, el * np * n);
@@ -1162,6 +1163,7 @@ cudaError_t sytrd_enqueue(SytrdPlan* sp, void* A, long long lda, void* d, void* 
 }
 
 int* sytrd_error_word(SytrdPlan* sp) { return sp->err; }
+size_t sytrd_plan_bytes(const SytrdPlan* sp) { return sp->bytes; }
 void sytrd_set_oz64(SytrdPlan* sp, Oz64* oz) { sp->oz = oz; }
 bool sytrd_set_cluster_only(SytrdPlan* sp) {
   sp->cluster_only = sp->cluster && sp->n <= kSideBySideMaxN;

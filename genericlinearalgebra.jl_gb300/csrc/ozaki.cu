@@ -96,6 +96,10 @@ int oz_create_f32(OzWork** out, int m, int n, int K) {
   return create(out, m, n, K, oz::CfgF32::S, oz::CfgF32::BN);
 }
 
+size_t oz_bytes(const OzWork* w) {
+  return w->abytes + w->bbytes + 2 * sizeof(int) * ((size_t)w->A.nblk * w->A.H + (size_t)w->B.nblk * w->B.H);
+}
+
 void oz_destroy(OzWork* w) {
   if (!w) return;
   cudaFree(w->A.base);

@@ -308,9 +308,9 @@ class _PlanPool:
     and streams, and freeing it waits for the device (0.8 ms at order 64, 4 ms
     at 2048 refined). A call takes a plan out, so a plan has one user at a
     time, and gives it back after its results have been waited for, so it is
-    idle on every stream. At most `entries` plans and `limit` bytes of
-    (estimated) device workspace are kept, the least recently used go first;
-    release_workspaces() closes all of them."""
+    idle on every stream. At most `entries` plans and `limit` bytes of device
+    memory are kept, the least recently used go first; release_workspaces()
+    closes all of them."""
 
     entries, limit = 32, 2 << 30
 
@@ -319,12 +319,6 @@ class _PlanPool:
         self._plans = OrderedDict()  # (key, serial) -> (plan, bytes)
         self._bytes = 0
         self._serial = 0
-
-    @staticmethod
-    def _size(plan):
-        large = np.unique(plan.ns[plan.ns > GLA_MAX_SMALL_N]).astype(np.float64)
-        staging = 2 * plan.a_elems * np.dtype(plan.dtype).itemsize
-        return int(plan.workspace_bytes() + staging + 128 * (large ** 2).sum())
 
     def take(self, ns, **kw):
         key = (_torch().cuda.current_device(), tuple(ns), tuple(sorted(kw.items())))
@@ -342,7 +336,7 @@ class _PlanPool:
             return key, Plan(ns, **kw)  # once more with the kept workspaces free
 
     def give(self, key, plan):
-        size, drop = self._size(plan), []
+        size, drop = plan.workspace_bytes(), []
         with self._lock:
             self._plans[key, self._serial] = (plan, size)
             self._serial += 1

@@ -138,7 +138,9 @@ const char* gla_status_string(int status);
 int gla_plan_create(gla_plan_t* plan, int precision, char jobz, char uplo, int64_t batch, const int64_t* n,
                     double tol, int flags);
 int gla_plan_destroy(gla_plan_t plan);
-/* Device workspace held by the plan, in bytes. */
+/* Device memory held by the plan now, in bytes: its workspace, the contexts of
+ * its orders above GLA_MAX_SMALL_N, and what the first adjoint and the first
+ * host-buffer call add. */
 int gla_plan_workspace_size(gla_plan_t plan, size_t* bytes);
 /* Total arena sizes (elements) of A/V and of w for this plan. */
 int gla_plan_arena_sizes(gla_plan_t plan, int64_t* a_elems, int64_t* w_elems);
