@@ -33,6 +33,7 @@
 #include "gla_adjoint.h"
 #include "gla_large.h"
 #include "gla_refine.h"
+#include "gla_status.h"
 
 using namespace gla;
 
@@ -55,10 +56,10 @@ constexpr int kMaxBuckets = 8;      // size buckets of width 16 over (0, 128]
 constexpr int kMaxChunks = 4;       // host-execute pipeline: chunks of the batch
 constexpr int kMaxSide = 8;         // large matrices solved side by side
 
-#define GLA_CUDA(x)                                  \
-  do {                                               \
-    cudaError_t e_ = (x);                            \
-    if (e_ != cudaSuccess) return -1000 - (int)e_;   \
+#define GLA_CUDA(x)                                \
+  do {                                             \
+    cudaError_t e_ = (x);                          \
+    if (e_ != cudaSuccess) return cuda_status(e_); \
   } while (0)
 
 // A lazily allocated cache buffer: *slot is set only on success, so a failed
@@ -368,7 +369,7 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (err != cudaSuccess) {
       delete p;
-      return -1000 - (int)err;
+      return cuda_status(err);
     }
     p->persist_grid = std::max(1, std::min(2 * nsm, p->nwork));
   }
@@ -412,7 +413,7 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
   err = cudaMalloc((void**)&p->ws, p->ws_bytes);
   if (err != cudaSuccess) {
     delete p;
-    return -1000 - (int)err;
+    return cuda_status(err);
   }
   char* w = p->ws;
   p->d_desc = (SmallDesc*)(w + o_desc);
@@ -479,7 +480,7 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
         for (int k = 0; k < 2 && err == cudaSuccess; k++) err = cudaEventCreate(&p->tev[b][ph][k]);
   if (err != cudaSuccess) {
     gla_plan_destroy(p);
-    return -1000 - (int)err;
+    return cuda_status(err);
   }
   if (flags & GLA_FLAG_AUTOTUNE) {
     int rc = autotune_plan(p, flags & (3 | GLA_FLAG_SMALL_LOG | GLA_FLAG_REFINE_QL | GLA_FLAG_REFINE_SIMT));
@@ -786,12 +787,12 @@ int execute_large(gla_plan_t p, const void* A, void* w, void* V, int* info, cuda
       cudaStream_t s = p->side_streams[t];
       cudaError_t e = cudaSetDevice(dev);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(s, p->fork, 0);
-      int rc = e == cudaSuccess ? 0 : -1000 - (int)e;
+      int rc = e == cudaSuccess ? 0 : cuda_status(e);
       for (int c; !rc && !status.load() && (c = next.fetch_add(1)) < nside;)
         for (int k : p->chains[c].items)
           if ((rc = solve_large(p, k, A, w, V, info, s, &stats[t + 1]))) break;
       e = cudaStreamSynchronize(s);
-      if (!rc && e != cudaSuccess) rc = -1000 - (int)e;
+      if (!rc && e != cudaSuccess) rc = cuda_status(e);
       int none = 0;
       if (rc) status.compare_exchange_strong(none, rc);
     };
@@ -1018,7 +1019,7 @@ int ensure_staging(gla_plan_t p) {
     cudaFree(p->h_V);
     p->h_A = p->h_w = p->h_V = nullptr;
     p->h_info = nullptr;
-    return -1000 - (int)e;
+    return cuda_status(e);
   }
   return 0;
 }
@@ -1276,7 +1277,7 @@ int gla_plan_adjoint(gla_plan_t p, const double* w, const double* V, const doubl
     if (!rc && sides > 1) {
       cudaError_t e = cudaStreamCreateWithFlags(&a.stream, cudaStreamNonBlocking);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a.join, cudaEventDisableTiming);
-      if (e != cudaSuccess) rc = -1000 - (int)e;
+      if (e != cudaSuccess) rc = cuda_status(e);
     }
     if (rc) {
       large_adjoint_destroy(a.ctx);
@@ -1445,7 +1446,7 @@ int single_entry(int prec, char jobz, char uplo, int64_t n, int flags, SingleEnt
   if (ce != cudaSuccess) {  // nothing is cached on failure
     cudaFree(e.buf);
     gla_plan_destroy(e.plan);
-    return -1000 - (int)ce;
+    return cuda_status(ce);
   }
   auto r = g_single.emplace(k, e);
   *out = &r.first->second;
@@ -1753,7 +1754,7 @@ int tune_measure(const TuneKey& k, int count, int base_flags, TuneVal* out) {
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
-  int rc = e == cudaSuccess ? 0 : -1000 - (int)e;
+  int rc = e == cudaSuccess ? 0 : cuda_status(e);
   const int nt = std::max(32, (n + 31) / 32 * 32);
   TuneVal best{1, k.fam == 0 ? 16 : 8, 1e30f, 1e30f};
   for (int mult = 1; mult <= 4 && rc == 0; mult *= 2) {

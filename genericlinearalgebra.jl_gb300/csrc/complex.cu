@@ -33,13 +33,14 @@
 
 #include "../../include/glagpu.h"
 #include "gla_large.h"
+#include "gla_status.h"
 
 namespace {
 
-#define Z_CUDA(x)                                   \
-  do {                                              \
-    cudaError_t e_ = (x);                           \
-    if (e_ != cudaSuccess) return -1000 - (int)e_;  \
+#define Z_CUDA(x)                                       \
+  do {                                                  \
+    cudaError_t e_ = (x);                               \
+    if (e_ != cudaSuccess) return gla::cuda_status(e_); \
   } while (0)
 
 // E (2n x 2n, leading dimension 2n) from the referenced triangle of the
@@ -373,13 +374,13 @@ int gla_zheev_host(char jobz, char uplo, int64_t n, const double* A, int64_t lda
   double *dA = buf, *dV = buf + cn, *dw = buf + 2 * cn;
   cudaError_t err = cudaMemcpy2D(dA, 2 * sizeof(double) * n, A, 2 * sizeof(double) * lda, 2 * sizeof(double) * n, n,
                                  cudaMemcpyHostToDevice);
-  int rc = err == cudaSuccess ? gla_zheev(jobz, uplo, n, dA, n, dw, dV, n, info, nullptr) : -1000 - (int)err;
+  int rc = err == cudaSuccess ? gla_zheev(jobz, uplo, n, dA, n, dw, dV, n, info, nullptr) : gla::cuda_status(err);
   if (rc >= 0) {
     err = cudaMemcpy(w, dw, sizeof(double) * n, cudaMemcpyDeviceToHost);
     if (err == cudaSuccess && jobz == 'V')
       err = cudaMemcpy2D(V, 2 * sizeof(double) * ldv, dV, 2 * sizeof(double) * n, 2 * sizeof(double) * n, n,
                          cudaMemcpyDeviceToHost);
-    if (err != cudaSuccess) rc = -1000 - (int)err;
+    if (err != cudaSuccess) rc = gla::cuda_status(err);
   }
   cudaFree(buf);
   return rc;

@@ -33,6 +33,7 @@
 
 #include "../../include/glagpu.h"
 #include "gla_large.h"
+#include "gla_status.h"
 
 namespace gla {
 namespace {
@@ -167,10 +168,10 @@ void release_eigenq_cache() {
 
 namespace {
 
-#define Q_CUDA(x)                                   \
-  do {                                              \
-    cudaError_t e_ = (x);                           \
-    if (e_ != cudaSuccess) return -1000 - (int)e_;  \
+#define Q_CUDA(x)                                  \
+  do {                                             \
+    cudaError_t e_ = (x);                          \
+    if (e_ != cudaSuccess) return cuda_status(e_); \
   } while (0)
 
 }  // namespace
@@ -299,13 +300,13 @@ int gla_dsytrd_host(char uplo, int64_t n, double* A, int64_t lda, double* d, dou
   double *dA = buf, *dd = buf + nn, *de = dd + n, *dt = de + ne;
   cudaError_t err = cudaMemcpy2D(dA, sizeof(double) * n, A, sizeof(double) * lda, sizeof(double) * n, n,
                                  cudaMemcpyHostToDevice);
-  int rc = err == cudaSuccess ? gla_dsytrd(uplo, n, dA, n, dd, de, dt, nullptr) : -1000 - (int)err;
+  int rc = err == cudaSuccess ? gla_dsytrd(uplo, n, dA, n, dd, de, dt, nullptr) : cuda_status(err);
   if (rc == 0) {
     err = cudaMemcpy2D(A, sizeof(double) * lda, dA, sizeof(double) * n, sizeof(double) * n, n, cudaMemcpyDeviceToHost);
     if (err == cudaSuccess) err = cudaMemcpy(d, dd, sizeof(double) * n, cudaMemcpyDeviceToHost);
     if (err == cudaSuccess && n > 1) err = cudaMemcpy(e, de, sizeof(double) * (n - 1), cudaMemcpyDeviceToHost);
     if (err == cudaSuccess && n > 1) err = cudaMemcpy(tau, dt, sizeof(double) * (n - 1), cudaMemcpyDeviceToHost);
-    if (err != cudaSuccess) rc = -1000 - (int)err;
+    if (err != cudaSuccess) rc = cuda_status(err);
   }
   cudaFree(buf);
   return rc;
@@ -335,10 +336,10 @@ int gla_dormtr_host(char side, char uplo, char trans, int64_t m, int64_t n, cons
   if (err == cudaSuccess) err = cudaMemcpy(dt, tau, sizeof(double) * (nq - 1), cudaMemcpyHostToDevice);
   if (err == cudaSuccess)
     err = cudaMemcpy2D(dC, sizeof(double) * m, C, sizeof(double) * ldc, sizeof(double) * m, n, cudaMemcpyHostToDevice);
-  int rc = err == cudaSuccess ? gla_dormtr(side, uplo, trans, m, n, dA, nq, dt, dC, m, nullptr) : -1000 - (int)err;
+  int rc = err == cudaSuccess ? gla_dormtr(side, uplo, trans, m, n, dA, nq, dt, dC, m, nullptr) : cuda_status(err);
   if (rc == 0) {
     err = cudaMemcpy2D(C, sizeof(double) * ldc, dC, sizeof(double) * m, sizeof(double) * m, n, cudaMemcpyDeviceToHost);
-    if (err != cudaSuccess) rc = -1000 - (int)err;
+    if (err != cudaSuccess) rc = cuda_status(err);
   }
   cudaFree(buf);
   return rc;

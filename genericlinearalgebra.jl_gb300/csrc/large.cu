@@ -19,6 +19,7 @@
 #include "gla_common.cuh"
 #include "gla_large.h"
 #include "gla_launch.h"
+#include "gla_status.h"
 
 namespace gla {
 
@@ -146,10 +147,10 @@ __global__ void k_large_store(const T* __restrict__ d, const T* __restrict__ Z, 
     V[i + (long long)j * ldv] = bad ? (Tout)NAN : (Tout)Z[i + (long long)j * n];
 }
 
-#define LG_CUDA(x)                                         \
-  do {                                                     \
-    cudaError_t e_ = (x);                                  \
-    if (e_ != cudaSuccess) return -1000 - (int)e_;         \
+#define LG_CUDA(x)                                 \
+  do {                                             \
+    cudaError_t e_ = (x);                          \
+    if (e_ != cudaSuccess) return cuda_status(e_); \
   } while (0)
 
 }  // namespace
@@ -162,7 +163,7 @@ int large_create(LargeCtx** out, int n, bool f64, bool refine_stage, bool side) 
   c->f64 = f64;
   const size_t el = f64 ? 8 : 4;
   cudaError_t err = sytrd_plan_create(&c->sy, n, f64, !f64 && refine_stage);
-  int rc = err == cudaSuccess ? 0 : -1000 - (int)err;
+  int rc = err == cudaSuccess ? 0 : cuda_status(err);
   if (!rc && side && !sytrd_set_cluster_only(c->sy)) rc = -1000 - (int)cudaErrorNotSupported;
   if (!rc) rc = dc_plan_create(&c->dc, n, f64, refine_stage);
   if (!rc) rc = backtr_plan_create(&c->bt, n, f64, !f64 && refine_stage);
@@ -178,7 +179,7 @@ int large_create(LargeCtx** out, int n, bool f64, bool refine_stage, bool side) 
   auto alloc = [&](void** p, size_t bytes) {
     if (!rc) {
       cudaError_t e2 = counted_malloc(p, bytes, &c->bytes);
-      if (e2 != cudaSuccess) rc = -1000 - (int)e2;
+      if (e2 != cudaSuccess) rc = cuda_status(e2);
     }
   };
   alloc(&c->Aw, el * (size_t)n * n);
@@ -191,7 +192,7 @@ int large_create(LargeCtx** out, int n, bool f64, bool refine_stage, bool side) 
   if (!rc) {
     cudaError_t e2 = cudaMallocHost((void**)&c->h_stat, 4 * sizeof(int));
     for (int i = 0; i < 4 && e2 == cudaSuccess; i++) e2 = cudaEventCreate(&c->ev[i]);
-    if (e2 != cudaSuccess) rc = -1000 - (int)e2;
+    if (e2 != cudaSuccess) rc = cuda_status(e2);
   }
   if (rc) {
     large_destroy(c);

@@ -18,6 +18,7 @@
 #include <new>
 
 #include "gla_large.h"
+#include "gla_status.h"
 
 namespace gla {
 
@@ -129,7 +130,7 @@ int large_adjoint_create(LargeAdjoint** out, int nmax) {
   if (e == cudaSuccess) e = cudaMalloc((void**)&a->M, (nn + 1) * sizeof(double));
   if (rc || e != cudaSuccess) {
     large_adjoint_destroy(a);
-    return rc ? rc : -1000 - (int)e;
+    return rc ? rc : cuda_status(e);
   }
   *out = a;
   return 0;

@@ -14,6 +14,7 @@
 
 #include "gla_common.cuh"
 #include "gla_large.h"
+#include "gla_status.h"
 #include "tc_gemm.cuh"
 
 namespace gla {
@@ -183,7 +184,7 @@ int backtr_plan_create(BacktrPlan** out, int n, bool f64, bool tc) {
                                      (int)larft_smem_bytes<float>());
   if (err != cudaSuccess) {
     backtr_plan_destroy(p);
-    return -1000 - (int)err;
+    return cuda_status(err);
   }
   *out = p;
   return 0;
@@ -222,13 +223,13 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
                   tc::tc_make_map(&mYt, p.Yt, n, n, ldy, tc::kBM);
   k_form_y<T><<<dim3((n + 255) / 256, n), 256, 0, st>>>(A, lda, Y, n, ldy, tc ? (T*)p.Yt : (T*)nullptr);
   cudaError_t err = cudaGetLastError();
-  if (err != cudaSuccess) return -1000 - (int)err;
+  if (err != cudaSuccess) return cuda_status(err);
   if (sizeof(T) == 8 && p.oz) {
     err = oz64_backtr(p.oz, (double*)Y, (const double*)tau, (double*)Zall, ldzu, ncol, trans, st);
-    return err == cudaSuccess ? 0 : -1000 - (int)err;
+    return err == cudaSuccess ? 0 : cuda_status(err);
   }
   k_larft<T><<<p.nblk, 256, larft_smem_bytes<T>(), st>>>(Y, ldy, tau, (T*)p.Tm, n);
-  if ((err = cudaGetLastError()) != cudaSuccess) return -1000 - (int)err;
+  if ((err = cudaGetLastError()) != cudaSuccess) return cuda_status(err);
   const bool f64 = sizeof(T) == 8;
   const int bk = f64 ? GemmCfg<double>::BK : GemmCfg<float>::BK;
   for (int c0 = 0; c0 < ncol; c0 += n) {
@@ -239,7 +240,7 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
   const long long ldz = copied ? ldy : ldzu;
   if (copied && (err = cudaMemcpy2DAsync(Z, sizeof(T) * ldz, Zuser, sizeof(T) * ldzu, sizeof(T) * n, nc,
                                          cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
-    return -1000 - (int)err;
+    return cuda_status(err);
   CUtensorMap mZ;
   const bool tcz = tc && tc::tc_make_map(&mZ, (const float*)Z, n, nc, ldz, tc::kBN);
   for (int bi = 0; bi < p.nblk; bi++) {
@@ -272,11 +273,11 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
       g.alpha = 1.f;
       g.beta = 0.f;
       g.err = p.err;
-      if ((err = tc::tc_gemm_launch(mY, mZ, g, splits, st)) != cudaSuccess) return -1000 - (int)err;
+      if ((err = tc::tc_gemm_launch(mY, mZ, g, splits, st)) != cudaSuccess) return cuda_status(err);
       k_tw<T><<<(nc + 15) / 16, 256, 0, st>>>((const T*)p.Wp, splits, (long long)kb * n,
                                               (const T*)p.Tm + (long long)b * kBT * kBT, (T*)p.W2, kb, nc,
                                               trans ? 1 : 0);
-      if ((err = cudaGetLastError()) != cudaSuccess) return -1000 - (int)err;
+      if ((err = cudaGetLastError()) != cudaSuccess) return cuda_status(err);
       // Z[r0:, :] -= Y_b W2: A operand rows = rows r0.. of Y (K-major through
       // Y'), B operand = W2 (K = the block's kb reflectors)
       CUtensorMap mW2;
@@ -295,7 +296,7 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
       h.alpha = -1.f;
       h.beta = 1.f;
       h.err = p.err;
-      if ((err = tc::tc_gemm_launch(mYt, mW2, h, 1, st)) != cudaSuccess) return -1000 - (int)err;
+      if ((err = tc::tc_gemm_launch(mYt, mW2, h, 1, st)) != cudaSuccess) return cuda_status(err);
       continue;
     }
     // W = Y_b' Z[r0:, :]
@@ -315,11 +316,11 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
     g.ksplit = splits > 1 ? ((mrows + splits - 1) / splits + bk - 1) / bk * bk : 0;
     if (splits > 1) splits = (mrows + g.ksplit - 1) / g.ksplit;
     g.split_stride = (long long)kb * n;
-    if ((err = gemm_launch(f64, true, false, false, g, splits, st)) != cudaSuccess) return -1000 - (int)err;
+    if ((err = gemm_launch(f64, true, false, false, g, splits, st)) != cudaSuccess) return cuda_status(err);
     k_tw<T><<<(nc + 15) / 16, 256, 0, st>>>((const T*)p.Wp, splits, (long long)kb * n,
                                             (const T*)p.Tm + (long long)b * kBT * kBT, (T*)p.W2, kb, nc,
                                             trans ? 1 : 0);
-    if ((err = cudaGetLastError()) != cudaSuccess) return -1000 - (int)err;
+    if ((err = cudaGetLastError()) != cudaSuccess) return cuda_status(err);
     // Z[r0:, :] -= Y_b W2
     GemmDesc h{};
     h.m = mrows;
@@ -333,11 +334,11 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
     h.ldc = ldz;
     h.alpha = -1.0;
     h.beta = 1.0;
-    if ((err = gemm_launch(f64, false, false, false, h, 1, st)) != cudaSuccess) return -1000 - (int)err;
+    if ((err = gemm_launch(f64, false, false, false, h, 1, st)) != cudaSuccess) return cuda_status(err);
   }
   if (copied && (err = cudaMemcpy2DAsync(Zuser, sizeof(T) * ldzu, Z, sizeof(T) * ldz, sizeof(T) * n, nc,
                                          cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
-    return -1000 - (int)err;
+    return cuda_status(err);
   }
   return 0;
 }

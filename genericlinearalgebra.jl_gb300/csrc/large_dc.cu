@@ -38,6 +38,7 @@
 #include "gla_large.h"
 #include "gla_launch.h"
 #include "gla_small.cuh"
+#include "gla_status.h"
 #include "../../include/glagpu.h"
 
 namespace gla {
@@ -800,9 +801,9 @@ int dc_run(DcPlan& p, T* d, const T* e, T* Z, int* info, cudaStream_t st) {
   const long long ldz = n;
   DcArrays<T>& a = *reinterpret_cast<DcArrays<T>*>(sizeof(T) == 8 ? (void*)&p.a64 : (void*)&p.a32);
   cudaError_t err;
-#define DC_CUDA(x)                                \
-  do {                                            \
-    if ((err = (x)) != cudaSuccess) return -1000 - (int)err; \
+#define DC_CUDA(x)                                           \
+  do {                                                       \
+    if ((err = (x)) != cudaSuccess) return cuda_status(err); \
   } while (0)
   DC_CUDA(cudaMemsetAsync(p.d_fail, 0, sizeof(int), st));
   // leaves
@@ -948,7 +949,7 @@ int dc_plan_create(DcPlan** out, int n, bool f64, bool bisect_leaves) {
   }
   if (err != cudaSuccess) {
     dc_plan_destroy(p);
-    return -1000 - (int)err;
+    return cuda_status(err);
   }
   if (f64)
     carve_arrays<double>(*p, p->a64, (char*)p->arrays, n);

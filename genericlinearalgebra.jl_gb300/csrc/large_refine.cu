@@ -51,6 +51,7 @@
 #include "df64.cuh"
 #include "gla_large.h"
 #include "gla_launch.h"
+#include "gla_status.h"
 
 namespace gla {
 
@@ -377,10 +378,10 @@ __global__ void k_ref_store(const float* __restrict__ Xhi, const float* __restri
   }
 }
 
-#define RF_CUDA(x)                                   \
-  do {                                               \
-    cudaError_t e_ = (x);                            \
-    if (e_ != cudaSuccess) return -1000 - (int)e_;   \
+#define RF_CUDA(x)                                 \
+  do {                                             \
+    cudaError_t e_ = (x);                          \
+    if (e_ != cudaSuccess) return cuda_status(e_); \
   } while (0)
 
 }  // namespace
@@ -412,7 +413,7 @@ int refine_large_create(RefineLarge** out, int n, bool side) {
   alloc((void**)&r->cinfo, sizeof(int) * n);
   if (err != cudaSuccess) {
     refine_large_destroy(r);
-    return -1000 - (int)err;
+    return cuda_status(err);
   }
   int orc = oz_create(&r->oz, n, n, n);
   if (!orc) orc = oz_create(&r->ozx, n, 0, n);

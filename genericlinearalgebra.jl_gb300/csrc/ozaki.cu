@@ -8,6 +8,7 @@
 #include <new>
 
 #include "gla_large.h"
+#include "gla_status.h"
 #include "ozaki.cuh"
 
 namespace gla {
@@ -72,7 +73,7 @@ int create(OzWork** out, int m, int n, int K, int S, int bn) {
   if (e == cudaSuccess) e = set_attributes();
   if (e != cudaSuccess) {
     oz_destroy(w);
-    return -1000 - (int)e;
+    return cuda_status(e);
   }
   *out = w;
   return 0;

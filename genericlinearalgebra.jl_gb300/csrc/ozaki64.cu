@@ -7,6 +7,7 @@
 #include <new>
 
 #include "gla_large.h"
+#include "gla_status.h"
 #include "ozaki64.cuh"
 
 namespace gla {
@@ -105,7 +106,7 @@ int oz64_create(Oz64** out, int n, int* err) {
   if (e == cudaSuccess) e = set_attributes();
   if (e != cudaSuccess) {
     oz64_destroy(w);
-    return -1000 - (int)e;
+    return cuda_status(e);
   }
   *out = w;
   return 0;
@@ -356,7 +357,7 @@ int oz64_gemm_status(Oz64Gemm* w, cudaStream_t st) {
     e = cudaMemsetAsync(w->err, 0, sizeof(int), st);
     if (e == cudaSuccess) e = cudaErrorLaunchTimeout;
   }
-  return e == cudaSuccess ? 0 : -1000 - (int)e;
+  return e == cudaSuccess ? 0 : cuda_status(e);
 }
 
 cudaError_t oz64_gemm_mark(Oz64Gemm* w) {

@@ -41,13 +41,14 @@
 
 #include "../../include/glagpu.h"
 #include "gla_large.h"
+#include "gla_status.h"
 
 namespace {
 
-#define Q_CUDA(x)                                   \
-  do {                                              \
-    cudaError_t e_ = (x);                           \
-    if (e_ != cudaSuccess) return -1000 - (int)e_;  \
+#define Q_CUDA(x)                                       \
+  do {                                                  \
+    cudaError_t e_ = (x);                               \
+    if (e_ != cudaSuccess) return gla::cuda_status(e_); \
   } while (0)
 
 // sign(r, c) of block (r, c) of L: bit (4 r + c) set means -1
@@ -417,13 +418,13 @@ int gla_qheev_host(char jobz, char uplo, int64_t n, const double* A, int64_t lda
   double *dA = buf, *dV = buf + qn, *dw = buf + 2 * qn;
   cudaError_t err = cudaMemcpy2D(dA, 4 * sizeof(double) * n, A, 4 * sizeof(double) * lda, 4 * sizeof(double) * n, n,
                                  cudaMemcpyHostToDevice);
-  int rc = err == cudaSuccess ? gla_qheev(jobz, uplo, n, dA, n, dw, dV, n, info, nullptr) : -1000 - (int)err;
+  int rc = err == cudaSuccess ? gla_qheev(jobz, uplo, n, dA, n, dw, dV, n, info, nullptr) : gla::cuda_status(err);
   if (rc >= 0) {
     err = cudaMemcpy(w, dw, sizeof(double) * n, cudaMemcpyDeviceToHost);
     if (err == cudaSuccess && jobz == 'V')
       err = cudaMemcpy2D(V, 4 * sizeof(double) * ldv, dV, 4 * sizeof(double) * n, 4 * sizeof(double) * n, n,
                          cudaMemcpyDeviceToHost);
-    if (err != cudaSuccess) rc = -1000 - (int)err;
+    if (err != cudaSuccess) rc = gla::cuda_status(err);
   }
   cudaFree(buf);
   return rc;

@@ -24,6 +24,7 @@
 
 #include "../../include/glagpu.h"
 #include "gla_launch.h"
+#include "gla_status.h"
 
 namespace gla {
 cudaError_t tridiag_kernels_init();
@@ -63,19 +64,19 @@ bool g_init[kMaxDevices] = {};
 int scratch_base(char** out) {
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return -1000 - (int)e;
+  if (e != cudaSuccess) return cuda_status(e);
   if (dev < 0 || dev >= kMaxDevices) return -1000 - (int)cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lk(g_mu);
   if (!g_addr[dev]) {
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_scratch);
-    if (e != cudaSuccess) return -1000 - (int)e;
+    if (e != cudaSuccess) return cuda_status(e);
     g_addr[dev] = static_cast<char*>(p);
   }
   if (!g_init[dev]) {
-    if ((e = tridiag_kernels_init()) != cudaSuccess) return -1000 - (int)e;
-    if ((e = chase_kernels_init()) != cudaSuccess) return -1000 - (int)e;
-    if ((e = apply_kernels_init()) != cudaSuccess) return -1000 - (int)e;
+    if ((e = tridiag_kernels_init()) != cudaSuccess) return cuda_status(e);
+    if ((e = chase_kernels_init()) != cudaSuccess) return cuda_status(e);
+    if ((e = apply_kernels_init()) != cudaSuccess) return cuda_status(e);
     g_init[dev] = true;
   }
   *out = g_addr[dev];
@@ -100,7 +101,7 @@ __global__ void k_static_setup(SmallDesc* desc, int* perm, int n) {
 #define GLA_CUDA(x)                                \
   do {                                             \
     cudaError_t e_ = (x);                          \
-    if (e_ != cudaSuccess) return -1000 - (int)e_; \
+    if (e_ != cudaSuccess) return cuda_status(e_); \
   } while (0)
 
 }  // namespace

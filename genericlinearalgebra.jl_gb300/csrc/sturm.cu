@@ -17,6 +17,7 @@
 #include <stdint.h>
 
 #include "../../include/glagpu.h"
+#include "gla_status.h"
 
 namespace {
 
@@ -100,11 +101,11 @@ int gla_numnegevals(int64_t n, const double* d, const double* e, int64_t m, cons
   cudaStream_t st = (cudaStream_t)stream;
   if (n == 0) {
     cudaError_t err = cudaMemsetAsync(counts, 0, sizeof(int64_t) * m, st);
-    return err == cudaSuccess ? 0 : -1000 - (int)err;
+    return err == cudaSuccess ? 0 : gla::cuda_status(err);
   }
   k_sturm_counts<<<(unsigned)((m + 127) / 128), 128, 0, st>>>(n, d, e, m, sigma, counts);
   const cudaError_t err = cudaGetLastError();
-  return err == cudaSuccess ? 0 : -1000 - (int)err;
+  return err == cudaSuccess ? 0 : gla::cuda_status(err);
 }
 
 int gla_dstebz(int64_t n, const double* d, const double* e, int64_t il, int64_t iu, double abstol, double* w,
@@ -121,7 +122,7 @@ int gla_dstebz(int64_t n, const double* d, const double* e, int64_t il, int64_t 
   const int64_t threads = count * 32;
   k_stebz<<<(unsigned)((threads + 127) / 128), 128, 0, (cudaStream_t)stream>>>(n, d, e, il, count, abstol, w);
   const cudaError_t err = cudaGetLastError();
-  return err == cudaSuccess ? 0 : -1000 - (int)err;
+  return err == cudaSuccess ? 0 : gla::cuda_status(err);
 }
 
 // Host-buffer forms (stage through the device, synchronize).
@@ -142,10 +143,10 @@ int gla_numnegevals_host(int64_t n, const double* d, const double* e, int64_t m,
   if (err == cudaSuccess && n) err = cudaMemcpy(buf, d, sizeof(double) * n, cudaMemcpyHostToDevice);
   if (err == cudaSuccess && ne) err = cudaMemcpy(buf + n, e, sizeof(double) * ne, cudaMemcpyHostToDevice);
   if (err == cudaSuccess) err = cudaMemcpy(buf + n + ne, sigma, sizeof(double) * m, cudaMemcpyHostToDevice);
-  int rc = err == cudaSuccess ? gla_numnegevals(n, buf, buf + n, m, buf + n + ne, dc, nullptr) : -1000 - (int)err;
+  int rc = err == cudaSuccess ? gla_numnegevals(n, buf, buf + n, m, buf + n + ne, dc, nullptr) : gla::cuda_status(err);
   if (rc == 0) {
     err = cudaMemcpy(counts, dc, sizeof(int64_t) * m, cudaMemcpyDeviceToHost);
-    if (err != cudaSuccess) rc = -1000 - (int)err;
+    if (err != cudaSuccess) rc = gla::cuda_status(err);
   }
   cudaFree(buf);
   cudaFree(dc);
@@ -167,10 +168,11 @@ int gla_dstebz_host(int64_t n, const double* d, const double* e, int64_t il, int
   cudaError_t err = cudaMalloc((void**)&buf, sizeof(double) * (n + ne + count + 1));
   if (err == cudaSuccess) err = cudaMemcpy(buf, d, sizeof(double) * n, cudaMemcpyHostToDevice);
   if (err == cudaSuccess && ne) err = cudaMemcpy(buf + n, e, sizeof(double) * ne, cudaMemcpyHostToDevice);
-  int rc = err == cudaSuccess ? gla_dstebz(n, buf, buf + n, il, iu, abstol, buf + n + ne, nullptr) : -1000 - (int)err;
+  int rc = err == cudaSuccess ? gla_dstebz(n, buf, buf + n, il, iu, abstol, buf + n + ne, nullptr)
+                              : gla::cuda_status(err);
   if (rc == 0) {
     err = cudaMemcpy(w, buf + n + ne, sizeof(double) * count, cudaMemcpyDeviceToHost);
-    if (err != cudaSuccess) rc = -1000 - (int)err;
+    if (err != cudaSuccess) rc = gla::cuda_status(err);
   }
   cudaFree(buf);
   return rc;

@@ -26,6 +26,7 @@
 
 #include "../../include/glagpu.h"
 #include "gla_common.cuh"
+#include "gla_status.h"
 #include "tc_gemm.cuh"
 
 namespace gla {
@@ -375,13 +376,13 @@ extern "C" int gla_sgemm_3xtf32(int64_t m, int64_t n, int64_t k, float alpha, co
   if (!g_sgemm_err_addr) {
     void* a = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&a, g_sgemm_err);
-    if (e != cudaSuccess) return -1000 - (int)e;
+    if (e != cudaSuccess) return gla::cuda_status(e);
     g_sgemm_err_addr = static_cast<int*>(a);
-    if ((e = cudaMemset(g_sgemm_err_addr, 0, sizeof(int))) != cudaSuccess) return -1000 - (int)e;
+    if ((e = cudaMemset(g_sgemm_err_addr, 0, sizeof(int))) != cudaSuccess) return gla::cuda_status(e);
   }
   int h = 0;  // a wait that ran out in an earlier call is reported now
   cudaError_t e = cudaMemcpy(&h, g_sgemm_err_addr, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return -1000 - (int)e;
+  if (e != cudaSuccess) return gla::cuda_status(e);
   if (h) {
     cudaMemset(g_sgemm_err_addr, 0, sizeof(int));
     return -1000 - (int)cudaErrorLaunchTimeout;
@@ -400,6 +401,6 @@ extern "C" int gla_sgemm_3xtf32(int64_t m, int64_t n, int64_t k, float alpha, co
   g.beta = beta;
   g.err = g_sgemm_err_addr;
   e = tc_gemm_launch(mA, mB, g, 1, (cudaStream_t)stream);
-  return e == cudaSuccess ? 0 : -1000 - (int)e;
+  return e == cudaSuccess ? 0 : gla::cuda_status(e);
 }
 
