@@ -148,6 +148,7 @@ struct gla_plan_s {
     cudaEvent_t join = nullptr;
   };
   std::vector<AdjointSide> adj_large;
+  bool adj_short = false;  // memory was short for more of them
   cudaEvent_t adj_fork = nullptr;
   // orders above GLA_MAX_SMALL_N: solved by the large path
   std::vector<int> large_idx;           // batch indices, in batch order
@@ -157,7 +158,7 @@ struct gla_plan_s {
   // kSideBySideMaxN, when there are several, run side by side, each on a
   // stream and a host thread of its own: one such matrix keeps a tenth of the
   // GPU busy. An order has as many chains then as it has matrices, at most
-  // kMaxSide; otherwise one.
+  // kMaxSide, or as many as the device's memory allows; otherwise one.
   struct LargeChain {
     int n = 0;
     bool side = false;
@@ -660,6 +661,7 @@ int make_chains(gla_plan_t p, const int64_t* n) {
   }
   // (phase times are sums over matrices that have the GPU to themselves)
   bool side = nside >= 2 && !p->timing;
+  int per_order = kMaxSide;  // chains of an order: fewer where memory is short
   p->large_chain.resize(p->large_idx.size());
   for (;;) {
     int rc = 0;
@@ -667,7 +669,7 @@ int make_chains(gla_plan_t p, const int64_t* n) {
       for (auto& kv : by_order) {
         const bool sd = side && kv.first <= kSideBySideMaxN;
         if (sd != (want == 1)) continue;
-        const int nch = sd ? std::min<int>(kMaxSide, (int)kv.second.size()) : 1;
+        const int nch = sd ? std::min<int>(per_order, (int)kv.second.size()) : 1;
         for (int c = 0; c < nch && !rc; c++) {
           p->chains.emplace_back();
           gla_plan_s::LargeChain& ch = p->chains.back();
@@ -682,13 +684,16 @@ int make_chains(gla_plan_t p, const int64_t* n) {
         }
         if (rc) break;
       }
-    if (rc == -1000 - (int)cudaErrorNotSupported && side) {  // no cluster: one after another
+    const bool no_cluster = rc == -1000 - (int)cudaErrorNotSupported && side;
+    const bool no_memory = rc == -1000 - (int)cudaErrorMemoryAllocation && side && per_order > 1;
+    if (no_cluster || no_memory) {
       for (auto& ch : p->chains) {
         large_destroy(ch.ctx);
         refine_large_destroy(ch.ref);
       }
       p->chains.clear();
-      side = false;
+      if (no_cluster) side = false;  // one after another
+      if (no_memory) per_order /= 2;
       continue;
     }
     if (rc) return rc;
@@ -1253,24 +1258,18 @@ int gla_plan_adjoint(gla_plan_t p, const double* w, const double* V, const doubl
   if (!(gap_rel == gap_rel)) return -7;
   const double gr = gap_rel > 0 ? gap_rel : 1e-10;
   cudaStream_t st = (cudaStream_t)stream;
-  if (!p->large_idx.empty()) {
-    if (!p->adj_fork) GLA_CUDA(cudaEventCreateWithFlags(&p->adj_fork, cudaEventDisableTiming));
-    GLA_CUDA(cudaEventRecord(p->adj_fork, st));
-  }
-  if (p->nwork > 0) {  // orders <= GLA_MAX_SMALL_N: one CTA per matrix
-    if (!p->d_adj) GLA_CUDA(cache_alloc(&p->d_adj, adjoint_workspace_bytes(p->a_elems)));
-    GLA_CUDA(launch_adjoint(p->nwork, st, p->d_desc, p->d_perm_bucket, w, V, wbar, Vbar, Abar, p->d_adj, p->a_elems,
-                            gr));
-  }
-  if (p->large_idx.empty()) return 0;
-  // larger orders: three FP64-accurate GEMMs each, about 17 launches. Those of
-  // an order up to kSideBySideMaxN leave most of the GPU idle, so several
-  // such matrices go over up to kMaxSide streams with a workspace each,
-  // beside the small orders (23 matrices of orders 129 .. 500 one after
-  // another: 4 ms); larger ones fill the GPU one at a time.
+  // Every workspace first: a call that gets none has written nothing.
+  if (p->nwork > 0 && !p->d_adj) GLA_CUDA(cache_alloc(&p->d_adj, adjoint_workspace_bytes(p->a_elems)));
+  // The larger orders take three FP64-accurate GEMMs each, about 17 launches.
+  // Those of an order up to kSideBySideMaxN leave most of the GPU idle, so
+  // several such matrices go over up to kMaxSide streams with a workspace each
+  // (fewer where memory is short), beside the small orders (23 matrices of
+  // orders 129 .. 500 one after another: 4 ms); larger ones fill the GPU one at
+  // a time.
   int nl = 0;
   for (int b : p->large_idx) nl = std::max(nl, (int)p->n[b]);
-  const size_t sides = nl <= kSideBySideMaxN ? std::min<size_t>(kMaxSide, p->large_idx.size()) : 1;
+  size_t sides = nl <= kSideBySideMaxN ? std::min<size_t>(kMaxSide, p->large_idx.size()) : std::min(nl, 1);
+  if (p->adj_short) sides = std::min(sides, p->adj_large.size());
   while (p->adj_large.size() < sides) {
     gla_plan_s::AdjointSide a;
     int rc = large_adjoint_create(&a.ctx, nl);
@@ -1283,10 +1282,21 @@ int gla_plan_adjoint(gla_plan_t p, const double* w, const double* V, const doubl
       large_adjoint_destroy(a.ctx);
       if (a.stream) cudaStreamDestroy(a.stream);
       if (a.join) cudaEventDestroy(a.join);
-      return rc;
+      if (rc != -1000 - (int)cudaErrorMemoryAllocation || p->adj_large.empty()) return rc;
+      p->adj_short = true;
+      sides = p->adj_large.size();
+      break;
     }
     p->adj_large.push_back(a);
   }
+  if (sides > 0) {
+    if (!p->adj_fork) GLA_CUDA(cudaEventCreateWithFlags(&p->adj_fork, cudaEventDisableTiming));
+    GLA_CUDA(cudaEventRecord(p->adj_fork, st));
+  }
+  if (p->nwork > 0)  // orders <= GLA_MAX_SMALL_N: one CTA per matrix
+    GLA_CUDA(launch_adjoint(p->nwork, st, p->d_desc, p->d_perm_bucket, w, V, wbar, Vbar, Abar, p->d_adj, p->a_elems,
+                            gr));
+  if (sides == 0) return 0;
   std::vector<int64_t> aoff(p->n.size() + 1, 0), woff(p->n.size() + 1, 0);
   for (size_t q = 0; q < p->n.size(); q++) {
     aoff[q + 1] = aoff[q] + p->n[q] * p->n[q];

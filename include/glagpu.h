@@ -201,8 +201,9 @@ int gla_plan_host_pipeline(gla_plan_t plan, int* chunks, int* last_pipelined);
  * maxima) on the tensor cores: one CTA per matrix for orders <=
  * GLA_MAX_SMALL_N, three tensor-core GEMMs per matrix above. The first call
  * allocates the adjoint workspace (32 bytes per arena element, plus about
- * 70 n^2 bytes for the largest order above GLA_MAX_SMALL_N); later calls
- * allocate nothing. A bounded tensor-core wait that ran out leaves the
+ * 70 n^2 bytes for the largest order n above GLA_MAX_SMALL_N, and that up to
+ * eight times, as memory allows, for several matrices of orders up to 1024,
+ * which run side by side); later calls allocate nothing. A bounded tensor-core wait that ran out leaves the
  * matrix's Abar NaN. Asynchronous on `stream`.
  */
 int gla_plan_adjoint(gla_plan_t plan, const double* w, const double* V, const double* wbar, const double* Vbar,

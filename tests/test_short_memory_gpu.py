@@ -48,3 +48,39 @@ def test_a_failed_allocation_is_told_once(G):
             G.Plan([2000])
         assert e.value.status == OUT_OF_MEMORY
     assert np.array_equal(G.symtri(A).diagonals.dv.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32_refined"])
+@pytest.mark.parametrize("ns", [[1000] * 8, [700, 700, 700, 300, 300, 500]])
+def test_repeated_orders_share_a_context(G, precision, ns):
+    # memory for one context an order, but not for one a matrix
+    import torch
+    G.release_workspaces()
+    plan = G.Plan(ns, precision=precision)
+    A = plan.pack([torch.tensor(goe(n, k + n), device="cuda") for k, n in enumerate(ns)], device="cuda")
+    outs = []
+    for short in (False, True):
+        w, V = torch.empty(plan.w_elems, dtype=A.dtype, device="cuda"), torch.empty_like(A)
+        wbar, Vbar, Abar = torch.ones_like(w), torch.ones_like(V), torch.empty_like(V)
+        info = torch.zeros(len(ns), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        need = plan.workspace_bytes() * 4 // 5 if not short else need
+        if short:
+            plan.close()
+        with only(need) if short else contextlib.nullcontext():
+            if short:
+                plan = G.Plan(ns, precision=precision)
+            plan.execute(A, w, V, info)
+            torch.cuda.synchronize()
+            if short:
+                assert plan.workspace_bytes() < need
+        assert (info.cpu().numpy() == 0).all()
+        # the adjoint's workspaces: 84 n^2 bytes each
+        with only((128 << 20) + 120 * max(ns) ** 2) if short else contextlib.nullcontext():
+            for _ in range(2):
+                plan.adjoint(w, V, wbar, Vbar, Abar)
+            torch.cuda.synchronize()
+        outs.append([x.cpu().numpy() for x in (w, V, Abar)])
+    plan.close()
+    for a, b in zip(*outs):
+        assert np.array_equal(a, b)
