@@ -91,6 +91,20 @@ class SymTridiagonal:
             raise DimensionMismatch(f"off-diagonal has length {len(ev)}, expected {max(n - 1, 0)}")
 
 
+_OUT_OF_MEMORY = -1002  # the status of cudaErrorMemoryAllocation
+
+
+def _call(name, *args):
+    """The library call `name`, and once more without the kept plans when device
+    memory was short for it. (Such a call allocates before it writes anything
+    that it reads.)"""
+    f = getattr(_lib.load(), name)
+    rc = f(*args)
+    if rc == _OUT_OF_MEMORY and _plan_pool.clear():
+        rc = f(*args)
+    return _lib.check(rc, name)
+
+
 def _raise_for_info(info):
     info = np.asarray(info)
     if (info == -1).any():
@@ -115,7 +129,6 @@ class Plan:
     def __init__(self, ns, precision="f64", jobz="V", uplo="L", tol=None, alg="QL", small_log=False,
                  timing=False, graph=False, autotune=False, refine_ql=False, bisect=False,
                  refine_simt=False):
-        L = _lib.load()
         ns = np.ascontiguousarray(np.asarray(ns, dtype=np.int64))
         if (ns < 0).any() or (ns > GLA_MAX_N).any():
             raise DimensionMismatch(f"orders must lie in [0, {GLA_MAX_N}]")
@@ -130,13 +143,12 @@ class Plan:
             (_lib.GLA_FLAG_F32_BISECT if bisect else 0) | (_lib.GLA_FLAG_REFINE_SIMT if refine_simt else 0)
         self.graph = graph
         h = C.c_void_p()
-        _lib.check(L.gla_plan_create(C.byref(h), PRECISIONS[precision], jobz.encode(), uplo.encode(), len(ns),
-                                     ns.ctypes.data_as(C.POINTER(C.c_int64)), float(tol or 0.0), flags),
-                   "gla_plan_create")
+        _call("gla_plan_create", C.byref(h), PRECISIONS[precision], jobz.encode(), uplo.encode(), len(ns),
+              ns.ctypes.data_as(C.POINTER(C.c_int64)), float(tol or 0.0), flags)
         self._h = h
         a = C.c_int64()
         w = C.c_int64()
-        L.gla_plan_arena_sizes(h, C.byref(a), C.byref(w))
+        _lib.load().gla_plan_arena_sizes(h, C.byref(a), C.byref(w))
         self.a_elems = a.value
         self.w_elems = w.value
         self.a_off = np.zeros(len(ns), np.int64)
@@ -194,10 +206,9 @@ class Plan:
     def execute_eigen2_host(self, A, w, V2, info, stream=None):
         """execute_eigen2 from and to numpy arenas (gla_plan_execute_eigen2_host);
         synchronizes. Returns the number of matrices with nonzero info."""
-        rc = _lib.load().gla_plan_execute_eigen2_host(self._h, C.c_void_p(A.ctypes.data), C.c_void_p(w.ctypes.data),
-                                                      C.c_void_p(V2.ctypes.data), C.c_void_p(info.ctypes.data),
-                                                      _stream_ptr(stream) if stream is not None else None)
-        return _lib.check(rc, "gla_plan_execute_eigen2_host")
+        return _call("gla_plan_execute_eigen2_host", self._h, C.c_void_p(A.ctypes.data), C.c_void_p(w.ctypes.data),
+                     C.c_void_p(V2.ctypes.data), C.c_void_p(info.ctypes.data),
+                     _stream_ptr(stream) if stream is not None else None)
 
     def capture(self, A, w, V, info):
         """Capture execute(A, w, V, info) into a torch.cuda.CUDAGraph (plan made
@@ -233,11 +244,9 @@ class Plan:
     def execute_host(self, A, w, V, info, stream=None):
         """Host-buffer run (numpy arenas); copies in/out and synchronizes.
         Returns the number of matrices with nonzero info."""
-        rc = _lib.load().gla_plan_execute_host(self._h, C.c_void_p(A.ctypes.data), C.c_void_p(w.ctypes.data),
-                                               C.c_void_p(V.ctypes.data) if V is not None else None,
-                                               C.c_void_p(info.ctypes.data),
-                                               _stream_ptr(stream) if stream is not None else None)
-        return _lib.check(rc, "gla_plan_execute_host")
+        return _call("gla_plan_execute_host", self._h, C.c_void_p(A.ctypes.data), C.c_void_p(w.ctypes.data),
+                     C.c_void_p(V.ctypes.data) if V is not None else None, C.c_void_p(info.ctypes.data),
+                     _stream_ptr(stream) if stream is not None else None)
 
     def host_pipeline(self):
         """(chunks, last_pipelined): the chunks execute_host overlaps its copies
@@ -249,10 +258,9 @@ class Plan:
     def adjoint(self, w, V, wbar, Vbar, Abar, gap_rel=0.0, stream=None):
         """Abar = V (diag(wbar) + sym(F o V'Vbar)) V' for every matrix (torch CUDA
         arenas, FP64, packed like execute's outputs). Asynchronous."""
-        rc = _lib.load().gla_plan_adjoint(self._h, C.c_void_p(w.data_ptr()), C.c_void_p(V.data_ptr()),
-                                          C.c_void_p(wbar.data_ptr()), C.c_void_p(Vbar.data_ptr()),
-                                          C.c_void_p(Abar.data_ptr()), float(gap_rel), _stream_ptr(stream))
-        return _lib.check(rc, "gla_plan_adjoint")
+        return _call("gla_plan_adjoint", self._h, C.c_void_p(w.data_ptr()), C.c_void_p(V.data_ptr()),
+                     C.c_void_p(wbar.data_ptr()), C.c_void_p(Vbar.data_ptr()), C.c_void_p(Abar.data_ptr()),
+                     float(gap_rel), _stream_ptr(stream))
 
     def adjoint_host(self, w, V, wbar, Vbar, Abar, gap_rel=0.0, stream=None):
         """adjoint() on host numpy arenas (float64, C-contiguous); the library
@@ -260,10 +268,9 @@ class Plan:
         arrs = [np.ascontiguousarray(x, dtype=np.float64) for x in (w, V, wbar, Vbar)]
         if not (Abar.dtype == np.float64 and Abar.flags.c_contiguous):
             raise ValueError("Abar must be a C-contiguous float64 array")
-        rc = _lib.load().gla_plan_adjoint_host(self._h, *[C.c_void_p(x.ctypes.data) for x in arrs],
-                                               C.c_void_p(Abar.ctypes.data), float(gap_rel),
-                                               _stream_ptr(stream) if stream is not None else None)
-        return _lib.check(rc, "gla_plan_adjoint_host")
+        return _call("gla_plan_adjoint_host", self._h, *[C.c_void_p(x.ctypes.data) for x in arrs],
+                     C.c_void_p(Abar.ctypes.data), float(gap_rel),
+                     _stream_ptr(stream) if stream is not None else None)
 
     def stats(self):
         """Work counters of the last execute (rotations, sweeps, row_rotations,
@@ -328,12 +335,7 @@ class _PlanPool:
                     plan, size = self._plans.pop(k)
                     self._bytes -= size
                     return key, plan
-        try:
-            return key, Plan(ns, **kw)
-        except GLAError as e:
-            if e.status > -1000 or not self.clear():
-                raise
-            return key, Plan(ns, **kw)  # once more with the kept workspaces free
+        return key, Plan(ns, **kw)
 
     def give(self, key, plan):
         size, drop = plan.workspace_bytes(), []
@@ -414,7 +416,6 @@ def eigvals_batched(mats, uplo="L", tol=None, precision="f64", check=True):
 def _tridiag(T, jobz, alg, tol):
     if tol is not None:
         raise ValueError("tol for SymTridiagonal input: only the default eps(Float64) is supported")
-    L = _lib.load()
     torch = _torch()
     on_dev = _is_torch(T.dv)
     dev = T.dv.device if on_dev else torch.device("cuda")
@@ -425,10 +426,9 @@ def _tridiag(T, jobz, alg, tol):
         e = torch.zeros(1, dtype=torch.float64, device=dev)
     Z = torch.empty((n, n), dtype=torch.float64, device=dev) if jobz == "V" else None
     info = C.c_int()
-    rc = L.gla_dstev(jobz.encode(), n, C.c_void_p(d.data_ptr()), C.c_void_p(e.data_ptr()),
-                     C.c_void_p(Z.data_ptr()) if Z is not None else None, max(n, 1),
-                     GLA_ALG_QR if alg == "QR" else GLA_ALG_QL, C.byref(info), _stream_ptr())
-    _lib.check(rc, "gla_dstev")
+    _call("gla_dstev", jobz.encode(), n, C.c_void_p(d.data_ptr()), C.c_void_p(e.data_ptr()),
+          C.c_void_p(Z.data_ptr()) if Z is not None else None, max(n, 1),
+          GLA_ALG_QR if alg == "QR" else GLA_ALG_QL, C.byref(info), _stream_ptr())
     _raise_for_info([info.value])
     if jobz == "V":
         Zt = Z.t()  # column-major buffer -> row-major view
@@ -502,10 +502,9 @@ def _zheev(A, jobz, uplo):
     w = torch.empty(max(n, 1), dtype=torch.float64, device=X.device)
     V = torch.empty((max(n, 1), max(n, 1)), dtype=torch.complex128, device=X.device) if jobz == "V" else None
     info = C.c_int()
-    rc = _lib.load().gla_zheev(jobz.encode(), uplo.encode(), n, C.c_void_p(Xc.data_ptr()), max(n, 1),
-                               C.c_void_p(w.data_ptr()), C.c_void_p(V.data_ptr()) if V is not None else None,
-                               max(n, 1), C.byref(info), _stream_ptr())
-    _lib.check(rc, "gla_zheev")
+    _call("gla_zheev", jobz.encode(), uplo.encode(), n, C.c_void_p(Xc.data_ptr()), max(n, 1),
+          C.c_void_p(w.data_ptr()), C.c_void_p(V.data_ptr()) if V is not None else None, max(n, 1),
+          C.byref(info), _stream_ptr())
     _raise_for_info([info.value])
     w = w[:n]
     if jobz == "V":
@@ -538,10 +537,9 @@ def _qheev(Q, jobz, uplo):
     w = torch.empty(max(n, 1), dtype=torch.float64, device=X.device)
     V = torch.empty((max(n, 1), max(n, 1), 4), dtype=torch.float64, device=X.device) if jobz == "V" else None
     info = C.c_int()
-    rc = _lib.load().gla_qheev(jobz.encode(), uplo.encode(), n, C.c_void_p(Xc.data_ptr()), max(n, 1),
-                               C.c_void_p(w.data_ptr()), C.c_void_p(V.data_ptr()) if V is not None else None,
-                               max(n, 1), C.byref(info), _stream_ptr())
-    _lib.check(rc, "gla_qheev")
+    _call("gla_qheev", jobz.encode(), uplo.encode(), n, C.c_void_p(Xc.data_ptr()), max(n, 1),
+          C.c_void_p(w.data_ptr()), C.c_void_p(V.data_ptr()) if V is not None else None, max(n, 1),
+          C.byref(info), _stream_ptr())
     _raise_for_info([info.value])
     w = w[:n]
     if jobz == "V":
@@ -671,9 +669,8 @@ class EigenQ:
         X = (B.to(torch.float64) if on_dev else torch.as_tensor(np.asarray(B, dtype=np.float64), device="cuda"))
         Xc = X.t().contiguous().clone()  # column-major storage of X
         F = self.factors.t().contiguous()
-        _lib.check(_lib.load().gla_dormtr(side.encode(), self.uplo.encode(), trans.encode(), m, k,
-                                          C.c_void_p(F.data_ptr()), self.n, C.c_void_p(self.tau.data_ptr()),
-                                          C.c_void_p(Xc.data_ptr()), max(m, 1), _stream_ptr()), "gla_dormtr")
+        _call("gla_dormtr", side.encode(), self.uplo.encode(), trans.encode(), m, k, C.c_void_p(F.data_ptr()), self.n,
+              C.c_void_p(self.tau.data_ptr()), C.c_void_p(Xc.data_ptr()), max(m, 1), _stream_ptr())
         out = Xc.t()
         return out if on_dev else out.cpu().numpy()
 
@@ -705,9 +702,8 @@ def symtri(A, uplo="L"):
     d = torch.empty(max(n, 1), dtype=torch.float64, device=X.device)
     e = torch.empty(max(n - 1, 1), dtype=torch.float64, device=X.device)
     tau = torch.empty(max(n - 1, 1), dtype=torch.float64, device=X.device)
-    _lib.check(_lib.load().gla_dsytrd(uplo.encode(), n, C.c_void_p(F.data_ptr()), max(n, 1), C.c_void_p(d.data_ptr()),
-                                      C.c_void_p(e.data_ptr()), C.c_void_p(tau.data_ptr()), _stream_ptr()),
-               "gla_dsytrd")
+    _call("gla_dsytrd", uplo.encode(), n, C.c_void_p(F.data_ptr()), max(n, 1), C.c_void_p(d.data_ptr()),
+          C.c_void_p(e.data_ptr()), C.c_void_p(tau.data_ptr()), _stream_ptr())
     return SymmetricTridiagonalFactorization(EigenQ(F.t(), tau, uplo), SymTridiagonal(d[:n], e[:max(n - 1, 0)]))
 
 

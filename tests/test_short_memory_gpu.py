@@ -84,3 +84,27 @@ def test_repeated_orders_share_a_context(G, precision, ns):
     plan.close()
     for a, b in zip(*outs):
         assert np.array_equal(a, b)
+
+
+def test_other_calls_take_the_kept_plans_memory(G):
+    # the kept plans hold 0.9 GB; what is left beside them is too little for a context of order 1000
+    import torch
+    rng = np.random.default_rng(1)
+    mats = [torch.tensor(goe(1000, k), device="cuda") for k in range(8)]
+    C = rng.standard_normal((500, 500)) + 1j * rng.standard_normal((500, 500))
+    Q = rng.standard_normal((250, 250, 4))
+    Q = np.concatenate([(Q + Q.swapaxes(0, 1))[..., :1], (Q - Q.swapaxes(0, 1))[..., 1:]], axis=-1) / 2
+    calls = [lambda: G.symtri(mats[0]).diagonals.dv, lambda: G.eigvals(torch.tensor(C + C.conj().T, device="cuda")),
+             lambda: G.eigvals(G.QuaternionMatrix(torch.tensor(Q, device="cuda"))),
+             lambda: G.eigvals(G.SymTridiagonal(mats[0][0], mats[0][1, 1:])),
+             lambda: torch.tensor(G.Plan([1000, 999]).workspace_bytes())]
+    for f in calls:
+        G.release_workspaces()
+        want = f()
+        G.release_workspaces()
+        G.eigen_batched(mats)
+        assert len(G._plan_pool._plans) == 1
+        with only(64 << 20):
+            got = f()
+        assert len(G._plan_pool._plans) == 0 and torch.equal(got, want)
+    G.release_workspaces()
