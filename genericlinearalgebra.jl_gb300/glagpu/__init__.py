@@ -328,6 +328,7 @@ class _PlanPool:
         self._serial = 0
 
     def take(self, ns, **kw):
+        kw["tol"] = float(kw["tol"] or 0.0)  # (an array or tensor of one value as well)
         key = (_torch().cuda.current_device(), tuple(ns), tuple(sorted(kw.items())))
         with self._lock:
             for k in reversed(self._plans):
