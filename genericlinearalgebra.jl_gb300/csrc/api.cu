@@ -24,7 +24,6 @@
 #include <mutex>
 #include <new>
 #include <numeric>
-#include <thread>
 #include <tuple>
 #include <vector>
 
@@ -34,6 +33,7 @@
 #include "gla_large.h"
 #include "gla_refine.h"
 #include "gla_status.h"
+#include "side_threads.h"
 
 using namespace gla;
 
@@ -795,22 +795,13 @@ int execute_large(gla_plan_t p, const void* A, void* w, void* V, int* info, cuda
       int rc = e == cudaSuccess ? 0 : cuda_status(e);
       for (int c; !rc && !status.load() && (c = next.fetch_add(1)) < nside;)
         for (int k : p->chains[c].items)
-          if ((rc = solve_large(p, k, A, w, V, info, s, &stats[t + 1]))) break;
+          if ((rc = guarded([&] { return solve_large(p, k, A, w, V, info, s, &stats[t + 1]); }))) break;
       e = cudaStreamSynchronize(s);
       if (!rc && e != cudaSuccess) rc = cuda_status(e);
       int none = 0;
       if (rc) status.compare_exchange_strong(none, rc);
     };
-    std::vector<std::thread> threads;
-    for (size_t t = 1; t < p->side_streams.size(); t++) {
-      try {
-        threads.emplace_back(worker, (int)t);
-      } catch (...) {
-        break;
-      }
-    }
-    worker(0);
-    for (std::thread& t : threads) t.join();
+    on_threads((int)p->side_streams.size(), worker);
     if (status.load()) return status.load();
   }
   for (const LargeStats& s : stats) {
@@ -904,7 +895,7 @@ int plan_execute(gla_plan_t p, const void* A, void* w, void* V, int* info, cudaS
     for (int ph = 0; ph < GLA_NUM_PHASES; ph++) p->tused[b][ph] = false;
   GLA_CUDA(cudaMemsetAsync(p->d_stats, 0, sizeof(unsigned long long) * 4, st));
   if (p->batch) GLA_CUDA(cudaMemsetAsync(info, 0, sizeof(int) * p->batch, st));
-  int rc_large = execute_large(p, A, w, V, info, st);
+  int rc_large = guarded([&] { return execute_large(p, A, w, V, info, st); });
   if (rc_large) return rc_large;
   if (p->nwork == 0) return 0;
   const int lower = p->uplo == 'L';
