@@ -32,6 +32,7 @@
 #include <mutex>
 
 #include "../../include/glagpu.h"
+#include "gla_common.cuh"
 #include "gla_large.h"
 #include "gla_status.h"
 
@@ -40,26 +41,50 @@ namespace {
 
 // Lower-stored working copy W (zeros above the diagonal) of the lower
 // triangle (lower) or of the reversed upper triangle, W[i, j] =
-// A[n-1-i, n-1-j] (!lower).
-__global__ void k_q_load(const double* __restrict__ A, long long lda, int n, int lower, double* __restrict__ W) {
+// A[n-1-i, n-1-j] (!lower); the bits of the largest |entry| into *amax (zero on
+// entry; those of an infinity or NaN are above all others).
+__global__ void k_q_load(const double* __restrict__ A, long long lda, int n, int lower, double* __restrict__ W,
+                         unsigned long long* amax) {
   const int j = blockIdx.y;
+  unsigned long long m = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double x = i < j ? 0.0 : (lower ? A[i + (long long)j * lda] : A[(n - 1 - i) + (long long)(n - 1 - j) * lda]);
+    W[i + (long long)j * n] = x;
+    m = max(m, (unsigned long long)__double_as_longlong(fabs(x)));
+  }
+  m = warp_max_u64(m);
+  if ((threadIdx.x & 31) == 0 && m > *(volatile unsigned long long*)amax) atomicMax(amax, m);
+}
+
+// The power of two that the reduction's matrix is divided by. It multiplies up
+// to three entries (the quadratic form of a column), so a matrix whose largest
+// is outside 2^-200 .. 2^200 is brought to [1, 2); the others stay as they are.
+GLA_DEV int q_scale(unsigned long long amax) {
+  if (amax == 0 || amax >= 0x7ff0000000000000ull) return 0;
+  const int ex = ilogb(__longlong_as_double((long long)amax));
+  return ex > 200 || ex < -200 ? ex : 0;
+}
+__global__ void k_q_scale(double* __restrict__ W, int n, const unsigned long long* __restrict__ amax) {
+  const int ex = q_scale(*amax), j = blockIdx.y;
+  if (ex == 0) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    W[i + (long long)j * n] =
-        i < j ? 0.0 : (lower ? A[i + (long long)j * lda] : A[(n - 1 - i) + (long long)(n - 1 - j) * lda]);
+    W[i + (long long)j * n] = ldexp(W[i + (long long)j * n], -ex);
 }
 
 // The factorisation into A's referenced triangle: d on the diagonal, e next
-// to it, the reflectors' stored parts beyond (reversed back for !lower).
-__global__ void k_q_store(const double* __restrict__ W, int n, const double* __restrict__ d,
-                          const double* __restrict__ e, int lower, double* __restrict__ A, long long lda) {
-  const int j = blockIdx.y;
+// to it, the reflectors' stored parts beyond (reversed back for !lower); d and
+// e back to the matrix's own size.
+__global__ void k_q_store(const double* __restrict__ W, int n, double* __restrict__ d, double* __restrict__ e,
+                          int lower, double* __restrict__ A, long long lda,
+                          const unsigned long long* __restrict__ amax) {
+  const int ex = q_scale(*amax), j = blockIdx.y;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (i < j) continue;
     double v;
     if (i == j)
-      v = d[j];
+      v = ex ? d[j] = ldexp(d[j], ex) : d[j];
     else if (i == j + 1)
-      v = e[j];
+      v = ex ? e[j] = ldexp(e[j], ex) : e[j];
     else
       v = W[i + (long long)j * n];
     if (lower)
@@ -198,7 +223,10 @@ int gla_dsytrd(char uplo, int64_t n, double* A, int64_t lda, double* d, double* 
   const int nn = (int)n, lower = uplo == 'L';
   const dim3 g2((nn + 255) / 256, nn);
   double* W = (double*)large_work_matrix(q->c);
-  k_q_load<<<g2, 256, 0, st>>>(A, lda, nn, lower, W);
+  unsigned long long* amax = large_amax(q->c);
+  Q_CUDA(cudaMemsetAsync(amax, 0, sizeof(*amax), st));
+  k_q_load<<<g2, 256, 0, st>>>(A, lda, nn, lower, W, amax);
+  k_q_scale<<<g2, 256, 0, st>>>(W, nn, amax);
   Q_CUDA(cudaGetLastError());
   if (n == 1) {
     Q_CUDA(cudaMemcpyAsync(d, W, sizeof(double), cudaMemcpyDeviceToDevice, st));
@@ -206,7 +234,7 @@ int gla_dsytrd(char uplo, int64_t n, double* A, int64_t lda, double* d, double* 
     rc = large_sytrd(q->c, W, nn, d, e, tau, st);
     if (rc) return rc;
   }
-  k_q_store<<<g2, 256, 0, st>>>(W, nn, d, n > 1 ? e : d, lower, A, lda);
+  k_q_store<<<g2, 256, 0, st>>>(W, nn, d, n > 1 ? e : d, lower, A, lda, amax);
   Q_CUDA(cudaGetLastError());
   if (!lower) {  // the upper form's d and e are the reversed matrix's, reversed
     k_q_reverse<<<(nn + 511) / 512, 256, 0, st>>>(d, nn);

@@ -192,6 +192,8 @@ void large_stage_ms(const LargeCtx* c, float* ms3);
 int large_sytrd(LargeCtx* c, void* A, long long lda, void* d, void* e, void* tau, cudaStream_t st);
 // The context's n x n working matrix (leading dimension n).
 void* large_work_matrix(LargeCtx* c);
+// Scratch for the bits of a matrix's largest |entry|.
+unsigned long long* large_amax(LargeCtx* c);
 // Eigenpairs of the symmetric tridiagonal (d, e): d becomes the ascending
 // eigenvalues, Z (ldz) the eigenvectors. info: 0, or > 0 if a subproblem
 // did not converge.

@@ -222,6 +222,7 @@ void large_destroy(LargeCtx* c) {
 }
 
 void* large_work_matrix(LargeCtx* c) { return c->Aw; }
+unsigned long long* large_amax(LargeCtx* c) { return reinterpret_cast<unsigned long long*>(c->flags); }
 
 void large_stage_ms(const LargeCtx* c, float* ms3) {
   for (int i = 0; i < 3; i++) ms3[i] = c->ms[i];
