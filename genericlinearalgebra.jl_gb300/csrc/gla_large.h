@@ -91,10 +91,9 @@ cudaError_t oz64_rank2k(Oz64* w, const double* VW, int nbp, int t, double* A, lo
 // Problems whose sizes are known on the device only: d[0 .. nprob), not
 // transposed, at most m1max x mmax with k <= mmax (a level of the tree).
 cudaError_t oz64_grouped(Oz64* w, const GemmDesc* d, int nprob, int m1max, int mmax, cudaStream_t st);
-// Z := Q Z (trans: Q' Z) from the reflectors Y (n x n columns with their unit
+// Z := Q Z (n x n) from the reflectors Y (n x n columns with their unit
 // elements, zeros above and in the last column; overwritten) and tau.
-cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Z, long long ldz, int ncol, bool trans,
-                        cudaStream_t st);
+cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Z, long long ldz, cudaStream_t st);
 
 // C = op(A) B (+ C when add), FP64, column-major, m x n x k: on the tensor
 // cores when every extent reaches kOz64MinGemm, by the SIMT GEMM below that
@@ -136,6 +135,7 @@ void sytrd_plan_destroy(SytrdPlan* p);
 cudaError_t sytrd_enqueue(SytrdPlan* p, void* A, long long lda, void* d, void* e, void* tau, cudaStream_t st);
 int* sytrd_error_word(SytrdPlan* p);
 void sytrd_set_oz64(SytrdPlan* p, Oz64* oz);
+void sytrd_keep_entries(SytrdPlan* p);  // no fixed-point panels
 // Every panel on one thread-block cluster, so that several reductions run on
 // SMs of their own; false (and unchanged) above kSideBySideMaxN or where the
 // device cannot hold the cluster.
@@ -181,6 +181,13 @@ struct LargeCtx;
 // cluster; cudaErrorNotSupported where they cannot).
 int large_create(LargeCtx** out, int n, bool f64, bool refine_stage = false, bool side = false);
 void large_destroy(LargeCtx* c);
+// For a context whose operands are the caller's own (gla_dsytrd, gla_dormtr):
+// the reduction's products and Z := Q Z in FP64 throughout. Fixed-point
+// operands are exact to 2^-57 of the largest entry of their unit or column,
+// which is what an eigen-decomposition's accuracy is measured by; but where Q
+// does not couple two groups of rows, the product on one of them owes nothing
+// to the size of the other.
+void large_keep_entries(LargeCtx* c);
 size_t large_workspace_bytes(const LargeCtx* c);  // device memory of the context, in bytes
 // Stage times of the last large_syev (ms): tridiagonalisation (with the
 // load), divide and conquer, back-transformation (with the store).
@@ -202,7 +209,7 @@ int large_stedc(LargeCtx* c, void* d, const void* e, void* Z, long long ldz, int
 int large_ormtr(LargeCtx* c, const void* A, long long lda, const void* tau, void* Z, long long ldz, cudaStream_t st,
                 int ncol = -1, bool trans = false);
 // Clears the word that bounded waits set (the reduction clears it itself):
-// before a back-transformation that does not follow a reduction.
+// before a divide and conquer that does not follow a reduction.
 int large_clear_error(LargeCtx* c, cudaStream_t st);
 // Full eigen-decomposition of one matrix. tcode: kF64, kF32 or kF32FromF64
 // (double input solved in FP32; outputs float). Ain has leading dimension

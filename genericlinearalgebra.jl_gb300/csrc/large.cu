@@ -202,6 +202,11 @@ int large_create(LargeCtx** out, int n, bool f64, bool refine_stage, bool side) 
   return 0;
 }
 
+void large_keep_entries(LargeCtx* c) {
+  sytrd_keep_entries(c->sy);
+  backtr_set_oz64(c->bt, nullptr);
+}
+
 void large_destroy(LargeCtx* c) {
   if (!c) return;
   sytrd_plan_destroy(c->sy);

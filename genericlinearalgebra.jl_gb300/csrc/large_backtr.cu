@@ -41,35 +41,20 @@ __global__ void k_form_y(const T* __restrict__ A, long long lda, T* __restrict__
   }
 }
 
-// One CTA per block: G = Y_b' Y_b, then T (kb x kb, leading dimension kBT):
-// T[i][i] = tau_i, T[0:i, i] = -tau_i T[0:i, 0:i] G[0:i, i]. Dynamic shared
-// memory: G (kBT x kBT+1), then the staging tile of Y rows, later reused
-// for T.
+// Rows i0 .. i1 - 1 of block b's Gram matrix G = Y_b' Y_b: this thread's
+// entries (r, c) = (tid % 64, tid / 64 + 4 q). Ys: staging tile of 32 rows.
 template <class T>
-size_t larft_smem_bytes() {
-  return sizeof(T) * (size_t)(2 * kBT * (kBT + 1));
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) k_larft(const T* __restrict__ Y, long long ldy, const T* __restrict__ tau,
-                                               T* __restrict__ Tm, int n) {
-  const int b = blockIdx.x, j0 = b * kBT, kb = min(kBT, n - 1 - j0);
-  extern __shared__ __align__(16) unsigned char larft_sm[];
-  T(*G)[kBT + 1] = reinterpret_cast<T(*)[kBT + 1]>(larft_sm);
-  T(*Ys)[kBT + 1] = reinterpret_cast<T(*)[kBT + 1]>(larft_sm + sizeof(T) * kBT * (kBT + 1));
-  T(*Ts)[kBT + 1] = Ys;
-  const int tid = threadIdx.x;
-  T acc[16];
+GLA_DEV void gram_rows(const T* __restrict__ Y, long long ldy, int j0, int kb, int i0, int i1, T (*Ys)[kBT + 1],
+                       T (&acc)[16]) {
+  const int tid = threadIdx.x, r = tid % kBT, cb = tid / kBT;
 #pragma unroll
   for (int q = 0; q < 16; q++) acc[q] = T(0);
-  // thread owns entries (r, c) = (tid % 64, tid / 64 + 4 q) of the 64 x 64 Gram matrix
-  const int r = tid % kBT, cb = tid / kBT;
-  for (int i0 = j0 + 1; i0 < n; i0 += 32) {
+  for (; i0 < i1; i0 += 32) {
     __syncthreads();
     for (int idx = tid; idx < 32 * kBT; idx += 256) {
       const int ii = idx % 32, c = idx / 32;
       const int i = i0 + ii;
-      Ys[ii][c] = (i < n && c < kb) ? Y[i + (j0 + c) * ldy] : T(0);
+      Ys[ii][c] = (i < i1 && c < kb) ? Y[i + (j0 + c) * ldy] : T(0);
     }
     __syncthreads();
 #pragma unroll 4
@@ -78,6 +63,55 @@ __global__ void __launch_bounds__(256) k_larft(const T* __restrict__ Y, long lon
 #pragma unroll
       for (int q = 0; q < 16; q++) acc[q] = fma(yr, Ys[ii][cb + 4 * q], acc[q]);
     }
+  }
+}
+
+// FP64: the Gram matrices' sums over chunks of the rows, each by a CTA of its
+// own (grid: block, chunk), Gp[chunk][block][64][64]. An SM does one FP64 warp
+// instruction in 16 cycles, and all rows in the one CTA of k_larft took 0.5 ms
+// at order 400 and 2.2 ms at 2048.
+__global__ void __launch_bounds__(256) k_gram(const double* __restrict__ Y, long long ldy, int n,
+                                              double* __restrict__ Gp) {
+  __shared__ double Ys[32][kBT + 1];
+  const int b = blockIdx.x, j0 = b * kBT, kb = min(kBT, n - 1 - j0), tid = threadIdx.x;
+  const int per = ((n - j0 - 1 + (int)gridDim.y - 1) / (int)gridDim.y + 31) & ~31;
+  const int i0 = j0 + 1 + (int)blockIdx.y * per;
+  double acc[16];
+  gram_rows<double>(Y, ldy, j0, kb, min(i0, n), min(i0 + per, n), Ys, acc);
+  double* out = Gp + ((size_t)blockIdx.y * gridDim.x + b) * kBT * kBT;
+#pragma unroll
+  for (int q = 0; q < 16; q++) out[tid % kBT + (tid / kBT + 4 * q) * kBT] = acc[q];
+}
+
+// One CTA per block: G = Y_b' Y_b (or the sum of k_gram's `chunks` parts), then
+// T (kb x kb, leading dimension kBT): T[i][i] = tau_i, T[0:i, i] = -tau_i
+// T[0:i, 0:i] G[0:i, i]. Dynamic shared memory: G (kBT x kBT+1), then the
+// staging tile of Y rows, later reused for T.
+template <class T>
+size_t larft_smem_bytes() {
+  return sizeof(T) * (size_t)(2 * kBT * (kBT + 1));
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) k_larft(const T* __restrict__ Y, long long ldy, const T* __restrict__ tau,
+                                               T* __restrict__ Tm, int n, const T* __restrict__ Gp, int chunks) {
+  const int b = blockIdx.x, j0 = b * kBT, kb = min(kBT, n - 1 - j0);
+  extern __shared__ __align__(16) unsigned char larft_sm[];
+  T(*G)[kBT + 1] = reinterpret_cast<T(*)[kBT + 1]>(larft_sm);
+  T(*Ys)[kBT + 1] = reinterpret_cast<T(*)[kBT + 1]>(larft_sm + sizeof(T) * kBT * (kBT + 1));
+  T(*Ts)[kBT + 1] = Ys;
+  const int tid = threadIdx.x, r = tid % kBT, cb = tid / kBT;
+  T acc[16];
+  if (Gp) {
+#pragma unroll
+    for (int q = 0; q < 16; q++) acc[q] = T(0);
+    for (int c = 0; c < chunks; c++) {
+      const T* g = Gp + ((size_t)c * gridDim.x + b) * kBT * kBT;
+#pragma unroll
+      for (int q = 0; q < 16; q++) acc[q] += g[r + (cb + 4 * q) * kBT];
+    }
+  } else {
+    gram_rows<T>(Y, ldy, j0, kb, j0 + 1, n, Ys, acc);
   }
 #pragma unroll
   for (int q = 0; q < 16; q++) G[r][cb + 4 * q] = acc[q];
@@ -146,7 +180,7 @@ struct BacktrPlan {
   float* Zp = nullptr;
   int* err = nullptr;   // error word of the tensor-core GEMMs (set by backtr_set_error_word)
   size_t bytes = 0;     // device memory held
-  Oz64* oz = nullptr;   // FP64: the whole application on the tensor cores (set by backtr_set_oz64)
+  Oz64* oz = nullptr;   // FP64: Q Z for a square Z on the tensor cores (set by backtr_set_oz64)
 };
 
 size_t backtr_plan_bytes(const BacktrPlan* p) { return p->bytes; }
@@ -224,11 +258,16 @@ int backtr_run(BacktrPlan& p, const T* A, long long lda, const T* tau, T* Zall, 
   k_form_y<T><<<dim3((n + 255) / 256, n), 256, 0, st>>>(A, lda, Y, n, ldy, tc ? (T*)p.Yt : (T*)nullptr);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return cuda_status(err);
-  if (sizeof(T) == 8 && p.oz) {
-    err = oz64_backtr(p.oz, (double*)Y, (const double*)tau, (double*)Zall, ldzu, ncol, trans, st);
+  if (sizeof(T) == 8 && p.oz && ncol == n && !trans) {
+    err = oz64_backtr(p.oz, (double*)Y, (const double*)tau, (double*)Zall, ldzu, st);
     return err == cudaSuccess ? 0 : cuda_status(err);
   }
-  k_larft<T><<<p.nblk, 256, larft_smem_bytes<T>(), st>>>(Y, ldy, tau, (T*)p.Tm, n);
+  // (the parts of the Gram matrices in Wp, which the products take over after it)
+  const int chunks = sizeof(T) == 8 ? std::min(16, (int)((long long)p.splits * n / ((long long)p.nblk * kBT))) : 0;
+  if constexpr (sizeof(T) == 8)
+    if (chunks > 1) k_gram<<<dim3(p.nblk, chunks), 256, 0, st>>>(Y, ldy, n, (double*)p.Wp);
+  k_larft<T><<<p.nblk, 256, larft_smem_bytes<T>(), st>>>(Y, ldy, tau, (T*)p.Tm, n,
+                                                         chunks > 1 ? (const T*)p.Wp : nullptr, chunks);
   if ((err = cudaGetLastError()) != cudaSuccess) return cuda_status(err);
   const bool f64 = sizeof(T) == 8;
   const int bk = f64 ? GemmCfg<double>::BK : GemmCfg<float>::BK;

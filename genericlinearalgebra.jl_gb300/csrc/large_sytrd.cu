@@ -1165,6 +1165,12 @@ cudaError_t sytrd_enqueue(SytrdPlan* sp, void* A, long long lda, void* d, void* 
 int* sytrd_error_word(SytrdPlan* sp) { return sp->err; }
 size_t sytrd_plan_bytes(const SytrdPlan* sp) { return sp->bytes; }
 void sytrd_set_oz64(SytrdPlan* sp, Oz64* oz) { sp->oz = oz; }
+void sytrd_keep_entries(SytrdPlan* sp) {
+  cudaFree(sp->F);
+  cudaFree(sp->fe);
+  sp->F = nullptr;
+  sp->fe = nullptr;
+}
 bool sytrd_set_cluster_only(SytrdPlan* sp) {
   sp->cluster_only = sp->cluster && sp->n <= kSideBySideMaxN;
   return sp->cluster_only;

@@ -194,13 +194,12 @@ cudaError_t oz64_grouped(Oz64* w, const GemmDesc* d, int nprob, int m1max, int m
   return cudaGetLastError();
 }
 
-// Z := Q Z or Q' Z, Q = B_0 B_1 ..., B_b = I - Y_b T_b Y_b' with 128 reflectors
-// a block. Y: the reflectors as columns with their unit elements and zeros
-// above (n x n; overwritten), tau their scalars. With V_b = Y_b T_b formed
-// once (T' for Q'), a block is W = Y_b' Z, Z -= V_b W. Block b touches rows
-// 128 b .. only, and its operands start on a slab there.
-cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Zall, long long ldz, int ncol, bool trans,
-                        cudaStream_t st) {
+// Z := Q Z, Q = B_0 B_1 ..., B_b = I - Y_b T_b Y_b' with 128 reflectors a
+// block. Y: the reflectors as columns with their unit elements and zeros above
+// (n x n; overwritten), tau their scalars. With V_b = Y_b T_b formed once, a
+// block is W = Y_b' Z, Z -= V_b W. Block b touches rows 128 b .. only, and its
+// operands start on a slab there.
+cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Z, long long ldz, cudaStream_t st) {
   const int n = w->n, nb = w->nb, nks = w->nks, nref = n - 1, nblk = blocks(nref);
   const size_t nbp = (size_t)nb * kBM;
   unsigned char* p = w->arena;
@@ -242,22 +241,12 @@ cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Zall, lon
   k_larft_leaf<<<dim3(kBM / kLeafT, nblk), 256, 0, st>>>(w->G, tau, w->T, nref);
   k_larft_merge<32><<<dim3(4, 2, nblk), 256, 0, st>>>(w->G, w->T);
   k_larft_merge<64><<<dim3(16, 1, nblk), 256, 0, st>>>(w->G, w->T);
-  // V_b = Y_b T_b (or Y_b T_b') over Y, then V by block columns
+  // V_b = Y_b T_b over Y, then V by block columns
   k_slice_blockcol<<<dim3(nb, nblk), 256, kSlab, st>>>(Y, n, n, (int)nbp, vr, vexp);
   const int trows = nblk * kBM;  // the T factors' columns, one after another
-  if (!trans) {
-    Source sT{w->T, kBM, trows, kBM, nullptr};
-    k_max_cols<<<(trows + 7) / 8, 256, 0, st>>>(sT, trows, ts.mx);
-    k_tile<false><<<dim3(nblk, 4), 256, kSlab, st>>>(sT, ts);
-  } else {
-    if ((e = cudaMemsetAsync(ts.mx, 0, sizeof(unsigned) * trows, st)) != cudaSuccess) return e;
-    for (int b = 0; b < nblk; b++) {
-      Source sT{w->T + (size_t)b * kBM * kBM, kBM, kBM, kBM, nullptr};
-      Operand tb{ts.base + (size_t)b * 4 * kSlab, ts.exps + b * kBM, ts.mx + b * kBM};
-      k_max_rows<<<dim3(1, 2), 256, 0, st>>>(sT, tb.mx);
-      k_tile<true><<<dim3(1, 4), 256, kSlab, st>>>(sT, tb);
-    }
-  }
+  Source sT{w->T, kBM, trows, kBM, nullptr};
+  k_max_cols<<<(trows + 7) / 8, 256, 0, st>>>(sT, trows, ts.mx);
+  k_tile<false><<<dim3(nblk, 4), 256, kSlab, st>>>(sT, ts);
   Args gv{};
   gv.seg[0] = Seg{vr, ts.base, vexp, ts.exps, 4, 4, 4};
   gv.M = n;
@@ -276,47 +265,41 @@ cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Zall, lon
   k_gemm_steps<<<dim3(2 * nb, nblk), kThreads, kSmem, st>>>(gv, sv);
   k_slice_blockcol<<<dim3(nb, nblk), 256, kSlab, st>>>(Y, n, n, (int)nbp, vr, vexp);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  for (int c0 = 0; c0 < ncol; c0 += n) {
-    const int nc = std::min(n, ncol - c0), cb = blocks(nc);
-    double* Z = Zall + (long long)c0 * ldz;
-    for (int bi = 0; bi < nblk; bi++) {
-      const int b = trans ? bi : nblk - 1 - bi;
-      const int r0 = b * kBM, len = n - r0, ks = slabs(len);
-      Source sz{Z + r0, ldz, nc, len, nullptr};
-      k_max_cols<<<cb * kBM / 8, 256, 0, st>>>(sz, cb * kBM, zs.mx);
-      k_tile<false><<<dim3(cb, ks), 256, kSlab, st>>>(sz, zs);
-      int per = ks, splits = 1;
-      if (w->splits > 1) {  // at least eight slabs a split
-        splits = std::max(1, std::min(w->splits, ks / 8));
-        per = (ks + splits - 1) / splits;
-        splits = (ks + per - 1) / per;
-      }
-      Args h{};
-      h.seg[0] = Seg{yc.base + ((size_t)b * nks + 4 * b) * kSlab, zs.base, yc.exps + r0, zs.exps, ks, nks, ks};
-      h.M = kBM;
-      h.N = nc;
-      h.C = w->Wp;
-      h.ldc = kBM;
-      h.ksplit = splits > 1 ? per : 0;
-      h.split_stride = (long long)kBM * (long long)nbp;
-      h.err = w->err;
-      k_gemm<1><<<dim3(tiles(kBM, nc), splits), kThreads, kSmem, st>>>(h);
-      k_slice_w<<<dim3(cb, 4), 256, kSlab, st>>>(w->Wp, splits, h.split_stride, nc, ws);
-      Args u{};
-      u.seg[0] = Seg{vr + ((size_t)b * nb + b) * 4 * kSlab, ws.base, vexp + (size_t)b * nbp + r0, ws.exps, 4, 4, 4};
-      u.M = len;
-      u.N = nc;
-      u.C = Z + r0;
-      u.ldc = ldz;
-      u.neg = u.add = 1;
-      u.err = w->err;
-      k_gemm<1><<<tiles(len, nc), kThreads, kSmem, st>>>(u);
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  for (int b = nblk - 1; b >= 0; b--) {
+    const int r0 = b * kBM, len = n - r0, ks = slabs(len);
+    Source sz{Z + r0, ldz, n, len, nullptr};
+    k_max_cols<<<nb * kBM / 8, 256, 0, st>>>(sz, nb * kBM, zs.mx);
+    k_tile<false><<<dim3(nb, ks), 256, kSlab, st>>>(sz, zs);
+    int per = ks, splits = 1;
+    if (w->splits > 1) {  // at least eight slabs a split
+      splits = std::max(1, std::min(w->splits, ks / 8));
+      per = (ks + splits - 1) / splits;
+      splits = (ks + per - 1) / per;
     }
+    Args h{};
+    h.seg[0] = Seg{yc.base + ((size_t)b * nks + 4 * b) * kSlab, zs.base, yc.exps + r0, zs.exps, ks, nks, ks};
+    h.M = kBM;
+    h.N = n;
+    h.C = w->Wp;
+    h.ldc = kBM;
+    h.ksplit = splits > 1 ? per : 0;
+    h.split_stride = (long long)kBM * (long long)nbp;
+    h.err = w->err;
+    k_gemm<1><<<dim3(tiles(kBM, n), splits), kThreads, kSmem, st>>>(h);
+    k_slice_w<<<dim3(nb, 4), 256, kSlab, st>>>(w->Wp, splits, h.split_stride, n, ws);
+    Args u{};
+    u.seg[0] = Seg{vr + ((size_t)b * nb + b) * 4 * kSlab, ws.base, vexp + (size_t)b * nbp + r0, ws.exps, 4, 4, 4};
+    u.M = len;
+    u.N = n;
+    u.C = Z + r0;
+    u.ldc = ldz;
+    u.neg = u.add = 1;
+    u.err = w->err;
+    k_gemm<1><<<tiles(len, n), kThreads, kSmem, st>>>(u);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
-
 
 // ---- a single product of any shape, with operand buffers that grow
 struct Oz64Gemm {
