@@ -77,12 +77,26 @@ GLA_DEV df64 df_mac(df64 acc, df64 a, float b) {
 
 GLA_DEV df64 df_mul(df64 a, df64 b) { return df_mac(df_make(0.f, 0.f), a, b); }
 
-// a - b rounded to a float once (the high parts' difference is exact in two
-// floats).
-GLA_DEV float df_diff(df64 a, df64 b) {
-  float s, e;
+// A double as three floats (all 53 bits), and the difference of two rounded to
+// a float: on the FP32 pipe and with no more error than a few of its roundings,
+// however close the two are (the differences of the first and of the second
+// parts are exact in two floats each, and what cancels, cancels exactly).
+struct f3 {
+  float hi, mid, lo;
+};
+GLA_DEV f3 f3_from(double x) {
+  f3 r;
+  r.hi = (float)x;
+  x -= (double)r.hi;
+  r.mid = (float)x;
+  r.lo = (float)(x - (double)r.mid);
+  return r;
+}
+GLA_DEV float f3_diff(f3 a, f3 b) {
+  float s, e, t, f;
   two_sum(a.hi, -b.hi, s, e);
-  return s + (e + (a.lo - b.lo));
+  two_sum(a.mid, -b.mid, t, f);
+  return (s + t) + (e + (f + (a.lo - b.lo)));
 }
 
 // Conversions (FP64 instructions: use outside inner loops only).

@@ -152,7 +152,7 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
   df64 *As = AsBs, *Bs2 = AsBs + 16 * kTP;
   static_assert(kTPF >= 2 * kTP, "both pair tiles");
   __shared__ double lam[kSmallMaxN];
-  __shared__ df64 lamdf[kSmallMaxN];
+  __shared__ f3 lam3[kSmallMaxN];
   __shared__ float red[kRT / 32];
   __shared__ unsigned long long keys[kSmallMaxN];
   __shared__ int rank[kSmallMaxN], ord[kSmallMaxN], cstart[kSmallMaxN + 1], cid[kSmallMaxN];
@@ -298,7 +298,7 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
     for (int i = tid; i < n; i += kRT) {
       const double l = df_to(cS[(size_t)i * n + i]) / (1.0 - df_to(cR[(size_t)i * n + i]));
       lam[i] = l;
-      lamdf[i] = df_from(l);
+      lam3[i] = f3_from(l);
       keys[i] = sort_key(l);
     }
     __syncthreads();
@@ -394,10 +394,11 @@ GLA_DEV void refine_body(int mid, const SmallDesc* __restrict__ descs, const dou
       rmax = fmaxf(rmax, fabsf(rhalf));
       float eij = rhalf, eji = rhalf;
       if (cid[i] != cid[j]) {
-        const float gap = df_diff(lamdf[j], lamdf[i]);
+        const f3 li = lam3[i], lj = lam3[j];
+        const float gap = f3_diff(lj, li);
         const float sij = x.s.hi + x.s.lo;
         if (!(fabsf(sij) <= tfloor && fabsf(sij) > 1e-8f * fabsf(gap))) {
-          const df64 nij = df_mac(x.s, lamdf[j], x.r), nji = df_mac(x.s, lamdf[i], x.r);
+          const df64 nij = df_mac(x.s, df_make(lj.hi, lj.mid), x.r), nji = df_mac(x.s, df_make(li.hi, li.mid), x.r);
           eij = (nij.hi + nij.lo) / gap;
           eji = (nji.hi + nji.lo) / -gap;
         }
