@@ -49,27 +49,48 @@ GLA_DEV float rcp_seed(float x) {
 }
 
 // Guarded pivot (LAPACK dlaebz / dstebz): a pivot smaller than pivmin in
-// magnitude is replaced by -pivmin. SIGNED: a positive one by pivmin, so that
-// the count is that of the pivot as it is and an entry that stands alone is met
-// exactly however small it is.
-template <bool SIGNED = false>
-GLA_DEV float guard_piv(float q, float pivmin) {
-  return fabsf(q) < pivmin ? (SIGNED && q > 0.f ? pivmin : -pivmin) : q;
+// magnitude is replaced by -pivmin.
+GLA_DEV float guard_piv(float q, float pivmin) { return fabsf(q) < pivmin ? -pivmin : q; }
+
+// The same for the negated pivot r = -q, which keeps its sign (zero: +), so
+// that the count is that of the pivot as it is and an entry that stands alone
+// is met exactly however small it is.
+GLA_DEV float guard_neg(float r, float pivmin) {
+  return __int_as_float(__float_as_int(fmaxf(fabsf(r), pivmin)) | (__float_as_int(r) & 0x80000000));
 }
 
 // Numbers of eigenvalues of T below x0, x1, x2 (three interleaved Sturm
 // sequences). d: diagonal, e2: squared off-diagonal (shared memory, read
-// by every thread at the same index: broadcast).
+// by every thread at the same index: broadcast). SIGNED: below or at them, by
+// guard_neg (one instruction a pivot less: the magnitude's maximum and the sign
+// bit take the place of two comparisons and two selects).
 template <bool SIGNED = false>
 GLA_DEV void sturm3(int n, const float* __restrict__ d, const float* __restrict__ e2, float x0, float x1, float x2,
                     float pivmin, int& c0, int& c1, int& c2) {
-  float q0 = guard_piv<SIGNED>(d[0] - x0, pivmin), q1 = guard_piv<SIGNED>(d[0] - x1, pivmin), q2 = guard_piv<SIGNED>(d[0] - x2, pivmin);
+  if constexpr (SIGNED) {
+    float r0 = guard_neg(x0 - d[0], pivmin), r1 = guard_neg(x1 - d[0], pivmin), r2 = guard_neg(x2 - d[0], pivmin);
+    unsigned a0 = __float_as_uint(r0) >> 31, a1 = __float_as_uint(r1) >> 31, a2 = __float_as_uint(r2) >> 31;
+    for (int i = 1; i < n; i++) {
+      const float di = d[i], ei = e2[i - 1];
+      r0 = guard_neg(fmaf(-ei, rcp_seed(r0), x0 - di), pivmin);
+      r1 = guard_neg(fmaf(-ei, rcp_seed(r1), x1 - di), pivmin);
+      r2 = guard_neg(fmaf(-ei, rcp_seed(r2), x2 - di), pivmin);
+      a0 += __float_as_uint(r0) >> 31;
+      a1 += __float_as_uint(r1) >> 31;
+      a2 += __float_as_uint(r2) >> 31;
+    }
+    c0 = n - (int)a0;
+    c1 = n - (int)a1;
+    c2 = n - (int)a2;
+    return;
+  }
+  float q0 = guard_piv(d[0] - x0, pivmin), q1 = guard_piv(d[0] - x1, pivmin), q2 = guard_piv(d[0] - x2, pivmin);
   int a0 = q0 < 0.f, a1 = q1 < 0.f, a2 = q2 < 0.f;
   for (int i = 1; i < n; i++) {
     const float di = d[i], ei = e2[i - 1];
-    q0 = guard_piv<SIGNED>(fmaf(-ei, rcp_seed(q0), di - x0), pivmin);
-    q1 = guard_piv<SIGNED>(fmaf(-ei, rcp_seed(q1), di - x1), pivmin);
-    q2 = guard_piv<SIGNED>(fmaf(-ei, rcp_seed(q2), di - x2), pivmin);
+    q0 = guard_piv(fmaf(-ei, rcp_seed(q0), di - x0), pivmin);
+    q1 = guard_piv(fmaf(-ei, rcp_seed(q1), di - x1), pivmin);
+    q2 = guard_piv(fmaf(-ei, rcp_seed(q2), di - x2), pivmin);
     a0 += q0 < 0.f;
     a1 += q1 < 0.f;
     a2 += q2 < 0.f;
