@@ -63,23 +63,12 @@ struct dc_eps<float> {
   static constexpr float u = 0x1p-24f;
 };
 
-// 1/x and 1/sqrt(x) to about one unit in the last place: FP64 from a hardware
-// seed and one cubic step (3 and 4 instructions of 64 cycles, where the IEEE
-// division takes 9), FP32 from the hardware's division and square root.
-GLA_DEV double dc_rcp(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
+// 1/x and sqrt(x): FP64 from a hardware seed, FP32 from the hardware's division
+// and square root.
+GLA_DEV double dc_rcp(double x) { return rcp64(x); }
 GLA_DEV float dc_rcp(float x) { return 1.f / x; }
 GLA_DEV double dc_sqrt(double x) {  // x >= 0
-  if (prec<double>::biased_exp(x) < 64) return sqrt(x);
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = x * y;
-  const double e = fma(-h, y, 1.0);
-  return fma(h * e, fma(e, 0.375, 0.5), h);
+  return prec<double>::biased_exp(x) < 64 ? sqrt(x) : sqrt64(x);
 }
 GLA_DEV float dc_sqrt(float x) { return sqrtf(x); }
 

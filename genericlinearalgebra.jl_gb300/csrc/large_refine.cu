@@ -237,16 +237,6 @@ __device__ __forceinline__ void atomic_max_pos(float* a, float v) {
   atomicMax(reinterpret_cast<int*>(a), __float_as_int(v));  // v >= 0
 }
 
-// 1/x to about one unit in the last place (a hardware seed and one cubic
-// step: 3 FP64 instructions, where the IEEE division takes 9); x far from the
-// ends of the range.
-__device__ __forceinline__ double ref_rcp(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-
 // The correction E (FP32); max |E_ij| over separated pairs into scal[0].
 // polish: the full Gram matrix X'X (lower triangle in G) is available and
 // separated pairs take the symmetric Ogita-Aishima form
@@ -280,10 +270,10 @@ __global__ void k_ref_e(const float* __restrict__ T, const float* __restrict__ G
         // tfloor; rotations below 1e-8 cost nothing in orthogonality and are
         // kept (they carry the residual's last bits)
         const double t = 0.5 * ((double)T[idx] + (double)T[j + (long long)i * n]);
-        const double rot = t * ref_rcp(gap);
+        const double rot = t * rcp64(gap);
         sep = (fabs(t) <= tfloor && fabs(rot) > 1e-8) ? 0.f : (float)rot;
       } else {
-        sep = (float)((double)T[idx] * ref_rcp(gap));
+        sep = (float)((double)T[idx] * rcp64(gap));
       }
       em = fmaxf(em, fabsf(sep));
       e = polish ? sep - 0.5f * (Ghi[g] + Glo[g]) : sep;

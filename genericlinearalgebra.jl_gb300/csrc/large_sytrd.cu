@@ -436,8 +436,8 @@ GLA_DEV __host__ int panel_rows(int k0, int n, int G) { return (n - k0 - 1 + G -
 // zeros when sigma is zero, or when the whole column is so small (2^-500 beside
 // a matrix of size 1; FP32 2^-60) that its square leaves the normal range and
 // the seeds below: leaving it out moves the matrix by no more than its norm.
-// FP64: one seed and one cubic step per square root and reciprocal, 10
-// instructions in a row; the norm in even lanes and its reciprocal in odd ones.
+// FP64: the steps of sqrt_rsqrt64 and rcp64, 10 instructions in a row; the norm
+// in even lanes and its reciprocal in odd ones.
 GLA_DEV void panel_scalars(double alpha, double sigma, double& beta, double& tau, double& scale) {
   const double nrm2 = fma(alpha, alpha, sigma);
   if ((__double_as_longlong(sigma) << 1) == 0 || prec<double>::biased_exp(nrm2) < 1023 - 1000) {
@@ -446,9 +446,7 @@ GLA_DEV void panel_scalars(double alpha, double sigma, double& beta, double& tau
     return;
   }
   const bool odd = threadIdx.x & 1;
-  double y, x;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(nrm2));
-  const double h = nrm2 * y;
+  const double y = rsqrt_seed64(nrm2), h = nrm2 * y;
   const double e = fma(-h, y, 1.0);
   const double q = e * fma(e, 0.375, 0.5);
   const double hy = odd ? y : h;
@@ -458,10 +456,7 @@ GLA_DEV void panel_scalars(double alpha, double sigma, double& beta, double& tau
   // even: alpha - beta = sign(alpha) (|alpha| + norm); odd: tau = 1 + |alpha| / norm
   const double d = fma(odd ? fabs(alpha) : 1.0, odd ? rn : nrm, odd ? 1.0 : fabs(alpha));
   tau = __shfl_sync(0xffffffffu, d, 1);
-  const double dd = copysign(__shfl_sync(0xffffffffu, d, 0), alpha);
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(dd));
-  const double ed = fma(-dd, x, 1.0);
-  scale = fma(x, fma(ed, ed, ed), x);
+  scale = rcp64(copysign(__shfl_sync(0xffffffffu, d, 0), alpha));
 }
 GLA_DEV void panel_scalars(float alpha, float sigma, float& beta, float& tau, float& scale) {
   const float nrm2 = fmaf(alpha, alpha, sigma);

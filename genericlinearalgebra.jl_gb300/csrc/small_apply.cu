@@ -38,15 +38,8 @@ size_t apply_smem_bytes(int n, int elem) {
          4 * (3 * (size_t)n + 4) + 16 + (elem == 8 ? 4 * (size_t)chunk : 0);
 }
 
-// t = s / (1 + c), 1 <= 1 + c <= 2: the reciprocal's seed and one cubic step.
-GLA_DEV double shear(double c, double s) {
-  const double q = 1.0 + c;
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(q));
-  const double e = fma(-q, x, 1.0);
-  x = fma(x, fma(e, e, e), x);
-  return s * x;
-}
+// t = s / (1 + c), 1 <= 1 + c <= 2.
+GLA_DEV double shear(double c, double s) { return s * rcp64(1.0 + c); }
 GLA_DEV double flip_sign(double x, unsigned m) {
   return __hiloint2double((int)((unsigned)__double2hiint(x) ^ m), __double2loint(x));
 }

@@ -540,8 +540,8 @@ __global__ void __launch_bounds__(32) k_chase(const SmallDesc* __restrict__ desc
 //   6      p' = nr y | c = p y     s = e y          r = r2 y
 //
 // with p, c1 the sweep's state, e and d the entries the step consumes, ee =
-// e^2, a = d - mu, y0 the hardware seed of 1/sqrt(r2) and y its cubic
-// (Halley) correction. p' = gam'/c with gam' = c^2 a - s^2 gam is computed
+// e^2, a = d - mu, y0 the hardware seed of 1/sqrt(r2) and y its
+// third-order correction. p' = gam'/c with gam' = c^2 a - s^2 gam is computed
 // as (p a - ee c1)/r, the same number since gam = p c1: it needs no division
 // and no case for c = 0. The chase of one matrix of order 64 (4840 rotations)
 // took about 8 ms with one lane per matrix, where a rotation was 58 FP64
@@ -564,16 +564,11 @@ GLA_DEV double flip(double x, unsigned mask) {
 GLA_DEV double pick(bool f, double x, double y) {
   return __hiloint2double(f ? __double2hiint(x) : __double2hiint(y), f ? __double2loint(x) : __double2loint(y));
 }
-GLA_DEV double rsqrt_seed(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  return y;
-}
 GLA_DEV int hi_exp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 
 // The shift of :271-273 / :324-326, mu = d0 - e / (m + sign(m) hypot(m, 1))
 // with m = (d1 - d0) / 2e, as d0 - 2 e^2 / (dd + sign(dd) sqrt(dd^2 + 4 e^2)),
-// dd = d1 - d0: one reciprocal and one rsqrt, each a seed and one cubic step.
+// dd = d1 - d0.
 GLA_DEV double wilkinson_shift(double d0, double d1, double e) {
   const double dd = d1 - d0;
   const double ee4 = (2.0 * e) * (2.0 * e);
@@ -583,16 +578,7 @@ GLA_DEV double wilkinson_shift(double d0, double d1, double e) {
     const double m = div_fast(dd, 2.0 * e);
     return d0 - div_fast(e, m + tcopysign(hypot1_fast(m), m));
   }
-  const double y0 = rsqrt_seed(q);
-  const double h = q * y0;
-  const double er = fma(-h, y0, 1.0);
-  const double sq = fma(h * er, fma(er, 0.375, 0.5), h);
-  const double den = dd + copysign(sq, dd);
-  double x0;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x0) : "d"(den));
-  const double ed = fma(-den, x0, 1.0);
-  const double x = fma(x0, fma(ed, ed, ed), x0);
-  return fma(-0.5 * ee4, x, d0);
+  return fma(-0.5 * ee4, rcp64(dd + copysign(sqrt64(q), dd)), d0);
 }
 
 constexpr int kGRows = kSmallMaxN + 4;  // rows of d and of e in shared memory: two of padding on either side
@@ -817,7 +803,7 @@ __global__ void __launch_bounds__(32) k_chase_grp(const SmallDesc* __restrict__ 
       const unsigned long long bp = prec<double>::bits(p) << 1, be2 = prec<double>::bits(ei) << 1;
       const unsigned neg = ((unsigned)__double2hiint(p) & (bp > be2 ? 0x80000000u : 0u)) |
                            ((unsigned)__double2hiint(ei) & (bp == 0 ? 0x80000000u : 0u));
-      const double y0 = flip(rsqrt_seed(v1), neg);
+      const double y0 = flip(rsqrt_seed64(v1), neg);
       // 2
       const double v2 = fma(pick(l01, v1, pick(l2, p, t)), pick(l01, y0, pick(l2, a, 1.0)),
                             pick(l01, 0.0, flip(v1, 0x80000000u)));

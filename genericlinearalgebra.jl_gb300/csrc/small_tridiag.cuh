@@ -66,24 +66,15 @@ GLA_DEV double block_sum8(double v, double* red) {
 
 // The reflector's scalars from x1 and the column's squared norm (FP64, both
 // well inside the normal range): nu = copysign(norm, x1), tau = (x1 + nu)/nu
-// and 1/(x1 + nu), each from one hardware seed and a cubic correction (12
-// FP64 instructions where the IEEE square root and divisions take about 45;
-// with block_sum8 and two threads per row, the reduction and Q of one matrix
+// and 1/(x1 + nu), each from one hardware seed (12 FP64 instructions; the IEEE
+// square root and two divisions have a latency of about 30; with block_sum8 and two threads per row, the reduction and Q of one matrix
 // of order 64 went from 0.62 to 0.42 ms, of 512 of order 128 from 7.7 to 5.8).
 GLA_DEV void reflector_scalars(double x0, double sumsq, double& nu, double& tau, double& scl) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(sumsq));
-  const double h = sumsq * y;
-  const double e = fma(-h, y, 1.0);
-  const double q = e * fma(e, 0.375, 0.5);
-  const double norm = fma(h, q, h), rnorm = fma(y, q, y);
+  double norm, rnorm;
+  sqrt_rsqrt64(sumsq, norm, rnorm);
   nu = copysign(norm, x0);
-  const double xi1 = x0 + nu;
   tau = fma(fabs(x0), rnorm, 1.0);
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(xi1));
-  const double d = fma(-xi1, x, 1.0);
-  scl = fma(x, fma(d, d, d), x);
+  scl = rcp64(x0 + nu);
 }
 
 // Leading dimension of the staged matrix: odd, so that transposed accesses

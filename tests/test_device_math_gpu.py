@@ -11,12 +11,19 @@ pytestmark = pytest.mark.gpu
 
 SOURCE = r"""
 #include "df64.cuh"
+#include "gla_common.cuh"
 using namespace gla;
 __global__ void k(int what, int n, const double* a, const double* b, double* out) {
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   const double x = a[i], y = b[i];
+  double r, s;
   if (what == 0) out[i] = f3_diff(f3_from(x), f3_from(y));
+  if (what == 1) out[i] = rcp64(x);
+  if (what == 2) out[i] = sqrt64(x);
+  if (what >= 3) sqrt_rsqrt64(x, r, s);
+  if (what == 3) out[i] = r;
+  if (what == 4) out[i] = s;
 }
 extern "C" int run(int what, int n, const double* a, const double* b, double* out) {
   double* d;
@@ -62,3 +69,20 @@ def test_differences_of_three_floats(device):
     exact = a.astype(np.longdouble) - b.astype(np.longdouble)
     got = device(0, a, b).astype(np.longdouble)
     assert (np.abs(got - exact) <= 4 * 2.0 ** -24 * np.abs(exact)).all()
+
+
+def test_seeded_reciprocals_and_roots(device):
+    # relative errors: the last rounding (2^-53) for 1/x; for the roots half of
+    # that of x y as well; 1% for what the third-order step leaves out
+    u = np.longdouble(2.0) ** -53
+    rng = np.random.default_rng(2)
+    x = rng.uniform(1, 2, 500000) * 2.0 ** rng.integers(-1000, 1001, 500000)
+    x[:5] = 1, 2, 4, 2.0 ** 1000, 2.0 ** -1000
+    X = x.astype(np.longdouble)
+    for sign in (1, -1):
+        got = device(1, sign * x).astype(np.longdouble)
+        assert (np.abs(sign * got * X - 1) <= 1.01 * u).all()
+    for what in (2, 3):
+        root = np.sqrt(X)
+        assert (np.abs(device(what, x).astype(np.longdouble) - root) <= 1.01 * 1.5 * u * root).all()
+    assert (np.abs(device(4, x).astype(np.longdouble) * np.sqrt(X) - 1) <= 1.01 * 1.5 * u).all()
