@@ -84,7 +84,11 @@ struct Oz64;
 int oz64_create(Oz64** out, int n, int* err);
 void oz64_destroy(Oz64* w);
 size_t oz64_bytes(const Oz64* w);
-constexpr int kOz64MinMerge = 256;   // smallest merge whose level runs on it
+// Smallest merge whose level runs on it: below, the FP64 loops' few tiles cost
+// about what the slicing and its four launches do (tridiagonals of order 300,
+// 500 and 1500 in 1.24, 1.65 and 2.47 ms; with 128 1.20, 1.58 and 2.42 and
+// operands for another level; with 512 1.33, 1.75 and 2.56).
+constexpr int kOz64MinMerge = 256;
 // A[t:, t:] -= V W' + W V' (lower triangle of the order-n matrix A): V the
 // first nbp <= 32 columns of VW (leading dimension n), W the next nbp.
 cudaError_t oz64_rank2k(Oz64* w, const double* VW, int nbp, int t, double* A, long long lda, cudaStream_t st);
@@ -97,7 +101,9 @@ cudaError_t oz64_backtr(Oz64* w, double* Y, const double* tau, double* Z, long l
 
 // C = op(A) B (+ C when add), FP64, column-major, m x n x k: on the tensor
 // cores when every extent reaches kOz64MinGemm, by the SIMT GEMM below that
-// (there the slicing and launches cost more than the product). *w, made by
+// (there a tile of 128 rows is half empty or more: complex order 128 in 4.07 ms
+// with the line at 128 and 4.48 at 256; order 96 3.58, and 3.30 with it at 64).
+// *w, made by
 // the first call, holds the operand buffers, which grow; calls that share it
 // run on one stream after another. Should a bounded wait run out, C is NaN and
 // oz64_gemm_status tells.
@@ -139,6 +145,10 @@ void sytrd_keep_entries(SytrdPlan* p);  // no fixed-point panels
 // Every panel on one thread-block cluster, so that several reductions run on
 // SMs of their own; false (and unchanged) above kSideBySideMaxN or where the
 // device cannot hold the cluster.
+// Eight matrices of order 1000 take 31 ms side by side in FP64 and two 24 ms,
+// one after another 11 to 12 ms each. Beyond the line a cluster's 16 SMs no
+// longer hold a column's work against the whole GPU's: two of order 1200 take
+// 34.5 ms side by side and 32.8 one after another, though four 36.6 and 66.1.
 constexpr int kSideBySideMaxN = 1024;
 bool sytrd_set_cluster_only(SytrdPlan* p);
 size_t sytrd_plan_bytes(const SytrdPlan* p);

@@ -62,6 +62,8 @@ constexpr int kMaxTC = kMaxOrder / 32;  // tile columns a launch may cover (560/
 // A plan that solves several matrices side by side runs all of their panels
 // so (SytrdPlan::cluster_only), each on SMs of its own.
 constexpr int kClusterG = 16, kClusterMaxF64 = 200, kClusterMaxF32 = 700;
+static_assert(kClusterMaxF64 <= kSideBySideMaxN && kClusterMaxF32 <= kSideBySideMaxN,
+              "the cluster kernels' shared memory is set for kSideBySideMaxN");
 // Rows per dot-product unit. An FP32 unit waits for L2 (eight rows a lane, in
 // two batches of loads, 6.6 us a column at order 2048; 32 rows 7.6); in FP64
 // the warps are occupied as it is, and shorter units add their reductions
@@ -263,7 +265,8 @@ __device__ T symv_unit(const SytrdArgs<T>& a, int j, int s, int J, int ch, T* sv
 // unit by unit. A product is then three 32 x 32 -> 64-bit multiply-adds of 4
 // cycles (the product of the low digits, 2^-58 of the unit's largest, is left
 // out), the sums are exact in 64 bits, and the reductions over lanes are
-// integer additions. What is rounded is the entries, at 2^-57 of their unit's
+// integer additions. (The matrix given to gla_dsytrd keeps the FP64 units: see
+// large_keep_entries.) What is rounded is the entries, at 2^-57 of their unit's
 // largest, and the unit's sums, at 2^-56: below the 2^-53 of each FP64 sum
 // (residual and orthogonality of orders 1100 .. 4096, also of graded
 // matrices, as with FP64 products to 3%).

@@ -237,7 +237,11 @@ int gla_plan_counters(gla_plan_t plan, int64_t* counters);
 /*
  * Milliseconds spent in each phase (GLA_PHASE_*) by the last execute, from
  * CUDA events recorded on the execute's stream (plan created with
- * GLA_FLAG_TIMING; otherwise all zero). Synchronizes that stream.
+ * GLA_FLAG_TIMING; otherwise all zero). Synchronizes that stream. A plan with
+ * that flag solves its orders above GLA_MAX_SMALL_N one after another, each
+ * with the GPU to itself, where one without it solves several of orders up to
+ * 1024 side by side: its phase times add up to its own execute, not to that
+ * plan's.
  */
 int gla_plan_phase_times(gla_plan_t plan, float* ms);
 
