@@ -410,12 +410,22 @@ int gla_plan_create(gla_plan_t* plan_out, int precision, char jobz, char uplo, i
   const size_t o_corder = carve(sizeof(int) * chunk_order.size());
   // the slices of the tensor-core products' operands, one set per persistent CTA;
   // a second one for the pipeline's odd chunks, whose CTAs
-  // run beside the even chunks' with the same block indices
+  // run beside the even chunks' with the same block indices. Where memory is
+  // short: no pipeline, then half the CTAs, and so on.
   const bool ops = p->persistent && p->refine_tc;
-  const size_t ops_set = ops ? (size_t)p->persist_grid * refine_ops_bytes() : 0;
-  const size_t o_ops = carve((p->nchunks ? 2 : 1) * ops_set);
-  p->ws_bytes = off;
-  err = cudaMalloc((void**)&p->ws, p->ws_bytes);
+  const size_t o_ops = off;
+  for (;;) {
+    off = o_ops;
+    if (ops) carve((p->nchunks ? 2 : 1) * (size_t)p->persist_grid * refine_ops_bytes());
+    p->ws_bytes = off;
+    err = cudaMalloc((void**)&p->ws, p->ws_bytes);
+    if (err != cudaErrorMemoryAllocation || !ops || (p->nchunks == 0 && p->persist_grid == 1)) break;
+    (void)cudaGetLastError();
+    if (p->nchunks)
+      p->nchunks = 0;
+    else
+      p->persist_grid /= 2;
+  }
   if (err != cudaSuccess) {
     delete p;
     return cuda_status(err);

@@ -108,3 +108,24 @@ def test_other_calls_take_the_kept_plans_memory(G):
             got = f()
         assert len(G._plan_pool._plans) == 0 and torch.equal(got, want)
     G.release_workspaces()
+
+
+def test_refined_batch_with_fewer_ctas(G):
+    # every CTA of the persistent kernel has 0.9 MB of slices (twice that where the host pipeline runs)
+    rng = np.random.default_rng(3)
+    ns = rng.integers(8, 17, 2000)
+    G.release_workspaces()
+    outs = []
+    for leave in (None, 400 << 20, 160 << 20):
+        with only(leave) if leave else contextlib.nullcontext():
+            plan = G.Plan(ns, precision="f32_refined")
+            A = plan.pack([goe(int(n), 10 * k + int(n)) for k, n in enumerate(ns)])
+            w, V, info = np.zeros(plan.w_elems), np.zeros(plan.a_elems), np.zeros(len(ns), np.int32)
+            plan.execute_host(A, w, V, info)
+            if leave:
+                assert plan.workspace_bytes() < leave
+            plan.close()
+        assert not info.any()
+        outs.append((w, V))
+    for w, V in outs[1:]:
+        assert np.array_equal(w, outs[0][0]) and np.array_equal(V, outs[0][1])
