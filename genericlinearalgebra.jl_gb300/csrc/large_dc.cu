@@ -100,8 +100,21 @@ struct MergeInfo {
   int k, nf, nrot;
   int ktop, kbot;
   int fail;
-  int pad;
+  int ex;  // kd, tau and rho of the merge are in units of 2^ex
 };
+
+// A merge is solved in units of 2^ex that bring the larger of max |D| and rho
+// to [1, 2): a matrix of rank one leaves blocks of 1e-14, a graded one of any
+// size, and the squares of z / (D - lambda), up to 2^42 / rho in FP32, leave
+// the range there. Powers of two change no bit of what stays inside.
+template <class T>
+GLA_DEV T dc_pow2(int k);
+template <>
+GLA_DEV double dc_pow2<double>(int k) { return __hiloint2double((1023 + k) << 20, 0); }
+template <>
+GLA_DEV float dc_pow2<float>(int k) { return __int_as_float((127 + k) << 23); }
+template <class T>
+constexpr int kDcMinEx = sizeof(T) == 8 ? -900 : -100;
 
 template <class T>
 struct DcArrays {
@@ -111,13 +124,13 @@ struct DcArrays {
   int* ssrc;    // local source column of each sorted entry
   int* zdef;    // z-deflation flag of each sorted entry
   int* ctype;   // per local column: 0 top, 1 bottom, 2 mixed
-  T *kd, *kz;   // kept entries
+  T *kd, *kz;   // kept entries (kd in units of 2^ex)
   int* ksrc;
   T* fd;        // deflated eigenvalues
   int* fsrc;
   T *rc, *rs;   // rotation list
   int *rp, *rt;
-  int* org;     // secular roots: origin (kept index) and offset
+  int* org;     // secular roots: origin (kept index) and offset (in units of 2^ex)
   T* tau;
   T* zh;
   int *opos_k, *opos_f;  // absolute output column of kept / deflated entries
@@ -174,7 +187,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_dc_prep(DcArrays<T> a) {
   const long long ld = a.ld;
   const T beta = a.e[o + m1 - 1];
   const T sgn = beta < T(0) ? T(-1) : T(1);
-  const T rho = T(2) * fabs(beta);
+  T rho = T(2) * fabs(beta);
   const T rs2 = T(0.70710678118654752440);
   __shared__ unsigned long long sred[kPrepThreads / 32];
   __shared__ int scnt[kPrepThreads / 32], sfirst;
@@ -220,7 +233,14 @@ __global__ void __launch_bounds__(kPrepThreads) k_dc_prep(DcArrays<T> a) {
   dbits = warp_max_u64(sred[lane]);
   T dmax;
   from_bits(dbits, dmax);
-  const T tol = T(8) * dc_eps<T>::u * fmax(dmax, rho);
+  // below 2^kDcMinEx of the matrix (which has its largest entry in [1, 2)) the
+  // coupling is left out: everything deflates
+  const unsigned long long mbits = dbits > abs_bits(rho) ? dbits : abs_bits(rho);
+  const int ex0 = (int)(mbits >> prec<T>::mant) - prec<T>::expbias;
+  const int ex = max(kDcMinEx<T>, min(ex0, -kDcMinEx<T>));
+  const T scl = dc_pow2<T>(-ex), up = dc_pow2<T>(ex);
+  rho *= scl;
+  const T tol = ex0 < kDcMinEx<T> ? T(INFINITY) : T(8) * dc_eps<T>::u * fmax(dmax * scl, rho);
   // entries that the size of z keeps, in order, and the others: thread t takes
   // `per` consecutive ones
   const int per = (m + kPrepThreads - 1) / kPrepThreads;
@@ -249,7 +269,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_dc_prep(DcArrays<T> a) {
       a.fd[o + t - before] = Dt;
       a.fsrc[o + t - before] = st;
     } else {
-      a.kd[o + before] = Dt;
+      a.kd[o + before] = Dt * scl;
       a.kz[o + before] = a.sZ[o + t];
       a.ksrc[o + before] = st;
       before++;
@@ -299,7 +319,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_dc_prep(DcArrays<T> a) {
               a.ctype[o + sp] = 2;
               a.ctype[o + st] = 2;
             }
-            a.fd[o + nf] = cs * cs * Dp + sn * sn * Dt;
+            a.fd[o + nf] = (cs * cs * Dp + sn * sn * Dt) * up;
             a.fsrc[o + nf] = sp;
             nf++;
             Dp = sn * sn * Dp + cs * cs * Dt;
@@ -329,6 +349,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_dc_prep(DcArrays<T> a) {
     mi->nf = nf;
     mi->nrot = nr;
     mi->fail = 0;
+    mi->ex = ex;
   }
 }
 
@@ -360,7 +381,7 @@ __global__ void __launch_bounds__(256) k_dc_secular(DcArrays<T> a) {
   if (j >= k) return;
   const T* __restrict__ D = a.kd + o;
   const T* __restrict__ Z = a.kz + o;
-  const T rho = T(2) * fabs(a.e[o + mp->m1 - 1]);
+  const T rho = T(2) * fabs(a.e[o + mp->m1 - 1]) * dc_pow2<T>(-mp->ex);
   const T irho = T(1) / rho;
   const T eps = dc_eps<T>::u;
   if (k == 1) {
@@ -483,7 +504,7 @@ __global__ void __launch_bounds__(256) k_dc_zhat(DcArrays<T> a) {
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= k) return;
   const T* __restrict__ D = a.kd + o;
-  const T rho = T(2) * fabs(a.e[o + mi.m1 - 1]);
+  const T rho = T(2) * fabs(a.e[o + mi.m1 - 1]) * dc_pow2<T>(-mi.ex);
   const T Di = D[i];
   // lambda_j - D_i = tau_j - (D_i - D_org(j))
   T prod = T(1);
@@ -542,13 +563,14 @@ __global__ void __launch_bounds__(1024) k_dc_post(DcArrays<T> a, int mpow2) {
   MergeInfo* mp = a.info + blockIdx.x;
   const int o = mp->o, m1 = mp->m1, m = m1 + mp->m2, k = mp->k;
   const int tid = threadIdx.x;
+  const T up = dc_pow2<T>(mp->ex);
   extern __shared__ unsigned char smraw[];
   unsigned long long* key = reinterpret_cast<unsigned long long*>(smraw);
   int* tag = reinterpret_cast<int*>(key + mpow2);
   // eigenvalue of entry t: kept roots first (t < k), then deflated
   for (int t = tid; t < mpow2; t += 1024) {
     if (t < m) {
-      T v = t < k ? a.kd[o + a.org[o + t]] + a.tau[o + t] : a.fd[o + (t - k)];
+      T v = t < k ? (a.kd[o + a.org[o + t]] + a.tau[o + t]) * up : a.fd[o + (t - k)];
       key[t] = sort_key(v);
       tag[t] = t;
     } else {
@@ -580,7 +602,7 @@ __global__ void __launch_bounds__(1024) k_dc_post(DcArrays<T> a, int mpow2) {
     const int t = tag[pos];
     T v;
     if (t < k) {
-      v = a.kd[o + a.org[o + t]] + a.tau[o + t];
+      v = (a.kd[o + a.org[o + t]] + a.tau[o + t]) * up;
       a.opos_k[o + t] = o + pos;
     } else {
       v = a.fd[o + (t - k)];

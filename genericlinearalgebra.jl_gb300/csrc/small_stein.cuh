@@ -311,6 +311,9 @@ GLA_DEV bool stein_solve(int n, const float* __restrict__ dd, const float* __res
   glo -= widen;
   ghi += widen;
   const float atol = 2.f * prec<float>::eps * tnorm + 4.f * pivmin;
+  // a matrix that the guarded pivots reach (a leaf far below the others of its
+  // tridiagonal) is the chase's as well
+  if (!(tnorm > 0x1p40f * pivmin)) return false;
   grid_bracket(n, dd, e2s, glo, ghi, pivmin, cnt);
   if (tid < n) lams[tid] = eig_bisect(n, dd, e2s, tid, glo, ghi, atol, pivmin);
   __syncthreads();
