@@ -317,10 +317,7 @@ GLA_DEV bool stein_solve(int n, const float* __restrict__ dd, const float* __res
   grid_bracket(n, dd, e2s, glo, ghi, pivmin, cnt);
   if (tid < n) lams[tid] = eig_bisect(n, dd, e2s, tid, glo, ghi, atol, pivmin);
   __syncthreads();
-  // strict: a zero gap is tight even when ||T|| = 0
-  if (tid + 1 < n && !(lams[tid + 1] - lams[tid] > kTightGap * tnorm)) misc[0] = 1;
-  __syncthreads();
-  if (misc[0] != 0) return false;
+  if (__syncthreads_or(tid + 1 < n && !(lams[tid + 1] - lams[tid] > kTightGap * tnorm))) return false;
   if (tid < n && !twisted_vector(n, dd, ee, e2s, lams[tid], pivmin, Ys, ldy, tid)) misc[0] = 1;
   if (tid == 0) {  // clusters of two or more eigenvalues within kLooseGap ||T||
     int nc = 0, s0 = 0;
