@@ -52,11 +52,16 @@ template <> struct prec<double> {
     r = fma(-h, y, 1.0);
     return fma(0.5 * y, r, y);
   }
-  // True when |x| lies in [2^-900, 2^900]: reciprocals and squares of such
-  // values stay normal, so the seeded Newton paths above are safe.
+  // True when |x| lies in [2^-900, 2^900]: reciprocals of such values stay
+  // normal, so the seeded Newton paths above are safe.
   GLA_DEV static bool tame(double x) {
     int be = biased_exp(x);
     return be >= expbias - 900 && be <= expbias + 900;
+  }
+  // The same for squares, and sums of two of them.
+  GLA_DEV static bool squares(double x) {
+    int be = biased_exp(x);
+    return be >= expbias - 480 && be <= expbias + 480;
   }
 };
 
@@ -124,6 +129,7 @@ template <> struct prec<float> {
     int be = biased_exp(x);
     return be >= expbias - 60 && be <= expbias + 60;
   }
+  GLA_DEV static bool squares(float x) { return tame(x); }
 };
 
 template <class T> GLA_DEV T tabs(T x) { return x < 0 ? -x : x; }

@@ -102,7 +102,7 @@ template <class T> GLA_DEV void givens(T f, T g, T& c, T& s, T& r) {
     r = g;
     return;
   }
-  if (prec<T>::tame(f) && prec<T>::tame(g)) {
+  if (prec<T>::squares(f) && prec<T>::squares(g)) {
     const T r2 = fma(f, f, g * g);
     const T y = prec<T>::rsqrt(r2);
     r = r2 * y;
@@ -183,7 +183,7 @@ GLA_DEV void store_rot(float* log, int k, float c, float s) {
 // the correctly rounded hypot here.
 template <class T> GLA_DEV T hypot1_fast(T m) {
   const T am = tabs(m);
-  if (!prec<T>::tame(am)) return am < T(1) ? T(1) : am;
+  if (!prec<T>::squares(am)) return am < T(1) ? T(1) : am;
   const T q = fma(m, m, T(1));
   return q * prec<T>::rsqrt(q);
 }
