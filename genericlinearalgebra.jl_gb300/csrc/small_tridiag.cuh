@@ -67,8 +67,9 @@ GLA_DEV double block_sum8(double v, double* red) {
 // The reflector's scalars from x1 and the column's squared norm (FP64, both
 // well inside the normal range): nu = copysign(norm, x1), tau = (x1 + nu)/nu
 // and 1/(x1 + nu), each from one hardware seed (12 FP64 instructions; the IEEE
-// square root and two divisions have a latency of about 30; with block_sum8 and two threads per row, the reduction and Q of one matrix
-// of order 64 went from 0.62 to 0.42 ms, of 512 of order 128 from 7.7 to 5.8).
+// square root and two divisions have a latency of about 30; with block_sum8
+// and two threads per row, the reduction and Q of one matrix of order 64 went
+// from 0.62 to 0.42 ms, of 512 of order 128 from 7.7 to 5.8).
 GLA_DEV void reflector_scalars(double x0, double sumsq, double& nu, double& tau, double& scl) {
   double norm, rnorm;
   sqrt_rsqrt64(sumsq, norm, rnorm);
@@ -206,37 +207,32 @@ GLA_DEV void tridiag_body_shared(const SmallDesc& dsc, double* S, int ld, double
   for (int k = 0; k + 2 < n; k++) {
     const int m = n - k - 1;
     T* xc = S + (size_t)k * ld + (k + 1);
-    const T xi = (tid < m) ? xc[tid] : T(0);
+    T xi = (tid < m) ? xc[tid] : T(0);
     const T x0 = xc[0];  // read before the reduction's barriers; thread 0 rewrites xc[0] below
     T sumsq;
     unsigned long long mb;
     block_sum_max(xi * xi, (tid < m) ? AbsBits<T>::get(xi) : 0ull, red, redm, sumsq, mb);
     T tau = 0;
     if (mb != 0) {
-      // LinearAlgebra.reflector!: norm (scaled only when maxabs^2 would
-      // overflow or underflow), nu = copysign(norm, x1), x1 += nu,
-      // x[2:] /= x1, tau = x1/nu, x[1] = -nu.
+      // LinearAlgebra.reflector!: nu = copysign(norm, x1), x1 += nu,
+      // x[2:] /= x1, tau = x1/nu, x[1] = -nu. A column far from 1 is brought
+      // there first by an exact power of two: its squares, 1/x1 and, where it
+      // is subnormal, nu keep their digits, and I - tau v v' stays orthogonal.
       T nu, scl;
       const int mbe = (int)(mb >> 52);  // (FP64) biased exponent of the largest entry
       if (mbe > 1023 - 400 && mbe < 1023 + 400) {
         reflector_scalars(x0, sumsq, nu, tau, scl);
       } else {
-        const T maxabs = AbsBits<T>::from(mb);
-        const T mm = maxabs * maxabs;
-        T normu;
-        if (isfinite((T)m * mm) && mm != 0) {
-          normu = prec<T>::sqrt_ieee(sumsq);
-        } else {
-          const T r = (tid < m) ? xi / maxabs : T(0);
-          T s2;
-          unsigned long long dummy;
-          block_sum_max(r * r, 0ull, red, redm, s2, dummy);
-          normu = maxabs * prec<T>::sqrt_ieee(s2);
-        }
-        nu = tcopysign(normu, x0);
-        const T xi1 = x0 + nu;
-        tau = prec<T>::div_ieee(xi1, nu);
-        scl = prec<T>::tame(xi1) ? prec<T>::rcp(xi1) : prec<T>::div_ieee(T(1), xi1);
+        const int ex = min(max(mbe - 1023, -1022), 1022);
+        const T dn = __hiloint2double((1023 - ex) << 20, 0), up = __hiloint2double((1023 + ex) << 20, 0);
+        xi *= dn;
+        T s2;
+        unsigned long long dummy;
+        block_sum_max(xi * xi, 0ull, red, redm, s2, dummy);
+        const T y0 = x0 * dn, nus = copysign(prec<T>::sqrt_ieee(s2), y0), y1 = y0 + nus;
+        tau = prec<T>::div_ieee(y1, nus);
+        scl = prec<T>::rcp(y1);
+        nu = nus * up;
       }
       if (tid < m) {
         const T v = (tid == 0) ? T(1) : xi * scl;

@@ -143,23 +143,28 @@ GLA_DEV void tridiag_regs_block(float (&a)[NB][NB], int n, float* dd, float* ee,
         float tau = 0.f, scl = 0.f, nu = 0.f;
         if (mb != 0) {  // (alike in the 16 lanes of a row)
           const float maxabs = __uint_as_float(mb), mm = maxabs * maxabs;
-          float norm;
-          if (isfinite((float)(n - k - 1) * mm) && mm != 0.f) {
-            norm = prec<float>::sqrt_ieee(s2);
-          } else {  // squares out of range: by an exact power of two
+          float y0 = x0, up = 1.f;
+          if (!(isfinite((float)(n - k - 1) * mm) && mm >= 0x1p-100f)) {
+            // squares (nearly) out of range: the column by an exact power of
+            // two, so that 1/x1 and, where it is subnormal, nu keep their digits
             const int ex = min(max((int)(mb >> 23) - 127, -126), 126);
-            const float dn = __int_as_float((127 - ex) << 23), up = __int_as_float((127 + ex) << 23);
-            float q2 = 0.f;
+            const float dn = __int_as_float((127 - ex) << 23);
+            up = __int_as_float((127 + ex) << 23);
+            y0 *= dn;
+            s2 = 0.f;
 #pragma unroll
-            for (int v = KB; v < NB; v++) q2 = fmaf(x[v] * dn, x[v] * dn, q2);
+            for (int v = KB; v < NB; v++) {
+              x[v] *= dn;
+              s2 = fmaf(x[v], x[v], s2);
+            }
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) q2 += __shfl_xor_sync(half, q2, o);
-            norm = up * prec<float>::sqrt_ieee(q2);
+            for (int o = 8; o > 0; o >>= 1) s2 += __shfl_xor_sync(half, s2, o);
           }
-          nu = copysignf(norm, x0);
-          const float xi1 = x0 + nu;
+          nu = copysignf(prec<float>::sqrt_ieee(s2), y0);
+          const float xi1 = y0 + nu;
           tau = prec<float>::div_ieee(xi1, nu);
           scl = prec<float>::tame(xi1) ? prec<float>::rcp(xi1) : prec<float>::div_ieee(1.f, xi1);
+          nu *= up;
         }
         if (mine) {
 #pragma unroll
