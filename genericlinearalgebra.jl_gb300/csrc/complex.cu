@@ -16,9 +16,10 @@
 // orthogonalisation keeps k orthonormal vectors. The complex inner
 // products of vectors from different groups carry the real subspaces'
 // departure from invariance under [x; y] -> [-y; x], about u ||A|| / gap,
-// so one symmetric Newton-Schulz step V <- V (I + R/2), R = I - V^H V, in
+// so a symmetric Newton-Schulz step V <- V (I + R/2), R = I - V^H V, in
 // real FP64 GEMMs on the real and imaginary parts, squares that defect (the
-// residual moves by (lambda_a - lambda_b) r_ab / 2 ~ u ||A||).
+// residual moves by (lambda_a - lambda_b) r_ab / 2 ~ u ||A||). Another one
+// follows where R had entries above kOrthoDone: at gaps below 1e-7 ||A|| or so.
 //
 // Costs: the real problem has order 2n (8 times the n^3 work of a real
 // solve of order n, twice that of complex Householder arithmetic), in
@@ -33,6 +34,7 @@
 
 #include "../../include/glagpu.h"
 #include "gla_large.h"
+#include "gla_ortho.cuh"
 #include "gla_status.h"
 
 namespace {
@@ -189,10 +191,13 @@ __global__ void k_zmerge(const double* __restrict__ XY, int n, double* __restric
   }
 }
 // From PQ = [re(V^H V), im(V^H V)] (n x 2n) the halves of R = I - V^H V as
-// the right operand of [X Y] (2n x 2n): [Rr Ri; -Ri Rr] / 2.
-__global__ void k_zresid(int n, const double* __restrict__ PQ, double* __restrict__ R) {
+// the right operand of [X Y] (2n x 2n): [Rr Ri; -Ri Rr] / 2; their largest
+// entry to *rmax.
+__global__ void k_zresid(int n, const double* __restrict__ PQ, double* __restrict__ R,
+                         unsigned long long* __restrict__ rmax) {
   const int j = blockIdx.y;
   const long long n2 = 2LL * n;
+  double m = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double rr = 0.5 * ((i == j ? 1.0 : 0.0) - PQ[i + (long long)j * n]);
     const double ri = -0.5 * PQ[i + (long long)(n + j) * n];
@@ -200,13 +205,16 @@ __global__ void k_zresid(int n, const double* __restrict__ PQ, double* __restric
     R[n + i + j * n2] = -ri;
     R[i + (n + j) * n2] = ri;
     R[n + i + (n + j) * n2] = rr;
+    m = fmax(m, fmax(fabs(rr), fabs(ri)));
   }
+  gla::warp_max_to(m, rmax);
 }
 
 // One Newton-Schulz step V (I + R/2) on V (n x n complex, interleaved), as
 // two real products with everything stacked (8 n^2 doubles of work in W):
 // V^H V = [X; Y]' [X Y; Y -X] and [X Y] [Rr Ri; -Ri Rr] / 2.
-int z_orthonormalise(double* V, long long ldv, int n, double* W, gla::Oz64Gemm** oz, cudaStream_t st) {
+int z_orthonormalise(double* V, long long ldv, int n, double* W, unsigned long long* rmax, gla::Oz64Gemm** oz,
+                     cudaStream_t st) {
   const long long nn = (long long)n * n;
   double *S = W, *PQ = W + 4 * nn, *XY = W + 6 * nn;
   const int n2 = 2 * n;
@@ -214,7 +222,8 @@ int z_orthonormalise(double* V, long long ldv, int n, double* W, gla::Oz64Gemm**
   k_zstack<<<g2, 256, 0, st>>>(V, ldv, n, S);
   Z_CUDA(cudaGetLastError());
   Z_CUDA(gla::oz64_gemm(oz, true, n, n2, n2, S, n2, S, n2, PQ, n, false, st));
-  k_zresid<<<g2, 256, 0, st>>>(n, PQ, S);
+  Z_CUDA(cudaMemsetAsync(rmax, 0, sizeof(*rmax), st));
+  k_zresid<<<g2, 256, 0, st>>>(n, PQ, S, rmax);
   k_zsplit<<<g2, 256, 0, st>>>(V, ldv, n, XY);
   Z_CUDA(cudaGetLastError());
   Z_CUDA(cudaMemcpyAsync(PQ, XY, sizeof(double) * 2 * nn, cudaMemcpyDeviceToDevice, st));
@@ -345,10 +354,15 @@ int gla_zheev(char jobz, char uplo, int64_t n, const double* A, int64_t lda, dou
       Z_CUDA(cudaGetLastError());
     }
     // E's real eigenvectors are consumed (stream order); its 8 n^2 doubles
-    // hold the work arrays of the orthonormalisation step
-    if (nn > 1) {
-      int rc2 = z_orthonormalise(V, ldv, nn, g_z.E, &g_z.oz, st);
-      if (rc2) return rc2;
+    // hold the work arrays of the orthonormalisation, its eigenvalues (read
+    // above) the largest entry of R / 2
+    unsigned long long* rmax = reinterpret_cast<unsigned long long*>(g_z.w2);
+    double r = 1.0;
+    for (int step = 0; nn > 1 && step < gla::kOrthoSteps && r > gla::kOrthoDone; step++) {
+      rc = z_orthonormalise(V, ldv, nn, g_z.E, rmax, &g_z.oz, st);
+      if (rc) return rc;
+      Z_CUDA(cudaMemcpyAsync(&r, rmax, sizeof(r), cudaMemcpyDeviceToHost, st));
+      Z_CUDA(cudaStreamSynchronize(st));
     }
   }
   return gla::oz64_gemm_status(g_z.oz, st);  // (the index tables live in host memory until it has waited)

@@ -22,9 +22,10 @@
 // four gives the quaternion vector of its first real eigenvector; a larger
 // group's 4k candidates span a k-dimensional (right) quaternion space, from
 // which modified Gram-Schmidt with re-orthogonalisation keeps k orthonormal
-// vectors. One symmetric Newton-Schulz step V <- V (I + R/2), R = I - V^H V,
+// vectors. A symmetric Newton-Schulz step V <- V (I + R/2), R = I - V^H V,
 // then squares the departure from orthogonality between groups (about
-// u ||A|| / gap). It runs as two real FP64 GEMMs of order 4n on L(V):
+// u ||A|| / gap); another one follows where R had entries above kOrthoDone.
+// A step runs as two real FP64 GEMMs of order 4n on L(V):
 // L(V)' [V0; V1; V2; V3] is the first block column [M0; M1; M2; M3] of
 // L(V^H V), and L(V) [R0; R1; R2; R3] that of L(V R).
 //
@@ -41,6 +42,7 @@
 
 #include "../../include/glagpu.h"
 #include "gla_large.h"
+#include "gla_ortho.cuh"
 #include "gla_status.h"
 
 namespace {
@@ -231,20 +233,25 @@ __global__ void k_qlmat(const double* __restrict__ Cc, int n, double* __restrict
       for (int c = 0; c < 4; c++) Lv[(r * n + i) + (long long)(c * n + j) * n4] = lsign(r, c) * a[r ^ c];
   }
 }
-// G = [M0; M1; M2; M3] -> R / 2 = (I - M) / 2 in place
-__global__ void k_qresid(int n, double* __restrict__ G) {
+// G = [M0; M1; M2; M3] -> R / 2 = (I - M) / 2 in place; its largest entry to *rmax
+__global__ void k_qresid(int n, double* __restrict__ G, unsigned long long* __restrict__ rmax) {
   const int j = blockIdx.y;
   const long long n4 = 4LL * n;
+  double mx = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 #pragma unroll
     for (int m = 0; m < 4; m++) {
       const long long idx = (m * n + i) + j * n4;
-      G[idx] = 0.5 * ((m == 0 && i == j ? 1.0 : 0.0) - G[idx]);
+      const double r = 0.5 * ((m == 0 && i == j ? 1.0 : 0.0) - G[idx]);
+      G[idx] = r;
+      mx = fmax(mx, fabs(r));
     }
+  gla::warp_max_to(mx, rmax);
 }
 
 // One Newton-Schulz step on V (n x n quaternions); W holds 28 n^2 doubles.
-int q_orthonormalise(double* V, long long ldv, int n, double* W, gla::Oz64Gemm** oz, cudaStream_t st) {
+int q_orthonormalise(double* V, long long ldv, int n, double* W, unsigned long long* rmax, gla::Oz64Gemm** oz,
+                     cudaStream_t st) {
   const long long nn = (long long)n * n, n4 = 4LL * n;
   double *Lv = W, *Cc = W + 16 * nn, *G = W + 20 * nn, *Out = W + 24 * nn;
   const dim3 g2((n + 255) / 256, n);
@@ -254,7 +261,8 @@ int q_orthonormalise(double* V, long long ldv, int n, double* W, gla::Oz64Gemm**
   Q_CUDA(cudaGetLastError());
   const int m4 = (int)n4;
   Q_CUDA(gla::oz64_gemm(oz, true, m4, n, m4, Lv, n4, Cc, n4, G, n4, false, st));  // G = L(V)' Cc
-  k_qresid<<<g2, 256, 0, st>>>(n, G);
+  Q_CUDA(cudaMemsetAsync(rmax, 0, sizeof(*rmax), st));
+  k_qresid<<<g2, 256, 0, st>>>(n, G, rmax);
   Q_CUDA(cudaGetLastError());
   Q_CUDA(cudaMemcpyAsync(Out, Cc, sizeof(double) * 4 * nn, cudaMemcpyDeviceToDevice, st));
   Q_CUDA(gla::oz64_gemm(oz, false, m4, n, m4, Lv, n4, G, n4, Out, n4, true, st));  // Out = Cc + L(V) R / 2
@@ -396,10 +404,15 @@ int gla_qheev(char jobz, char uplo, int64_t n, const double* A, int64_t lda, dou
       Q_CUDA(cudaGetLastError());
     }
     // L(A)'s real eigenvectors are consumed (stream order); its buffer holds
-    // the work arrays of the orthonormalisation step
-    if (nn > 1) {
-      const int rc2 = q_orthonormalise(V, ldv, nn, g_qh.E, &g_qh.oz, st);
-      if (rc2) return rc2;
+    // the work arrays of the orthonormalisation, that of the eigenvalues (read
+    // above) the largest entry of R / 2
+    unsigned long long* rmax = reinterpret_cast<unsigned long long*>(g_qh.w4);
+    double r = 1.0;
+    for (int step = 0; nn > 1 && step < gla::kOrthoSteps && r > gla::kOrthoDone; step++) {
+      rc = q_orthonormalise(V, ldv, nn, g_qh.E, rmax, &g_qh.oz, st);
+      if (rc) return rc;
+      Q_CUDA(cudaMemcpyAsync(&r, rmax, sizeof(r), cudaMemcpyDeviceToHost, st));
+      Q_CUDA(cudaStreamSynchronize(st));
     }
   }
   return gla::oz64_gemm_status(g_qh.oz, st);  // (the index tables live in host memory until it has waited)
